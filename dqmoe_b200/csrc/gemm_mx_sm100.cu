@@ -192,7 +192,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
       ptx::setmaxnreg_dec<kRegsControl>();
       if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             ptx::prefetch_tensormap(&tma_a);
             ptx::prefetch_tensormap(&tma_b);
             uint32_t it = 0;
@@ -226,8 +226,10 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
         __syncwarp();
       } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             constexpr uint32_t idesc = kFp4 ? ptx::make_idesc_nvf4(kBM, kN) : ptx::make_idesc_mx(kBM, kN);
+            const uint64_t desc0 = ptx::smem_desc_sw128(ptx::smem_u32(smem));
+            const uint64_t desc_sf0 = ptx::smem_desc_sf(ptx::smem_u32(&st.sf[0][0]));
             uint32_t it = 0;
             uint32_t acc_it = 0;
             bool ok = true;
@@ -248,9 +250,9 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
                         break;
                     }
                     ptx::tc_fence_after();
-                    const uint32_t a_addr = ptx::smem_u32(smem + size_t(s) * kStageBytes);
-                    const uint32_t b_addr = a_addr + kABytes;
-                    const uint32_t sf_addr = ptx::smem_u32(&st.sf[s][0]);
+                    const uint64_t da = ptx::smem_desc_advance(desc0, uint32_t(s) * kStageBytes);
+                    const uint64_t db = ptx::smem_desc_advance(da, kABytes);
+                    const uint64_t dsf = ptx::smem_desc_advance(desc_sf0, uint32_t(s) * kSfStage);
                     const uint32_t sf_col = tmem_base + kSfCol + (it & 1u) * kSfCols;
                     // scale bytes of this stage -> TMEM (executed in order with the MMAs around them). MXFP8: one block
                     // per 128 rows serves the stage's four instructions (byte k of a column each); NVFP4: block k
@@ -258,17 +260,17 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
 #pragma unroll
                     for (int k = 0; k < kSfAtoms; ++k) {
                         const uint32_t col_b = sf_col + (kFp4 ? 16 + 8 * k : 4);
-                        ptx::tmem_cp_sf(sf_col + 4 * k, ptx::smem_desc_sf(sf_addr + k * kSfBlock));
-                        ptx::tmem_cp_sf(col_b, ptx::smem_desc_sf(sf_addr + kSfPart + k * kSfBlock));
-                        ptx::tmem_cp_sf(col_b + 4, ptx::smem_desc_sf(sf_addr + 2 * kSfPart + k * kSfBlock));
+                        ptx::tmem_cp_sf(sf_col + 4 * k, ptx::smem_desc_advance(dsf, k * kSfBlock));
+                        ptx::tmem_cp_sf(col_b, ptx::smem_desc_advance(dsf, kSfPart + k * kSfBlock));
+                        ptx::tmem_cp_sf(col_b + 4, ptx::smem_desc_advance(dsf, 2 * kSfPart + k * kSfBlock));
                     }
 #pragma unroll
                     for (int k = 0; k < kBK / kUmmaK; ++k) {
-                        const uint64_t da = ptx::smem_desc_sw128(a_addr + k * kUmmaK), db = ptx::smem_desc_sw128(b_addr + k * kUmmaK);
+                        const uint64_t dak = ptx::smem_desc_advance(da, k * kUmmaK), dbk = ptx::smem_desc_advance(db, k * kUmmaK);
                         if constexpr (kFp4)
-                            ptx::umma_nvf4(d_tmem, da, db, idesc, sf_col + 4 * k, sf_col + 16 + 8 * k, (kb | k) != 0 ? 1u : 0u);
+                            ptx::umma_nvf4(d_tmem, dak, dbk, idesc, sf_col + 4 * k, sf_col + 16 + 8 * k, (kb | k) != 0 ? 1u : 0u);
                         else
-                            ptx::umma_mx(d_tmem, da, db, ptx::idesc_mx_with_sf_id(idesc, k), sf_col, sf_col + 4,
+                            ptx::umma_mx(d_tmem, dak, dbk, ptx::idesc_mx_with_sf_id(idesc, k), sf_col, sf_col + 4,
                                          (kb | k) != 0 ? 1u : 0u);
                     }
                     ptx::umma_commit(&st.empty[s]);

@@ -291,7 +291,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
       ptx::setmaxnreg_dec<kRegsControl>();
       if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             ptx::prefetch_tensormap(&tma_a);
             ptx::prefetch_tensormap(&tma_b);
             uint32_t it = 0;
@@ -330,16 +330,25 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
         __syncwarp();
       } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0 && leader) {
+        if (leader && ptx::elect_one()) {
             // operand format code: e4m3 = 0 (kind::f8f6f4); f16 = 0, bf16 = 1 (kind::f16); tf32 = 2 (kind::tf32)
             constexpr uint32_t idesc =
                 ptx::make_idesc(kFp8 || kElem == kElemHalf ? 0u : (kElem == kElemF32 ? 2u : 1u), kPair ? 2 * kBM : kBM, kN);
-            // issue one K step; in a pair the same call drives both CTAs' tensor cores
-            auto mma_step = [&](uint32_t d_tmem, uint32_t a_addr, uint32_t b_addr, uint32_t accumulate) {
-                if constexpr (kPair)
-                    ptx::umma_pair<kKind>(d_tmem, ptx::smem_desc_sw128(a_addr), ptx::smem_desc_sw128(b_addr), idesc, accumulate);
-                else
-                    ptx::umma<kKind>(d_tmem, ptx::smem_desc_sw128(a_addr), ptx::smem_desc_sw128(b_addr), idesc, accumulate);
+            // the four K steps of a stage; in a pair the same instructions drive both CTAs' tensor cores
+            const uint64_t desc0 = ptx::smem_desc_sw128(ptx::smem_u32(smem));
+            auto mma_stage = [&](uint32_t d_tmem, int s, bool first) {
+                const uint64_t da = ptx::smem_desc_advance(desc0, uint32_t(s) * kStageSz);
+                const uint64_t db = ptx::smem_desc_advance(da, kABytes);
+#pragma unroll
+                for (int k = 0; k < kBKBytes / kUmmaKBytes; ++k) {
+                    const uint32_t accumulate = first && k == 0 ? 0u : 1u;
+                    if constexpr (kPair)
+                        ptx::umma_pair<kKind>(d_tmem, ptx::smem_desc_advance(da, k * kUmmaKBytes),
+                                              ptx::smem_desc_advance(db, k * kUmmaKBytes), idesc, accumulate);
+                    else
+                        ptx::umma<kKind>(d_tmem, ptx::smem_desc_advance(da, k * kUmmaKBytes),
+                                         ptx::smem_desc_advance(db, k * kUmmaKBytes), idesc, accumulate);
+                }
             };
             // completion of everything issued so far -> one barrier (of both CTAs in a pair)
             auto commit = [&](uint64_t* bar) {
@@ -368,12 +377,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                             break;
                         }
                         ptx::tc_fence_after();
-                        const uint32_t a_addr = ptx::smem_u32(smem + size_t(s) * kStageSz);
-                        const uint32_t b_addr = a_addr + kABytes;
-#pragma unroll
-                        for (int k = 0; k < kBKBytes / kUmmaKBytes; ++k)
-                            mma_step(tmem_base + buf * kUmmaN, a_addr + k * kUmmaKBytes, b_addr + k * kUmmaKBytes,
-                                     (kb | k) != 0 ? 1u : 0u);
+                        mma_stage(tmem_base + buf * kUmmaN, s, kb == 0);
                         commit(&st.empty[s]);
                     }
                     if (!ok) break;
@@ -393,12 +397,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                             break;
                         }
                         ptx::tc_fence_after();
-                        const uint32_t a_addr = ptx::smem_u32(smem + size_t(s) * kStageSz);
-                        const uint32_t b_addr = a_addr + kABytes;
-#pragma unroll
-                        for (int k = 0; k < kBKBytes / kUmmaKBytes; ++k)
-                            mma_step(tmem_base + buf * kUmmaN, a_addr + k * kUmmaKBytes, b_addr + k * kUmmaKBytes,
-                                     k != 0 ? 1u : 0u);
+                        mma_stage(tmem_base + buf * kUmmaN, s, true);
                         commit(&st.tmem_full[buf]);
                         commit(&st.empty[s]);
                     }

@@ -13,6 +13,22 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// True in exactly one lane of a converged warp. Branching on elect.sync instead of `lane == 0` tells the compiler that a
+// single thread executes the branch, so the uniform-register operands of tcgen05 and TMA instructions need no handling
+// of divergent lanes: a K stage of four 128x256 MMAs issued under `lane == 0` took 580-630 cycles whatever N was (and
+// eight 128-column ones 825-920), under elect.sync with descriptors formed by addition 512, the tensor pipe's own time.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}"
+        : "=r"(p));
+    return p != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -175,6 +191,9 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr) {
     d |= static_cast<uint64_t>(2) << 61;                       // layout type: 128-byte swizzle
     return d;
 }
+// The descriptor of an operand `bytes` (a multiple of 16) further on: shared memory ends below 2^18 bytes, so the
+// address field takes the addition without a carry.
+__device__ __forceinline__ uint64_t smem_desc_advance(uint64_t desc, uint32_t bytes) { return desc + (bytes >> 4); }
 
 // Instruction descriptor: D fp32, A and B both K-major, M x N tile.
 // ab_format: kind::f8f6f4 -> 0 = e4m3 ; kind::f16 -> 0 = f16, 1 = bf16 ; kind::tf32 -> 2 = tf32.
