@@ -45,6 +45,7 @@ constexpr int kEpiWarps = 8;
 constexpr int kMaxExperts = 1024;
 constexpr int kMaxDevices = 64;
 constexpr int kScaleSlots = 8;                     // ring of per-K-block scale sets (block mode)
+static_assert(kScaleSlots >= kStages + 2, "a slot must be drained when its stage is refilled");
 constexpr int kTmemCols = 512;                    // two accumulator buffers of 256 columns
 constexpr long long kWaitLimit = 1000000000LL;    // clock cycles before a wait gives up (~0.5 s)
 
@@ -79,8 +80,6 @@ struct SharedTail {
     uint64_t tmem_full[2];
     uint64_t tmem_empty[2];
     uint64_t epi_sync[4];    // per TMEM lane quarter: the two warps that share a row's 1x128 group
-    uint64_t sc_full[kScaleSlots];
-    uint64_t sc_empty[kScaleSlots];
     uint32_t tmem_base;
     int abort_flag;
     alignas(16) float amax[2][2][kBM];
@@ -217,6 +216,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
     constexpr int kBKElems = kFp8 ? kBKBytes : (kElem == kElemF32 ? kBKBytes / 4 : kBKBytes / 2);
     constexpr int kKind = kFp8 ? 0 : (kElem == kElemF32 ? 2 : 1);  // kind::f8f6f4, kind::f16, kind::tf32
     static_assert(kBox == 128 || (kBox == 64 && !kPair && kMode != kBlock), "narrow tiles: single CTA, non-block modes");
+    static_assert(kMode != kBlock || !kPair, "block mode: single CTAs only");
     static_assert(kElem == kElemBf16 || (!kFp8 && kMode == kNone), "fp16 / fp32 operands: the unquantised path only");
     static_assert(kElem != kElemF32 || (!kPair && kBox == 128), "fp32 operands: single-CTA 256-column tiles only");
     constexpr int kN = 2 * kBox;                      // accumulator columns of a tile
@@ -232,7 +232,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kNumStages; ++s) {
-            ptx::mbar_init(&st.full[s], 1);
+            ptx::mbar_init(&st.full[s], kMode == kBlock ? 1 + 32 : 1);  // block mode: and every lane of the scale loader
             ptx::mbar_init(&st.empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -240,10 +240,6 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
             ptx::mbar_init(&st.tmem_empty[b], kPair ? 2 * kEpiWarps : kEpiWarps);  // both CTAs' epilogue warps
         }
         for (int i = 0; i < 4; ++i) ptx::mbar_init(&st.epi_sync[i], 2);
-        for (int i = 0; i < kScaleSlots; ++i) {
-            ptx::mbar_init(&st.sc_full[i], 32);         // every lane of the scale-loader warp
-            ptx::mbar_init(&st.sc_empty[i], kEpiWarps);
-        }
         st.abort_flag = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async();
@@ -407,8 +403,14 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
         __syncwarp();
       } else if (warp == 2) {
         // ------------------------------------------------------------ scale loader (block mode)
-        // Stages the scales of every K block in shared memory ahead of the epilogue warps with
-        // 4-byte asynchronous copies, so no global-load latency sits in the accumulation loop.
+        // Stages the scales of every K block in shared memory with 4-byte asynchronous copies. They belong to the K
+        // block's stage: the copies arrive on its full barrier, so that the barrier of the accumulator buffer, which the
+        // MMA thread signals after it has seen the stage full, covers them too, and the epilogue warps need no wait of
+        // their own for them (an mbarrier wait costs ~100 cycles even when it is over already: with one for the scales and
+        // one for the buffer a K block took 987 / 940 cycles in fc1 / fc2 at the Mixtral shape with T = 4096, now 885 /
+        // 817; 1132 / 556 us -> 1100 / 514 us). The ring has more slots
+        // than the kNumStages + 2 K blocks that can lie between a stage being refilled and the oldest undrained
+        // accumulator, so a slot is free when its stage is.
         if constexpr (kMode == kBlock) {
             const int KB = kb_count;
             const int NB = (p.w_rows + 127) / 128;
@@ -425,15 +427,15 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                 const int nb = lane == 0 ? sr.nb0 : (lane == 1 ? sr.nb1_lo : sr.nb1_hi);
                 const float* src_b = p.sb + (size_t(tl.e) * NB + nb) * KB;
                 for (int kb = 0; kb < KB; ++kb, ++it) {
-                    const int slot = it % kScaleSlots;
-                    if (!ptx::mbar_wait(&st.sc_empty[slot], ((it / kScaleSlots) & 1u) ^ 1u, abort_flag, kWaitLimit)) {
+                    const int slot = it % kScaleSlots, s = it % kNumStages;
+                    if (!ptx::mbar_wait(&st.empty[s], ((it / kNumStages) & 1u) ^ 1u, abort_flag, kWaitLimit)) {
                         ok = false;
                         break;
                     }
 #pragma unroll
                     for (int j = 0; j < 4; ++j) ptx::cp_async4(&st.sc_a[slot][lane + 32 * j], src_a[j] + kb);
                     if (lane < 3) ptx::cp_async4(&st.sc_b[slot][lane], src_b + kb);
-                    ptx::cp_async_arrive(&st.sc_full[slot]);
+                    ptx::cp_async_arrive(&st.full[s]);
                 }
             }
             ptx::cp_async_wait_all();
@@ -447,7 +449,6 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
         const int r_in_tile = q * 32 + lane;
         const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
         uint32_t acc_it = 0;
-        uint32_t sc_it = 0;
         uint32_t tile_it = 0;
         uint32_t epi_phase = 0;
         int e_cursor = 0;
@@ -661,21 +662,18 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         }
                     };
                     uint32_t r0[32], r1[32];
-                    for (int kb = 0; kb < KB; ++kb, ++acc_it, ++sc_it) {
-                        const int slot = sc_it % kScaleSlots;
-                        if (!ptx::mbar_wait(&st.sc_full[slot], (sc_it / kScaleSlots) & 1u, abort_flag, kWaitLimit)) return false;
-                        const float a_s = st.sc_a[slot][r_in_tile];
-                        const float s0 = a_s * st.sc_b[slot][0], s1l = a_s * st.sc_b[slot][1];
-                        const float s1h = kOneScale ? 0.0f : a_s * st.sc_b[slot][2];
-                        __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive(&st.sc_empty[slot]);
-
+                    bool ready = false;
+                    for (int kb = 0; kb < KB; ++kb, ++acc_it) {
+                        const int slot = acc_it % kScaleSlots;
                         const uint32_t buf = acc_it & 1u;
-                        if (!ptx::mbar_wait(&st.tmem_full[buf], (acc_it >> 1) & 1u, abort_flag, kWaitLimit)) return false;
+                        if (!ready && !ptx::mbar_wait(&st.tmem_full[buf], (acc_it >> 1) & 1u, abort_flag, kWaitLimit)) return false;
                         ptx::tc_fence_after();
                         const uint32_t t_buf = t_lane + buf * kUmmaN;
                         ptx::tmem_ld32(t_buf + tcol(0), r0);
                         ptx::tmem_ld32(t_buf + tcol(1), r1);
+                        const float a_s = st.sc_a[slot][r_in_tile];
+                        const float s0 = a_s * st.sc_b[slot][0], s1l = a_s * st.sc_b[slot][1];
+                        const float s1h = kOneScale ? 0.0f : a_s * st.sc_b[slot][2];
                         ptx::tmem_wait_ld2(r0, r1);
                         fma_chunk(0, r0, s0, s1l, s1h);
                         ptx::tmem_ld32(t_buf + tcol(2), r0);
@@ -685,6 +683,8 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         ptx::tc_fence_before();
                         __syncwarp();
                         if (lane == 0) release_tmem(buf);
+                        // ask for the next buffer now: the answer arrives under the FMAs
+                        ready = ptx::mbar_test_wait(&st.tmem_full[buf ^ 1u], ((acc_it + 1) >> 1) & 1u);
                         fma_chunk(2, r0, s0, s1l, s1h);
                         fma_chunk(3, r1, s0, s1l, s1h);
                     }
@@ -934,7 +934,7 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
         case DQMOE_QUANT_NONE: DQ_GEMM_CASE(false, kNone);
         case DQMOE_QUANT_FP8_TENSOR: DQ_GEMM_CASE(true, kTensor);
         case DQMOE_QUANT_FP8_CHANNEL: DQ_GEMM_CASE(true, kChannel);
-        default: return pair ? DQ_GEMM_LAUNCH(true, kBlock, true, 128) : DQ_GEMM_LAUNCH(true, kBlock, false, 128);
+        default: return DQ_GEMM_LAUNCH(true, kBlock, false, 128);
     }
 #undef DQ_GEMM_CASE
 #undef DQ_GEMM_LAUNCH
