@@ -50,8 +50,8 @@ constexpr int kBBytes = kN * kBK;        // 32 KiB
 constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kSfBlock = 512;            // scale bytes of 128 rows x 4 groups, in tcgen05.cp order
 constexpr int kThreads = 384;
-constexpr int kRegsControl = 56;
-constexpr int kRegsEpilogue = 224;
+constexpr int kRegsControl = 88;  // the control threads spilled at 56
+constexpr int kRegsEpilogue = 208;
 constexpr int kEpiWarps = 8;
 constexpr int kMaxExperts = 1024;
 constexpr int kMaxDevices = 64;
@@ -347,27 +347,34 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
                         const int col0 = tl.nt * kBox + h * 64 + j * 32;
-                        float act[32];
-                        float amax[2] = {0.0f, 0.0f};
+                        uint32_t act2[16];  // bf16 pairs
+                        uint32_t amax2[2] = {0, 0};
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const float bg = has_bias ? __ldg(bias_e + col0 + i) : 0.0f;
-                            const float bv = has_bias ? __ldg(bias_e + N + col0 + i) : 0.0f;
-                            const float gate = bf_round_cvt(__uint_as_float(r[j][i]) * alpha + bg);
-                            const float val = bf_round_cvt(__uint_as_float(r[2 + j][i]) * alpha + bv);
-                            act[i] = bf_round_cvt(bf_round_cvt(__fdividef(gate, 1.0f + __expf(-gate))) * val);
-                            amax[i >> 4] = fmaxf(amax[i >> 4], fabsf(act[i]));
+                        for (int i = 0; i < 32; i += 2) {
+                            float bg[2] = {0.0f, 0.0f}, bv[2] = {0.0f, 0.0f};
+                            if (has_bias) {
+#pragma unroll
+                                for (int u = 0; u < 2; ++u) bg[u] = __ldg(bias_e + col0 + i + u), bv[u] = __ldg(bias_e + N + col0 + i + u);
+                            }
+                            act2[i >> 1] = swiglu_bf16x2(__uint_as_float(r[j][i]) * alpha + bg[0], __uint_as_float(r[j][i + 1]) * alpha + bg[1],
+                                                         __uint_as_float(r[2 + j][i]) * alpha + bv[0],
+                                                         __uint_as_float(r[2 + j][i + 1]) * alpha + bv[1]);
+                            amax_bf16x2(amax2[i >> 4], act2[i >> 1]);
                         }
                         uint32_t w4[4];
 #pragma unroll
                         for (int b = 0; b < 2; ++b) {
                             float inv;
-                            sf_bytes |= nvfp4_scale_byte(amax[b], gout, &inv) << (16 * j + 8 * b);
+                            sf_bytes |= nvfp4_scale_byte(amax_bf16x2_value(amax2[b]), gout, &inv) << (16 * j + 8 * b);
 #pragma unroll
                             for (int hf = 0; hf < 2; ++hf) {
                                 float x8[8];
 #pragma unroll
-                                for (int i = 0; i < 8; ++i) x8[i] = act[16 * b + 8 * hf + i] * inv;
+                                for (int i = 0; i < 8; i += 2) {
+                                    const uint32_t a2 = act2[8 * b + 4 * hf + (i >> 1)];
+                                    x8[i] = bf16_lo(a2) * inv;
+                                    x8[i + 1] = bf16_hi(a2) * inv;
+                                }
                                 w4[2 * b + hf] = f2e2m1x8(x8);
                             }
                         }
@@ -427,8 +434,8 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
                     ptx::tmem_wait_ld(g);
                     ptx::tmem_wait_ld(v);
                     overlap_drained(jj + 1);
-                    float act[32];
-                    float amax = 0.0f;
+                    uint32_t act2[16];  // bf16 pairs
+                    uint32_t amax2 = 0;
 #pragma unroll
                     for (int i = 0; i < 32; i += 4) {
                         float bg[4] = {0.0f, 0.0f, 0.0f, 0.0f}, bv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -438,22 +445,22 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
                             bv[0] = b.x, bv[1] = b.y, bv[2] = b.z, bv[3] = b.w;
                         }
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
+                        for (int u = 0; u < 4; u += 2) {
                             // roundings as in the fp32-scaled block mode: product, silu and their product to bf16
-                            const float gate = bf_round_cvt(__uint_as_float(g[i + u]) + bg[u]);
-                            const float val = bf_round_cvt(__uint_as_float(v[i + u]) + bv[u]);
-                            float a = bf_round_cvt(bf_round_cvt(__fdividef(gate, 1.0f + __expf(-gate))) * val);
-                            if (col0 + i + u >= N) a = 0.0f;
-                            act[i + u] = a;
-                            amax = fmaxf(amax, fabsf(a));
+                            uint32_t a2 = swiglu_bf16x2(__uint_as_float(g[i + u]) + bg[u], __uint_as_float(g[i + u + 1]) + bg[u + 1],
+                                                        __uint_as_float(v[i + u]) + bv[u], __uint_as_float(v[i + u + 1]) + bv[u + 1]);
+                            if (col0 + i + u >= N) a2 = 0;
+                            act2[(i + u) >> 1] = a2;
+                            amax_bf16x2(amax2, a2);
                         }
                     }
                     float inv;
-                    const uint32_t e8 = mx_scale_byte(amax, &inv);
+                    const uint32_t e8 = mx_scale_byte(amax_bf16x2_value(amax2), &inv);
                     sf_bytes |= e8 << (8 * j);
 #pragma unroll
                     for (int i = 0; i < 32; i += 4)
-                        pk[jj][i >> 2] = f2e4m3x4(act[i] * inv, act[i + 1] * inv, act[i + 2] * inv, act[i + 3] * inv);
+                        pk[jj][i >> 2] = f2e4m3x4(bf16_lo(act2[i >> 1]) * inv, bf16_hi(act2[i >> 1]) * inv,
+                                                  bf16_lo(act2[(i >> 1) + 1]) * inv, bf16_hi(act2[(i >> 1) + 1]) * inv);
                 }
                 uint32_t packed[16];  // back into column order (buffer 0 drains its second group first)
 #pragma unroll

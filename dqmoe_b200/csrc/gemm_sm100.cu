@@ -39,8 +39,14 @@ constexpr int kStageBytes = kABytes + kBBytes;    // 48 KiB
 constexpr int kStageBytesPair = kABytes + kBBytes / 2;  // 32 KiB per CTA of a pair
 static_assert(kStages * kStageBytes == kStagesPair * kStageBytesPair, "both layouts fill the same stage area");
 constexpr int kThreads = 384;                     // warp 0 TMA, warp 1 MMA, warp 2 scale loader (block mode), warp 3 idle, warps 4..11 epilogue
-constexpr int kRegsControl = 56;                  // registers per thread of the TMA/MMA warpgroup
-constexpr int kRegsEpilogue = 224;                // registers per thread of the two epilogue warpgroups
+// Registers per thread of the control warpgroup and of the two epilogue warpgroups; 128 * control + 256 * epilogue stay
+// within the launch's 384 * 168. Block mode keeps 128 accumulators and 64 loaded values in registers; the other modes
+// need less, and their control threads spilled at 56.
+template <bool kBlockMode>
+struct Regs {
+    static constexpr int kControl = kBlockMode ? 56 : 88;
+    static constexpr int kEpilogue = kBlockMode ? 224 : 208;
+};
 constexpr int kEpiWarps = 8;
 constexpr int kMaxExperts = 1024;
 constexpr int kMaxDevices = 64;
@@ -138,11 +144,6 @@ __device__ __forceinline__ ScaleRows scale_rows(bool gated, int nt, int N, int N
     r.nb1_lo = min(r.nb1_lo, NB - 1);
     r.nb1_hi = min(r.nb1_hi, NB - 1);
     return r;
-}
-
-__device__ __forceinline__ float silu_bf16(float g) {
-    // the torch oracle evaluates silu on bf16 and rounds the result to bf16 (test/util.py:141-142)
-    return bf_round_cvt(__fdividef(g, 1.0f + __expf(-g)));
 }
 
 // One 32-column chunk of a tile row per lane: 32 values of 16 bits (packed[16]) or of 32 bits (packed[32], two
@@ -284,7 +285,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
     // The launch gives every thread 168 registers; the control warpgroup hands most of its
     // share to the epilogue warpgroups, whose block-scaled accumulators live in registers.
     if (warp < 4) {
-      ptx::setmaxnreg_dec<kRegsControl>();
+      ptx::setmaxnreg_dec<Regs<kMode == kBlock>::kControl>();
       if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         if (ptx::elect_one()) {
@@ -442,7 +443,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
         }
       }
     } else {
-        ptx::setmaxnreg_inc<kRegsEpilogue>();
+        ptx::setmaxnreg_inc<Regs<kMode == kBlock>::kEpilogue>();
         // ------------------------------------------------------------ epilogue warps
         const int q = warp & 3;            // TMEM lane quarter this warp may read
         const int h = (warp - 4) >> 2;     // which 64-column half of each 128-column group
@@ -467,6 +468,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
             const int grow = tl.row0 + r_in_tile;
             const bool row_ok = grow < tl.row_end;
             const int grow_ld = min(grow, p.n_rows - 1);
+            const bool live = tl.row0 + q * 32 < tl.row_end;  // some of this warp's rows exist; else it only hands buffers back
 
             if constexpr (kMode != kBlock) {
                 const uint32_t buf = acc_it & 1u;
@@ -493,9 +495,9 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
 
                 if constexpr (kGated) {
                     // columns [h*kHalf, (h+1)*kHalf) of the gate group and of the value group
-                    float amax_local = 0.0f;
+                    uint32_t amax2 = 0;  // running maximum of |act|, bf16 pairs
 #pragma unroll 1
-                    for (int j = 0; j < kChunks; ++j) {
+                    for (int j = 0; j < (live ? kChunks : 0); ++j) {
                         uint32_t g[32], v[32];
                         const int c0 = h * kHalf + j * 32;  // column inside the kBox-wide act tile
                         ptx::tmem_ld32(t_buf + c0, g);
@@ -517,8 +519,6 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         ptx::tmem_wait_ld(g);
                         ptx::tmem_wait_ld(v);
                         uint32_t packed[kElem == kElemF32 ? 32 : 16];
-                        // This epilogue runs beside the next tile's MMAs; its roundings use the conversion
-                        // instruction (one issue slot each), which measured faster here than bf_round.
 #pragma unroll
                         for (int i = 0; i < 32; i += 4) {
                             float sg[4] = {row_scale, row_scale, row_scale, row_scale};
@@ -534,24 +534,32 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                                 bg[0] = a.x, bg[1] = a.y, bg[2] = a.z, bg[3] = a.w;
                                 bv[0] = b.x, bv[1] = b.y, bv[2] = b.z, bv[3] = b.w;
                             }
-                            float a4[4];
+                            if constexpr (kElem == kElemBf16) {
 #pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                const float gate = round16<kElem>(__uint_as_float(g[i + u]) * sg[u] + bg[u]);
-                                const float val = round16<kElem>(__uint_as_float(v[i + u]) * sv[u] + bv[u]);
-                                const float act = round16<kElem>(round16<kElem>(__fdividef(gate, 1.0f + __expf(-gate))) * val);
-                                a4[u] = act;
-                                if (col0 + i + u < I_or_H) amax_local = fmaxf(amax_local, fabsf(act));
-                            }
-                            if constexpr (kElem == kElemF32) {
-#pragma unroll
-                                for (int u = 0; u < 4; ++u) packed[i + u] = __float_as_uint(a4[u]);
-                            } else if constexpr (kElem == kElemHalf) {
-                                packed[i >> 1] = pack16x2<kElemHalf>(a4[0], a4[1]);
-                                packed[(i >> 1) + 1] = pack16x2<kElemHalf>(a4[2], a4[3]);
+                                for (int u = 0; u < 4; u += 2) {
+                                    const uint32_t a2 = swiglu_bf16x2(__uint_as_float(g[i + u]) * sg[u] + bg[u],
+                                                                      __uint_as_float(g[i + u + 1]) * sg[u + 1] + bg[u + 1],
+                                                                      __uint_as_float(v[i + u]) * sv[u] + bv[u],
+                                                                      __uint_as_float(v[i + u + 1]) * sv[u + 1] + bv[u + 1]);
+                                    packed[(i + u) >> 1] = a2;
+                                    if constexpr (kMode == kChannel || kMode == kTensor)
+                                        if (col0 + i + u < I_or_H) amax_bf16x2(amax2, a2);  // I is a multiple of 8
+                                }
                             } else {
-                                packed[i >> 1] = pack_bf16x2_exact(a4[0], a4[1]);  // act is already rounded to bf16
-                                packed[(i >> 1) + 1] = pack_bf16x2_exact(a4[2], a4[3]);
+                                float a4[4];
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) {
+                                    const float gate = round16<kElem>(__uint_as_float(g[i + u]) * sg[u] + bg[u]);
+                                    const float val = round16<kElem>(__uint_as_float(v[i + u]) * sv[u] + bv[u]);
+                                    a4[u] = round16<kElem>(round16<kElem>(__fdividef(gate, 1.0f + __expf(-gate))) * val);
+                                }
+                                if constexpr (kElem == kElemF32) {
+#pragma unroll
+                                    for (int u = 0; u < 4; ++u) packed[i + u] = __float_as_uint(a4[u]);
+                                } else {
+                                    packed[i >> 1] = pack16x2<kElemHalf>(a4[0], a4[1]);
+                                    packed[(i >> 1) + 1] = pack16x2<kElemHalf>(a4[2], a4[3]);
+                                }
                             }
                         }
                         uint8_t* optr = row_ok ? static_cast<uint8_t*>(p.out) + (size_t(grow) * I_or_H + col0) * kOutBytes
@@ -559,10 +567,10 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         store_chunk<kElem == kElemF32>(st.stage[warp - 4], packed, optr, I_or_H - col0, lane);
                     }
                     if constexpr (kMode == kChannel) {
-                        if (row_ok) atomic_max_nonneg(p.amax + grow, amax_local);
+                        if (row_ok) atomic_max_nonneg(p.amax + grow, amax_bf16x2_value(amax2));
                     }
                     if constexpr (kMode == kTensor) {
-                        float m = row_ok ? amax_local : 0.0f;
+                        float m = row_ok ? amax_bf16x2_value(amax2) : 0.0f;
                         m = warp_max(m);
                         if (lane == 0) atomic_max_nonneg(p.amax, m);
                     }
@@ -576,7 +584,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         orow_idx = orow != nullptr ? 0 : -1;
                     }
 #pragma unroll 1
-                    for (int c = 0; c < 2 * kChunks; ++c) {
+                    for (int c = 0; c < (live ? 2 * kChunks : 0); ++c) {
                         uint32_t r[32];
                         const int tc = (c / kChunks) * kBox + h * kHalf + (c % kChunks) * 32;
                         ptx::tmem_ld32(t_buf + tc, r);
@@ -690,7 +698,12 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                     }
                     return true;
                 };
-                if (!kGated || c_switch == 128)
+                if (!live) {
+                    for (int kb = 0; ok && kb < KB; ++kb, ++acc_it) {
+                        ok = ptx::mbar_wait(&st.tmem_full[acc_it & 1u], (acc_it >> 1) & 1u, abort_flag, kWaitLimit);
+                        if (lane == 0) release_tmem(acc_it & 1u);
+                    }
+                } else if (!kGated || c_switch == 128)
                     ok = k_loop(std::true_type{});
                 else
                     ok = k_loop(std::false_type{});
@@ -708,35 +721,16 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                 if constexpr (kGated) {
                     // act columns nt*128 + h*64 + [0, 64): gate = acc[0..63], value = acc[64..127]
                     const int col0 = tl.nt * kBoxRows + h * 64;
-                    float amax_local = 0.0f;
-                    // The tensor pipe idles during this part (the same warps drain its buffers), so it is
-                    // written for throughput: bf16 roundings on the fp32 pipe (bf_round), eight elements
-                    // per step and stage by stage so that the exp / reciprocal latencies overlap.
-                    auto swiglu = [&](auto full_tag) {
-                        constexpr bool kFullTile = decltype(full_tag)::value;  // all 64 columns inside the matrix
+                    uint32_t act2[32];   // bf16 pairs
+                    uint32_t amax2 = 0;
+                    // The tensor pipe idles during this part: the same warps drain its buffers.
+                    const int cols_ok = I_or_H - col0;  // a multiple of 16
 #pragma unroll
-                        for (int i0 = 0; i0 < 64; i0 += 8) {
-                            float g8[8], e8[8];
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                g8[j] = bf_round(acc[i0 + j]);
-                                e8[j] = __expf(-g8[j]);
-                            }
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) e8[j] = bf_round(__fdividef(g8[j], 1.0f + e8[j]));
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                float act = bf_round(e8[j] * bf_round(acc[64 + i0 + j]));
-                                if (!kFullTile && col0 + i0 + j >= I_or_H) act = 0.0f;
-                                acc[i0 + j] = act;
-                                amax_local = fmaxf(amax_local, fabsf(act));
-                            }
-                        }
-                    };
-                    if (col0 + 64 <= I_or_H)
-                        swiglu(std::true_type{});
-                    else
-                        swiglu(std::false_type{});
+                    for (int i = 0; i < 64; i += 2) {
+                        act2[i >> 1] = swiglu_bf16x2(acc[i], acc[i + 1], acc[64 + i], acc[64 + i + 1]);
+                        if (i < cols_ok) amax_bf16x2(amax2, act2[i >> 1]);
+                    }
+                    const float amax_local = amax_bf16x2_value(amax2);
                     // the 1x128 group spans both halves: exchange the partial amax through shared memory
                     st.amax[tile_it & 1u][h][r_in_tile] = amax_local;
                     __syncwarp();
@@ -752,10 +746,9 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                     {
                         uint32_t packed[16];  // 64 e4m3 bytes of this row
 #pragma unroll
-                        for (int g4 = 0; g4 < 16; ++g4) {
-                            const float* a = acc + g4 * 4;
-                            packed[g4] = f2e4m3x4(a[0] * inv, a[1] * inv, a[2] * inv, a[3] * inv);
-                        }
+                        for (int g4 = 0; g4 < 16; ++g4)
+                            packed[g4] = f2e4m3x4(bf16_lo(act2[2 * g4]) * inv, bf16_hi(act2[2 * g4]) * inv,
+                                                  bf16_lo(act2[2 * g4 + 1]) * inv, bf16_hi(act2[2 * g4 + 1]) * inv);
                         store_rows_staged(st.stage[warp - 4], packed,
                                           row_ok ? reinterpret_cast<uint8_t*>(p.out) + size_t(grow) * I_or_H + col0 : nullptr,
                                           min(4, max(0, (I_or_H - col0 + 15) / 16)), lane);
