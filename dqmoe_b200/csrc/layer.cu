@@ -16,6 +16,11 @@ int route_sort(const int* ids, int n, int E, int* counts, int* offsets, int* mti
 int route_topk(const float* logits, int T, int E, int k, int n_shared, int scoring, int* indices, float* weights,
                cudaStream_t stream);
 }  // namespace route
+namespace permute {
+int scatter_rows(const void* src, size_t row_bytes, int T, int k, const int* src_to_dest, void* dst, const float* src_scale,
+                 int scale_cols, float* dst_scale, cudaStream_t stream);
+int scatter_quant_1x128(const void* x_bf16, int T, int k, int H, const int* src_to_dest, void* q, float* scale, cudaStream_t stream);
+}  // namespace permute
 namespace gemm {
 int grouped_gemm(const void* a, const float* a_scale, const void* w, const float* w_scale, const int* offsets,
                  const int* mtile_prefix, int n, int N, int K, int E, int quant_mode, int gated, void* out,
@@ -44,7 +49,7 @@ constexpr size_t kAlign = 256;  // CUDA_MEM_ALIGN of the reference (csrc/util.h:
 constexpr int kDecodeRows = 8;  // up to this many expanded rows the GEMV path of decode.cu is used (bf16, per-tensor FP8)
 
 struct Layout {
-    size_t offsets, counts, mtile_prefix, sort_ws, dest_to_src, perm_a, perm_a_scale, act, act_scale, act_bf16, amax;
+    size_t offsets, counts, mtile_prefix, sort_ws, dest_to_src, src_to_dest, perm_a, perm_a_scale, act, act_scale, act_bf16, amax;
     size_t total;
     size_t sort_ws_bytes;
     int perm_scale_cols;
@@ -74,6 +79,7 @@ static Layout make_layout(int T, int H, int I, int E, int k, int quant_mode, int
     L.sort_ws_bytes = route::sort_workspace_bytes(int(n), E);
     L.sort_ws = add(L.sort_ws_bytes);
     L.dest_to_src = add(n * sizeof(int));
+    L.src_to_dest = add(n * sizeof(int));
     const bool fp4 = quant_mode == DQMOE_QUANT_NVFP4;  // two elements per byte; scales tiled like MXFP8's, per 64 K elements
     L.perm_a = add(fp4 ? n * H / 2 : n * H * esz);
     L.perm_scale_cols = quant_mode == DQMOE_QUANT_FP8_BLOCK ? ceil_div(H, 128)
@@ -160,6 +166,7 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
     int* counts = reinterpret_cast<int*>(ws + L.counts);
     int* mtile_prefix = reinterpret_cast<int*>(ws + L.mtile_prefix);
     int* dest_to_src = reinterpret_cast<int*>(ws + L.dest_to_src);
+    int* src_to_dest = reinterpret_cast<int*>(ws + L.src_to_dest);
     void* perm_a = ws + L.perm_a;
     float* perm_a_scale = reinterpret_cast<float*>(ws + L.perm_a_scale);
     void* act = ws + L.act;
@@ -172,12 +179,11 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
         return decode::forward(a, a_scale, b, b_scale, b1, b1_scale, d, m_indices, fp8 ? act_bf16 : act, amax, T, H, I,
                                E, k, fp8, stream);
 
-    int rc = route::route_sort(m_indices, n, E, counts, offsets, mtile_prefix, dest_to_src, nullptr, ws + L.sort_ws,
+    int rc = route::route_sort(m_indices, n, E, counts, offsets, mtile_prefix, dest_to_src, src_to_dest, ws + L.sort_ws,
                                L.sort_ws_bytes, stream);
     if (rc != DQMOE_OK) return rc;
 
-    rc = dqmoe_permute_rows(a, size_t(H) * esz, k, dest_to_src, n, perm_a, L.perm_scale_cols ? a_scale : nullptr,
-                            L.perm_scale_cols, L.perm_scale_cols ? perm_a_scale : nullptr, stream);
+    rc = permute::scatter_rows(a, size_t(H) * esz, T, k, src_to_dest, perm_a, a_scale, L.perm_scale_cols, perm_a_scale, stream);
     if (rc != DQMOE_OK) return rc;
 
     if (quant_mode == DQMOE_QUANT_FP8_MX) {
@@ -258,14 +264,15 @@ int dqmoe_moe_forward_nvfp4(const void* a, const uint8_t* a_sf, const float* a_g
     int* counts = reinterpret_cast<int*>(ws + L.counts);
     int* mtile_prefix = reinterpret_cast<int*>(ws + L.mtile_prefix);
     int* dest_to_src = reinterpret_cast<int*>(ws + L.dest_to_src);
+    int* src_to_dest = reinterpret_cast<int*>(ws + L.src_to_dest);
     void* perm_a = ws + L.perm_a;
     uint8_t* perm_a_sf = reinterpret_cast<uint8_t*>(ws + L.perm_a_scale);
     void* act = ws + L.act;
     uint8_t* act_sf = reinterpret_cast<uint8_t*>(ws + L.act_scale);
-    int rc = route::route_sort(m_indices, n, E, counts, offsets, mtile_prefix, dest_to_src, nullptr, ws + L.sort_ws,
+    int rc = route::route_sort(m_indices, n, E, counts, offsets, mtile_prefix, dest_to_src, src_to_dest, ws + L.sort_ws,
                                L.sort_ws_bytes, stream);
     if (rc != DQMOE_OK) return rc;
-    rc = dqmoe_permute_rows(a, size_t(H) / 2, k, dest_to_src, n, perm_a, nullptr, 0, nullptr, stream);
+    rc = permute::scatter_rows(a, size_t(H) / 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, stream);
     if (rc != DQMOE_OK) return rc;
     // one scale byte per 16 elements: the tiling kernel sees them as the scales of a row twice as long
     rc = dqmoe_mx_tile_scales(a_sf, n, 2 * H, dest_to_src, k, offsets, mtile_prefix, E, perm_a_sf, stream);
@@ -374,6 +381,7 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
     int* counts = reinterpret_cast<int*>(lws + L.counts);
     int* mtile_prefix = reinterpret_cast<int*>(lws + L.mtile_prefix);
     int* dest_to_src = reinterpret_cast<int*>(lws + L.dest_to_src);
+    int* src_to_dest = reinterpret_cast<int*>(lws + L.src_to_dest);
     void* perm_a = lws + L.perm_a;
     float* perm_a_scale = reinterpret_cast<float*>(lws + L.perm_a_scale);
     void* act = lws + L.act;
@@ -394,7 +402,7 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
         if (rc != DQMOE_OK) return rc;
         return dqmoe_finalize_weighted(d, weights, out_bf16, T, k, H, stream);
     }
-    rc = route::route_sort(indices, n, E, counts, offsets, mtile_prefix, dest_to_src, nullptr, lws + L.sort_ws,
+    rc = route::route_sort(indices, n, E, counts, offsets, mtile_prefix, dest_to_src, src_to_dest, lws + L.sort_ws,
                            L.sort_ws_bytes, stream);
     if (rc != DQMOE_OK) return rc;
     if (quant_mode == DQMOE_QUANT_FP8_MX) {  // the same fusion with 1x32 power-of-two scales
@@ -412,10 +420,10 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
         if (rc != DQMOE_OK) return rc;
         return dqmoe_finalize_weighted(d, weights, out_bf16, T, k, H, stream);
     }
-    if (fp8)  // quantise while gathering: each expanded row is read as bf16 and written as e4m3 + 1x128 scales
-        rc = dqmoe_permute_quant_block_1x128(x_bf16, H, k, dest_to_src, n, perm_a, perm_a_scale, stream);
+    if (fp8)  // quantise on the way into expert order: a token is read as bf16 once, its k rows written as e4m3 + 1x128 scales
+        rc = permute::scatter_quant_1x128(x_bf16, T, k, H, src_to_dest, perm_a, perm_a_scale, stream);
     else
-        rc = dqmoe_permute_rows(x_bf16, size_t(H) * 2, k, dest_to_src, n, perm_a, nullptr, 0, nullptr, stream);
+        rc = permute::scatter_rows(x_bf16, size_t(H) * 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, stream);
     if (rc != DQMOE_OK) return rc;
     rc = gemm::grouped_gemm(perm_a, perm_a_scale, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, act,
                             act_scale, nullptr, nullptr, nullptr, stream);

@@ -56,7 +56,12 @@ __global__ void __launch_bounds__(kThreads) row_move_kernel(const uint8_t* __res
     }
 }
 
-// out[t, :] = sum_j w[t, j] * d[t, j, :]; one warp per (token, 256-column strip)
+// out[t, :] = sum_j w[t, j] * d[t, j, :]; one warp per (token, 256-column strip). HBM-bound; the slots of a token are
+// fetched kSlotBatch at a time before the first is used, so that a lane has that many 16-byte loads in flight (T = 8192,
+// k = 8, H = 7168: one slot after the other 246 us, batches of eight 194 us = 5.4 TB/s). The batch is the power of two that
+// holds k, at most 8: with two slots in a batch of eight the registers of the empty ones cost occupancy (T = 2049, k = 2,
+// H = 4096: 25.9 us against 13.1).
+template <int kSlotBatch>
 __global__ void __launch_bounds__(kThreads) finalize_weighted_kernel(const uint8_t* __restrict__ d,
                                                                      const float* __restrict__ w,
                                                                      uint8_t* __restrict__ out, int T, int k,
@@ -70,22 +75,130 @@ __global__ void __launch_bounds__(kThreads) finalize_weighted_kernel(const uint8
         const int v = int(it % strips) * 32 + lane;
         if (v >= row_vecs) continue;
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int j = 0; j < k; ++j) {
-            const float wj = w[size_t(t) * k + j];
-            if (wj == 0.0f) continue;
-            const Vec16 x = ld_nc16(d + ((size_t(t) * k + j) * row_vecs + v) * 16);
-            acc[0] = fmaf(wj, bf16_lo(x.x), acc[0]);
-            acc[1] = fmaf(wj, bf16_hi(x.x), acc[1]);
-            acc[2] = fmaf(wj, bf16_lo(x.y), acc[2]);
-            acc[3] = fmaf(wj, bf16_hi(x.y), acc[3]);
-            acc[4] = fmaf(wj, bf16_lo(x.z), acc[4]);
-            acc[5] = fmaf(wj, bf16_hi(x.z), acc[5]);
-            acc[6] = fmaf(wj, bf16_lo(x.w), acc[6]);
-            acc[7] = fmaf(wj, bf16_hi(x.w), acc[7]);
+        for (int j0 = 0; j0 < k; j0 += kSlotBatch) {
+            float wj[kSlotBatch];
+            Vec16 x[kSlotBatch];
+#pragma unroll
+            for (int u = 0; u < kSlotBatch; ++u) wj[u] = j0 + u < k ? __ldg(w + size_t(t) * k + j0 + u) : 0.0f;
+#pragma unroll
+            for (int u = 0; u < kSlotBatch; ++u)
+                if (wj[u] != 0.0f) x[u] = ld_nc16(d + ((size_t(t) * k + j0 + u) * row_vecs + v) * 16);
+#pragma unroll
+            for (int u = 0; u < kSlotBatch; ++u) {
+                if (wj[u] == 0.0f) continue;  // a dropped slot's row is never written
+                acc[0] = fmaf(wj[u], bf16_lo(x[u].x), acc[0]);
+                acc[1] = fmaf(wj[u], bf16_hi(x[u].x), acc[1]);
+                acc[2] = fmaf(wj[u], bf16_lo(x[u].y), acc[2]);
+                acc[3] = fmaf(wj[u], bf16_hi(x[u].y), acc[3]);
+                acc[4] = fmaf(wj[u], bf16_lo(x[u].z), acc[4]);
+                acc[5] = fmaf(wj[u], bf16_hi(x[u].z), acc[5]);
+                acc[6] = fmaf(wj[u], bf16_lo(x[u].w), acc[6]);
+                acc[7] = fmaf(wj[u], bf16_hi(x[u].w), acc[7]);
+            }
         }
         Vec16 o{pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]),
                 pack_bf16x2(acc[6], acc[7])};
         st16(out + (size_t(t) * row_vecs + v) * 16, o);
+    }
+}
+
+// The layer's way into expert order: token t's row goes to rows src_to_dest[t*k + j] of the sorted matrix (negative: a
+// dropped slot). One warp per (token, strip of 128 16-byte vectors); a token is read - and in the quantising form
+// converted - once for its k copies, where the gathers above and below read it k times (HBM-bound: k + 1 rows of traffic
+// per token, the k writes dominating. 8192 tokens of 7168, k = 8, quantising: gather 353 us, scatter 111 us = 5.3 TB/s;
+// 16384 bf16 rows of 2880, k = 3: 102 / 62 us; 16384 e4m3 rows of 2048, k = 8: 82 / 50 us).
+__device__ __forceinline__ int slot_dest(const int* __restrict__ src_to_dest, int t, int k, int j0, int lane) {
+    if (src_to_dest == nullptr) return t;  // rows stay where they are (k = 1)
+    return j0 + lane < k ? src_to_dest[size_t(t) * k + j0 + lane] : -1;
+}
+
+__global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
+                                                                const int* __restrict__ src_to_dest, int T, int k, int row_vecs,
+                                                                const float* __restrict__ src_scale,
+                                                                float* __restrict__ dst_scale, int scale_cols) {
+    const int lane = threadIdx.x & 31;
+    const int strips = (row_vecs + 127) / 128;
+    const int64_t items = int64_t(T) * strips;
+    const int64_t warps = int64_t(gridDim.x) * kWarpsPerBlock;
+    for (int64_t it = int64_t(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5); it < items; it += warps) {
+        const int t = int(it / strips);
+        const int strip = int(it % strips);
+        const int v0 = strip * 128 + lane;
+        Vec16 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (v0 + 32 * u < row_vecs) x[u] = ld_nc16(src + (size_t(t) * row_vecs + v0 + 32 * u) * 16);
+        for (int j0 = 0; j0 < k; j0 += 32) {
+            const int mine = slot_dest(src_to_dest, t, k, j0, lane);
+            const int jn = min(32, k - j0);
+            for (int j = 0; j < jn; ++j) {
+                const int r = __shfl_sync(0xffffffffu, mine, j);
+                if (r < 0) continue;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (v0 + 32 * u < row_vecs) st16(dst + (size_t(r) * row_vecs + v0 + 32 * u) * 16, x[u]);
+                if (strip == 0)
+                    for (int c = lane; c < scale_cols; c += 32) dst_scale[size_t(r) * scale_cols + c] = src_scale[size_t(t) * scale_cols + c];
+            }
+        }
+    }
+}
+
+// The same with 1x128 FP8 quantisation of the bf16 row on the way: a lane owns 16 consecutive columns per step, so a
+// 128-column group is 8 lanes; two steps of 512 columns per strip. cols is a multiple of 16.
+__global__ void __launch_bounds__(kThreads) scatter_quant_1x128_kernel(const uint8_t* __restrict__ x, int T, int k, int cols,
+                                                                       const int* __restrict__ src_to_dest,
+                                                                       uint8_t* __restrict__ q, float* __restrict__ scale) {
+    const int lane = threadIdx.x & 31;
+    const int groups = (cols + 127) / 128;
+    const int strips = (cols + 1023) / 1024;
+    const int64_t items = int64_t(T) * strips;
+    const int64_t warps = int64_t(gridDim.x) * kWarpsPerBlock;
+    for (int64_t it = int64_t(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5); it < items; it += warps) {
+        const int t = int(it / strips);
+        const int c0 = int(it % strips) * 1024 + lane * 16;
+        Vec16 raw[2][2];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const uint8_t* xr = x + (size_t(t) * cols + c0 + 512 * s) * 2;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) raw[s][u] = c0 + 512 * s < cols ? ld_nc16(xr + 16 * u) : Vec16{0, 0, 0, 0};
+        }
+        Vec16 o[2];
+        float sf[2];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const uint32_t w[8] = {raw[s][0].x, raw[s][0].y, raw[s][0].z, raw[s][0].w,
+                                   raw[s][1].x, raw[s][1].y, raw[s][1].z, raw[s][1].w};
+            float amax = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fmaxf(fabsf(bf16_lo(w[i])), fabsf(bf16_hi(w[i]))));
+#pragma unroll
+            for (int d = 4; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
+            sf[s] = scale_from_amax(amax);
+            const float inv = inv_scale(sf[s]);
+            uint32_t b[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                b[i] = f2e4m3x4(bf16_lo(w[2 * i]) * inv, bf16_hi(w[2 * i]) * inv, bf16_lo(w[2 * i + 1]) * inv, bf16_hi(w[2 * i + 1]) * inv);
+            o[s] = Vec16{b[0], b[1], b[2], b[3]};
+        }
+        for (int j0 = 0; j0 < k; j0 += 32) {
+            const int mine = slot_dest(src_to_dest, t, k, j0, lane);
+            const int jn = min(32, k - j0);
+            for (int j = 0; j < jn; ++j) {
+                const int r = __shfl_sync(0xffffffffu, mine, j);
+                if (r < 0) continue;
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const int c = c0 + 512 * s;
+                    if (c < cols) {
+                        st16(q + size_t(r) * cols + c, o[s]);
+                        if ((lane & 7) == 0) scale[size_t(r) * groups + (c >> 7)] = sf[s];
+                    }
+                }
+            }
+        }
     }
 }
 
@@ -133,6 +246,24 @@ __global__ void __launch_bounds__(kThreads) quant_1x128_kernel(const uint8_t* __
     }
 }
 
+// Arguments have been checked by the layer (layer.cu).
+int scatter_rows(const void* src, size_t row_bytes, int T, int k, const int* src_to_dest, void* dst, const float* src_scale,
+                 int scale_cols, float* dst_scale, cudaStream_t stream) {
+    const int row_vecs = int(row_bytes / 16);
+    DQ_CHECK(is_aligned(src, 16) && is_aligned(dst, 16));
+    scatter_rows_kernel<<<grid_for_rows(int64_t(T) * ceil_div(row_vecs, 128)), kThreads, 0, stream>>>(
+        static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), src_to_dest, T, k, row_vecs, src_scale, dst_scale, scale_cols);
+    DQ_LAUNCH_CHECK();
+    return DQMOE_OK;
+}
+int scatter_quant_1x128(const void* x_bf16, int T, int k, int H, const int* src_to_dest, void* q, float* scale, cudaStream_t stream) {
+    DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 16) && H % 16 == 0);
+    scatter_quant_1x128_kernel<<<grid_for_rows(int64_t(T) * ceil_div(H, 1024)), kThreads, 0, stream>>>(
+        static_cast<const uint8_t*>(x_bf16), T, k, H, src_to_dest, static_cast<uint8_t*>(q), scale);
+    DQ_LAUNCH_CHECK();
+    return DQMOE_OK;
+}
+
 }  // namespace permute
 }  // namespace dq
 
@@ -178,8 +309,11 @@ int dqmoe_finalize_weighted(const void* d_bf16, const float* weights, void* out_
     DQ_CHECK(is_aligned(d_bf16, 16) && is_aligned(out_bf16, 16));
     const int row_vecs = H / 8;
     const int64_t items = int64_t(T) * ((row_vecs + 31) / 32);
-    permute::finalize_weighted_kernel<<<permute::grid_for_rows(items), permute::kThreads, 0,
-                                        static_cast<cudaStream_t>(stream)>>>(
+    auto* kern = k == 1   ? permute::finalize_weighted_kernel<1>
+                 : k == 2 ? permute::finalize_weighted_kernel<2>
+                 : k <= 4 ? permute::finalize_weighted_kernel<4>
+                          : permute::finalize_weighted_kernel<8>;
+    kern<<<permute::grid_for_rows(items), permute::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const uint8_t*>(d_bf16), weights, static_cast<uint8_t*>(out_bf16), T, k, row_vecs);
     DQ_LAUNCH_CHECK();
     return DQMOE_OK;
@@ -192,6 +326,10 @@ int dqmoe_quant_fp8_block_1x128(const void* x_bf16, int64_t rows, int cols, void
     DQ_CHECK(x_bf16 != nullptr && q != nullptr && scale != nullptr);
     DQ_CHECK_FMT(cols % 8 == 0, "cols=%d must be a multiple of 8", cols);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
+    // strips of a row with 16 columns per lane where rows and output allow it: more loads in flight than a warp per row has
+    // (4096 x 4096: 15.0 us, in strips 9.8 us)
+    if (cols % 16 == 0 && is_aligned(q, 16) && rows < (int64_t(1) << 31))
+        return permute::scatter_quant_1x128(x_bf16, int(rows), 1, cols, nullptr, q, scale, static_cast<cudaStream_t>(stream));
     permute::quant_1x128_kernel<<<permute::grid_for_rows(rows), permute::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const uint8_t*>(x_bf16), rows, cols, 1, nullptr, static_cast<uint8_t*>(q), scale);
     DQ_LAUNCH_CHECK();

@@ -69,8 +69,46 @@ __global__ void __launch_bounds__(kThreads) rowwise_kernel(const uint8_t* __rest
     }
 }
 
-// Second pass over the bf16 intermediate when stage 1 already produced the amax: one warp per row
-// (grid-stride), four 16-byte vectors per lane in flight, the scale arithmetic once per row.
+// Short rows (up to 2048 columns): one warp per row, the row's vectors (at most eight per lane) fetched together and kept
+// in registers between the amax and the conversion. Above, a warp would have to read the row twice and the block form,
+// whose 256 threads hold the row's loads in flight, is the better one. (16384 x 2048: block form 30.2 us, warp form 17.6 us.)
+constexpr int kShortRowVecs = 256;
+__global__ void __launch_bounds__(kThreads) rowwise_short_kernel(const uint8_t* __restrict__ x, int64_t rows, int cols,
+                                                                 uint8_t* __restrict__ q, float* __restrict__ scale) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nwarps = int64_t(gridDim.x) * (kThreads / 32);
+    const int vecs = cols / 8;
+    for (int64_t r = (int64_t(blockIdx.x) * kThreads + threadIdx.x) >> 5; r < rows; r += nwarps) {
+        const uint8_t* xr = x + size_t(r) * cols * 2;
+        Vec16 raw[kShortRowVecs / 32];
+#pragma unroll
+        for (int i = 0; i < kShortRowVecs / 32; ++i)
+            raw[i] = lane + 32 * i < vecs ? ld_nc16(xr + size_t(lane + 32 * i) * 16) : Vec16{0, 0, 0, 0};
+        float m = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kShortRowVecs / 32; ++i) {
+            float v[8];
+            unpack8(raw[i], v);
+            m = amax8(v, m);
+        }
+        const float sf = scale_from_amax(warp_max(m));
+        const float inv = inv_scale(sf);
+        if (lane == 0) scale[r] = sf;
+        uint8_t* qr = q + size_t(r) * cols;
+#pragma unroll
+        for (int i = 0; i < kShortRowVecs / 32; ++i) {
+            if (lane + 32 * i < vecs) {
+                float v[8];
+                unpack8(raw[i], v);
+                *reinterpret_cast<uint2*>(qr + size_t(lane + 32 * i) * 8) = quant8(v, inv);
+            }
+        }
+    }
+}
+
+// Second pass over the bf16 intermediate when stage 1 already produced the amax: one warp per (row, strip of 128 16-byte
+// vectors), four vectors per lane in flight. A warp per whole row left most of the chip idle when there are few long rows
+// (32 rows of 14336: 13.4 us; in strips 2.7 us).
 __global__ void __launch_bounds__(kThreads) requant_rows_kernel(const uint8_t* __restrict__ x, int64_t rows, int cols,
                                                                 uint8_t* __restrict__ q, float* __restrict__ scale,
                                                                 const float* __restrict__ amax_in, int amax_per_row,
@@ -80,67 +118,93 @@ __global__ void __launch_bounds__(kThreads) requant_rows_kernel(const uint8_t* _
     const int64_t warp = (int64_t(blockIdx.x) * kThreads + threadIdx.x) >> 5;
     const int64_t nwarps = int64_t(gridDim.x) * (kThreads / 32);
     const int vecs = cols / 8;
-    for (int64_t r = warp; r < rows; r += nwarps) {
-        const float sf = scale_from_amax(amax_in[amax_per_row ? r : 0]);
-        const float inv = inv_scale(sf);
-        if (lane == 0 && (amax_per_row || r == 0)) scale[amax_per_row ? r : 0] = sf;
+    const int strips = (vecs + 127) / 128;
+    for (int64_t it = warp; it < rows * strips; it += nwarps) {
+        const int64_t r = it / strips;
+        const int strip = int(it - r * strips);
+        const int i0 = strip * 128 + lane;
         const uint8_t* xr = x + size_t(r) * cols * 2;
         uint8_t* qr = q + size_t(r) * cols;
-        for (int i0 = lane; i0 < vecs; i0 += 128) {
-            Vec16 raw[4];
+        Vec16 raw[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (i0 + 32 * j < vecs) raw[j] = ld_nc16(xr + size_t(i0 + 32 * j) * 16);
+        for (int j = 0; j < 4; ++j)
+            if (i0 + 32 * j < vecs) raw[j] = ld_nc16(xr + size_t(i0 + 32 * j) * 16);
+        const float sf = scale_from_amax(amax_in[amax_per_row ? r : 0]);
+        const float inv = inv_scale(sf);
+        if (lane == 0 && strip == 0 && (amax_per_row || r == 0)) scale[amax_per_row ? r : 0] = sf;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (i0 + 32 * j < vecs) {
-                    float v[8];
-                    unpack8(raw[j], v);
-                    *reinterpret_cast<uint2*>(qr + size_t(i0 + 32 * j) * 8) = quant8(v, inv);
-                }
+        for (int j = 0; j < 4; ++j) {
+            if (i0 + 32 * j < vecs) {
+                float v[8];
+                unpack8(raw[j], v);
+                *reinterpret_cast<uint2*>(qr + size_t(i0 + 32 * j) * 8) = quant8(v, inv);
             }
         }
     }
 }
 
-// One block per 128x128 weight block: 256 threads = 16 column-vectors x 16 row lanes.
+// One block per 128x128 weight block: 256 threads = 16 column-vectors x 16 row lanes. A thread's eight 16-byte vectors
+// are fetched together and stay in registers between the amax and the conversion, and the next block's are on their way
+// while this one is reduced and written (HBM-bound: 3 B per element; 8 x 4096 x 14336: fetched one by one and read a second
+// time for the conversion 417 us, in one pass 284 us, with the next block's loads ahead 269 us = 5.2 TB/s).
 __global__ void __launch_bounds__(kThreads) block128_kernel(const uint8_t* __restrict__ w, int e, int rows, int cols,
                                                             uint8_t* __restrict__ q, float* __restrict__ scale) {
     __shared__ float s_red[kThreads / 32];
     const int bc = (cols + 127) / 128, br = (rows + 127) / 128;
     const int64_t blocks = int64_t(e) * br * bc;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    for (int64_t b = blockIdx.x; b < blocks; b += gridDim.x) {
+    struct Place {
+        size_t first;   // this thread's first element
+        int rows_left;  // rows of the matrix from it on, 0 beyond the last column
+    };
+    auto place = [&](int64_t b) {
         const int ei = int(b / (int64_t(br) * bc));
-        const int rb = int((b / bc) % br), cb = int(b % bc);
-        const int c = cb * 128 + tx * 8;
-        const uint8_t* base = w + size_t(ei) * rows * cols * 2;
+        const int r0 = int((b / bc) % br) * 128 + ty, c = int(b % bc) * 128 + tx * 8;
+        return Place{(size_t(ei) * rows + r0) * cols + c, c < cols ? max(0, rows - r0) : 0};
+    };
+    auto fetch = [&](const Place& pl, Vec16 (&raw)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            raw[i] = 16 * i < pl.rows_left ? ld_nc16(w + (pl.first + size_t(16 * i) * cols) * 2) : Vec16{0, 0, 0, 0};
+    };
+    Vec16 raw[8];
+    int64_t b = blockIdx.x;
+    if (b >= blocks) return;
+    Place pl = place(b);
+    fetch(pl, raw);
+    while (true) {
         float m = 0.0f;
-        if (c < cols) {
-            for (int rr = ty; rr < 128; rr += 16) {
-                const int r = rb * 128 + rr;
-                if (r < rows) {
-                    float v[8];
-                    unpack8(ld_nc16(base + (size_t(r) * cols + c) * 2), v);
-                    m = amax8(v, m);
-                }
-            }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float v[8];
+            unpack8(raw[i], v);
+            m = amax8(v, m);
+        }
+        const int64_t next = b + gridDim.x;
+        const bool more = next < blocks;
+        Place pn{0, 0};
+        Vec16 ahead[8];
+        if (more) {
+            pn = place(next);
+            fetch(pn, ahead);
         }
         const float amax = block_max(m, s_red);
         const float sf = scale_from_amax(amax);
         const float inv = inv_scale(sf);
         if (threadIdx.x == 0) scale[b] = sf;
-        if (c < cols) {
-            uint8_t* qbase = q + size_t(ei) * rows * cols;
-            for (int rr = ty; rr < 128; rr += 16) {
-                const int r = rb * 128 + rr;
-                if (r < rows) {
-                    float v[8];
-                    unpack8(ld_nc16(base + (size_t(r) * cols + c) * 2), v);
-                    *reinterpret_cast<uint2*>(qbase + size_t(r) * cols + c) = quant8(v, inv);
-                }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (16 * i < pl.rows_left) {
+                float v[8];
+                unpack8(raw[i], v);
+                *reinterpret_cast<uint2*>(q + pl.first + size_t(16 * i) * cols) = quant8(v, inv);
             }
         }
+        if (!more) break;
+        b = next;
+        pl = pn;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) raw[i] = ahead[i];
     }
 }
 
@@ -221,6 +285,12 @@ int dqmoe_quant_fp8_rowwise(const void* x_bf16, int64_t rows, int cols, void* q,
     DQ_CHECK(x_bf16 != nullptr && q != nullptr && scale != nullptr);
     DQ_CHECK_FMT(cols % 8 == 0, "cols=%d must be a multiple of 8", cols);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
+    if (cols / 8 <= quant::kShortRowVecs) {
+        quant::rowwise_short_kernel<<<quant::grid_cap((rows + 7) / 8, 8), quant::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+            static_cast<const uint8_t*>(x_bf16), rows, cols, static_cast<uint8_t*>(q), scale);
+        DQ_LAUNCH_CHECK();
+        return DQMOE_OK;
+    }
     quant::rowwise_kernel<<<quant::grid_cap(rows, 16), quant::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const uint8_t*>(x_bf16), rows, cols, static_cast<uint8_t*>(q), scale);
     DQ_LAUNCH_CHECK();
@@ -234,7 +304,7 @@ int dqmoe_requant_from_amax_dev(const void* act_bf16, int64_t n_max, int I, cons
     DQ_CHECK(act_bf16 != nullptr && q != nullptr && scale != nullptr && amax != nullptr);
     DQ_CHECK_FMT(I % 8 == 0, "I=%d must be a multiple of 8", I);
     DQ_CHECK(is_aligned(act_bf16, 16) && is_aligned(q, 8));
-    quant::requant_rows_kernel<<<quant::grid_cap((n_max + 7) / 8, 8), quant::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    quant::requant_rows_kernel<<<quant::grid_cap((n_max * ((I / 8 + 127) / 128) + 7) / 8, 8), quant::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const uint8_t*>(act_bf16), n_max, I, static_cast<uint8_t*>(q), scale, amax, per_row ? 1 : 0,
         n_rows_device);
     DQ_LAUNCH_CHECK();
@@ -254,7 +324,7 @@ int dqmoe_quant_fp8_block_128x128(const void* w_bf16, int e, int rows, int cols,
     DQ_CHECK_FMT(cols % 8 == 0, "cols=%d must be a multiple of 8", cols);
     DQ_CHECK(is_aligned(w_bf16, 16) && is_aligned(q, 8));
     const int64_t blocks = int64_t(e) * ((rows + 127) / 128) * ((cols + 127) / 128);
-    quant::block128_kernel<<<quant::grid_cap(blocks, 16), quant::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    quant::block128_kernel<<<quant::grid_cap(blocks, 3), quant::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const uint8_t*>(w_bf16), e, rows, cols, static_cast<uint8_t*>(q), scale);
     DQ_LAUNCH_CHECK();
     return DQMOE_OK;
