@@ -149,6 +149,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
     constexpr int kSfAtoms = F::kSfAtoms, kSfStage = F::kSfStage, kSfCols = F::kSfCols, kSfCol = F::kSfCol,
                   kAccCol1 = F::kAccCol1;
     constexpr int kSfPart = kSfAtoms * kSfBlock;  // scale bytes of 128 rows and one stage
+    pdl_launch();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     Shared<kFp4>& st = *reinterpret_cast<Shared<kFp4>*>(smem + size_t(kStages) * kStageBytes);
@@ -174,6 +175,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
         ptx::tmem_alloc(&st.tmem_base, kTmemCols);
         ptx::tmem_relinquish();
     }
+    pdl_wait();  // from here on global memory is read
     for (int i = threadIdx.x; i <= p.E; i += kThreads) {
         st.mprefix[i] = p.mtile_prefix[i];
         st.offsets[i] = p.offsets[i];
@@ -552,6 +554,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p,
             configured[dev] = true;
         }
     }
+    if (p.n_rows <= kPdlGemmRows) return launch_pdl(kern, dim3(sm_count()), kThreads, smem_bytes<kFp4>(), stream, ma, mb, p);
     kern<<<sm_count(), kThreads, smem_bytes<kFp4>(), stream>>>(ma, mb, p);
     DQ_LAUNCH_CHECK();
     return DQMOE_OK;

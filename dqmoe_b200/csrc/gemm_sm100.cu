@@ -208,6 +208,7 @@ template <bool kFp8, int kMode, bool kGated, bool kPair, int kBox, int kElem = k
 __global__ void __launch_bounds__(kThreads, 1)
 moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                                       const __grid_constant__ CUtensorMap tma_b, const Params p) {
+    pdl_launch();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     SharedTail& st = *reinterpret_cast<SharedTail*>(smem + size_t(kStages) * kStageBytes);
@@ -255,6 +256,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
             ptx::tmem_relinquish();
         }
     }
+    pdl_wait();  // from here on global memory is read
     for (int i = threadIdx.x; i <= p.E; i += kThreads) {
         st.mprefix[i] = p.mtile_prefix[i];
         st.offsets[i] = p.offsets[i];
@@ -816,25 +818,21 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p,
             configured[dev] = true;
         }
     }
-    if constexpr (kPair) {
-        // clusters of two CTAs on neighbouring SMs; an even grid
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(unsigned(sm_count() & ~1), 1, 1);
-        cfg.blockDim = dim3(kThreads, 1, 1);
-        cfg.dynamicSmemBytes = kSmemBytes;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        DQ_CUDA(cudaLaunchKernelEx(&cfg, kern, ma, mb, p));
-    } else {
-        kern<<<sm_count(), kThreads, kSmemBytes, stream>>>(ma, mb, p);
-    }
-    DQ_LAUNCH_CHECK();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(kPair ? sm_count() & ~1 : sm_count()), 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = p.n_rows <= kPdlGemmRows ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;  // pairs: clusters of two CTAs on neighbouring SMs; an even grid
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = kPair ? 2 : 1;
+    DQ_CUDA(cudaLaunchKernelEx(&cfg, kern, ma, mb, p));
     return DQMOE_OK;
 }
 

@@ -18,7 +18,7 @@ int route_topk(const float* logits, int T, int E, int k, int n_shared, int scori
 }  // namespace route
 namespace permute {
 int scatter_rows(const void* src, size_t row_bytes, int T, int k, const int* src_to_dest, void* dst, const float* src_scale,
-                 int scale_cols, float* dst_scale, cudaStream_t stream);
+                 int scale_cols, float* dst_scale, float* amax, int amax_per_row, cudaStream_t stream);
 int scatter_quant_1x128(const void* x_bf16, int T, int k, int H, const int* src_to_dest, void* q, float* scale, cudaStream_t stream);
 }  // namespace permute
 namespace gemm {
@@ -183,7 +183,9 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
                                L.sort_ws_bytes, stream);
     if (rc != DQMOE_OK) return rc;
 
-    rc = permute::scatter_rows(a, size_t(H) * esz, T, k, src_to_dest, perm_a, a_scale, L.perm_scale_cols, perm_a_scale, stream);
+    const bool two_pass = quant_mode == DQMOE_QUANT_FP8_TENSOR || quant_mode == DQMOE_QUANT_FP8_CHANNEL;
+    rc = permute::scatter_rows(a, size_t(H) * esz, T, k, src_to_dest, perm_a, a_scale, L.perm_scale_cols, perm_a_scale,
+                               two_pass ? amax : nullptr, quant_mode == DQMOE_QUANT_FP8_CHANNEL, stream);
     if (rc != DQMOE_OK) return rc;
 
     if (quant_mode == DQMOE_QUANT_FP8_MX) {
@@ -202,11 +204,6 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
                                         nullptr, dest_to_src, nullptr, bias2, false, nullptr, nullptr, nullptr, stream);
     }
     const float* sa1 = quant_mode == DQMOE_QUANT_FP8_TENSOR ? a_scale : perm_a_scale;
-    const bool two_pass = quant_mode == DQMOE_QUANT_FP8_TENSOR || quant_mode == DQMOE_QUANT_FP8_CHANNEL;
-    if (two_pass) {
-        const size_t amax_bytes = quant_mode == DQMOE_QUANT_FP8_CHANNEL ? size_t(n) * sizeof(float) : sizeof(float);
-        DQ_CUDA(cudaMemsetAsync(amax, 0, amax_bytes, stream));
-    }
     rc = gemm::grouped_gemm(perm_a, sa1, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1,
                             two_pass ? act_bf16 : act, act_scale, amax, nullptr, nullptr, stream, elem, bias1);
     if (rc != DQMOE_OK) return rc;
@@ -272,7 +269,7 @@ int dqmoe_moe_forward_nvfp4(const void* a, const uint8_t* a_sf, const float* a_g
     int rc = route::route_sort(m_indices, n, E, counts, offsets, mtile_prefix, dest_to_src, src_to_dest, ws + L.sort_ws,
                                L.sort_ws_bytes, stream);
     if (rc != DQMOE_OK) return rc;
-    rc = permute::scatter_rows(a, size_t(H) / 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, stream);
+    rc = permute::scatter_rows(a, size_t(H) / 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, nullptr, 0, stream);
     if (rc != DQMOE_OK) return rc;
     // one scale byte per 16 elements: the tiling kernel sees them as the scales of a row twice as long
     rc = dqmoe_mx_tile_scales(a_sf, n, 2 * H, dest_to_src, k, offsets, mtile_prefix, E, perm_a_sf, stream);
@@ -423,7 +420,7 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
     if (fp8)  // quantise on the way into expert order: a token is read as bf16 once, its k rows written as e4m3 + 1x128 scales
         rc = permute::scatter_quant_1x128(x_bf16, T, k, H, src_to_dest, perm_a, perm_a_scale, stream);
     else
-        rc = permute::scatter_rows(x_bf16, size_t(H) * 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, stream);
+        rc = permute::scatter_rows(x_bf16, size_t(H) * 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, nullptr, 0, stream);
     if (rc != DQMOE_OK) return rc;
     rc = gemm::grouped_gemm(perm_a, perm_a_scale, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, act,
                             act_scale, nullptr, nullptr, nullptr, stream);

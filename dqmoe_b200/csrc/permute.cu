@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(kThreads) row_move_kernel(const uint8_t* __res
                                                             const int* __restrict__ map, int n, int k, int row_vecs,
                                                             const float* __restrict__ src_scale,
                                                             float* __restrict__ dst_scale, int scale_cols) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int warps = gridDim.x * kWarpsPerBlock;
     for (int r = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); r < n; r += warps) {
@@ -66,6 +67,7 @@ __global__ void __launch_bounds__(kThreads) finalize_weighted_kernel(const uint8
                                                                      const float* __restrict__ w,
                                                                      uint8_t* __restrict__ out, int T, int k,
                                                                      int row_vecs) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int strips = (row_vecs + 31) / 32;
     const int64_t items = int64_t(T) * strips;
@@ -105,7 +107,8 @@ __global__ void __launch_bounds__(kThreads) finalize_weighted_kernel(const uint8
 // The layer's way into expert order: token t's row goes to rows src_to_dest[t*k + j] of the sorted matrix (negative: a
 // dropped slot). One warp per (token, strip of 128 16-byte vectors); a token is read - and in the quantising form
 // converted - once for its k copies, where the gathers above and below read it k times (HBM-bound: k + 1 rows of traffic
-// per token, the k writes dominating. 8192 tokens of 7168, k = 8, quantising: gather 353 us, scatter 111 us = 5.3 TB/s;
+// per token, the k writes dominating. It also clears the amax words fc1 collects into, one per row or one in all, which
+// saves a memset between two kernels. 8192 tokens of 7168, k = 8, quantising: gather 353 us, scatter 111 us = 5.3 TB/s;
 // 16384 bf16 rows of 2880, k = 3: 102 / 62 us; 16384 e4m3 rows of 2048, k = 8: 82 / 50 us).
 __device__ __forceinline__ int slot_dest(const int* __restrict__ src_to_dest, int t, int k, int j0, int lane) {
     if (src_to_dest == nullptr) return t;  // rows stay where they are (k = 1)
@@ -115,8 +118,11 @@ __device__ __forceinline__ int slot_dest(const int* __restrict__ src_to_dest, in
 __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
                                                                 const int* __restrict__ src_to_dest, int T, int k, int row_vecs,
                                                                 const float* __restrict__ src_scale,
-                                                                float* __restrict__ dst_scale, int scale_cols) {
+                                                                float* __restrict__ dst_scale, int scale_cols,
+                                                                float* __restrict__ amax, int amax_per_row) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
+    if (amax != nullptr && !amax_per_row && blockIdx.x == 0 && threadIdx.x == 0) amax[0] = 0.0f;
     const int strips = (row_vecs + 127) / 128;
     const int64_t items = int64_t(T) * strips;
     const int64_t warps = int64_t(gridDim.x) * kWarpsPerBlock;
@@ -137,6 +143,7 @@ __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* _
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
                     if (v0 + 32 * u < row_vecs) st16(dst + (size_t(r) * row_vecs + v0 + 32 * u) * 16, x[u]);
+                if (amax_per_row && strip == 0 && lane == 0) amax[r] = 0.0f;
                 if (strip == 0)
                     for (int c = lane; c < scale_cols; c += 32) dst_scale[size_t(r) * scale_cols + c] = src_scale[size_t(t) * scale_cols + c];
             }
@@ -149,6 +156,7 @@ __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* _
 __global__ void __launch_bounds__(kThreads) scatter_quant_1x128_kernel(const uint8_t* __restrict__ x, int T, int k, int cols,
                                                                        const int* __restrict__ src_to_dest,
                                                                        uint8_t* __restrict__ q, float* __restrict__ scale) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int groups = (cols + 127) / 128;
     const int strips = (cols + 1023) / 1024;
@@ -207,6 +215,7 @@ __global__ void __launch_bounds__(kThreads) scatter_quant_1x128_kernel(const uin
 __global__ void __launch_bounds__(kThreads) quant_1x128_kernel(const uint8_t* __restrict__ x, int64_t rows, int cols,
                                                                int k, const int* __restrict__ map,
                                                                uint8_t* __restrict__ q, float* __restrict__ scale) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int groups = (cols + 127) / 128;
     const int64_t warps = int64_t(gridDim.x) * kWarpsPerBlock;
@@ -248,19 +257,15 @@ __global__ void __launch_bounds__(kThreads) quant_1x128_kernel(const uint8_t* __
 
 // Arguments have been checked by the layer (layer.cu).
 int scatter_rows(const void* src, size_t row_bytes, int T, int k, const int* src_to_dest, void* dst, const float* src_scale,
-                 int scale_cols, float* dst_scale, cudaStream_t stream) {
+                 int scale_cols, float* dst_scale, float* amax, int amax_per_row, cudaStream_t stream) {
     const int row_vecs = int(row_bytes / 16);
     DQ_CHECK(is_aligned(src, 16) && is_aligned(dst, 16));
-    scatter_rows_kernel<<<grid_for_rows(int64_t(T) * ceil_div(row_vecs, 128)), kThreads, 0, stream>>>(
-        static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), src_to_dest, T, k, row_vecs, src_scale, dst_scale, scale_cols);
-    DQ_LAUNCH_CHECK();
+    DQ_RC(launch_pdl(scatter_rows_kernel, dim3(grid_for_rows(int64_t(T) * ceil_div(row_vecs, 128))), kThreads, 0, stream, static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), src_to_dest, T, k, row_vecs, src_scale, dst_scale, scale_cols, amax, amax_per_row));
     return DQMOE_OK;
 }
 int scatter_quant_1x128(const void* x_bf16, int T, int k, int H, const int* src_to_dest, void* q, float* scale, cudaStream_t stream) {
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 16) && H % 16 == 0);
-    scatter_quant_1x128_kernel<<<grid_for_rows(int64_t(T) * ceil_div(H, 1024)), kThreads, 0, stream>>>(
-        static_cast<const uint8_t*>(x_bf16), T, k, H, src_to_dest, static_cast<uint8_t*>(q), scale);
-    DQ_LAUNCH_CHECK();
+    DQ_RC(launch_pdl(scatter_quant_1x128_kernel, dim3(grid_for_rows(int64_t(T) * ceil_div(H, 1024))), kThreads, 0, stream, static_cast<const uint8_t*>(x_bf16), T, k, H, src_to_dest, static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 
@@ -279,10 +284,7 @@ int dqmoe_permute_rows(const void* src, size_t row_bytes, int k, const int32_t* 
     DQ_CHECK_FMT(row_bytes % 16 == 0 && row_bytes > 0, "row_bytes=%zu must be a multiple of 16", row_bytes);
     DQ_CHECK(is_aligned(src, 16) && is_aligned(dst, 16));
     if (scale_cols > 0) DQ_CHECK(src_scale != nullptr && dst_scale != nullptr);
-    permute::row_move_kernel<true><<<permute::grid_for_rows(n), permute::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), dest_to_src, n, k, int(row_bytes / 16), src_scale,
-        dst_scale, scale_cols);
-    DQ_LAUNCH_CHECK();
+    DQ_RC(launch_pdl(permute::row_move_kernel<true>, dim3(permute::grid_for_rows(n)), permute::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), dest_to_src, n, k, int(row_bytes / 16), src_scale, dst_scale, scale_cols));
     return DQMOE_OK;
 }
 
@@ -293,10 +295,7 @@ int dqmoe_finalize_scatter(const void* rows, size_t row_bytes, const int32_t* de
     DQ_CHECK(rows != nullptr && d != nullptr && dest_to_src != nullptr);
     DQ_CHECK_FMT(row_bytes % 16 == 0 && row_bytes > 0, "row_bytes=%zu must be a multiple of 16", row_bytes);
     DQ_CHECK(is_aligned(rows, 16) && is_aligned(d, 16));
-    permute::row_move_kernel<false><<<permute::grid_for_rows(n), permute::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(rows), static_cast<uint8_t*>(d), dest_to_src, n, 1, int(row_bytes / 16), nullptr,
-        nullptr, 0);
-    DQ_LAUNCH_CHECK();
+    DQ_RC(launch_pdl(permute::row_move_kernel<false>, dim3(permute::grid_for_rows(n)), permute::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(rows), static_cast<uint8_t*>(d), dest_to_src, n, 1, int(row_bytes / 16), nullptr, nullptr, 0));
     return DQMOE_OK;
 }
 
@@ -313,9 +312,8 @@ int dqmoe_finalize_weighted(const void* d_bf16, const float* weights, void* out_
                  : k == 2 ? permute::finalize_weighted_kernel<2>
                  : k <= 4 ? permute::finalize_weighted_kernel<4>
                           : permute::finalize_weighted_kernel<8>;
-    kern<<<permute::grid_for_rows(items), permute::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(d_bf16), weights, static_cast<uint8_t*>(out_bf16), T, k, row_vecs);
-    DQ_LAUNCH_CHECK();
+    DQ_RC(launch_pdl(kern, dim3(permute::grid_for_rows(items)), permute::kThreads, 0, static_cast<cudaStream_t>(stream),
+                     static_cast<const uint8_t*>(d_bf16), weights, static_cast<uint8_t*>(out_bf16), T, k, row_vecs));
     return DQMOE_OK;
 }
 
@@ -330,9 +328,7 @@ int dqmoe_quant_fp8_block_1x128(const void* x_bf16, int64_t rows, int cols, void
     // (4096 x 4096: 15.0 us, in strips 9.8 us)
     if (cols % 16 == 0 && is_aligned(q, 16) && rows < (int64_t(1) << 31))
         return permute::scatter_quant_1x128(x_bf16, int(rows), 1, cols, nullptr, q, scale, static_cast<cudaStream_t>(stream));
-    permute::quant_1x128_kernel<<<permute::grid_for_rows(rows), permute::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(x_bf16), rows, cols, 1, nullptr, static_cast<uint8_t*>(q), scale);
-    DQ_LAUNCH_CHECK();
+    DQ_RC(launch_pdl(permute::quant_1x128_kernel, dim3(permute::grid_for_rows(rows)), permute::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows, cols, 1, nullptr, static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 
@@ -343,9 +339,7 @@ int dqmoe_permute_quant_block_1x128(const void* x_bf16, int H, int k, const int3
     DQ_CHECK(x_bf16 != nullptr && q != nullptr && scale != nullptr && dest_to_src != nullptr);
     DQ_CHECK_FMT(H % 8 == 0, "H=%d must be a multiple of 8", H);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
-    permute::quant_1x128_kernel<<<permute::grid_for_rows(n), permute::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(x_bf16), n, H, k, dest_to_src, static_cast<uint8_t*>(q), scale);
-    DQ_LAUNCH_CHECK();
+    DQ_RC(launch_pdl(permute::quant_1x128_kernel, dim3(permute::grid_for_rows(n)), permute::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), n, H, k, dest_to_src, static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 

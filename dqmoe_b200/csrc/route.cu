@@ -25,6 +25,7 @@ __device__ __forceinline__ int bucket_of(int id, int E) { return (id >= 0 && id 
 // ---------------------------------------------------------------- pass 1: chunk histograms
 __global__ void __launch_bounds__(kSortThreads) sort_hist_kernel(const int* __restrict__ ids, int n, int E,
                                                                  int* __restrict__ chunk_hist /*[chunks][E+1]*/) {
+    pdl_enter();
     extern __shared__ int s_hist[];  // E+1
     for (int i = threadIdx.x; i <= E; i += kSortThreads) s_hist[i] = 0;
     __syncthreads();
@@ -88,6 +89,7 @@ template <bool kStaged>
 __global__ void __launch_bounds__(1024) sort_scan_kernel(int* __restrict__ chunk_hist, int chunks, int E,
                                                          int* __restrict__ counts, int* __restrict__ offsets,
                                                          int* __restrict__ mtile_prefix) {
+    pdl_enter();
     extern __shared__ int s_hist[];  // kStaged: [chunks][E + 1]
     __shared__ int s_tot[kMaxExperts + 2];
     __shared__ int s_tiles[kMaxExperts + 2];
@@ -139,6 +141,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* _
                                                                     int* __restrict__ mtile_prefix,
                                                                     int* __restrict__ dest_to_src,
                                                                     int* __restrict__ src_to_dest) {
+    pdl_enter();
     extern __shared__ int s_mem[];
     // s_warp_hist[w][E+1]: rows of bucket b seen so far by warp w, then exclusive prefix over warps
     int* s_warp_hist = s_mem;
@@ -277,26 +280,20 @@ int route_sort(const int* ids, int n, int E, int* counts, int* offsets, int* mti
         }
     }
     if (chunks == 1) {
-        sort_scatter_kernel<true><<<1, kSortThreads, smem_scatter, stream>>>(ids, n, E, nullptr, counts, offsets,
-                                                                            mtile_prefix, dest_to_src, src_to_dest);
-        DQ_LAUNCH_CHECK();
+        DQ_RC(launch_pdl(sort_scatter_kernel<true>, dim3(1), kSortThreads, smem_scatter, stream, ids, n, E, nullptr, counts, offsets, mtile_prefix, dest_to_src, src_to_dest));
         return DQMOE_OK;
     }
     if (ws == nullptr || ws_bytes < sort_workspace_bytes(n, E) || !is_aligned(ws, 16))
         return fail(DQMOE_ERR_WORKSPACE, __FILE__, __LINE__, "ws_bytes >= sort_workspace_bytes(n, E)",
                     "sort workspace %zu bytes, need %zu", ws_bytes, sort_workspace_bytes(n, E));
     int* chunk_hist = static_cast<int*>(ws);
-    sort_hist_kernel<<<chunks, kSortThreads, (E + 1) * sizeof(int), stream>>>(ids, n, E, chunk_hist);
-    DQ_LAUNCH_CHECK();
+    DQ_RC(launch_pdl(sort_hist_kernel, dim3(chunks), kSortThreads, (E + 1) * sizeof(int), stream, ids, n, E, chunk_hist));
     const size_t smem_scan = size_t(chunks) * (E + 1) * sizeof(int);
     if (smem_scan <= size_t(kScanSmemMax))
-        sort_scan_kernel<true><<<1, 1024, smem_scan, stream>>>(chunk_hist, chunks, E, counts, offsets, mtile_prefix);
+        DQ_RC(launch_pdl(sort_scan_kernel<true>, dim3(1), 1024, smem_scan, stream, chunk_hist, chunks, E, counts, offsets, mtile_prefix));
     else
-        sort_scan_kernel<false><<<1, 1024, 0, stream>>>(chunk_hist, chunks, E, counts, offsets, mtile_prefix);
-    DQ_LAUNCH_CHECK();
-    sort_scatter_kernel<false><<<chunks, kSortThreads, smem_scatter, stream>>>(ids, n, E, chunk_hist, counts, offsets,
-                                                                              mtile_prefix, dest_to_src, src_to_dest);
-    DQ_LAUNCH_CHECK();
+        DQ_RC(launch_pdl(sort_scan_kernel<false>, dim3(1), 1024, 0, stream, chunk_hist, chunks, E, counts, offsets, mtile_prefix));
+    DQ_RC(launch_pdl(sort_scatter_kernel<false>, dim3(chunks), kSortThreads, smem_scatter, stream, ids, n, E, chunk_hist, counts, offsets, mtile_prefix, dest_to_src, src_to_dest));
     return DQMOE_OK;
 }
 
@@ -309,6 +306,7 @@ template <int kPerLane>
 __global__ void __launch_bounds__(256) route_topk_kernel(const float* __restrict__ logits, int T, int E, int k,
                                                          int slots, int scoring, int* __restrict__ indices,
                                                          float* __restrict__ weights) {
+    pdl_enter();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= T) return;
@@ -376,13 +374,12 @@ int route_topk(const float* logits, int T, int E, int k, int n_shared, int scori
     if (T == 0) return DQMOE_OK;
     DQ_CHECK(logits != nullptr && indices != nullptr && weights != nullptr);
     const int blocks = ceil_div(T, 8);
-    if (E <= 32) route_topk_kernel<1><<<blocks, 256, 0, stream>>>(logits, T, E, k, slots, scoring, indices, weights);
-    else if (E <= 64) route_topk_kernel<2><<<blocks, 256, 0, stream>>>(logits, T, E, k, slots, scoring, indices, weights);
-    else if (E <= 128) route_topk_kernel<4><<<blocks, 256, 0, stream>>>(logits, T, E, k, slots, scoring, indices, weights);
-    else if (E <= 256) route_topk_kernel<8><<<blocks, 256, 0, stream>>>(logits, T, E, k, slots, scoring, indices, weights);
-    else if (E <= 512) route_topk_kernel<16><<<blocks, 256, 0, stream>>>(logits, T, E, k, slots, scoring, indices, weights);
-    else route_topk_kernel<32><<<blocks, 256, 0, stream>>>(logits, T, E, k, slots, scoring, indices, weights);
-    DQ_LAUNCH_CHECK();
+    if (E <= 32) DQ_RC(launch_pdl(route_topk_kernel<1>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
+    else if (E <= 64) DQ_RC(launch_pdl(route_topk_kernel<2>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
+    else if (E <= 128) DQ_RC(launch_pdl(route_topk_kernel<4>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
+    else if (E <= 256) DQ_RC(launch_pdl(route_topk_kernel<8>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
+    else if (E <= 512) DQ_RC(launch_pdl(route_topk_kernel<16>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
+    else DQ_RC(launch_pdl(route_topk_kernel<32>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
     return DQMOE_OK;
 }
 

@@ -1,0 +1,20 @@
+"""Per-tensor FP8 quantiser on both sides of the size its single-launch cluster form holds (524288 elements per slice)."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import bits
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("e,numel", [(1, 8), (1, 8 * 8191), (3, 8 * 8193), (2, 524288), (1, 524288 + 8)])
+def test_per_tensor_quantiser_bit_exact(e, numel):
+    from dqmoe_b200 import ops
+    g = torch.Generator().manual_seed(numel % 1000)
+    x = (torch.randn(e, 1, numel, generator=g) * 3).to(torch.bfloat16)
+    x[0, 0, -1] = 77.0  # the amax in the last element: every block and thread counts
+    sf = x.float().abs().amax((1, 2)).clamp(1e-4) / 448.0
+    ref = (x.float() * (1.0 / sf)[:, None, None]).to(torch.float8_e4m3fn)
+    q, s = ops.per_tensor_cast_to_fp8(x.to("cuda"), per_expert=True)
+    assert np.array_equal(bits(s.reshape(-1)), bits(sf)) and np.array_equal(bits(q.view(e, 1, numel)), bits(ref))
