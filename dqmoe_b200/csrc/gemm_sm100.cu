@@ -70,9 +70,11 @@ struct Params {
     const int* offsets;       // [E+1] first row of each expert
     const int* mtile_prefix;  // [E+1] cumulative 128-row tiles
     const float* sa;          // activation scales
+    const float* sa_t;        // block mode: the same by tile, [row tile][K block][128], or nullptr
     const float* sb;          // weight scales
     void* out;
     float* out_scale;         // stage 1 block mode: [n, ceil(I/128)]
+    float* out_scale_t;       // stage 1 block mode: the same by tile, [row tile][ceil(I/128)][128], or nullptr
     float* amax;              // stage 1 channel: [n]; tensor: [1]
     const float* bias;        // [E, w_rows] fp32 added to the dequantised product, or nullptr
     const int* dest_to_src;   // stage 2 scatter map or nullptr
@@ -100,6 +102,7 @@ constexpr size_t kSmemBytes = 1024 + size_t(kStages) * kStageBytes + sizeof(Shar
 
 struct Tile {
     int e, row0, row_end, nt;
+    int mtile;  // index of the row tile among all row tiles (single CTAs)
 };
 
 // Tiles are numbered expert-major; inside an expert the row tile runs fastest so
@@ -115,6 +118,7 @@ __device__ __forceinline__ Tile decode_tile(int t, int& e_cursor, const SharedTa
     Tile tl;
     tl.e = e_cursor;
     tl.nt = local / mtiles;
+    tl.mtile = st.mprefix[e_cursor] + local % mtiles;
     tl.row0 = st.offsets[e_cursor] + ((local % mtiles) * (kPair ? 2 : 1) + sub) * kBM;
     tl.row_end = st.offsets[e_cursor + 1];
     return tl;
@@ -234,7 +238,8 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kNumStages; ++s) {
-            ptx::mbar_init(&st.full[s], kMode == kBlock ? 1 + 32 : 1);  // block mode: and every lane of the scale loader
+            // block mode: and the lanes of the scale loader that copy something
+            ptx::mbar_init(&st.full[s], kMode == kBlock ? 1 + (p.sa_t != nullptr ? 3 : 32) : 1);
             ptx::mbar_init(&st.empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -318,7 +323,15 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         ptx::tma_load_2d_pair(sa, &tma_a, k0, tl.row0, full_leader);
                         ptx::tma_load_2d_pair(sb, &tma_b, k0, leader ? wrow0 : wrow1, full_leader);
                     } else {
-                        ptx::mbar_arrive_expect_tx(&st.full[s], kStageSz);
+                        if constexpr (kMode == kBlock) {
+                            const bool tiled = p.sa_t != nullptr;
+                            ptx::mbar_arrive_expect_tx(&st.full[s], kStageSz + (tiled ? uint32_t(sizeof(st.sc_a[0])) : 0u));
+                            if (tiled)
+                                ptx::bulk_load(st.sc_a[it % kScaleSlots], p.sa_t + (size_t(tl.mtile) * kb_count + kb) * kBM,
+                                               sizeof(st.sc_a[0]), &st.full[s]);
+                        } else {
+                            ptx::mbar_arrive_expect_tx(&st.full[s], kStageSz);
+                        }
                         ptx::tma_load_2d(sa, &tma_a, k0, tl.row0, &st.full[s]);
                         ptx::tma_load_2d(sb, &tma_b, k0, wrow0, &st.full[s]);
                         ptx::tma_load_2d(sb + kBox * kBKBytes, &tma_b, k0, wrow1, &st.full[s]);
@@ -414,6 +427,10 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
         // 817; 1132 / 556 us -> 1100 / 514 us). The ring has more slots
         // than the kNumStages + 2 K blocks that can lie between a stage being refilled and the oldest undrained
         // accumulator, so a slot is free when its stage is.
+        // Where the caller has the activation scales by tile as well (the layer does), the TMA producer fetches a K block's 128
+        // of them with one bulk copy and this warp copies three weight scales: the row-major form costs four scattered
+        // copies and 32 barrier arrivals per K block, which the epilogue warps' shared-memory traffic queues behind
+        // (4096 tokens x 2 at the Mixtral shape: fc1 1080 -> 1022 us, fc2 530 -> 521).
         if constexpr (kMode == kBlock) {
             const int KB = kb_count;
             const int NB = (p.w_rows + 127) / 128;
@@ -435,10 +452,12 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         ok = false;
                         break;
                     }
+                    if (p.sa_t == nullptr) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) ptx::cp_async4(&st.sc_a[slot][lane + 32 * j], src_a[j] + kb);
+                        for (int j = 0; j < 4; ++j) ptx::cp_async4(&st.sc_a[slot][lane + 32 * j], src_a[j] + kb);
+                    }
                     if (lane < 3) ptx::cp_async4(&st.sc_b[slot][lane], src_b + kb);
-                    ptx::cp_async_arrive(&st.full[s]);
+                    if (p.sa_t == nullptr || lane < 3) ptx::cp_async_arrive(&st.full[s]);
                 }
             }
             ptx::cp_async_wait_all();
@@ -754,7 +773,11 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         store_rows_staged(st.stage[warp - 4], packed,
                                           row_ok ? reinterpret_cast<uint8_t*>(p.out) + size_t(grow) * I_or_H + col0 : nullptr,
                                           min(4, max(0, (I_or_H - col0 + 15) / 16)), lane);
-                        if (row_ok && h == 0) p.out_scale[size_t(grow) * ((I_or_H + 127) / 128) + tl.nt] = sf;
+                        if (h == 0) {
+                            const int groups = (I_or_H + 127) / 128;
+                            if (row_ok) p.out_scale[size_t(grow) * groups + tl.nt] = sf;
+                            if (p.out_scale_t != nullptr) p.out_scale_t[(size_t(tl.mtile) * groups + tl.nt) * kBM + r_in_tile] = sf;
+                        }
                     }
                 } else {
                     int orow_idx = grow;
@@ -849,7 +872,7 @@ static bool use_pairs(int n, int E, int quant_mode) {
 int grouped_gemm(const void* a, const float* a_scale, const void* w, const float* w_scale, const int* offsets,
                  const int* mtile_prefix, int n, int N, int K, int E, int quant_mode, int gated, void* out,
                  float* out_scale, float* amax, const int* dest_to_src, const void* row_dst, cudaStream_t stream,
-                 int elem, const float* bias) {
+                 int elem, const float* bias, const float* a_scale_t, float* out_scale_t) {
     DQ_CHECK(elem == kElemBf16 || ((elem == kElemHalf || elem == kElemF32) && quant_mode == DQMOE_QUANT_NONE));
     DQ_CHECK(quant_mode == DQMOE_QUANT_NONE || quant_mode == DQMOE_QUANT_FP8_TENSOR ||
              quant_mode == DQMOE_QUANT_FP8_CHANNEL || quant_mode == DQMOE_QUANT_FP8_BLOCK);
@@ -863,6 +886,7 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
     DQ_CHECK(is_aligned(a, 16) && is_aligned(w, 16) && is_aligned(out, 16) && is_aligned(row_dst, 8));
     DQ_CHECK(a != nullptr && w != nullptr && (out != nullptr || row_dst != nullptr) && offsets != nullptr && mtile_prefix != nullptr);
     DQ_CHECK(row_dst == nullptr || !gated);
+    DQ_CHECK(is_aligned(a_scale_t, 16));
     if (fp8) DQ_CHECK(a_scale != nullptr && w_scale != nullptr);
     if (gated && quant_mode == DQMOE_QUANT_FP8_BLOCK) DQ_CHECK(out_scale != nullptr);
     if (gated && (quant_mode == DQMOE_QUANT_FP8_TENSOR || quant_mode == DQMOE_QUANT_FP8_CHANNEL)) DQ_CHECK(amax != nullptr);
@@ -891,9 +915,11 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
     p.offsets = offsets;
     p.mtile_prefix = mtile_prefix;
     p.sa = a_scale;
+    p.sa_t = a_scale_t;
     p.sb = w_scale;
     p.out = out;
     p.out_scale = out_scale;
+    p.out_scale_t = out_scale_t;
     p.amax = amax;
     p.bias = bias;
     p.dest_to_src = dest_to_src;
@@ -940,7 +966,7 @@ extern "C" int dqmoe_grouped_gemm(const void* a, const float* a_scale, const voi
                                   const int32_t* dest_to_src, dqmoe_stream_t stream) {
     return dq::gemm::grouped_gemm(a, a_scale, w, w_scale, offsets, mtile_prefix, n, N, K, E, quant_mode, gated, out,
                                   out_scale, amax, dest_to_src, nullptr, static_cast<cudaStream_t>(stream),
-                                  dq::gemm::kElemBf16, nullptr);
+                                  dq::gemm::kElemBf16, nullptr, nullptr, nullptr);
 }
 
 extern "C" int dqmoe_grouped_gemm_rows(const void* a, const float* a_scale, const void* w, const float* w_scale,
@@ -948,5 +974,5 @@ extern "C" int dqmoe_grouped_gemm_rows(const void* a, const float* a_scale, cons
                                        int quant_mode, const void* row_dst, dqmoe_stream_t stream) {
     return dq::gemm::grouped_gemm(a, a_scale, w, w_scale, offsets, mtile_prefix, n, N, K, E, quant_mode, 0, nullptr,
                                   nullptr, nullptr, nullptr, row_dst, static_cast<cudaStream_t>(stream), dq::gemm::kElemBf16,
-                                  nullptr);
+                                  nullptr, nullptr, nullptr);
 }

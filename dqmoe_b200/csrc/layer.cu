@@ -19,13 +19,15 @@ int route_topk(const float* logits, int T, int E, int k, int n_shared, int scori
 namespace permute {
 int scatter_rows(const void* src, size_t row_bytes, int T, int k, const int* src_to_dest, void* dst, const float* src_scale,
                  int scale_cols, float* dst_scale, float* amax, int amax_per_row, cudaStream_t stream);
+int scale_tiles(const float* scale, int n, int cols, const int* offsets, const int* mtile_prefix, int E, float* out,
+                cudaStream_t stream);
 int scatter_quant_1x128(const void* x_bf16, int T, int k, int H, const int* src_to_dest, void* q, float* scale, cudaStream_t stream);
 }  // namespace permute
 namespace gemm {
 int grouped_gemm(const void* a, const float* a_scale, const void* w, const float* w_scale, const int* offsets,
                  const int* mtile_prefix, int n, int N, int K, int E, int quant_mode, int gated, void* out,
                  float* out_scale, float* amax, const int* dest_to_src, const void* row_dst, cudaStream_t stream,
-                 int elem = 0, const float* bias = nullptr);
+                 int elem = 0, const float* bias = nullptr, const float* a_scale_t = nullptr, float* out_scale_t = nullptr);
 enum Elem : int { kElemBf16 = 0, kElemHalf = 1, kElemF32 = 2 };  // element type of the unquantised path
 }  // namespace gemm
 
@@ -46,10 +48,14 @@ bool eligible(int H, int I, bool fp8);  // row sizes the decode path serves (16-
 namespace layer {
 
 constexpr size_t kAlign = 256;  // CUDA_MEM_ALIGN of the reference (csrc/util.h:54-59)
+// From this many expanded rows on, block mode lays the activation scales out by tile a second time (a launch before fc1; fc1
+// itself writes fc2's): 8192 rows, H 4096, I 14336 1985 -> 1852 us per call, 65536 rows, H 7168, I 2048 6084 -> 5999. Below,
+// the GEMMs wait for weights and nothing is gained (864 rows: 326.7 / 326.8 us; 10 rows: 35.0 / 35.8).
+constexpr int kTiledScaleRows = 4096;
 constexpr int kDecodeRows = 8;  // up to this many expanded rows the GEMV path of decode.cu is used (bf16, per-tensor FP8)
 
 struct Layout {
-    size_t offsets, counts, mtile_prefix, sort_ws, dest_to_src, src_to_dest, perm_a, perm_a_scale, act, act_scale, act_bf16, amax;
+    size_t offsets, counts, mtile_prefix, sort_ws, dest_to_src, src_to_dest, perm_a, perm_a_scale, perm_a_scale_t, act_scale_t, act, act_scale, act_bf16, amax;
     size_t total;
     size_t sort_ws_bytes;
     int perm_scale_cols;
@@ -95,6 +101,10 @@ static Layout make_layout(int T, int H, int I, int E, int k, int quant_mode, int
                                    : quant_mode == DQMOE_QUANT_FP8_CHANNEL ? n
                                    : quant_mode == DQMOE_QUANT_FP8_TENSOR ? 1 : 0;
     L.act_scale = add(act_scale_elems * sizeof(float));
+    // block mode: the scale matrices a second time by tile, for the grouped GEMMs (every expert may add a partly filled tile)
+    const size_t tile_rows = quant_mode == DQMOE_QUANT_FP8_BLOCK && n >= size_t(kTiledScaleRows) ? ((n + 127) / 128 + (size_t(E) < n ? size_t(E) : n)) * 128 : 0;
+    L.perm_a_scale_t = add(tile_rows * ceil_div(H, 128) * sizeof(float));
+    L.act_scale_t = add(tile_rows * ceil_div(I, 128) * sizeof(float));
     const bool two_pass = quant_mode == DQMOE_QUANT_FP8_TENSOR || quant_mode == DQMOE_QUANT_FP8_CHANNEL;
     L.act_bf16 = add(two_pass ? n * I * 2 : 0);
     L.amax = add(quant_mode == DQMOE_QUANT_FP8_CHANNEL ? n * sizeof(float)
@@ -171,6 +181,9 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
     float* perm_a_scale = reinterpret_cast<float*>(ws + L.perm_a_scale);
     void* act = ws + L.act;
     float* act_scale = reinterpret_cast<float*>(ws + L.act_scale);
+    const bool block = quant_mode == DQMOE_QUANT_FP8_BLOCK;
+    float* perm_a_scale_t = block && n >= layer::kTiledScaleRows ? reinterpret_cast<float*>(ws + L.perm_a_scale_t) : nullptr;
+    float* act_scale_t = perm_a_scale_t != nullptr ? reinterpret_cast<float*>(ws + L.act_scale_t) : nullptr;
     void* act_bf16 = ws + L.act_bf16;
     float* amax = reinterpret_cast<float*>(ws + L.amax);
 
@@ -204,8 +217,12 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
                                         nullptr, dest_to_src, nullptr, bias2, false, nullptr, nullptr, nullptr, stream);
     }
     const float* sa1 = quant_mode == DQMOE_QUANT_FP8_TENSOR ? a_scale : perm_a_scale;
+    if (perm_a_scale_t != nullptr) {
+        rc = permute::scale_tiles(perm_a_scale, n, L.perm_scale_cols, offsets, mtile_prefix, E, perm_a_scale_t, stream);
+        if (rc != DQMOE_OK) return rc;
+    }
     rc = gemm::grouped_gemm(perm_a, sa1, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1,
-                            two_pass ? act_bf16 : act, act_scale, amax, nullptr, nullptr, stream, elem, bias1);
+                            two_pass ? act_bf16 : act, act_scale, amax, nullptr, nullptr, stream, elem, bias1, perm_a_scale_t, act_scale_t);
     if (rc != DQMOE_OK) return rc;
     if (two_pass) {
         rc = dqmoe_requant_from_amax(act_bf16, n, I, amax, quant_mode == DQMOE_QUANT_FP8_CHANNEL ? 1 : 0, act,
@@ -213,7 +230,7 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
         if (rc != DQMOE_OK) return rc;
     }
     rc = gemm::grouped_gemm(act, act_scale, b1, b1_scale, offsets, mtile_prefix, n, H, I, E, quant_mode, 0, d, nullptr,
-                            nullptr, dest_to_src, nullptr, stream, elem, bias2);
+                            nullptr, dest_to_src, nullptr, stream, elem, bias2, act_scale_t);
     return rc;
 }
 
@@ -383,6 +400,9 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
     float* perm_a_scale = reinterpret_cast<float*>(lws + L.perm_a_scale);
     void* act = lws + L.act;
     float* act_scale = reinterpret_cast<float*>(lws + L.act_scale);
+    const bool block = quant_mode == DQMOE_QUANT_FP8_BLOCK;
+    float* perm_a_scale_t = block && n >= layer::kTiledScaleRows ? reinterpret_cast<float*>(lws + L.perm_a_scale_t) : nullptr;
+    float* act_scale_t = perm_a_scale_t != nullptr ? reinterpret_cast<float*>(lws + L.act_scale_t) : nullptr;
 
     int rc = route::route_topk(logits, T, E_routed, k_routed, n_shared, scoring, indices, weights, stream);
     if (rc != DQMOE_OK) return rc;
@@ -422,11 +442,15 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
     else
         rc = permute::scatter_rows(x_bf16, size_t(H) * 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, nullptr, 0, stream);
     if (rc != DQMOE_OK) return rc;
+    if (perm_a_scale_t != nullptr) {
+        rc = permute::scale_tiles(perm_a_scale, n, L.perm_scale_cols, offsets, mtile_prefix, E, perm_a_scale_t, stream);
+        if (rc != DQMOE_OK) return rc;
+    }
     rc = gemm::grouped_gemm(perm_a, perm_a_scale, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, act,
-                            act_scale, nullptr, nullptr, nullptr, stream);
+                            act_scale, nullptr, nullptr, nullptr, stream, gemm::kElemBf16, nullptr, perm_a_scale_t, act_scale_t);
     if (rc != DQMOE_OK) return rc;
     rc = gemm::grouped_gemm(act, act_scale, b1, b1_scale, offsets, mtile_prefix, n, H, I, E, quant_mode, 0, d, nullptr,
-                            nullptr, dest_to_src, nullptr, stream);
+                            nullptr, dest_to_src, nullptr, stream, gemm::kElemBf16, nullptr, act_scale_t);
     if (rc != DQMOE_OK) return rc;
     return dqmoe_finalize_weighted(d, weights, out_bf16, T, k, H, stream);
 }

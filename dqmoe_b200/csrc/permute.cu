@@ -255,7 +255,49 @@ __global__ void __launch_bounds__(kThreads) quant_1x128_kernel(const uint8_t* __
     }
 }
 
+// Block scales a second time by tile, for the grouped GEMM, which then fetches the 128 scales of a row tile and K block in
+// one piece: out[tile][c][r] = scale[first row of the tile + r][c], every expert starting a new 128-row tile. One block per
+// tile and 32 columns, transposed through shared memory. (Written by the scatter itself, four bytes at a time, the same
+// matrix cost 56 us at 65536 rows x 56 columns; here ~15 us.)
+__global__ void __launch_bounds__(kThreads) scale_tiles_kernel(const float* __restrict__ scale, int cols,
+                                                               const int* __restrict__ offsets,
+                                                               const int* __restrict__ mtile_prefix, int E,
+                                                               float* __restrict__ out) {
+    pdl_enter();
+    __shared__ float s[128][33];
+    const int chunks = (cols + 31) / 32;
+    const int total = mtile_prefix[E] * chunks;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int it = blockIdx.x; it < total; it += gridDim.x) {
+        const int tile = it / chunks, c0 = (it % chunks) * 32;
+        int lo = 0, hi = E;  // expert of the tile: last e with mtile_prefix[e] <= tile
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (mtile_prefix[mid] <= tile) lo = mid; else hi = mid;
+        }
+        const int row0 = offsets[lo] + (tile - mtile_prefix[lo]) * 128;
+        const int rows = min(128, offsets[lo + 1] - row0);
+#pragma unroll 4
+        for (int r = warp; r < 128; r += kWarpsPerBlock)
+            s[r][lane] = r < rows && c0 + lane < cols ? scale[size_t(row0 + r) * cols + c0 + lane] : 0.0f;
+        __syncthreads();
+        const int r = threadIdx.x & 127;
+#pragma unroll 4
+        for (int c = threadIdx.x >> 7; c < 32; c += kThreads / 128)
+            if (c0 + c < cols) out[(size_t(tile) * cols + c0 + c) * 128 + r] = s[r][c];
+        __syncthreads();
+    }
+}
+
 // Arguments have been checked by the layer (layer.cu).
+int scale_tiles(const float* scale, int n, int cols, const int* offsets, const int* mtile_prefix, int E, float* out,
+                cudaStream_t stream) {
+    const int64_t blocks = (int64_t(ceil_div(n, 128)) + (E < n ? E : n)) * ceil_div(cols, 32);
+    const int64_t cap = int64_t(sm_count()) * 8;
+    DQ_RC(launch_pdl(scale_tiles_kernel, dim3(unsigned(blocks < cap ? blocks : cap)), kThreads, 0, stream, scale, cols, offsets,
+                     mtile_prefix, E, out));
+    return DQMOE_OK;
+}
 int scatter_rows(const void* src, size_t row_bytes, int T, int k, const int* src_to_dest, void* dst, const float* src_scale,
                  int scale_cols, float* dst_scale, float* amax, int amax_per_row, cudaStream_t stream) {
     const int row_vecs = int(row_bytes / 16);
