@@ -859,13 +859,20 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p,
     return DQMOE_OK;
 }
 
-// CTA pairs halve the weight bytes each SM stages per flop; they pay off once experts have
-// several row tiles.
-static bool use_pairs(int n, int E, int quant_mode) {
-    // Block mode hands a TMEM buffer back every K block and is bound by that round trip, not by the
-    // shared-memory traffic a pair saves (measured: +1 % with pairs, while ragged experts waste more
-    // rows in 256-row tiles), so it stays on single CTAs.
-    return quant_mode != DQMOE_QUANT_FP8_BLOCK && n / E >= 512;
+// CTA pairs: a 256-row tile shares its weight tile between two SMs, which halves the weight bytes each stages. They pay off
+// when the experts' rows fill 256-row tiles about as well as 128-row ones, that is when the average lies in the upper half
+// of a 256-row period (with some room below the period's end, as the counts scatter), or when there are so many rows that the
+// last tile hardly counts. Single CTAs / pairs, us per layer call, per-tensor FP8 at H 4096, I 14336, E 8: 105 rows per
+// expert 272 / 324, 150: 368 / 322, 225: 438 / 391, 250: 430 / 442, 300: 559 / 615, 425: 670 / 607, 512: 731 / 782, 650:
+// 890 / 857; bf16 (2880 x 2880, E 64) 140: 772 / 681, 281: 1146 / 1221; per-channel (2048 x 768, E 128) 312: 329 / 390,
+// 437: 459 / 429.
+// Below 560 rows the launch must also have two rounds of single-CTA tiles (wide_tiles): with fewer, halving the number of
+// tiles leaves SMs idle.
+static bool use_pairs(int n, int E, int quant_mode, int wide_tiles) {
+    // Block mode is bound by the trip of every K block through registers, not by the traffic a pair saves.
+    if (quant_mode == DQMOE_QUANT_FP8_BLOCK) return false;
+    const int rows = n / E;
+    return rows >= 560 || ((rows & 255) > 128 && (rows & 255) <= 240 && wide_tiles >= 2 * sm_count());
 }
 
 // elem: element type of the unquantised path (kElemBf16 / kElemHalf / kElemF32); bias: [E, gated ? 2N : N] fp32 or nullptr.
@@ -893,9 +900,9 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
 
     // Tile width: 256 accumulator columns, or 128 when the launch would leave many SMs without a tile.
     // The row-tile count is known only on the device; ceil(n/128) + min(E, n) - 1 bounds it.
-    const bool pair = elem != kElemF32 && use_pairs(n, E, quant_mode);
     const int mtiles_max = ceil_div(n, kBM) + (E < n ? E : n) - 1;
     const int wide_tiles = mtiles_max * (gated ? ceil_div(N, kBoxRows) : ceil_div(N, kUmmaN));
+    const bool pair = elem != kElemF32 && use_pairs(n, E, quant_mode, wide_tiles);
     // measured on decode shapes: 128-column tiles win when 256-column tiles would fill at most half of
     // the SMs, or when there are at most two row tiles (one or two tokens); otherwise 256 columns win
     const bool narrow = quant_mode != DQMOE_QUANT_FP8_BLOCK && !pair && elem != kElemF32 &&
