@@ -280,8 +280,8 @@ def quantize_activations_gpu(ops, x, mode):
 
 def launches_per_step(n, mode):
     sort = 1 if n <= 2048 else 3
-    # sort, gather, fc1, [re-quantisation pass | scale tiling of the MXFP8 mode], fc2
-    return sort + 1 + 1 + (1 if mode in (256, 512, 2048) else 0) + 1
+    # sort, scatter into expert order, [scale tiling: MXFP8, block FP8 from 4096 rows on], fc1, [re-quantisation pass], fc2
+    return sort + 1 + 1 + (1 if mode in (256, 512, 2048) or (mode == 1024 and n >= 4096) else 0) + 1
 
 
 def config_of(name, wl, world, T=None):

@@ -1,6 +1,6 @@
 // Layer orchestrator: carves the caller's workspace and enqueues the MoE layer
 // pipeline on one stream with no host synchronisation:
-//   expert sort -> row (+scale) gather -> grouped fc1 with fused SwiGLU and
+//   expert sort -> rows (+scales) scattered into expert order -> grouped fc1 with fused SwiGLU and
 //   intermediate quantisation -> [re-quantisation pass for tensor/channel modes]
 //   -> grouped fc2 with fused dequantisation and scatter into d[T, k, H].
 // Replaces MoeFCRunner::getWorkspaceDeviceBufferSizes / runMoe / Gemm of the
@@ -55,7 +55,8 @@ constexpr int kTiledScaleRows = 4096;
 constexpr int kDecodeRows = 8;  // up to this many expanded rows the GEMV path of decode.cu is used (bf16, per-tensor FP8)
 
 struct Layout {
-    size_t offsets, counts, mtile_prefix, sort_ws, dest_to_src, src_to_dest, perm_a, perm_a_scale, perm_a_scale_t, act_scale_t, act, act_scale, act_bf16, amax;
+    size_t offsets, counts, mtile_prefix, sort_ws, dest_to_src, src_to_dest, perm_a, perm_a_scale, perm_a_scale_t, act_scale_t, act,
+        act_scale, act_bf16, amax;
     size_t total;
     size_t sort_ws_bytes;
     int perm_scale_cols;
@@ -102,7 +103,8 @@ static Layout make_layout(int T, int H, int I, int E, int k, int quant_mode, int
                                    : quant_mode == DQMOE_QUANT_FP8_TENSOR ? 1 : 0;
     L.act_scale = add(act_scale_elems * sizeof(float));
     // block mode: the scale matrices a second time by tile, for the grouped GEMMs (every expert may add a partly filled tile)
-    const size_t tile_rows = quant_mode == DQMOE_QUANT_FP8_BLOCK && n >= size_t(kTiledScaleRows) ? ((n + 127) / 128 + (size_t(E) < n ? size_t(E) : n)) * 128 : 0;
+    const bool tiled = quant_mode == DQMOE_QUANT_FP8_BLOCK && n >= size_t(kTiledScaleRows);
+    const size_t tile_rows = tiled ? ((n + 127) / 128 + (size_t(E) < n ? size_t(E) : n)) * 128 : 0;
     L.perm_a_scale_t = add(tile_rows * ceil_div(H, 128) * sizeof(float));
     L.act_scale_t = add(tile_rows * ceil_div(I, 128) * sizeof(float));
     const bool two_pass = quant_mode == DQMOE_QUANT_FP8_TENSOR || quant_mode == DQMOE_QUANT_FP8_CHANNEL;

@@ -1,8 +1,9 @@
-// Streaming row kernels around the grouped GEMM: expert-order gather of
-// activations and their scales, the scatter back to slot order, the weighted
-// combine over the k slots of a token, and the gather fused with 1x128 FP8
-// quantisation. All are HBM-bound: one warp per row, 16-byte accesses, a grid
-// that is a multiple of the SM count.
+// Streaming row kernels around the grouped GEMM: activations and their scales
+// into expert order (by token in the layer, by sorted row as stand-alone
+// operators), also fused with 1x128 FP8 quantisation, the scatter back to slot
+// order and the weighted combine over the k slots of a token. All are HBM-bound:
+// one warp per row or strip of a row, 16-byte accesses, a grid that is a
+// multiple of the SM count.
 //
 // Replaces expandInputRowsGatherKernel, expandInputScale{,Block}GatherKernel and
 // finalizeScatterKernel of the reference (csrc/moe_kernels.h:487-620).
@@ -302,12 +303,15 @@ int scatter_rows(const void* src, size_t row_bytes, int T, int k, const int* src
                  int scale_cols, float* dst_scale, float* amax, int amax_per_row, cudaStream_t stream) {
     const int row_vecs = int(row_bytes / 16);
     DQ_CHECK(is_aligned(src, 16) && is_aligned(dst, 16));
-    DQ_RC(launch_pdl(scatter_rows_kernel, dim3(grid_for_rows(int64_t(T) * ceil_div(row_vecs, 128))), kThreads, 0, stream, static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), src_to_dest, T, k, row_vecs, src_scale, dst_scale, scale_cols, amax, amax_per_row));
+    DQ_RC(launch_pdl(scatter_rows_kernel, dim3(grid_for_rows(int64_t(T) * ceil_div(row_vecs, 128))), kThreads, 0, stream,
+                     static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), src_to_dest, T, k, row_vecs, src_scale,
+                     dst_scale, scale_cols, amax, amax_per_row));
     return DQMOE_OK;
 }
 int scatter_quant_1x128(const void* x_bf16, int T, int k, int H, const int* src_to_dest, void* q, float* scale, cudaStream_t stream) {
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 16) && H % 16 == 0);
-    DQ_RC(launch_pdl(scatter_quant_1x128_kernel, dim3(grid_for_rows(int64_t(T) * ceil_div(H, 1024))), kThreads, 0, stream, static_cast<const uint8_t*>(x_bf16), T, k, H, src_to_dest, static_cast<uint8_t*>(q), scale));
+    DQ_RC(launch_pdl(scatter_quant_1x128_kernel, dim3(grid_for_rows(int64_t(T) * ceil_div(H, 1024))), kThreads, 0, stream,
+                     static_cast<const uint8_t*>(x_bf16), T, k, H, src_to_dest, static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 
@@ -326,7 +330,9 @@ int dqmoe_permute_rows(const void* src, size_t row_bytes, int k, const int32_t* 
     DQ_CHECK_FMT(row_bytes % 16 == 0 && row_bytes > 0, "row_bytes=%zu must be a multiple of 16", row_bytes);
     DQ_CHECK(is_aligned(src, 16) && is_aligned(dst, 16));
     if (scale_cols > 0) DQ_CHECK(src_scale != nullptr && dst_scale != nullptr);
-    DQ_RC(launch_pdl(permute::row_move_kernel<true>, dim3(permute::grid_for_rows(n)), permute::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), dest_to_src, n, k, int(row_bytes / 16), src_scale, dst_scale, scale_cols));
+    DQ_RC(launch_pdl(permute::row_move_kernel<true>, dim3(permute::grid_for_rows(n)), permute::kThreads, 0,
+                     static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst),
+                     dest_to_src, n, k, int(row_bytes / 16), src_scale, dst_scale, scale_cols));
     return DQMOE_OK;
 }
 
@@ -337,7 +343,9 @@ int dqmoe_finalize_scatter(const void* rows, size_t row_bytes, const int32_t* de
     DQ_CHECK(rows != nullptr && d != nullptr && dest_to_src != nullptr);
     DQ_CHECK_FMT(row_bytes % 16 == 0 && row_bytes > 0, "row_bytes=%zu must be a multiple of 16", row_bytes);
     DQ_CHECK(is_aligned(rows, 16) && is_aligned(d, 16));
-    DQ_RC(launch_pdl(permute::row_move_kernel<false>, dim3(permute::grid_for_rows(n)), permute::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(rows), static_cast<uint8_t*>(d), dest_to_src, n, 1, int(row_bytes / 16), nullptr, nullptr, 0));
+    DQ_RC(launch_pdl(permute::row_move_kernel<false>, dim3(permute::grid_for_rows(n)), permute::kThreads, 0,
+                     static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(rows), static_cast<uint8_t*>(d),
+                     dest_to_src, n, 1, int(row_bytes / 16), nullptr, nullptr, 0));
     return DQMOE_OK;
 }
 
@@ -370,7 +378,9 @@ int dqmoe_quant_fp8_block_1x128(const void* x_bf16, int64_t rows, int cols, void
     // (4096 x 4096: 15.0 us, in strips 9.8 us)
     if (cols % 16 == 0 && is_aligned(q, 16) && rows < (int64_t(1) << 31))
         return permute::scatter_quant_1x128(x_bf16, int(rows), 1, cols, nullptr, q, scale, static_cast<cudaStream_t>(stream));
-    DQ_RC(launch_pdl(permute::quant_1x128_kernel, dim3(permute::grid_for_rows(rows)), permute::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows, cols, 1, nullptr, static_cast<uint8_t*>(q), scale));
+    DQ_RC(launch_pdl(permute::quant_1x128_kernel, dim3(permute::grid_for_rows(rows)), permute::kThreads, 0,
+                     static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows, cols, 1, nullptr,
+                     static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 
@@ -381,7 +391,9 @@ int dqmoe_permute_quant_block_1x128(const void* x_bf16, int H, int k, const int3
     DQ_CHECK(x_bf16 != nullptr && q != nullptr && scale != nullptr && dest_to_src != nullptr);
     DQ_CHECK_FMT(H % 8 == 0, "H=%d must be a multiple of 8", H);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
-    DQ_RC(launch_pdl(permute::quant_1x128_kernel, dim3(permute::grid_for_rows(n)), permute::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), n, H, k, dest_to_src, static_cast<uint8_t*>(q), scale));
+    DQ_RC(launch_pdl(permute::quant_1x128_kernel, dim3(permute::grid_for_rows(n)), permute::kThreads, 0,
+                     static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), n, H, k, dest_to_src,
+                     static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 

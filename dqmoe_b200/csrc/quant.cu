@@ -368,10 +368,14 @@ int dqmoe_quant_fp8_rowwise(const void* x_bf16, int64_t rows, int cols, void* q,
     DQ_CHECK_FMT(cols % 8 == 0, "cols=%d must be a multiple of 8", cols);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
     if (cols / 8 <= quant::kShortRowVecs) {
-        DQ_RC(launch_pdl(quant::rowwise_short_kernel, dim3(quant::grid_cap((rows + 7) / 8, 8)), quant::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows, cols, static_cast<uint8_t*>(q), scale));
+        DQ_RC(launch_pdl(quant::rowwise_short_kernel, dim3(quant::grid_cap((rows + 7) / 8, 8)), quant::kThreads, 0,
+                         static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows, cols,
+                         static_cast<uint8_t*>(q), scale));
         return DQMOE_OK;
     }
-    DQ_RC(launch_pdl(quant::rowwise_kernel, dim3(quant::grid_cap(rows, 16)), quant::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows, cols, static_cast<uint8_t*>(q), scale));
+    DQ_RC(launch_pdl(quant::rowwise_kernel, dim3(quant::grid_cap(rows, 16)), quant::kThreads, 0,
+                     static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows, cols,
+                     static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 
@@ -382,7 +386,9 @@ int dqmoe_requant_from_amax_dev(const void* act_bf16, int64_t n_max, int I, cons
     DQ_CHECK(act_bf16 != nullptr && q != nullptr && scale != nullptr && amax != nullptr);
     DQ_CHECK_FMT(I % 8 == 0, "I=%d must be a multiple of 8", I);
     DQ_CHECK(is_aligned(act_bf16, 16) && is_aligned(q, 8));
-    DQ_RC(launch_pdl(quant::requant_rows_kernel, dim3(quant::grid_cap((n_max * ((I / 8 + 127) / 128) + 7) / 8, 8)), quant::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(act_bf16), n_max, I, static_cast<uint8_t*>(q), scale, amax, per_row ? 1 : 0, n_rows_device));
+    DQ_RC(launch_pdl(quant::requant_rows_kernel, dim3(quant::grid_cap((n_max * ((I / 8 + 127) / 128) + 7) / 8, 8)),
+                     quant::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(act_bf16), n_max, I,
+                     static_cast<uint8_t*>(q), scale, amax, per_row ? 1 : 0, n_rows_device));
     return DQMOE_OK;
 }
 
@@ -399,7 +405,9 @@ int dqmoe_quant_fp8_block_128x128(const void* w_bf16, int e, int rows, int cols,
     DQ_CHECK_FMT(cols % 8 == 0, "cols=%d must be a multiple of 8", cols);
     DQ_CHECK(is_aligned(w_bf16, 16) && is_aligned(q, 8));
     const int64_t blocks = int64_t(e) * ((rows + 127) / 128) * ((cols + 127) / 128);
-    DQ_RC(launch_pdl(quant::block128_kernel, dim3(quant::grid_cap(blocks, 3)), quant::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(w_bf16), e, rows, cols, static_cast<uint8_t*>(q), scale));
+    DQ_RC(launch_pdl(quant::block128_kernel, dim3(quant::grid_cap(blocks, 3)), quant::kThreads, 0,
+                     static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(w_bf16), e, rows, cols,
+                     static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 
@@ -416,8 +424,10 @@ int dqmoe_quant_fp8_tensor(const void* x_bf16, int e, int64_t numel_per, void* q
     const int64_t vecs = numel_per / 8;
     const int gx = quant::grid_cap((vecs + quant::kThreads - 1) / quant::kThreads, e >= 8 ? 2 : 8);
     dim3 grid(gx, e);
-    DQ_RC(launch_pdl(quant::tensor_amax_kernel, dim3(grid), quant::kThreads, 0, s, static_cast<const uint8_t*>(x_bf16), vecs, amax_scratch));
-    DQ_RC(launch_pdl(quant::tensor_quant_kernel, dim3(grid), quant::kThreads, 0, s, static_cast<const uint8_t*>(x_bf16), vecs, amax_scratch, static_cast<uint8_t*>(q), scale));
+    DQ_RC(launch_pdl(quant::tensor_amax_kernel, dim3(grid), quant::kThreads, 0, s, static_cast<const uint8_t*>(x_bf16), vecs,
+                     amax_scratch));
+    DQ_RC(launch_pdl(quant::tensor_quant_kernel, dim3(grid), quant::kThreads, 0, s, static_cast<const uint8_t*>(x_bf16), vecs,
+                     amax_scratch, static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 
@@ -449,8 +459,10 @@ int dqmoe_quant_fp8_tensor_static(const void* x_bf16, int e, int64_t numel_per, 
     const int64_t vecs = numel_per / 8;
     const int gx = quant::grid_cap((vecs + quant::kThreads - 1) / quant::kThreads, e >= 8 ? 2 : 8);
     dim3 grid(gx, e);
-    DQ_RC(launch_pdl(quant::tensor_amax_kernel, dim3(grid), quant::kThreads, 0, s, static_cast<const uint8_t*>(x_bf16), vecs, amax));
-    DQ_RC(launch_pdl(quant::tensor_quant_kernel, dim3(grid), quant::kThreads, 0, s, static_cast<const uint8_t*>(x_bf16), vecs, amax, static_cast<uint8_t*>(q), scale));
+    DQ_RC(launch_pdl(quant::tensor_amax_kernel, dim3(grid), quant::kThreads, 0, s, static_cast<const uint8_t*>(x_bf16), vecs,
+                     amax));
+    DQ_RC(launch_pdl(quant::tensor_quant_kernel, dim3(grid), quant::kThreads, 0, s, static_cast<const uint8_t*>(x_bf16), vecs,
+                     amax, static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 

@@ -213,7 +213,9 @@ int dqmoe_quant_mxfp8(const void* x_bf16, int64_t rows, int cols, void* q, uint8
     DQ_CHECK(x_bf16 != nullptr && q != nullptr && scale != nullptr);
     DQ_CHECK_FMT(cols % 32 == 0, "cols=%d: MXFP8 rows are made of 32-element groups", cols);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
-    DQ_RC(launch_pdl(quant_mx::quant_rows_kernel<false>, dim3(quant_mx::grid_for(rows, quant_mx::kThreads / 32)), quant_mx::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows, cols, nullptr, 1, nullptr, nullptr, 0, static_cast<uint8_t*>(q), scale));
+    DQ_RC(launch_pdl(quant_mx::quant_rows_kernel<false>, dim3(quant_mx::grid_for(rows, quant_mx::kThreads / 32)),
+                     quant_mx::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows,
+                     cols, nullptr, 1, nullptr, nullptr, 0, static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 
@@ -225,7 +227,10 @@ int dqmoe_permute_quant_mxfp8(const void* x_bf16, int H, int k, const int32_t* d
              scale_tiled != nullptr);
     DQ_CHECK_FMT(H % 128 == 0, "H=%d: the tiled scale layout needs rows of whole 128-column blocks", H);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8) && is_aligned(scale_tiled, 16));
-    DQ_RC(launch_pdl(quant_mx::quant_rows_kernel<true>, dim3(quant_mx::grid_for(n, quant_mx::kThreads / 32)), quant_mx::kThreads, size_t(2 * (E + 1)) * sizeof(int), static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), n, H, dest_to_src, k, offsets, mtile_prefix, E, static_cast<uint8_t*>(q), scale_tiled));
+    DQ_RC(launch_pdl(quant_mx::quant_rows_kernel<true>, dim3(quant_mx::grid_for(n, quant_mx::kThreads / 32)),
+                     quant_mx::kThreads, size_t(2 * (E + 1)) * sizeof(int), static_cast<cudaStream_t>(stream),
+                     static_cast<const uint8_t*>(x_bf16), n, H, dest_to_src, k, offsets, mtile_prefix, E,
+                     static_cast<uint8_t*>(q), scale_tiled));
     return DQMOE_OK;
 }
 
@@ -245,7 +250,10 @@ int dqmoe_mx_tile_scales(const uint8_t* scale_rows, int64_t rows, int cols, cons
         DQ_CHECK_FMT(rows % 128 == 0, "rows=%lld: rows that form blocks by their index must fill whole 128-row blocks",
                      (long long) rows);
     const int kblocks = cols / 128;
-    DQ_RC(launch_pdl(quant_mx::tile_scales_kernel, dim3(quant_mx::grid_for(rows * kblocks, quant_mx::kThreads)), quant_mx::kThreads, offsets != nullptr ? size_t(2 * (E + 1)) * sizeof(int) : 0, static_cast<cudaStream_t>(stream), reinterpret_cast<const uint32_t*>(scale_rows), rows, kblocks, dest_to_src, k, offsets, mtile_prefix, E, scale_tiled));
+    DQ_RC(launch_pdl(quant_mx::tile_scales_kernel, dim3(quant_mx::grid_for(rows * kblocks, quant_mx::kThreads)),
+                     quant_mx::kThreads, offsets != nullptr ? size_t(2 * (E + 1)) * sizeof(int) : 0,
+                     static_cast<cudaStream_t>(stream), reinterpret_cast<const uint32_t*>(scale_rows), rows, kblocks,
+                     dest_to_src, k, offsets, mtile_prefix, E, scale_tiled));
     return DQMOE_OK;
 }
 
@@ -256,7 +264,9 @@ int dqmoe_quant_nvfp4(const void* x_bf16, int64_t rows, int cols, const float* g
     DQ_CHECK(x_bf16 != nullptr && gscale != nullptr && q != nullptr && scale != nullptr);
     DQ_CHECK_FMT(cols % 16 == 0, "cols=%d: NVFP4 rows are made of 16-element groups", cols);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
-    DQ_RC(launch_pdl(quant_mx::quant_nvfp4_kernel, dim3(quant_mx::grid_for(rows * (cols / 16), quant_mx::kThreads)), quant_mx::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows, cols, gscale, rows_per_gscale, static_cast<uint8_t*>(q), scale));
+    DQ_RC(launch_pdl(quant_mx::quant_nvfp4_kernel, dim3(quant_mx::grid_for(rows * (cols / 16), quant_mx::kThreads)),
+                     quant_mx::kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows,
+                     cols, gscale, rows_per_gscale, static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
 

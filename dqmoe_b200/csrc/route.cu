@@ -280,7 +280,8 @@ int route_sort(const int* ids, int n, int E, int* counts, int* offsets, int* mti
         }
     }
     if (chunks == 1) {
-        DQ_RC(launch_pdl(sort_scatter_kernel<true>, dim3(1), kSortThreads, smem_scatter, stream, ids, n, E, nullptr, counts, offsets, mtile_prefix, dest_to_src, src_to_dest));
+        DQ_RC(launch_pdl(sort_scatter_kernel<true>, dim3(1), kSortThreads, smem_scatter, stream, ids, n, E, nullptr, counts,
+                         offsets, mtile_prefix, dest_to_src, src_to_dest));
         return DQMOE_OK;
     }
     if (ws == nullptr || ws_bytes < sort_workspace_bytes(n, E) || !is_aligned(ws, 16))
@@ -290,10 +291,13 @@ int route_sort(const int* ids, int n, int E, int* counts, int* offsets, int* mti
     DQ_RC(launch_pdl(sort_hist_kernel, dim3(chunks), kSortThreads, (E + 1) * sizeof(int), stream, ids, n, E, chunk_hist));
     const size_t smem_scan = size_t(chunks) * (E + 1) * sizeof(int);
     if (smem_scan <= size_t(kScanSmemMax))
-        DQ_RC(launch_pdl(sort_scan_kernel<true>, dim3(1), 1024, smem_scan, stream, chunk_hist, chunks, E, counts, offsets, mtile_prefix));
+        DQ_RC(launch_pdl(sort_scan_kernel<true>, dim3(1), 1024, smem_scan, stream, chunk_hist, chunks, E, counts, offsets,
+                         mtile_prefix));
     else
-        DQ_RC(launch_pdl(sort_scan_kernel<false>, dim3(1), 1024, 0, stream, chunk_hist, chunks, E, counts, offsets, mtile_prefix));
-    DQ_RC(launch_pdl(sort_scatter_kernel<false>, dim3(chunks), kSortThreads, smem_scatter, stream, ids, n, E, chunk_hist, counts, offsets, mtile_prefix, dest_to_src, src_to_dest));
+        DQ_RC(launch_pdl(sort_scan_kernel<false>, dim3(1), 1024, 0, stream, chunk_hist, chunks, E, counts, offsets,
+                         mtile_prefix));
+    DQ_RC(launch_pdl(sort_scatter_kernel<false>, dim3(chunks), kSortThreads, smem_scatter, stream, ids, n, E, chunk_hist,
+                     counts, offsets, mtile_prefix, dest_to_src, src_to_dest));
     return DQMOE_OK;
 }
 
@@ -374,12 +378,18 @@ int route_topk(const float* logits, int T, int E, int k, int n_shared, int scori
     if (T == 0) return DQMOE_OK;
     DQ_CHECK(logits != nullptr && indices != nullptr && weights != nullptr);
     const int blocks = ceil_div(T, 8);
-    if (E <= 32) DQ_RC(launch_pdl(route_topk_kernel<1>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
-    else if (E <= 64) DQ_RC(launch_pdl(route_topk_kernel<2>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
-    else if (E <= 128) DQ_RC(launch_pdl(route_topk_kernel<4>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
-    else if (E <= 256) DQ_RC(launch_pdl(route_topk_kernel<8>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
-    else if (E <= 512) DQ_RC(launch_pdl(route_topk_kernel<16>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
-    else DQ_RC(launch_pdl(route_topk_kernel<32>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices, weights));
+    if (E <= 32) DQ_RC(launch_pdl(route_topk_kernel<1>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring,
+                                  indices, weights));
+    else if (E <= 64) DQ_RC(launch_pdl(route_topk_kernel<2>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring,
+                                       indices, weights));
+    else if (E <= 128) DQ_RC(launch_pdl(route_topk_kernel<4>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring,
+                                        indices, weights));
+    else if (E <= 256) DQ_RC(launch_pdl(route_topk_kernel<8>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring,
+                                        indices, weights));
+    else if (E <= 512) DQ_RC(launch_pdl(route_topk_kernel<16>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring,
+                                        indices, weights));
+    else DQ_RC(launch_pdl(route_topk_kernel<32>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices,
+                          weights));
     return DQMOE_OK;
 }
 

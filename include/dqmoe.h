@@ -92,7 +92,7 @@ int dqmoe_device_status(int* code);
 size_t dqmoe_moe_workspace_bytes(int T, int H, int I, int E, int k, int quant_mode);
 
 /*
- * One MoE layer: expert sort -> row gather -> grouped fc1 + SwiGLU (+ dynamic
+ * One MoE layer: expert sort -> rows into expert order -> grouped fc1 + SwiGLU (+ dynamic
  * FP8 re-quantisation of the intermediate) -> grouped fc2 -> scatter into d.
  * Replaces m_grouped_moe_nt_contiguous<T,W,O> / MoeFCRunner::runMoe
  * (csrc/pybind11_register.h:99-151, csrc/moe_kernels.h:770-892).
@@ -176,7 +176,7 @@ void* dqmoe_moe_workspace_ptr(void* workspace, int which, int T, int H, int I, i
 
 /*
  * The whole MoE block from bf16 activations x [T, H] and fp32 router logits [T, E] to
- * out [T, H] bf16: top-k router, expert sort, gather fused with the dynamic 1x128 FP8
+ * out [T, H] bf16: top-k router, expert sort, rows into expert order fused with the dynamic 1x128 FP8
  * quantisation of the activations (block mode) or plain gather (bf16 mode), grouped fc1 +
  * SwiGLU (+ re-quantisation), grouped fc2, weighted combine of the k slots. quant_mode is
  * DQMOE_QUANT_NONE (bf16 weights), DQMOE_QUANT_FP8_BLOCK (e4m3 weights with 128x128
@@ -366,7 +366,8 @@ int dqmoe_quant_fp8_tensor(const void* x_bf16, int e, int64_t numel_per, void* q
  * e is limited to 1024 slices; a larger e returns DQMOE_ERR_INVALID. The first call on a
  * device queries the array's address from the runtime and should happen before any stream
  * capture begins. All calls on a device share the array (it is zeroed per call): calls that
- * overlap on the GPU race. Results are identical to dqmoe_quant_fp8_tensor.
+ * overlap on the GPU race. Slices of up to 524288 elements are quantised without the array and fall under neither rule.
+ * Results are identical to dqmoe_quant_fp8_tensor.
  */
 int dqmoe_quant_fp8_tensor_static(const void* x_bf16, int e, int64_t numel_per, void* q, float* scale,
                                   dqmoe_stream_t stream);
