@@ -303,7 +303,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
             const int grow = tl.row0 + r_in_tile;
             const bool row_ok = grow < tl.row_end;
             const uint32_t buf = acc_it & 1u;
-            if (!ptx::mbar_wait(&st.tmem_full[buf], (acc_it >> 1) & 1u, abort_flag, kWaitLimit)) {
+            if (!ptx::mbar_wait_warp(&st.tmem_full[buf], (acc_it >> 1) & 1u, abort_flag, kWaitLimit)) {
                 ok = false;
                 break;
             }

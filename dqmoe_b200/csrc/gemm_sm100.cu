@@ -448,7 +448,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                 const float* src_b = p.sb + (size_t(tl.e) * NB + nb) * KB;
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int slot = it % kScaleSlots, s = it % kNumStages;
-                    if (!ptx::mbar_wait(&st.empty[s], ((it / kNumStages) & 1u) ^ 1u, abort_flag, kWaitLimit)) {
+                    if (!ptx::mbar_wait_warp(&st.empty[s], ((it / kNumStages) & 1u) ^ 1u, abort_flag, kWaitLimit)) {
                         ok = false;
                         break;
                     }
@@ -476,8 +476,11 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
         int e_cursor = 0;
         bool ok = true;
         const int I_or_H = p.N;
-        // hand a drained accumulator buffer back to the MMA thread (which lives in the leader CTA)
+        // hand a drained accumulator buffer back to the MMA thread (which lives in the leader CTA): one arrival per warp,
+        // after all of its lanes are done with the buffer
         auto release_tmem = [&](uint32_t b) {
+            __syncwarp();
+            if (lane != 0) return;
             if constexpr (kPair)
                 ptx::mbar_arrive_cluster(ptx::map_to_cta(&st.tmem_empty[b], 0));
             else
@@ -493,7 +496,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
 
             if constexpr (kMode != kBlock) {
                 const uint32_t buf = acc_it & 1u;
-                if (!ptx::mbar_wait(&st.tmem_full[buf], (acc_it >> 1) & 1u, abort_flag, kWaitLimit)) {
+                if (!ptx::mbar_wait_warp(&st.tmem_full[buf], (acc_it >> 1) & 1u, abort_flag, kWaitLimit)) {
                     ok = false;
                     break;
                 }
@@ -648,8 +651,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                     }
                 }
                 ptx::tc_fence_before();
-                __syncwarp();
-                if (lane == 0) release_tmem(buf);
+                release_tmem(buf);
             } else {
                 // ---------------------------------------------------- block-scaled accumulation
                 // acc[c*32 + i]: chunk c of this thread's four 32-column chunks.
@@ -695,7 +697,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                     for (int kb = 0; kb < KB; ++kb, ++acc_it) {
                         const int slot = acc_it % kScaleSlots;
                         const uint32_t buf = acc_it & 1u;
-                        if (!ready && !ptx::mbar_wait(&st.tmem_full[buf], (acc_it >> 1) & 1u, abort_flag, kWaitLimit)) return false;
+                        if (!ptx::mbar_wait_warp(&st.tmem_full[buf], (acc_it >> 1) & 1u, abort_flag, kWaitLimit, ready)) return false;
                         ptx::tc_fence_after();
                         const uint32_t t_buf = t_lane + buf * kUmmaN;
                         ptx::tmem_ld32(t_buf + tcol(0), r0);
@@ -710,8 +712,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         ptx::tmem_ld32(t_buf + tcol(3), r1);
                         ptx::tmem_wait_ld2(r0, r1);
                         ptx::tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) release_tmem(buf);
+                        release_tmem(buf);
                         // ask for the next buffer now: the answer arrives under the FMAs
                         ready = ptx::mbar_test_wait(&st.tmem_full[buf ^ 1u], ((acc_it + 1) >> 1) & 1u);
                         fma_chunk(2, r0, s0, s1l, s1h);
@@ -720,9 +721,10 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                     return true;
                 };
                 if (!live) {
-                    for (int kb = 0; ok && kb < KB; ++kb, ++acc_it) {
-                        ok = ptx::mbar_wait(&st.tmem_full[acc_it & 1u], (acc_it >> 1) & 1u, abort_flag, kWaitLimit);
-                        if (lane == 0) release_tmem(acc_it & 1u);
+                    for (int kb = 0; kb < KB; ++kb, ++acc_it) {
+                        ok = ptx::mbar_wait_warp(&st.tmem_full[acc_it & 1u], (acc_it >> 1) & 1u, abort_flag, kWaitLimit);
+                        if (!ok) break;
+                        release_tmem(acc_it & 1u);
                     }
                 } else if (!kGated || c_switch == 128)
                     ok = k_loop(std::true_type{});
@@ -756,7 +758,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                     st.amax[tile_it & 1u][h][r_in_tile] = amax_local;
                     __syncwarp();
                     if (lane == 0) ptx::mbar_arrive(&st.epi_sync[q]);
-                    if (!ptx::mbar_wait(&st.epi_sync[q], epi_phase, abort_flag, kWaitLimit)) {
+                    if (!ptx::mbar_wait_warp(&st.epi_sync[q], epi_phase, abort_flag, kWaitLimit)) {
                         ok = false;
                         break;
                     }

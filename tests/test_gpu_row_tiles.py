@@ -34,3 +34,43 @@ def test_ragged_row_counts_match_oracle(mode, H, I):
     assert ops.device_status() == 0
     # the layer tolerance: a rounding of the intermediate that flips moves one e4m3 step (2^-3 relative) of one of I terms
     assert orc.cosine(d.cpu(), ref) >= 0.999 and orc.max_rel_err(d.cpu(), ref) <= 2e-2
+
+
+@pytest.mark.parametrize("H,I,drop", [(1408, 192, False), (2048, 320, True)])
+def test_quarters_without_rows_over_long_reductions(H, I, drop):
+    """Block mode from 4096 rows on (scales by tile), row tiles of 1 to 128 rows and K loops of 11 and 16 blocks: warps without
+    rows, and the lanes of the scale loader without a copy, go round the same barriers as the others. With dropped slots the
+    kept tiles are fewer than the layout's bound. Rows are bit-identical to the same rows in a small call."""
+    from dqmoe_b200 import ops
+    rows = ROWS * 4
+    E, T = len(rows), sum(rows)
+    assert T >= 4096
+    g = torch.Generator().manual_seed(H)
+    a = torch.randn(T, H, generator=g).to(torch.bfloat16).to(DEV)
+    b = ops.per_block_cast_to_fp8((torch.randn(E, 2 * I, H, generator=g) * 0.05).to(torch.bfloat16).to(DEV))
+    b1 = ops.per_block_cast_to_fp8((torch.randn(E, H, I, generator=g) * 0.05).to(torch.bfloat16).to(DEV))
+    q, s = ops.per_token_block_cast_to_fp8(a)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(rows))[torch.randperm(T, generator=g)].to(torch.int32)
+    if drop:
+        ids[::3] = -1
+        ids[1::7] = E
+    ids = ids.view(T, 1)
+
+    def run(sel):
+        n = len(sel)
+        ws = torch.empty(ops.moe_workspace_bytes(n, H, I, E, 1, 1024), dtype=torch.uint8, device=DEV)
+        d = torch.zeros(n, 1, H, dtype=torch.bfloat16, device=DEV)
+        qd = q.view(torch.uint8)[sel.to(DEV)].contiguous().view(q.dtype)
+        ops.moe_forward(qd, s[sel.to(DEV)].contiguous(), *b, *b1, d, ids[sel].contiguous().to(DEV), ws, 1024)
+        assert ops.device_status() == 0
+        return d.cpu()
+
+    sample = torch.arange(0, T, 23)
+    full, small = run(torch.arange(T)), run(sample)
+    assert torch.equal(full[sample], small)
+    kept = (ids[:, 0] >= 0) & (ids[:, 0] < E)
+    assert not full[~kept].any()
+    sample = sample[kept[sample]]
+    ref = orc.moe_layer_fp8(q.cpu()[sample], s.cpu()[sample], *[t.cpu() for t in b], *[t.cpu() for t in b1], ids[sample], E, 1024)
+    # the layer tolerance (see above)
+    assert orc.cosine(full[sample], ref) >= 0.999 and orc.max_rel_err(full[sample], ref) <= 2e-2

@@ -1,0 +1,47 @@
+"""Rules of the kernel sources that no run can show to be kept: what breaks when one is broken depends on how the lanes of a
+warp happen to be scheduled, or on which cache a load is served from."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "dqmoe_b200", "csrc")
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())  # without comments
+
+
+def braces(text, start):
+    """The block that opens at the first '{' from `start` on."""
+    at = text.index("{", start)
+    depth = 0
+    for i in range(at, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[at:i + 1]
+    raise AssertionError("unbalanced braces")
+
+
+def test_roles_of_a_whole_warp_wait_together():
+    """A role that one elected thread plays may poll a barrier alone. In one that a whole warp plays, a lane that goes on
+    alone can let the barrier pass twice before another lane polls again, which then waits for a parity that is gone."""
+    for name, roles in (("gemm_sm100.cu", ["else if (warp == 2)", "setmaxnreg_inc"]), ("gemm_mx_sm100.cu", ["setmaxnreg_inc"])):
+        text = source(name)
+        for role in roles:
+            at = text.index(role)
+            if role == "setmaxnreg_inc":
+                at = text.rindex("else {", 0, at)
+            body = braces(text, at)
+            assert "mbar_wait_warp(" in body, (name, role)
+            assert not re.search(r"\bmbar_wait\(", body), (name, role)
+
+
+def test_buffers_are_released_by_a_converged_warp():
+    """One lane arrives for its warp, so the others must be known to have read the buffer and to have seen the phase."""
+    text = source("gemm_sm100.cu")
+    release = braces(text, text.index("auto release_tmem"))
+    assert release.index("__syncwarp()") < release.index("mbar_arrive")
+    assert not re.search(r"if \(lane == 0\)\s*release_tmem", text)
+    mx = source("gemm_mx_sm100.cu")
+    for m in re.finditer(r"mbar_arrive\(&st\.(tmem_empty|overlap_free)", mx):
+        assert "__syncwarp()" in mx[max(0, m.start() - 200):m.start()], mx[m.start() - 200:m.end()]
