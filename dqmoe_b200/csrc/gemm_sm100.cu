@@ -697,7 +697,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                     for (int kb = 0; kb < KB; ++kb, ++acc_it) {
                         const int slot = acc_it % kScaleSlots;
                         const uint32_t buf = acc_it & 1u;
-                        if (!ptx::mbar_wait_warp(&st.tmem_full[buf], (acc_it >> 1) & 1u, abort_flag, kWaitLimit, ready)) return false;
+                        if (!ready && !ptx::mbar_wait_warp(&st.tmem_full[buf], (acc_it >> 1) & 1u, abort_flag, kWaitLimit)) return false;
                         ptx::tc_fence_after();
                         const uint32_t t_buf = t_lane + buf * kUmmaN;
                         ptx::tmem_ld32(t_buf + tcol(0), r0);
@@ -713,9 +713,10 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         ptx::tmem_wait_ld2(r0, r1);
                         ptx::tc_fence_before();
                         release_tmem(buf);
-                        // ask for the next buffer now: the answer arrives under the FMAs
-                        ready = ptx::mbar_test_wait(&st.tmem_full[buf ^ 1u], ((acc_it + 1) >> 1) & 1u);
+                        // ask for the next buffer now: the answers arrive under the FMAs, and the lanes agree on one
+                        const bool over = ptx::mbar_test_wait(&st.tmem_full[buf ^ 1u], ((acc_it + 1) >> 1) & 1u);
                         fma_chunk(2, r0, s0, s1l, s1h);
+                        ready = __all_sync(0xffffffffu, over);
                         fma_chunk(3, r1, s0, s1l, s1h);
                     }
                     return true;

@@ -98,10 +98,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 // The same for a whole warp that goes on together: every lane polls for itself (each needs the acquire), then all of them
 // leave with one answer. Polling lanes may part, and a lane that goes on alone - to release a buffer, or merely to the next
 // wait - can let the barrier complete twice before another lane polls again; that lane then finds the parity it waits for
-// gone and waits for good. `over`: this lane has already seen the phase complete.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, long long limit,
-                                               bool over = false) {
-    if (__all_sync(0xffffffffu, over)) return true;
+// gone and waits for good.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, long long limit) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, limit));
 }
 
