@@ -65,7 +65,9 @@ constexpr int kAmaxParts = 4096;  // floats the layer workspace holds for the pe
 
 // Programmatic dependent launch. Every kernel launched through launch_pdl calls pdl_launch() and pdl_wait() first thing
 // (the grouped GEMMs set up their barriers and TMEM in between): the next kernel's blocks may become resident while this
-// one runs, and no thread touches global memory before all earlier kernels of the stream have completed. Between the short
+// one runs, and no thread touches global memory before all earlier kernels of the stream have completed. What such a kernel
+// reads may therefore still be written while it is resident: its pointers are not __restrict__ and its loads are plain ones
+// (ld_stream16). Between the short
 // kernels of the layer the gap shrinks from ~2 us to below 1 us (MoE block of 5 tokens, H 1024, I 2048: 45.8 -> 34.6 us).
 // The grouped GEMMs are launched this way up to kPdlGemmRows rows only. Their blocks, one per SM, would otherwise take the
 // SMs in the order in which the kernel before leaves them instead of in the launch order, which spreads the blocks that
@@ -105,9 +107,20 @@ struct __align__(16) Vec16 {
     uint32_t x, y, z, w;
 };
 
+// For data that nobody writes as long as the kernel is resident: in kernels that start only after their predecessors' end.
 __device__ __forceinline__ Vec16 ld_nc16(const void* p) {
     Vec16 v;
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+    return v;
+}
+// The same as a plain load, for kernels launched through launch_pdl. They are resident while their predecessors still write
+// what they read after pdl_wait, which the non-coherent path (ld.global.nc, __ldg, a const __restrict__ argument) does not
+// allow for. Volatile, so that it stays behind the wait.
+__device__ __forceinline__ Vec16 ld_stream16(const void* p) {
+    Vec16 v;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
     return v;

@@ -67,7 +67,7 @@ __device__ __forceinline__ uint32_t e4m3x2_to_half2(uint32_t two) {
 // xs[piece * vecs + v] holds 8 16-bit values, piece 0 / 1 = elements 0-7 / 8-15 of weight vector v (e4m3 weights);
 // bf16 weights have 8 elements per vector and one piece.
 template <bool kFp8>
-__device__ __forceinline__ void dot16x2(const uint4& w0, const uint4& w1, const uint4* __restrict__ xs, int vecs, int v,
+__device__ __forceinline__ void dot16x2(const uint4& w0, const uint4& w1, const uint4* xs, int vecs, int v,
                                         float& acc0, float& acc1) {
     if constexpr (kFp8) {
         const uint32_t a[4] = {w0.x, w0.y, w0.z, w0.w}, b[4] = {w1.x, w1.y, w1.z, w1.w};
@@ -102,12 +102,12 @@ __device__ __forceinline__ void dot16x2(const uint4& w0, const uint4& w1, const 
 //                    intermediate), then kept as IEEE half
 //   neither          the row is bf16 and is copied
 template <bool kFp8Src, bool kQuant>
-__device__ __forceinline__ void stage_row(const uint8_t* __restrict__ src, int K, uint4* xs, float inv) {
+__device__ __forceinline__ void stage_row(const uint8_t* src, int K, uint4* xs, float inv) {
     const int tid = threadIdx.x;
     if constexpr (kFp8Src) {
         const int vecs = K / 16;
         for (int v = tid; v < vecs; v += kConsumers) {
-            const Vec16 raw = ld_nc16(src + size_t(v) * 16);
+            const Vec16 raw = ld_nc16(src + size_t(v) * 16);  // fc1 only, which starts after its predecessors' end
             const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
             uint32_t h[8];
 #pragma unroll

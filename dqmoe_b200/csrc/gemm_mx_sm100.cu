@@ -356,7 +356,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
                             float bg[2] = {0.0f, 0.0f}, bv[2] = {0.0f, 0.0f};
                             if (has_bias) {
 #pragma unroll
-                                for (int u = 0; u < 2; ++u) bg[u] = __ldg(bias_e + col0 + i + u), bv[u] = __ldg(bias_e + N + col0 + i + u);
+                                for (int u = 0; u < 2; ++u) bg[u] = bias_e[col0 + i + u], bv[u] = bias_e[N + col0 + i + u];
                             }
                             act2[i >> 1] = swiglu_bf16x2(__uint_as_float(r[j][i]) * alpha + bg[0], __uint_as_float(r[j][i + 1]) * alpha + bg[1],
                                                          __uint_as_float(r[2 + j][i]) * alpha + bv[0],
@@ -405,7 +405,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
 #pragma unroll
                                     for (int u = 0; u < 8; ++u)
                                         y[u] = __uint_as_float(r[c][i + u]) * alpha +
-                                               (has_bias ? __ldg(bias_e + min(col0 + i + u, N - 1)) : 0.0f);
+                                               (has_bias ? bias_e[min(col0 + i + u, N - 1)] : 0.0f);
                                     st16(orow + size_t(col0 + i) * 2, Vec16{pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]),
                                                                           pack_bf16x2(y[4], y[5]), pack_bf16x2(y[6], y[7])});
                                 }

@@ -738,7 +738,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                     for (int i = 0; i < 128; ++i) {
                         const int cg = kGated ? (i >> 6) * I_or_H + tl.nt * kBoxRows + h * 64 + (i & 63)
                                               : tl.nt * kUmmaN + tcol(i >> 5) + (i & 31);
-                        acc[i] += __ldg(bias_e + min(cg, p.w_rows - 1));
+                        acc[i] += bias_e[min(cg, p.w_rows - 1)];
                     }
                 }
 

@@ -21,28 +21,27 @@ static int grid_for_rows(int64_t rows) {
     return int(want < cap ? (want > 0 ? want : 1) : cap);
 }
 
-__device__ __forceinline__ void copy_row16(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int vecs,
+__device__ __forceinline__ void copy_row16(const uint8_t* src, uint8_t* dst, int vecs,
                                            int lane) {
     int i = lane;
     for (; i + 96 < vecs; i += 128) {
-        const Vec16 a = ld_nc16(src + size_t(i) * 16);
-        const Vec16 b = ld_nc16(src + size_t(i + 32) * 16);
-        const Vec16 c = ld_nc16(src + size_t(i + 64) * 16);
-        const Vec16 d = ld_nc16(src + size_t(i + 96) * 16);
+        const Vec16 a = ld_stream16(src + size_t(i) * 16);
+        const Vec16 b = ld_stream16(src + size_t(i + 32) * 16);
+        const Vec16 c = ld_stream16(src + size_t(i + 64) * 16);
+        const Vec16 d = ld_stream16(src + size_t(i + 96) * 16);
         st16(dst + size_t(i) * 16, a);
         st16(dst + size_t(i + 32) * 16, b);
         st16(dst + size_t(i + 64) * 16, c);
         st16(dst + size_t(i + 96) * 16, d);
     }
-    for (; i < vecs; i += 32) st16(dst + size_t(i) * 16, ld_nc16(src + size_t(i) * 16));
+    for (; i < vecs; i += 32) st16(dst + size_t(i) * 16, ld_stream16(src + size_t(i) * 16));
 }
 
 // dst[r] = src[map[r] / k]  (kGather)   or   dst[map[r]] = src[r]  (!kGather)
 template <bool kGather>
-__global__ void __launch_bounds__(kThreads) row_move_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
-                                                            const int* __restrict__ map, int n, int k, int row_vecs,
-                                                            const float* __restrict__ src_scale,
-                                                            float* __restrict__ dst_scale, int scale_cols) {
+__global__ void __launch_bounds__(kThreads) row_move_kernel(const uint8_t* src, uint8_t* dst, const int* map, int n,
+                                                            int k, int row_vecs, const float* src_scale,
+                                                            float* dst_scale, int scale_cols) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int warps = gridDim.x * kWarpsPerBlock;
@@ -64,10 +63,8 @@ __global__ void __launch_bounds__(kThreads) row_move_kernel(const uint8_t* __res
 // holds k, at most 8: with two slots in a batch of eight the registers of the empty ones cost occupancy (T = 2049, k = 2,
 // H = 4096: 25.9 us against 13.1).
 template <int kSlotBatch>
-__global__ void __launch_bounds__(kThreads) finalize_weighted_kernel(const uint8_t* __restrict__ d,
-                                                                     const float* __restrict__ w,
-                                                                     uint8_t* __restrict__ out, int T, int k,
-                                                                     int row_vecs) {
+__global__ void __launch_bounds__(kThreads) finalize_weighted_kernel(const uint8_t* d, const float* w, uint8_t* out,
+                                                                     int T, int k, int row_vecs) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int strips = (row_vecs + 31) / 32;
@@ -82,10 +79,10 @@ __global__ void __launch_bounds__(kThreads) finalize_weighted_kernel(const uint8
             float wj[kSlotBatch];
             Vec16 x[kSlotBatch];
 #pragma unroll
-            for (int u = 0; u < kSlotBatch; ++u) wj[u] = j0 + u < k ? __ldg(w + size_t(t) * k + j0 + u) : 0.0f;
+            for (int u = 0; u < kSlotBatch; ++u) wj[u] = j0 + u < k ? w[size_t(t) * k + j0 + u] : 0.0f;
 #pragma unroll
             for (int u = 0; u < kSlotBatch; ++u)
-                if (wj[u] != 0.0f) x[u] = ld_nc16(d + ((size_t(t) * k + j0 + u) * row_vecs + v) * 16);
+                if (wj[u] != 0.0f) x[u] = ld_stream16(d + ((size_t(t) * k + j0 + u) * row_vecs + v) * 16);
 #pragma unroll
             for (int u = 0; u < kSlotBatch; ++u) {
                 if (wj[u] == 0.0f) continue;  // a dropped slot's row is never written
@@ -111,16 +108,15 @@ __global__ void __launch_bounds__(kThreads) finalize_weighted_kernel(const uint8
 // per token, the k writes dominating. It also clears the amax words fc1 collects into, one per row or one in all, which
 // saves a memset between two kernels. 8192 tokens of 7168, k = 8, quantising: gather 353 us, scatter 111 us = 5.3 TB/s;
 // 16384 bf16 rows of 2880, k = 3: 102 / 62 us; 16384 e4m3 rows of 2048, k = 8: 82 / 50 us).
-__device__ __forceinline__ int slot_dest(const int* __restrict__ src_to_dest, int t, int k, int j0, int lane) {
+__device__ __forceinline__ int slot_dest(const int* src_to_dest, int t, int k, int j0, int lane) {
     if (src_to_dest == nullptr) return t;  // rows stay where they are (k = 1)
     return j0 + lane < k ? src_to_dest[size_t(t) * k + j0 + lane] : -1;
 }
 
-__global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
-                                                                const int* __restrict__ src_to_dest, int T, int k, int row_vecs,
-                                                                const float* __restrict__ src_scale,
-                                                                float* __restrict__ dst_scale, int scale_cols,
-                                                                float* __restrict__ amax, int amax_per_row) {
+__global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* src, uint8_t* dst,
+                                                                const int* src_to_dest, int T, int k, int row_vecs,
+                                                                const float* src_scale, float* dst_scale,
+                                                                int scale_cols, float* amax, int amax_per_row) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     if (amax != nullptr && !amax_per_row && blockIdx.x == 0 && threadIdx.x == 0) amax[0] = 0.0f;
@@ -134,7 +130,7 @@ __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* _
         Vec16 x[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-            if (v0 + 32 * u < row_vecs) x[u] = ld_nc16(src + (size_t(t) * row_vecs + v0 + 32 * u) * 16);
+            if (v0 + 32 * u < row_vecs) x[u] = ld_stream16(src + (size_t(t) * row_vecs + v0 + 32 * u) * 16);
         for (int j0 = 0; j0 < k; j0 += 32) {
             const int mine = slot_dest(src_to_dest, t, k, j0, lane);
             const int jn = min(32, k - j0);
@@ -154,9 +150,9 @@ __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* _
 
 // The same with 1x128 FP8 quantisation of the bf16 row on the way: a lane owns 16 consecutive columns per step, so a
 // 128-column group is 8 lanes; two steps of 512 columns per strip. cols is a multiple of 16.
-__global__ void __launch_bounds__(kThreads) scatter_quant_1x128_kernel(const uint8_t* __restrict__ x, int T, int k, int cols,
-                                                                       const int* __restrict__ src_to_dest,
-                                                                       uint8_t* __restrict__ q, float* __restrict__ scale) {
+__global__ void __launch_bounds__(kThreads) scatter_quant_1x128_kernel(const uint8_t* x, int T, int k, int cols,
+                                                                       const int* src_to_dest, uint8_t* q,
+                                                                       float* scale) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int groups = (cols + 127) / 128;
@@ -171,7 +167,7 @@ __global__ void __launch_bounds__(kThreads) scatter_quant_1x128_kernel(const uin
         for (int s = 0; s < 2; ++s) {
             const uint8_t* xr = x + (size_t(t) * cols + c0 + 512 * s) * 2;
 #pragma unroll
-            for (int u = 0; u < 2; ++u) raw[s][u] = c0 + 512 * s < cols ? ld_nc16(xr + 16 * u) : Vec16{0, 0, 0, 0};
+            for (int u = 0; u < 2; ++u) raw[s][u] = c0 + 512 * s < cols ? ld_stream16(xr + 16 * u) : Vec16{0, 0, 0, 0};
         }
         Vec16 o[2];
         float sf[2];
@@ -213,9 +209,8 @@ __global__ void __launch_bounds__(kThreads) scatter_quant_1x128_kernel(const uin
 
 // q[r, :], scale[r, :] = 1x128 FP8 quantisation of bf16 row map[r] / k (map == nullptr: row r).
 // One warp per row; a lane owns 8 consecutive columns, so a 128-column group is 16 lanes.
-__global__ void __launch_bounds__(kThreads) quant_1x128_kernel(const uint8_t* __restrict__ x, int64_t rows, int cols,
-                                                               int k, const int* __restrict__ map,
-                                                               uint8_t* __restrict__ q, float* __restrict__ scale) {
+__global__ void __launch_bounds__(kThreads) quant_1x128_kernel(const uint8_t* x, int64_t rows, int cols, int k,
+                                                               const int* map, uint8_t* q, float* scale) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int groups = (cols + 127) / 128;
@@ -233,7 +228,7 @@ __global__ void __launch_bounds__(kThreads) quant_1x128_kernel(const uint8_t* __
             const int c = c0 + lane * 8;
             float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             if (c < cols) {
-                const Vec16 raw = ld_nc16(xr + size_t(c) * 2);
+                const Vec16 raw = ld_stream16(xr + size_t(c) * 2);
                 v[0] = bf16_lo(raw.x); v[1] = bf16_hi(raw.x); v[2] = bf16_lo(raw.y); v[3] = bf16_hi(raw.y);
                 v[4] = bf16_lo(raw.z); v[5] = bf16_hi(raw.z); v[6] = bf16_lo(raw.w); v[7] = bf16_hi(raw.w);
             }
@@ -260,10 +255,8 @@ __global__ void __launch_bounds__(kThreads) quant_1x128_kernel(const uint8_t* __
 // one piece: out[tile][c][r] = scale[first row of the tile + r][c], every expert starting a new 128-row tile. One block per
 // tile and 32 columns, transposed through shared memory. (Written by the scatter itself, four bytes at a time, the same
 // matrix cost 56 us at 65536 rows x 56 columns; here ~15 us.)
-__global__ void __launch_bounds__(kThreads) scale_tiles_kernel(const float* __restrict__ scale, int cols,
-                                                               const int* __restrict__ offsets,
-                                                               const int* __restrict__ mtile_prefix, int E,
-                                                               float* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) scale_tiles_kernel(const float* scale, int cols, const int* offsets,
+                                                               const int* mtile_prefix, int E, float* out) {
     pdl_enter();
     __shared__ float s[128][33];
     const int chunks = (cols + 31) / 32;

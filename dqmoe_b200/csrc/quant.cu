@@ -45,8 +45,8 @@ __device__ __forceinline__ float block_max(float v, float* s_red) {
 }
 
 // One block per row (grid-stride): amax pass, then quantise pass (second read hits L1/L2).
-__global__ void __launch_bounds__(kThreads) rowwise_kernel(const uint8_t* __restrict__ x, int64_t rows, int cols,
-                                                           uint8_t* __restrict__ q, float* __restrict__ scale) {
+__global__ void __launch_bounds__(kThreads) rowwise_kernel(const uint8_t* x, int64_t rows, int cols, uint8_t* q,
+                                                           float* scale) {
     pdl_enter();
     __shared__ float s_red[kThreads / 32];
     const int vecs = cols / 8;
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kThreads) rowwise_kernel(const uint8_t* __rest
         float m = 0.0f;
         for (int i = threadIdx.x; i < vecs; i += kThreads) {
             float v[8];
-            unpack8(ld_nc16(xr + size_t(i) * 16), v);
+            unpack8(ld_stream16(xr + size_t(i) * 16), v);
             m = amax8(v, m);
         }
         const float amax = block_max(m, s_red);
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kThreads) rowwise_kernel(const uint8_t* __rest
         uint8_t* qr = q + size_t(r) * cols;
         for (int i = threadIdx.x; i < vecs; i += kThreads) {
             float v[8];
-            unpack8(ld_nc16(xr + size_t(i) * 16), v);
+            unpack8(ld_stream16(xr + size_t(i) * 16), v);
             *reinterpret_cast<uint2*>(qr + size_t(i) * 8) = quant8(v, inv);
         }
     }
@@ -75,8 +75,8 @@ __global__ void __launch_bounds__(kThreads) rowwise_kernel(const uint8_t* __rest
 // in registers between the amax and the conversion. Above, a warp would have to read the row twice and the block form,
 // whose 256 threads hold the row's loads in flight, is the better one. (16384 x 2048: block form 30.2 us, warp form 17.6 us.)
 constexpr int kShortRowVecs = 256;
-__global__ void __launch_bounds__(kThreads) rowwise_short_kernel(const uint8_t* __restrict__ x, int64_t rows, int cols,
-                                                                 uint8_t* __restrict__ q, float* __restrict__ scale) {
+__global__ void __launch_bounds__(kThreads) rowwise_short_kernel(const uint8_t* x, int64_t rows, int cols, uint8_t* q,
+                                                                 float* scale) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = int64_t(gridDim.x) * (kThreads / 32);
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kThreads) rowwise_short_kernel(const uint8_t* 
         Vec16 raw[kShortRowVecs / 32];
 #pragma unroll
         for (int i = 0; i < kShortRowVecs / 32; ++i)
-            raw[i] = lane + 32 * i < vecs ? ld_nc16(xr + size_t(lane + 32 * i) * 16) : Vec16{0, 0, 0, 0};
+            raw[i] = lane + 32 * i < vecs ? ld_stream16(xr + size_t(lane + 32 * i) * 16) : Vec16{0, 0, 0, 0};
         float m = 0.0f;
 #pragma unroll
         for (int i = 0; i < kShortRowVecs / 32; ++i) {
@@ -112,10 +112,9 @@ __global__ void __launch_bounds__(kThreads) rowwise_short_kernel(const uint8_t* 
 // Second pass over the bf16 intermediate when stage 1 already produced the amax: one warp per (row, strip of 128 16-byte
 // vectors), four vectors per lane in flight. A warp per whole row left most of the chip idle when there are few long rows
 // (32 rows of 14336: 13.4 us; in strips 2.7 us).
-__global__ void __launch_bounds__(kThreads) requant_rows_kernel(const uint8_t* __restrict__ x, int64_t rows, int cols,
-                                                                uint8_t* __restrict__ q, float* __restrict__ scale,
-                                                                const float* __restrict__ amax_in, int amax_per_row,
-                                                                const int* __restrict__ rows_dev) {
+__global__ void __launch_bounds__(kThreads) requant_rows_kernel(const uint8_t* x, int64_t rows, int cols, uint8_t* q,
+                                                                float* scale, const float* amax_in, int amax_per_row,
+                                                                const int* rows_dev) {
     pdl_enter();
     if (rows_dev != nullptr) rows = rows < *rows_dev ? rows : *rows_dev;  // row count known only on the device
     const int lane = threadIdx.x & 31;
@@ -132,7 +131,7 @@ __global__ void __launch_bounds__(kThreads) requant_rows_kernel(const uint8_t* _
         Vec16 raw[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (i0 + 32 * j < vecs) raw[j] = ld_nc16(xr + size_t(i0 + 32 * j) * 16);
+            if (i0 + 32 * j < vecs) raw[j] = ld_stream16(xr + size_t(i0 + 32 * j) * 16);
         const float sf = scale_from_amax(amax_in[amax_per_row ? r : 0]);
         const float inv = inv_scale(sf);
         if (lane == 0 && strip == 0 && (amax_per_row || r == 0)) scale[amax_per_row ? r : 0] = sf;
@@ -151,8 +150,8 @@ __global__ void __launch_bounds__(kThreads) requant_rows_kernel(const uint8_t* _
 // are fetched together and stay in registers between the amax and the conversion, and the next block's are on their way
 // while this one is reduced and written (HBM-bound: 3 B per element; 8 x 4096 x 14336: fetched one by one and read a second
 // time for the conversion 417 us, in one pass 284 us, with the next block's loads ahead 269 us = 5.2 TB/s).
-__global__ void __launch_bounds__(kThreads) block128_kernel(const uint8_t* __restrict__ w, int e, int rows, int cols,
-                                                            uint8_t* __restrict__ q, float* __restrict__ scale) {
+__global__ void __launch_bounds__(kThreads) block128_kernel(const uint8_t* w, int e, int rows, int cols, uint8_t* q,
+                                                            float* scale) {
     pdl_enter();
     __shared__ float s_red[kThreads / 32];
     const int bc = (cols + 127) / 128, br = (rows + 127) / 128;
@@ -170,7 +169,7 @@ __global__ void __launch_bounds__(kThreads) block128_kernel(const uint8_t* __res
     auto fetch = [&](const Place& pl, Vec16 (&raw)[8]) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-            raw[i] = 16 * i < pl.rows_left ? ld_nc16(w + (pl.first + size_t(16 * i) * cols) * 2) : Vec16{0, 0, 0, 0};
+            raw[i] = 16 * i < pl.rows_left ? ld_stream16(w + (pl.first + size_t(16 * i) * cols) * 2) : Vec16{0, 0, 0, 0};
     };
     Vec16 raw[8];
     int64_t b = blockIdx.x;
@@ -214,8 +213,7 @@ __global__ void __launch_bounds__(kThreads) block128_kernel(const uint8_t* __res
 }
 
 // per-tensor pass 1: amax of each of e slices into amax[e] (zeroed before)
-__global__ void __launch_bounds__(kThreads) tensor_amax_kernel(const uint8_t* __restrict__ x, int64_t vecs_per,
-                                                               float* __restrict__ amax) {
+__global__ void __launch_bounds__(kThreads) tensor_amax_kernel(const uint8_t* x, int64_t vecs_per, float* amax) {
     pdl_enter();
     __shared__ float s_red[kThreads / 32];
     const int ei = blockIdx.y;
@@ -223,16 +221,15 @@ __global__ void __launch_bounds__(kThreads) tensor_amax_kernel(const uint8_t* __
     float m = 0.0f;
     for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < vecs_per; i += int64_t(gridDim.x) * kThreads) {
         float v[8];
-        unpack8(ld_nc16(xe + size_t(i) * 16), v);
+        unpack8(ld_stream16(xe + size_t(i) * 16), v);
         m = amax8(v, m);
     }
     m = block_max(m, s_red);
     if (threadIdx.x == 0) atomic_max_nonneg(amax + ei, m);
 }
 // per-tensor pass 2
-__global__ void __launch_bounds__(kThreads) tensor_quant_kernel(const uint8_t* __restrict__ x, int64_t vecs_per,
-                                                                const float* __restrict__ amax,
-                                                                uint8_t* __restrict__ q, float* __restrict__ scale) {
+__global__ void __launch_bounds__(kThreads) tensor_quant_kernel(const uint8_t* x, int64_t vecs_per, const float* amax,
+                                                                uint8_t* q, float* scale) {
     pdl_enter();
     const int ei = blockIdx.y;
     const float sf = scale_from_amax(amax[ei]);
@@ -242,7 +239,7 @@ __global__ void __launch_bounds__(kThreads) tensor_quant_kernel(const uint8_t* _
     uint8_t* qe = q + size_t(ei) * vecs_per * 8;
     for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < vecs_per; i += int64_t(gridDim.x) * kThreads) {
         float v[8];
-        unpack8(ld_nc16(xe + size_t(i) * 16), v);
+        unpack8(ld_stream16(xe + size_t(i) * 16), v);
         *reinterpret_cast<uint2*>(qe + size_t(i) * 8) = quant8(v, inv);
     }
 }
@@ -251,8 +248,8 @@ __global__ void __launch_bounds__(kThreads) tensor_quant_kernel(const uint8_t* _
 // takes the amax through distributed shared memory and converts what it holds, one launch in place of a memset and two
 // passes. Latency-bound at these sizes (16 x 4096: 14 us from the first operation to the end of the last, now 5.3).
 constexpr int kSmallBlocks = 8, kSmallThreads = 1024, kSmallVecs = 8;
-__global__ void __launch_bounds__(kSmallThreads, 1) tensor_small_kernel(const uint8_t* __restrict__ x, int64_t vecs_per,
-                                                                        uint8_t* __restrict__ q, float* __restrict__ scale) {
+__global__ void __launch_bounds__(kSmallThreads, 1) tensor_small_kernel(const uint8_t* x, int64_t vecs_per,
+                                                                        uint8_t* q, float* scale) {
     pdl_enter();
     __shared__ float s_red[kSmallThreads / 32];
     __shared__ float s_block;
@@ -264,7 +261,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) tensor_small_kernel(const ui
 #pragma unroll
     for (int j = 0; j < kSmallVecs; ++j) {
         const int64_t i = int64_t(j) * (kSmallBlocks * kSmallThreads) + rank * kSmallThreads + threadIdx.x;
-        raw[j] = i < vecs_per ? ld_nc16(xe + size_t(i) * 16) : Vec16{0, 0, 0, 0};
+        raw[j] = i < vecs_per ? ld_stream16(xe + size_t(i) * 16) : Vec16{0, 0, 0, 0};
     }
 #pragma unroll
     for (int j = 0; j < kSmallVecs; ++j) {

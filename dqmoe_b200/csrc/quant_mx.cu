@@ -52,11 +52,9 @@ __device__ __forceinline__ size_t tiled_row_base(int64_t r, const int* s_off, co
 // dest_to_src[r] / k of the expert sort and its scales go to the tiled layout; otherwise rows map to themselves
 // and the scales are row-major.
 template <bool kGather>
-__global__ void __launch_bounds__(kThreads) quant_rows_kernel(const uint8_t* __restrict__ x, int64_t rows, int cols,
-                                                              const int* __restrict__ dest_to_src, int k,
-                                                              const int* __restrict__ offsets,
-                                                              const int* __restrict__ mtile_prefix, int E,
-                                                              uint8_t* __restrict__ q, uint8_t* __restrict__ sf) {
+__global__ void __launch_bounds__(kThreads) quant_rows_kernel(const uint8_t* x, int64_t rows, int cols,
+                                                              const int* dest_to_src, int k, const int* offsets,
+                                                              const int* mtile_prefix, int E, uint8_t* q, uint8_t* sf) {
     pdl_enter();
     extern __shared__ int s_tab[];  // kGather: offsets[E+1] then mtile_prefix[E+1]
     if constexpr (kGather) {
@@ -86,7 +84,7 @@ __global__ void __launch_bounds__(kThreads) quant_rows_kernel(const uint8_t* __r
             float f[8];
             float amax = 0.0f;
             if (v < vecs) {
-                const Vec16 raw = ld_nc16(xr + size_t(v) * 16);
+                const Vec16 raw = ld_stream16(xr + size_t(v) * 16);
                 const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -118,11 +116,9 @@ __global__ void __launch_bounds__(kThreads) quant_rows_kernel(const uint8_t* __r
 
 // Row-major scales [*, kblocks * 4] -> tiled. One thread per (output row, K block): a 4-byte word each way.
 // dest_to_src != null: output row r takes the scales of input row dest_to_src[r] / k (negative: skipped).
-__global__ void __launch_bounds__(kThreads) tile_scales_kernel(const uint32_t* __restrict__ sf_rows, int64_t rows, int kblocks,
-                                                               const int* __restrict__ dest_to_src, int k,
-                                                               const int* __restrict__ offsets,
-                                                               const int* __restrict__ mtile_prefix, int E,
-                                                               uint8_t* __restrict__ tiled) {
+__global__ void __launch_bounds__(kThreads) tile_scales_kernel(const uint32_t* sf_rows, int64_t rows, int kblocks,
+                                                               const int* dest_to_src, int k, const int* offsets,
+                                                               const int* mtile_prefix, int E, uint8_t* tiled) {
     pdl_enter();
     extern __shared__ int s_tab[];
     const bool sorted = offsets != nullptr;
@@ -162,15 +158,15 @@ static int grid_for(int64_t work_items, int per_block) {
 //   scale byte  = e4m3_rne((amax / 6) / g), saturating at 448
 //   nibbles     = e2m1_rne(x * (1 / (e4m3 * g))), saturating at 6; an all-zero group stores zeros
 // All divisions IEEE fp32. Scale bytes row-major [rows, cols / 16].
-__global__ void __launch_bounds__(kThreads) quant_nvfp4_kernel(const uint8_t* __restrict__ x, int64_t rows, int cols,
-                                                               const float* __restrict__ g, int64_t rows_per_g,
-                                                               uint8_t* __restrict__ q, uint8_t* __restrict__ sf) {
+__global__ void __launch_bounds__(kThreads) quant_nvfp4_kernel(const uint8_t* x, int64_t rows, int cols,
+                                                               const float* g, int64_t rows_per_g, uint8_t* q,
+                                                               uint8_t* sf) {
     pdl_enter();
     const int groups = cols / 16;
     const int64_t total = rows * groups;
     for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < total; i += int64_t(gridDim.x) * kThreads) {
         const int64_t r = i / groups;
-        const Vec16 v0 = ld_nc16(x + i * 32), v1 = ld_nc16(x + i * 32 + 16);
+        const Vec16 v0 = ld_stream16(x + i * 32), v1 = ld_stream16(x + i * 32 + 16);
         const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
         float f[16];
         float amax = 0.0f;

@@ -23,17 +23,19 @@ constexpr int kMaxExperts = 1024;
 __device__ __forceinline__ int bucket_of(int id, int E) { return (id >= 0 && id < E) ? id : E; }
 
 // ---------------------------------------------------------------- pass 1: chunk histograms
-__global__ void __launch_bounds__(kSortThreads) sort_hist_kernel(const int* __restrict__ ids, int n, int E,
-                                                                 int* __restrict__ chunk_hist /*[chunks][E+1]*/) {
+__global__ void __launch_bounds__(kSortThreads) sort_hist_kernel(const int* ids, int n, int E,
+                                                                 int* chunk_hist /*[chunks][E+1]*/) {
     pdl_enter();
     extern __shared__ int s_hist[];  // E+1
     for (int i = threadIdx.x; i <= E; i += kSortThreads) s_hist[i] = 0;
     __syncthreads();
-    const int base = blockIdx.x * kChunk;
-    for (int i = threadIdx.x; i < kChunk; i += kSortThreads) {
-        const int r = base + i;
-        if (r < n) atomicAdd(&s_hist[bucket_of(ids[r], E)], 1);  // integer counts: order-independent
-    }
+    const int base = blockIdx.x * kChunk + threadIdx.x;
+    int id[kChunk / kSortThreads];  // all of a thread's loads before the first use
+#pragma unroll
+    for (int i = 0; i < kChunk / kSortThreads; ++i) id[i] = base + i * kSortThreads < n ? ids[base + i * kSortThreads] : 0;
+#pragma unroll
+    for (int i = 0; i < kChunk / kSortThreads; ++i)
+        if (base + i * kSortThreads < n) atomicAdd(&s_hist[bucket_of(id[i], E)], 1);  // integer counts: order-independent
     __syncthreads();
     for (int i = threadIdx.x; i <= E; i += kSortThreads) chunk_hist[size_t(blockIdx.x) * (E + 1) + i] = s_hist[i];
 }
@@ -86,9 +88,8 @@ __device__ void block_exclusive_scan(int* s_val, int len, int* s_warp_tot) {
 // kStaged: the whole table fits shared memory and is scanned there (coalesced in, coalesced out; walking the table
 // bucket by bucket in global memory is a chain of strided round trips: 15.7 us at 64 chunks x 129 buckets).
 template <bool kStaged>
-__global__ void __launch_bounds__(1024) sort_scan_kernel(int* __restrict__ chunk_hist, int chunks, int E,
-                                                         int* __restrict__ counts, int* __restrict__ offsets,
-                                                         int* __restrict__ mtile_prefix) {
+__global__ void __launch_bounds__(1024) sort_scan_kernel(int* chunk_hist, int chunks, int E, int* counts,
+                                                         int* offsets, int* mtile_prefix) {
     pdl_enter();
     extern __shared__ int s_hist[];  // kStaged: [chunks][E + 1]
     __shared__ int s_tot[kMaxExperts + 2];
@@ -135,12 +136,10 @@ __global__ void __launch_bounds__(1024) sort_scan_kernel(int* __restrict__ chunk
 // ---------------------------------------------------------------- pass 3: scatter
 // kSingle: the whole problem is one chunk; histogram, scan and scatter in one block.
 template <bool kSingle>
-__global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* __restrict__ ids, int n, int E,
-                                                                    const int* __restrict__ chunk_base,
-                                                                    int* __restrict__ counts, int* __restrict__ offsets,
-                                                                    int* __restrict__ mtile_prefix,
-                                                                    int* __restrict__ dest_to_src,
-                                                                    int* __restrict__ src_to_dest) {
+__global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* ids, int n, int E,
+                                                                    const int* chunk_base, int* counts, int* offsets,
+                                                                    int* mtile_prefix, int* dest_to_src,
+                                                                    int* src_to_dest) {
     pdl_enter();
     extern __shared__ int s_mem[];
     // s_warp_hist[w][E+1]: rows of bucket b seen so far by warp w, then exclusive prefix over warps
@@ -158,10 +157,12 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* _
     int bucket[kRowsPerWarp / 32];
     int rank[kRowsPerWarp / 32];
 #pragma unroll
+    for (int it = 0; it < kRowsPerWarp / 32; ++it)  // all loads before the first use
+        bucket[it] = base + it * 32 + lane < n ? bucket_of(ids[base + it * 32 + lane], E) : -1;
+#pragma unroll
     for (int it = 0; it < kRowsPerWarp / 32; ++it) {
-        const int r = base + it * 32 + lane;
-        const bool live = r < n;
-        const int b = live ? bucket_of(ids[r], E) : -1;
+        const bool live = base + it * 32 + lane < n;
+        const int b = bucket[it];
         // lanes holding the same bucket, in row order
         const unsigned peers = __match_any_sync(0xffffffffu, b);
         const int before = __popc(peers & ((1u << lane) - 1u));
@@ -170,7 +171,6 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* _
         __syncwarp();
         if (live && before == 0) my_hist[b] = seen + __popc(peers);
         __syncwarp();
-        bucket[it] = b;
         rank[it] = seen + before;
     }
     __syncthreads();
@@ -228,8 +228,9 @@ __global__ void mtile_prefix_kernel(const int* __restrict__ offsets, int E, int*
 
 // out[r] = values[s] for the rows r of segment s, segments laid out back to back with
 // counts[s] rows each (S <= kMaxExperts). Every block rebuilds the small prefix in shared memory.
-__global__ void __launch_bounds__(256) segment_ids_kernel(const int* __restrict__ counts, const int* __restrict__ values,
-                                                         int S, int* __restrict__ out, int n) {
+__global__ void __launch_bounds__(256) segment_ids_kernel(const int* __restrict__ counts,
+                                                          const int* __restrict__ values, int S,
+                                                          int* __restrict__ out, int n) {
     __shared__ int s_pref[kMaxExperts + 2];
     __shared__ int s_warp_tot[33];
     for (int i = threadIdx.x; i < S; i += blockDim.x) s_pref[i] = counts[i];
@@ -307,9 +308,8 @@ int route_sort(const int* ids, int n, int E, int* counts, int* offsets, int* mti
 // normalised to sum 1. Output rows have `slots` >= k entries: entries k.. name the shared
 // experts E, E+1, ... (every token, weight 1), which the layer then treats like routed ones.
 template <int kPerLane>
-__global__ void __launch_bounds__(256) route_topk_kernel(const float* __restrict__ logits, int T, int E, int k,
-                                                         int slots, int scoring, int* __restrict__ indices,
-                                                         float* __restrict__ weights) {
+__global__ void __launch_bounds__(256) route_topk_kernel(const float* logits, int T, int E, int k, int slots,
+                                                         int scoring, int* indices, float* weights) {
     pdl_enter();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;

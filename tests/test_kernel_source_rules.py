@@ -45,3 +45,26 @@ def test_buffers_are_released_by_a_converged_warp():
     mx = source("gemm_mx_sm100.cu")
     for m in re.finditer(r"mbar_arrive\(&st\.(tmem_empty|overlap_free)", mx):
         assert "__syncwarp()" in mx[max(0, m.start() - 200):m.start()], mx[m.start() - 200:m.end()]
+
+
+def test_dependents_read_their_predecessors_output_with_plain_loads():
+    """A programmatic dependent is resident while the kernels before it still write what it reads behind its wait. Non-coherent
+    loads (and what the compiler makes of const __restrict__ arguments) are for data that stays unchanged in that time."""
+    found = 0
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith(".cu"):
+            continue
+        text = source(name)
+        for m in re.finditer(r"__global__", text):
+            signature = text[m.start():text.find("{", m.start())]
+            if ";" in signature:
+                continue
+            body = braces(text, m.start())
+            if not re.search(r"\b(pdl_enter|pdl_wait|wait_for_primary)\(", body):
+                continue
+            found += 1
+            for word in ("__restrict__", "__ldg", "ld_nc16", ".nc"):
+                assert word not in signature + body, (name, signature[:120], word)
+        if name in ("permute.cu", "quant.cu", "quant_mx.cu"):  # device helpers of such kernels
+            assert "ld_nc16" not in text and "__ldg" not in text, name
+    assert found >= 18
