@@ -240,10 +240,11 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
         for (int s = 0; s < kNumStages; ++s) {
             // block mode: and the lanes of the scale loader that copy something
             ptx::mbar_init(&st.full[s], kMode == kBlock ? 1 + (p.sa_t != nullptr ? 3 : 32) : 1);
-            ptx::mbar_init(&st.empty[s], 1);
+            // block mode: the MMAs' completion and the MMA thread itself, which passes on what it has seen (scale loader)
+            ptx::mbar_init(&st.empty[s], kMode == kBlock ? 2 : 1);
         }
         for (int b = 0; b < 2; ++b) {
-            ptx::mbar_init(&st.tmem_full[b], 1);
+            ptx::mbar_init(&st.tmem_full[b], kMode == kBlock ? 2 : 1);
             ptx::mbar_init(&st.tmem_empty[b], kPair ? 2 * kEpiWarps : kEpiWarps);  // both CTAs' epilogue warps
         }
         for (int i = 0; i < 4; ++i) ptx::mbar_init(&st.epi_sync[i], 2);
@@ -412,6 +413,9 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         mma_stage(tmem_base + buf * kUmmaN, s, true);
                         commit(&st.tmem_full[buf]);
                         commit(&st.empty[s]);
+                        // both also by this thread: see the scale loader
+                        ptx::mbar_arrive(&st.tmem_full[buf]);
+                        ptx::mbar_arrive(&st.empty[s]);
                     }
                 }
             }
@@ -420,13 +424,17 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
       } else if (warp == 2) {
         // ------------------------------------------------------------ scale loader (block mode)
         // Stages the scales of every K block in shared memory with 4-byte asynchronous copies. They belong to the K
-        // block's stage: the copies arrive on its full barrier, so that the barrier of the accumulator buffer, which the
-        // MMA thread signals after it has seen the stage full, covers them too, and the epilogue warps need no wait of
-        // their own for them (an mbarrier wait costs ~100 cycles even when it is over already: with one for the scales and
-        // one for the buffer a K block took 987 / 940 cycles in fc1 / fc2 at the Mixtral shape with T = 4096, now 885 /
-        // 817; 1132 / 556 us -> 1100 / 514 us). The ring has more slots
-        // than the kNumStages + 2 K blocks that can lie between a stage being refilled and the oldest undrained
-        // accumulator, so a slot is free when its stage is.
+        // block's stage: the copies arrive on its full barrier, which only the MMA thread waits for, and the epilogue warps
+        // have one wait per K block, for the accumulator buffer (a wait for an mbarrier costs ~100 cycles even when it is
+        // over already: with a second one for the scales a K block took 987 / 940 cycles in fc1 / fc2 at the Mixtral shape
+        // with T = 4096, without 885 / 817; 1132 / 556 us -> 1100 / 514 us).
+        // Why the epilogue sees the scales: a completed copy is visible to whoever observes the full barrier's phase, that
+        // is to the MMA thread; its own arrival on the buffer's barrier (a release) comes after that, and the epilogue
+        // warps acquire this barrier. The commit's arrival alone would not do: it tracks the completion of MMAs, and nothing
+        // says that it also publishes what the issuing thread has seen. Why a slot may be refilled: a warp reads its scales before
+        // it releases the buffer, the MMA thread acquires that release before it issues the K block two further on, and
+        // then arrives on that block's empty barrier, which the refill acquires. The ring has more slots than the
+        // kNumStages + 2 K blocks that can lie between a stage being refilled and the oldest undrained accumulator.
         // Where the caller has the activation scales by tile as well (the layer does), the TMA producer fetches a K block's 128
         // of them with one bulk copy and this warp copies three weight scales: the row-major form costs four scattered
         // copies and 32 barrier arrivals per K block, which the epilogue warps' shared-memory traffic queues behind

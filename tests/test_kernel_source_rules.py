@@ -68,3 +68,17 @@ def test_dependents_read_their_predecessors_output_with_plain_loads():
         if name in ("permute.cu", "quant.cu", "quant_mx.cu"):  # device helpers of such kernels
             assert "ld_nc16" not in text and "__ldg" not in text, name
     assert found >= 18
+
+
+def test_block_scales_are_passed_on_by_a_release():
+    """Block mode's scales arrive on the stage's barrier, which only the MMA thread observes; the epilogue warps read them behind
+    the accumulator buffer's. A tcgen05.commit tracks the completion of MMAs and publishes nothing else, so the thread arrives
+    there itself, and on the barrier that lets the ring slot be refilled."""
+    text = source("gemm_sm100.cu")
+    at = text.index("else if (warp == 1)", text.index("setmaxnreg_dec"))
+    issuer = braces(text, at)
+    block = issuer[issuer.index("acc_it) {", issuer.index("} else {\n", issuer.index("commit(&st.tmem_full"))):]
+    for bar in ("tmem_full[buf]", "empty[s]"):
+        assert f"commit(&st.{bar})" in block and f"mbar_arrive(&st.{bar})" in block, bar
+    for bar in ("empty[s]", "tmem_full[b]"):
+        assert f"mbar_init(&st.{bar}, kMode == kBlock ? 2 : 1)" in text, bar
