@@ -317,7 +317,12 @@ static int tensor_small(const void* x, int e, int64_t vecs, void* q, float* scal
     DQ_CUDA(cudaLaunchKernelEx(&cfg, tensor_small_kernel, static_cast<const uint8_t*>(x), vecs, static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
 }
-static bool tensor_small_fits(int64_t vecs) { return vecs <= int64_t(kSmallBlocks) * kSmallThreads * kSmallVecs; }
+// Only as many slices as run at once, one block per SM: every slice, however short, costs a cluster of eight blocks, and from
+// the second wave on the general form is the faster one (general / cluster, us: 1 slice of 65536 11.1 / 7.9, 18 slices of 64
+// 11.3 / 8.9, of 524288 18.5 / 12.5; 32 of 65536 11.2 / 14.1, 256 of 8192 11.5 / 76.6, 1024 of 131072 175 / 329).
+static bool tensor_small_fits(int e, int64_t vecs) {
+    return vecs <= int64_t(kSmallBlocks) * kSmallThreads * kSmallVecs && int64_t(e) * kSmallBlocks <= sm_count();
+}
 
 // Scratch of dqmoe_quant_fp8_tensor_static: lives in the library image of every GPU that
 // loads it (4 KiB per device) so that the call needs no caller- or library-made allocation.
@@ -416,7 +421,7 @@ int dqmoe_quant_fp8_tensor(const void* x_bf16, int e, int64_t numel_per, void* q
     DQ_CHECK_FMT(numel_per % 8 == 0, "numel_per=%lld must be a multiple of 8", (long long) numel_per);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (quant::tensor_small_fits(numel_per / 8)) return quant::tensor_small(x_bf16, e, numel_per / 8, q, scale, s);
+    if (quant::tensor_small_fits(e, numel_per / 8)) return quant::tensor_small(x_bf16, e, numel_per / 8, q, scale, s);
     DQ_CUDA(cudaMemsetAsync(amax_scratch, 0, size_t(e) * sizeof(float), s));
     const int64_t vecs = numel_per / 8;
     const int gx = quant::grid_cap((vecs + quant::kThreads - 1) / quant::kThreads, e >= 8 ? 2 : 8);
@@ -445,7 +450,7 @@ int dqmoe_quant_fp8_tensor_static(const void* x_bf16, int e, int64_t numel_per, 
     DQ_CHECK(x_bf16 != nullptr && q != nullptr && scale != nullptr);
     DQ_CHECK_FMT(numel_per % 8 == 0, "numel_per=%lld must be a multiple of 8", (long long) numel_per);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
-    if (quant::tensor_small_fits(numel_per / 8))
+    if (quant::tensor_small_fits(e, numel_per / 8))
         return quant::tensor_small(x_bf16, e, numel_per / 8, q, scale, static_cast<cudaStream_t>(stream));
     float* amax = nullptr;
     const int rc = quant::static_amax_address(&amax);

@@ -39,3 +39,13 @@ def bits(t: torch.Tensor) -> np.ndarray:
     if t.dtype == torch.float8_e4m3fn:
         return t.view(torch.uint8).numpy()
     return t.numpy()
+
+
+def kernels_of(fn):
+    """Names of the CUDA kernels that fn() launches, in order of their start."""
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    events = [e for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    return [e.name for e in sorted(events, key=lambda e: e.time_range.start)]

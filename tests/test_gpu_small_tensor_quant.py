@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import bits
+from helpers import bits, kernels_of
 
 pytestmark = pytest.mark.gpu
 
@@ -18,3 +18,19 @@ def test_per_tensor_quantiser_bit_exact(e, numel):
     ref = (x.float() * (1.0 / sf)[:, None, None]).to(torch.float8_e4m3fn)
     q, s = ops.per_tensor_cast_to_fp8(x.to("cuda"), per_expert=True)
     assert np.array_equal(bits(s.reshape(-1)), bits(sf)) and np.array_equal(bits(q.view(e, 1, numel)), bits(ref))
+
+
+@pytest.mark.parametrize("numel", [64, 131072])
+def test_cluster_form_only_while_all_slices_run_at_once(numel):
+    """A slice takes eight SMs in the cluster form: more slices than that go through the general one, however short they are."""
+    from dqmoe_b200 import ops
+    most = torch.cuda.get_device_properties(0).multi_processor_count // 8
+    for e in (most, most + 1, 8 * most):
+        x = torch.randn(e, 1, numel, generator=torch.Generator().manual_seed(e)).to(torch.bfloat16)
+        sf = x.float().abs().amax((1, 2)).clamp(1e-4) / 448.0
+        ref = (x.float() * (1.0 / sf)[:, None, None]).to(torch.float8_e4m3fn)
+        xd, out = x.to("cuda"), []
+        names = kernels_of(lambda: out.append(ops.per_tensor_cast_to_fp8(xd, per_expert=True)))
+        q, s = out[0]
+        assert np.array_equal(bits(s.reshape(-1)), bits(sf)) and np.array_equal(bits(q), bits(ref))
+        assert any("tensor_small" in n for n in names) == (e <= most), (e, names)
