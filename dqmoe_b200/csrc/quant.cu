@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kThreads) tensor_quant_kernel(const uint8_t* x
 // passes. Latency-bound at these sizes (16 x 4096: 14 us from the first operation to the end of the last, now 5.3).
 constexpr int kSmallBlocks = 8, kSmallThreads = 1024, kSmallVecs = 8;
 __global__ void __launch_bounds__(kSmallThreads, 1) tensor_small_kernel(const uint8_t* x, int64_t vecs_per,
-                                                                        uint8_t* q, float* scale) {
+                                                                        uint8_t* q, float* scale, float* amax) {
     pdl_enter();
     __shared__ float s_red[kSmallThreads / 32];
     __shared__ float s_block;
@@ -286,7 +286,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) tensor_small_kernel(const ui
     }
     const float sf = scale_from_amax(m);
     const float inv = inv_scale(sf);
-    if (rank == 0 && threadIdx.x == 0) scale[ei] = sf;
+    if (rank == 0 && threadIdx.x == 0) {
+        scale[ei] = sf;
+        if (amax != nullptr) amax[ei] = m;  // as the general form leaves it
+    }
     uint8_t* qe = q + size_t(ei) * vecs_per * 8;
 #pragma unroll
     for (int j = 0; j < kSmallVecs; ++j) {
@@ -300,7 +303,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) tensor_small_kernel(const ui
     ptx::cluster_sync();  // no block leaves while another may still read its word
 }
 
-static int tensor_small(const void* x, int e, int64_t vecs, void* q, float* scale, cudaStream_t stream) {
+static int tensor_small(const void* x, int e, int64_t vecs, void* q, float* scale, float* amax, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kSmallBlocks, unsigned(e), 1);
     cfg.blockDim = dim3(kSmallThreads, 1, 1);
@@ -314,7 +317,8 @@ static int tensor_small(const void* x, int e, int64_t vecs, void* q, float* scal
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    DQ_CUDA(cudaLaunchKernelEx(&cfg, tensor_small_kernel, static_cast<const uint8_t*>(x), vecs, static_cast<uint8_t*>(q), scale));
+    DQ_CUDA(cudaLaunchKernelEx(&cfg, tensor_small_kernel, static_cast<const uint8_t*>(x), vecs, static_cast<uint8_t*>(q), scale,
+                               amax));
     return DQMOE_OK;
 }
 // Only as many slices as run at once, one block per SM: every slice, however short, costs a cluster of eight blocks, and from
@@ -421,7 +425,7 @@ int dqmoe_quant_fp8_tensor(const void* x_bf16, int e, int64_t numel_per, void* q
     DQ_CHECK_FMT(numel_per % 8 == 0, "numel_per=%lld must be a multiple of 8", (long long) numel_per);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (quant::tensor_small_fits(e, numel_per / 8)) return quant::tensor_small(x_bf16, e, numel_per / 8, q, scale, s);
+    if (quant::tensor_small_fits(e, numel_per / 8)) return quant::tensor_small(x_bf16, e, numel_per / 8, q, scale, amax_scratch, s);
     DQ_CUDA(cudaMemsetAsync(amax_scratch, 0, size_t(e) * sizeof(float), s));
     const int64_t vecs = numel_per / 8;
     const int gx = quant::grid_cap((vecs + quant::kThreads - 1) / quant::kThreads, e >= 8 ? 2 : 8);
@@ -451,7 +455,7 @@ int dqmoe_quant_fp8_tensor_static(const void* x_bf16, int e, int64_t numel_per, 
     DQ_CHECK_FMT(numel_per % 8 == 0, "numel_per=%lld must be a multiple of 8", (long long) numel_per);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
     if (quant::tensor_small_fits(e, numel_per / 8))
-        return quant::tensor_small(x_bf16, e, numel_per / 8, q, scale, static_cast<cudaStream_t>(stream));
+        return quant::tensor_small(x_bf16, e, numel_per / 8, q, scale, nullptr, static_cast<cudaStream_t>(stream));
     float* amax = nullptr;
     const int rc = quant::static_amax_address(&amax);
     if (rc != DQMOE_OK) return rc;

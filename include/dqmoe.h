@@ -351,7 +351,7 @@ int dqmoe_quant_fp8_block_128x128(const void* w_bf16, int e, int rows, int cols,
                                   float* scale, dqmoe_stream_t stream);
 /*
  * One scale per tensor (or per expert when e > 1: x is [e, numel_per] and scale [e]).
- * amax_scratch is e floats of caller-owned device memory, overwritten.
+ * amax_scratch is e floats of caller-owned device memory, overwritten with the slices' largest absolute values.
  * The reference has this mode only for the intermediate (csrc/moe_kernels.h:136-221).
  */
 int dqmoe_quant_fp8_tensor(const void* x_bf16, int e, int64_t numel_per, void* q, float* scale,

@@ -34,3 +34,18 @@ def test_cluster_form_only_while_all_slices_run_at_once(numel):
         q, s = out[0]
         assert np.array_equal(bits(s.reshape(-1)), bits(sf)) and np.array_equal(bits(q), bits(ref))
         assert any("tensor_small" in n for n in names) == (e <= most), (e, names)
+
+
+@pytest.mark.parametrize("e,numel", [(3, 1024), (40, 1024), (1, 524288 + 8)])
+def test_scratch_receives_the_largest_values(e, numel):
+    """Whichever form runs, the scratch holds each slice's largest absolute value afterwards."""
+    import ctypes
+    from dqmoe_b200 import _lib
+    x = torch.randn(e, numel, generator=torch.Generator().manual_seed(e)).to(torch.bfloat16)
+    xd = x.to("cuda")
+    q = torch.empty(e, numel, dtype=torch.uint8, device="cuda")
+    s, scratch = torch.empty(e, device="cuda"), torch.full((e,), 1e30, device="cuda")
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    _lib.check(_lib.load().dqmoe_quant_fp8_tensor(p(xd), e, numel, p(q), p(s), p(scratch),
+                                                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    assert torch.equal(scratch.cpu(), x.float().abs().amax(1))
