@@ -367,9 +367,11 @@ int dqmoe_quant_fp8_block_1x128(const void* x_bf16, int64_t rows, int cols, void
     DQ_CHECK(x_bf16 != nullptr && q != nullptr && scale != nullptr);
     DQ_CHECK_FMT(cols % 8 == 0, "cols=%d must be a multiple of 8", cols);
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 8));
-    // strips of a row with 16 columns per lane where rows and output allow it: more loads in flight than a warp per row has
-    // (4096 x 4096: 15.0 us, in strips 9.8 us)
-    if (cols % 16 == 0 && is_aligned(q, 16) && rows < (int64_t(1) << 31))
+    // Strips of a row with 16 columns per lane where rows and output allow it: more loads in flight than a warp per row has
+    // (row form / strips, us: 4096 x 4096 15.0 / 9.8, 100000 x 1024 81 / 54, 100000 x 528 54 / 42). Up to 512 columns half a
+    // strip stays empty or more, and the row form is as fast or faster (100000 rows of 512 41.5 / 39.9, 20000 rows of 512
+    // 8.3 / 8.6, 100000 rows of 256 20.9 / 36.1).
+    if (cols > 512 && cols % 16 == 0 && is_aligned(q, 16) && rows < (int64_t(1) << 31))
         return permute::scatter_quant_1x128(x_bf16, int(rows), 1, cols, nullptr, q, scale, static_cast<cudaStream_t>(stream));
     DQ_RC(launch_pdl(permute::quant_1x128_kernel, dim3(permute::grid_for_rows(rows)), permute::kThreads, 0,
                      static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows, cols, 1, nullptr,

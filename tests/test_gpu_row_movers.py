@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import bits
+from helpers import bits, kernels_of
 from oracle import moe_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -110,3 +110,14 @@ def test_128x128_quantiser_bit_exact(ops, E, rows, cols):
     ref = (blk * (1.0 / sf)[:, :, None, :, None]).view(E, R * 128, Cb * 128)[:, :rows, :cols].contiguous().to(torch.float8_e4m3fn)
     q, s = ops.per_block_cast_to_fp8(w.to(DEV))
     assert np.array_equal(bits(s), bits(sf)) and np.array_equal(bits(q), bits(ref))
+
+
+@pytest.mark.parametrize("rows,cols,strips", [(3, 512, False), (1000, 128, False), (3, 528, True), (700, 1040, True), (5, 1032, False)])
+def test_1x128_quantiser_takes_strips_for_rows_that_fill_them(ops, rows, cols, strips):
+    g = torch.Generator().manual_seed(cols)
+    x = torch.randn(rows, cols, generator=g).to(torch.bfloat16)
+    xd, out = x.to(DEV), []
+    names = kernels_of(lambda: out.append(ops.per_token_block_cast_to_fp8(xd)))
+    assert any("scatter_quant" in n for n in names) == strips, names
+    q, s = orc.quant_block_1x128(x)
+    assert np.array_equal(bits(out[0][1]), bits(s)) and np.array_equal(bits(out[0][0]), bits(q))
