@@ -59,9 +59,10 @@ __global__ void __launch_bounds__(kThreads) row_move_kernel(const uint8_t* src, 
 
 // out[t, :] = sum_j w[t, j] * d[t, j, :]; one warp per (token, 256-column strip). HBM-bound; the slots of a token are
 // fetched kSlotBatch at a time before the first is used, so that a lane has that many 16-byte loads in flight (T = 8192,
-// k = 8, H = 7168: one slot after the other 246 us, batches of eight 194 us = 5.4 TB/s). The batch is the power of two that
-// holds k, at most 8: with two slots in a batch of eight the registers of the empty ones cost occupancy (T = 2049, k = 2,
-// H = 4096: 25.9 us against 13.1).
+// k = 8, H = 7168: one slot after the other 246 us, batches of eight 194 us = 5.4 TB/s). The batch is k itself, at most 8: the
+// registers of empty slots cost occupancy (T = 2049, k = 2, H = 4096: in batches of eight 25.9 us, of two 13.1; T = 4096, k = 5,
+// H = 2048: one after the other 22.7, in batches of eight 25.6, of five 16.6). Three slots take the batch of four
+// (T = 4096, H = 2880: 16.6 us, in a batch of three 17.1).
 template <int kSlotBatch>
 __global__ void __launch_bounds__(kThreads) finalize_weighted_kernel(const uint8_t* d, const float* w, uint8_t* out,
                                                                      int T, int k, int row_vecs) {
@@ -351,10 +352,12 @@ int dqmoe_finalize_weighted(const void* d_bf16, const float* weights, void* out_
     DQ_CHECK(is_aligned(d_bf16, 16) && is_aligned(out_bf16, 16));
     const int row_vecs = H / 8;
     const int64_t items = int64_t(T) * ((row_vecs + 31) / 32);
-    auto* kern = k == 1   ? permute::finalize_weighted_kernel<1>
-                 : k == 2 ? permute::finalize_weighted_kernel<2>
-                 : k <= 4 ? permute::finalize_weighted_kernel<4>
-                          : permute::finalize_weighted_kernel<8>;
+    using Kernel = void (*)(const uint8_t*, const float*, uint8_t*, int, int, int);
+    static const Kernel kernels[8] = {permute::finalize_weighted_kernel<1>, permute::finalize_weighted_kernel<2>,
+                                      permute::finalize_weighted_kernel<4>, permute::finalize_weighted_kernel<4>,
+                                      permute::finalize_weighted_kernel<5>, permute::finalize_weighted_kernel<6>,
+                                      permute::finalize_weighted_kernel<7>, permute::finalize_weighted_kernel<8>};
+    const Kernel kern = kernels[(k < 8 ? k : 8) - 1];
     DQ_RC(launch_pdl(kern, dim3(permute::grid_for_rows(items)), permute::kThreads, 0, static_cast<cudaStream_t>(stream),
                      static_cast<const uint8_t*>(d_bf16), weights, static_cast<uint8_t*>(out_bf16), T, k, row_vecs));
     return DQMOE_OK;

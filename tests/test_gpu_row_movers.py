@@ -121,3 +121,10 @@ def test_1x128_quantiser_takes_strips_for_rows_that_fill_them(ops, rows, cols, s
     assert any("scatter_quant" in n for n in names) == strips, names
     q, s = orc.quant_block_1x128(x)
     assert np.array_equal(bits(out[0][1]), bits(s)) and np.array_equal(bits(out[0][0]), bits(q))
+
+
+@pytest.mark.parametrize("k", [1, 3, 5, 6, 7, 8, 9])
+def test_combine_batches_as_many_slots_as_there_are(ops, k):
+    d, w = torch.randn(33, k, 264, device=DEV).to(torch.bfloat16), torch.rand(33, k, device=DEV)
+    names = kernels_of(lambda: ops.finalize_weighted(d, w))
+    assert any(f"finalize_weighted_kernel<{4 if k == 3 else min(k, 8)}>" in n for n in names), names
