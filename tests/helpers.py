@@ -42,10 +42,14 @@ def bits(t: torch.Tensor) -> np.ndarray:
 
 
 def kernels_of(fn):
-    """Names of the CUDA kernels that fn() launches, in order of their start."""
-    torch.cuda.synchronize()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        fn()
+    """Names of the CUDA kernels that fn() launches, in order of their start. The profiler now and then comes back empty from a
+    short session; fn() is then called again."""
+    for _ in range(5):
         torch.cuda.synchronize()
-    events = [e for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            fn()
+            torch.cuda.synchronize()
+        events = [e for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+        if events:
+            break
     return [e.name for e in sorted(events, key=lambda e: e.time_range.start)]
