@@ -278,10 +278,13 @@ def quantize_activations_gpu(ops, x, mode):
     return x, None
 
 
-def launches_per_step(n, mode):
+def launches_per_step(n, mode, H, I, E):
     sort = 1 if n <= 2048 else 3
-    # sort, scatter into expert order, [scale tiling: MXFP8, block FP8 from 4096 rows on], fc1, [re-quantisation pass], fc2
-    return sort + 1 + 1 + (1 if mode in (256, 512, 2048) or (mode == 1024 and n >= 4096) else 0) + 1
+    kh, ki = -(-H // 128), -(-I // 128)
+    # block FP8 lays the activation scales out by tile in calls of many K blocks (tiled_scales in layer.cu)
+    tiled = mode == 1024 and min(H, I) >= 2048 and n >= 192 * E and (n // 128 + E // 2) * (ki * kh + -(-H // 256) * ki) >= 44000
+    # sort, scatter into expert order, [scale tiling: MXFP8, block FP8 where it pays], fc1, [re-quantisation pass], fc2
+    return sort + 1 + 1 + (1 if mode in (256, 512, 2048) or tiled else 0) + 1
 
 
 def config_of(name, wl, world, T=None):
@@ -524,7 +527,7 @@ def decode_sweep(args, dev, ops, with_cpu=True):
         "config": {"workload": "c5: decode-shape sweep, Mixtral shape, T in {1,16,64,256}; headline = fp8-tensor T=64",
                    "H": H, "I": I, "E": E, "k": k, "l2": "256 MB flush write before every timed call"},
         "clocks": clocks, "sweep": rows, "e2e": e2e, "cpu_baseline": base,
-        "gpu_launches": launches_per_step(64 * k, 256) * steps,
+        "gpu_launches": launches_per_step(64 * k, 256, H, I, E) * steps,
         "roofline": {"bound": "hbm", "achieved": head["gbs"], "peak": pk["hbm_gbs"], "unit": "GB/s",
                      "frac": head["gbs"] / pk["hbm_gbs"], "traffic": None,
                      "peak_note": f"of {pk['source']} copy bandwidth; nominal 8000 GB/s"}}
@@ -645,7 +648,7 @@ def run_prefill(args, name, wl, ops, dev, rank, world, local_rank, dist=None, ep
 
         def step():
             ops.moe_forward(aq, as_, bq, bs, b1q, b1s, d, idx, ws, mode)
-        per_step_launches = launches_per_step(n, mode)
+        per_step_launches = launches_per_step(n, mode, wl["H"], wl["I"], wl["E"])
     else:
         layer = EPModel(wl, T, dev, 0, ops, ep, dist, out_buffers=2 if headline else 1)
         sort_l = 1 if n <= 2048 else 3
@@ -1051,7 +1054,7 @@ def run_nvfp4(args, ops, dev, name="c2"):
     return {"metric": "moe_layer_tflops", "value": flops / (ms * 1e-3) / 1e12, "unit": "TFLOP/s", "n_gpus": 1,
             "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": ms, "tokens_per_s": T / (ms * 1e-3),
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "e2m1 x e2m1 -> f32 (ue4m3 scales per 16)",
-            "data": "synthetic", "parity": par, "clocks": clocks, "gpu_launches": args.steps * (launches_per_step(n, 2048)),
+            "data": "synthetic", "parity": par, "clocks": clocks, "gpu_launches": args.steps * (launches_per_step(n, 2048, H, I, E)),
             "roofline": {"bound": "tensor", "kernel": "fc1 grouped GEMM (gated, NVFP4 re-quantisation)", "achieved": fl1 / (ms1 * 1e-3) / 1e12,
                          "peak": peak, "unit": "TFLOP/s", "frac": fl1 / (ms1 * 1e-3) / 1e12 / peak,
                          "peak_note": "4 x measured bf16 burst (no FP4 peak measured; nominal dense FP4 9 000)",

@@ -48,10 +48,21 @@ bool eligible(int H, int I, bool fp8);  // row sizes the decode path serves (16-
 namespace layer {
 
 constexpr size_t kAlign = 256;  // CUDA_MEM_ALIGN of the reference (csrc/util.h:54-59)
-// From this many expanded rows on, block mode lays the activation scales out by tile a second time (a launch before fc1; fc1
-// itself writes fc2's): 8192 rows, H 4096, I 14336 1985 -> 1852 us per call, 65536 rows, H 7168, I 2048 6084 -> 5999. Below,
-// the GEMMs wait for weights and nothing is gained (864 rows: 326.7 / 326.8 us; 10 rows: 35.0 / 35.8).
-constexpr int kTiledScaleRows = 4096;
+// Block mode may lay the activation scales out by tile a second time, a launch before fc1 (fc1 itself writes fc2's). What it
+// shortens is the trip of every K block, by about 4 %, so it pays where the GEMMs are bound by these trips for long: with
+// reductions of at least 2048 (in short ones the start and end of a tile count for more), more than one and a half row tiles
+// per expert (below, the GEMMs wait for weights) and at least kTiledTrips K blocks over all tiles (some 300 per SM; a smaller
+// call does not win back the launch). Row-major / by tile, us per layer call: H 4096, I 14336, E 8, 1536 rows 525 / 505, 8192
+// rows 1883 / 1798; H 7168, I 2048, E 32 16384 rows 1050 / 1036, 65536 rows 3609 / 3526; E 256 65536 rows 5120 / 4989;
+// H 2048, I 4096, E 8 8192 rows 300 / 296. On the other side of the three lines: H 2048, I 768, E 128 32768 rows 334 / 341;
+// H 1024, I 2048, E 4 4096 rows 60 / 64; H 7168, I 2048, E 32 4096 rows 378 / 385; H 2048, I 4096, E 8 4096 rows 163 / 168.
+constexpr int64_t kTiledTrips = 44000;
+static bool tiled_scales(int64_t n, int H, int I, int E, int quant_mode) {
+    if (quant_mode != DQMOE_QUANT_FP8_BLOCK || H < 2048 || I < 2048 || n < 192 * int64_t(E)) return false;
+    const int64_t tiles = n / 128 + E / 2;  // an expert's last row tile is on average half full
+    const int64_t kh = ceil_div(H, 128), ki = ceil_div(I, 128);
+    return tiles * (ki * kh + ceil_div(H, 256) * ki) >= kTiledTrips;
+}
 constexpr int kDecodeRows = 8;  // up to this many expanded rows the GEMV path of decode.cu is used (bf16, per-tensor FP8)
 
 struct Layout {
@@ -103,7 +114,7 @@ static Layout make_layout(int T, int H, int I, int E, int k, int quant_mode, int
                                    : quant_mode == DQMOE_QUANT_FP8_TENSOR ? 1 : 0;
     L.act_scale = add(act_scale_elems * sizeof(float));
     // block mode: the scale matrices a second time by tile, for the grouped GEMMs (every expert may add a partly filled tile)
-    const bool tiled = quant_mode == DQMOE_QUANT_FP8_BLOCK && n >= size_t(kTiledScaleRows);
+    const bool tiled = tiled_scales(int64_t(n), H, I, E, quant_mode);
     const size_t tile_rows = tiled ? ((n + 127) / 128 + (size_t(E) < n ? size_t(E) : n)) * 128 : 0;
     L.perm_a_scale_t = add(tile_rows * ceil_div(H, 128) * sizeof(float));
     L.act_scale_t = add(tile_rows * ceil_div(I, 128) * sizeof(float));
@@ -183,8 +194,7 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
     float* perm_a_scale = reinterpret_cast<float*>(ws + L.perm_a_scale);
     void* act = ws + L.act;
     float* act_scale = reinterpret_cast<float*>(ws + L.act_scale);
-    const bool block = quant_mode == DQMOE_QUANT_FP8_BLOCK;
-    float* perm_a_scale_t = block && n >= layer::kTiledScaleRows ? reinterpret_cast<float*>(ws + L.perm_a_scale_t) : nullptr;
+    float* perm_a_scale_t = layer::tiled_scales(n, H, I, E, quant_mode) ? reinterpret_cast<float*>(ws + L.perm_a_scale_t) : nullptr;
     float* act_scale_t = perm_a_scale_t != nullptr ? reinterpret_cast<float*>(ws + L.act_scale_t) : nullptr;
     void* act_bf16 = ws + L.act_bf16;
     float* amax = reinterpret_cast<float*>(ws + L.amax);
@@ -402,8 +412,7 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
     float* perm_a_scale = reinterpret_cast<float*>(lws + L.perm_a_scale);
     void* act = lws + L.act;
     float* act_scale = reinterpret_cast<float*>(lws + L.act_scale);
-    const bool block = quant_mode == DQMOE_QUANT_FP8_BLOCK;
-    float* perm_a_scale_t = block && n >= layer::kTiledScaleRows ? reinterpret_cast<float*>(lws + L.perm_a_scale_t) : nullptr;
+    float* perm_a_scale_t = layer::tiled_scales(n, H, I, E, quant_mode) ? reinterpret_cast<float*>(lws + L.perm_a_scale_t) : nullptr;
     float* act_scale_t = perm_a_scale_t != nullptr ? reinterpret_cast<float*>(lws + L.act_scale_t) : nullptr;
 
     int rc = route::route_topk(logits, T, E_routed, k_routed, n_shared, scoring, indices, weights, stream);

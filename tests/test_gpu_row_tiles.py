@@ -3,6 +3,7 @@
 import pytest
 import torch
 
+from helpers import kernels_of
 from oracle import moe_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -36,37 +37,40 @@ def test_ragged_row_counts_match_oracle(mode, H, I):
     assert orc.cosine(d.cpu(), ref) >= 0.999 and orc.max_rel_err(d.cpu(), ref) <= 2e-2
 
 
-@pytest.mark.parametrize("H,I,drop", [(1408, 192, False), (2048, 320, True)])
-def test_quarters_without_rows_over_long_reductions(H, I, drop):
-    """Block mode from 4096 rows on (scales by tile), row tiles of 1 to 128 rows and K loops of 11 and 16 blocks: warps without
-    rows, and the lanes of the scale loader without a copy, go round the same barriers as the others. With dropped slots the
-    kept tiles are fewer than the layout's bound. Rows are bit-identical to the same rows in a small call."""
+@pytest.mark.parametrize("drop", [False, True])
+def test_quarters_without_rows_over_long_reductions(drop):
+    """Block mode with the scales by tile, last row tiles of 1 to 128 rows and K loops of 33 and 23 blocks: warps without rows,
+    and the lanes of the scale loader without a copy, go round the same barriers as the others. With dropped slots the kept
+    tiles are fewer than the layout's bound. Rows are bit-identical to the same rows in a small call."""
     from dqmoe_b200 import ops
-    rows = ROWS * 4
+    H, I = 4112, 2832
+    rows = [r + 128 * (1 + i % 3) for i, r in enumerate(ROWS)]
     E, T = len(rows), sum(rows)
-    assert T >= 4096
-    g = torch.Generator().manual_seed(H)
-    a = torch.randn(T, H, generator=g).to(torch.bfloat16).to(DEV)
-    b = ops.per_block_cast_to_fp8((torch.randn(E, 2 * I, H, generator=g) * 0.05).to(torch.bfloat16).to(DEV))
-    b1 = ops.per_block_cast_to_fp8((torch.randn(E, H, I, generator=g) * 0.05).to(torch.bfloat16).to(DEV))
+    g = torch.Generator(device=DEV).manual_seed(H)
+    a = torch.randn(T, H, generator=g, device=DEV).to(torch.bfloat16)
+    b = ops.per_block_cast_to_fp8((torch.randn(E, 2 * I, H, generator=g, device=DEV) * 0.05).to(torch.bfloat16))
+    b1 = ops.per_block_cast_to_fp8((torch.randn(E, H, I, generator=g, device=DEV) * 0.05).to(torch.bfloat16))
     q, s = ops.per_token_block_cast_to_fp8(a)
-    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(rows))[torch.randperm(T, generator=g)].to(torch.int32)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(rows))[torch.randperm(T, generator=torch.Generator().manual_seed(H))]
+    ids = ids.to(torch.int32)
     if drop:
         ids[::3] = -1
         ids[1::7] = E
     ids = ids.view(T, 1)
 
-    def run(sel):
+    def run(sel, tiled):
         n = len(sel)
         ws = torch.empty(ops.moe_workspace_bytes(n, H, I, E, 1, 1024), dtype=torch.uint8, device=DEV)
         d = torch.zeros(n, 1, H, dtype=torch.bfloat16, device=DEV)
         qd = q.view(torch.uint8)[sel.to(DEV)].contiguous().view(q.dtype)
-        ops.moe_forward(qd, s[sel.to(DEV)].contiguous(), *b, *b1, d, ids[sel].contiguous().to(DEV), ws, 1024)
+        sd, idd = s[sel.to(DEV)].contiguous(), ids[sel].contiguous().to(DEV)
+        names = kernels_of(lambda: ops.moe_forward(qd, sd, *b, *b1, d, idd, ws, 1024))
         assert ops.device_status() == 0
+        assert any("scale_tiles" in k for k in names) == tiled, names
         return d.cpu()
 
     sample = torch.arange(0, T, 23)
-    full, small = run(torch.arange(T)), run(sample)
+    full, small = run(torch.arange(T), True), run(sample, False)
     assert torch.equal(full[sample], small)
     kept = (ids[:, 0] >= 0) & (ids[:, 0] < E)
     assert not full[~kept].any()
