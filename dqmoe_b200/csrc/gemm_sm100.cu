@@ -55,6 +55,9 @@ static_assert(kScaleSlots >= kStages + 2, "a slot must be drained when its stage
 constexpr int kTmemCols = 512;                    // two accumulator buffers of 256 columns
 constexpr long long kWaitLimit = 1000000000LL;    // clock cycles before a wait gives up (~0.5 s)
 
+// CTA pairs are taken where 2 x (256-row tiles) <= 1.16 x (128-row tiles): see tile_form.
+constexpr int kPairsWeight = 50, kSinglesWeight = 29;
+
 enum Mode : int { kNone = 0, kTensor = 1, kChannel = 2, kBlock = 3 };
 
 struct Params {
@@ -67,6 +70,7 @@ struct Params {
     int tile_w_rows;     // weight rows advanced per column tile (stage 1: 128, stage 2: 256)
     int box2_off;        // row offset of the second weight box (stage 1: I, stage 2: 128)
     int kb_count;        // ceil(K bytes / 128)
+    int by_counts;       // this launch works only if the experts' row counts favour its tile form (see tile_form)
     const int* offsets;       // [E+1] first row of each expert
     const int* mtile_prefix;  // [E+1] cumulative 128-row tiles
     const float* sa;          // activation scales
@@ -206,6 +210,15 @@ __device__ __forceinline__ void ffma2(float& a0, float& a1, uint32_t x0, uint32_
     a1 = r.y;
 }
 
+// Whether the experts' rows fill 256-row tiles well enough for CTA pairs (see tile_form); the same answer in every lane.
+__device__ __forceinline__ bool pairs_suit(const int* mtile_prefix, int E, int lane) {
+    pdl_wait();
+    int pairs = 0;
+    for (int e = lane; e < E; e += 32) pairs += (mtile_prefix[e + 1] - mtile_prefix[e] + 1) >> 1;
+    pairs = __reduce_add_sync(0xffffffffu, pairs);
+    return kPairsWeight * pairs <= kSinglesWeight * mtile_prefix[E];
+}
+
 // kBox = weight rows per TMA box (two boxes per stage, 2*kBox accumulator columns): 128 for
 // throughput, 64 when a launch would otherwise have fewer tiles than SMs (decode shapes).
 template <bool kFp8, int kMode, bool kGated, bool kPair, int kBox, int kElem = kElemBf16>
@@ -219,6 +232,9 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
+    if constexpr (kMode != kBlock && kElem != kElemF32 && kBox == 128) {
+        if (p.by_counts && pairs_suit(p.mtile_prefix, p.E, lane) != kPair) return;  // the other tile form's launch works
+    }
     constexpr int kBKElems = kFp8 ? kBKBytes : (kElem == kElemF32 ? kBKBytes / 4 : kBKBytes / 2);
     constexpr int kKind = kFp8 ? 0 : (kElem == kElemF32 ? 2 : 1);  // kind::f8f6f4, kind::f16, kind::tf32
     static_assert(kBox == 128 || (kBox == 64 && !kPair && kMode != kBlock), "narrow tiles: single CTA, non-block modes");
@@ -870,20 +886,32 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p,
     return DQMOE_OK;
 }
 
-// CTA pairs: a 256-row tile shares its weight tile between two SMs, which halves the weight bytes each stages. They pay off
-// when the experts' rows fill 256-row tiles about as well as 128-row ones, that is when the average lies in the upper half
-// of a 256-row period (with some room below the period's end, as the counts scatter), or when there are so many rows that the
-// last tile hardly counts. Single CTAs / pairs, us per layer call, per-tensor FP8 at H 4096, I 14336, E 8: 105 rows per
-// expert 272 / 324, 150: 368 / 322, 225: 438 / 391, 250: 430 / 442, 300: 559 / 615, 425: 670 / 607, 512: 731 / 782, 650:
-// 890 / 857; bf16 (2880 x 2880, E 64) 140: 772 / 681, 281: 1146 / 1221; per-channel (2048 x 768, E 128) 312: 329 / 390,
-// 437: 459 / 429.
-// Below 560 rows the launch must also have two rounds of single-CTA tiles (wide_tiles): with fewer, halving the number of
-// tiles leaves SMs idle.
-static bool use_pairs(int n, int E, int quant_mode, int wide_tiles) {
-    // Block mode is bound by the trip of every K block through registers, not by the traffic a pair saves.
-    if (quant_mode == DQMOE_QUANT_FP8_BLOCK) return false;
+// Tile forms. A 256-row tile on a CTA pair shares its weight tile between two SMs, which halves the weight bytes each stages;
+// it pays off when the experts' rows fill 256-row tiles about as well as 128-row ones. How they do depends on every expert's
+// count, which is known only on the device: the average says little when the routing is skewed, experts are empty or a shared
+// expert takes every token. So where it can go either way both forms are launched, and each kernel compares, from the sort's
+// table, the numbers of 256-row and 128-row tiles before it sets anything up: the pairs work up to 2 x 256-row tiles = 1.16 x
+// 128-row tiles, the singles beyond, and the other kernel leaves at once.
+// Measured, singles / pairs in us per layer call, by that ratio: 1.00 per-tensor (H 4096, I 14336, E 8, 194 rows per expert)
+// 430 / 391, bf16 (7168 x 2048, E 32, 192) 883 / 788, per-channel (2880 x 2880, E 64, 178) 581 / 479; 1.13 per-channel (2880 x
+// 2880, 690, skewed) 1528 / 1342, bf16 (7168 x 2048, 801) 2235 / 2267; 1.20 per-channel (7168 x 2048, 297, half the experts empty)
+// 484 / 502, per-tensor (4096 x 14336, 511, one expert for every token) 811 / 866; 1.33 per-tensor (2880 x 2880, 284) 751 / 791;
+// 1.54 per-channel (4096 x 14336, 165, one for all) 392 / 459; 1.72 per-tensor (2880 x 2880, 139, one for all) 437 / 495. Over
+// 540 calls of five models and these routings, 128 to 1024 rows per expert, against pairs from an average of 512 rows on: the
+// form on the right side of the line 0.972 of the time, with the launch that leaves (4 to 8 us) 0.990; a rule on the average
+// 0.994, but up to 1.25 for skewed calls.
+// Below kByCountsTrips K blocks over all tiles (200 per SM) the second launch costs more than the choice gives. Below an average
+// of 128 rows most experts have one tile; from 800 on the counts cannot say otherwise (every expert adds at most one empty
+// half: 2 x 256-row tiles <= 128-row tiles + E <= (1 + 128 / 800) x 128-row tiles).
+enum TileForm { kSingles, kPairs, kByCounts };
+constexpr int64_t kByCountsTrips = 30000;
+static TileForm tile_form(int n, int E, int quant_mode, int elem, int wide_tiles, int kb_count) {
+    // Block mode is bound by the trip of every K block through registers, not by the traffic a pair saves; fp32 has no pairs.
+    if (quant_mode == DQMOE_QUANT_FP8_BLOCK || elem == kElemF32) return kSingles;
     const int rows = n / E;
-    return rows >= 560 || ((rows & 255) > 128 && (rows & 255) <= 240 && wide_tiles >= 2 * sm_count());
+    if (rows >= 128 && rows < 800 && wide_tiles >= 2 * sm_count() && int64_t(wide_tiles) * kb_count >= kByCountsTrips)
+        return kByCounts;
+    return rows >= 512 ? kPairs : kSingles;
 }
 
 // elem: element type of the unquantised path (kElemBf16 / kElemHalf / kElemF32); bias: [E, gated ? 2N : N] fp32 or nullptr.
@@ -913,10 +941,11 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
     // The row-tile count is known only on the device; ceil(n/128) + min(E, n) - 1 bounds it.
     const int mtiles_max = ceil_div(n, kBM) + (E < n ? E : n) - 1;
     const int wide_tiles = mtiles_max * (gated ? ceil_div(N, kBoxRows) : ceil_div(N, kUmmaN));
-    const bool pair = elem != kElemF32 && use_pairs(n, E, quant_mode, wide_tiles);
+    const int kb_count = ceil_div(K * esz, kBKBytes);
+    const TileForm form = tile_form(n, E, quant_mode, elem, wide_tiles, kb_count);
     // measured on decode shapes: 128-column tiles win when 256-column tiles would fill at most half of
     // the SMs, or when there are at most two row tiles (one or two tokens); otherwise 256 columns win
-    const bool narrow = quant_mode != DQMOE_QUANT_FP8_BLOCK && !pair && elem != kElemF32 &&
+    const bool narrow = quant_mode != DQMOE_QUANT_FP8_BLOCK && form == kSingles && elem != kElemF32 &&
                         (2 * wide_tiles <= sm_count() || (mtiles_max <= 2 && wide_tiles < 2 * sm_count()));
     const int box = narrow ? 64 : kBoxRows;
 
@@ -929,7 +958,8 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
     p.n_tiles = gated ? ceil_div(N, box) : ceil_div(N, 2 * box);
     p.tile_w_rows = gated ? box : 2 * box;
     p.box2_off = gated ? N : box;
-    p.kb_count = ceil_div(K * esz, kBKBytes);
+    p.kb_count = kb_count;
+    p.by_counts = form == kByCounts ? 1 : 0;
     p.offsets = offsets;
     p.mtile_prefix = mtile_prefix;
     p.sa = a_scale;
@@ -951,25 +981,25 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
     rc = make_map(&mb, w, esz, uint64_t(E) * p.w_rows, uint64_t(K), box);
     if (rc != DQMOE_OK) return rc;
 
-#define DQ_GEMM_LAUNCH(FP8, MODE, PAIR, BOX)                                                 \
-    (gated ? launch<FP8, MODE, true, PAIR, BOX>(ma, mb, p, stream) : launch<FP8, MODE, false, PAIR, BOX>(ma, mb, p, stream))
-#define DQ_GEMM_CASE(FP8, MODE)                                                              \
-    return pair ? DQ_GEMM_LAUNCH(FP8, MODE, true, 128)                                        \
-                : (narrow ? DQ_GEMM_LAUNCH(FP8, MODE, false, 64) : DQ_GEMM_LAUNCH(FP8, MODE, false, 128))
-#define DQ_GEMM_LAUNCH_F16(PAIR, BOX)                                                          \
-    (gated ? launch<false, kNone, true, PAIR, BOX, kElemHalf>(ma, mb, p, stream)                   \
-           : launch<false, kNone, false, PAIR, BOX, kElemHalf>(ma, mb, p, stream))
-    if (elem == kElemHalf)
-        return pair ? DQ_GEMM_LAUNCH_F16(true, 128) : (narrow ? DQ_GEMM_LAUNCH_F16(false, 64) : DQ_GEMM_LAUNCH_F16(false, 128));
-#undef DQ_GEMM_LAUNCH_F16
+#define DQ_GEMM_LAUNCH(FP8, MODE, PAIR, BOX, ELEM)                                           \
+    (gated ? launch<FP8, MODE, true, PAIR, BOX, ELEM>(ma, mb, p, stream)                      \
+           : launch<FP8, MODE, false, PAIR, BOX, ELEM>(ma, mb, p, stream))
+#define DQ_GEMM_CASE(FP8, MODE, ELEM)                                                        \
+    do {                                                                                     \
+        if (narrow) return DQ_GEMM_LAUNCH(FP8, MODE, false, 64, ELEM);                        \
+        if (form != kPairs) rc = DQ_GEMM_LAUNCH(FP8, MODE, false, 128, ELEM);                 \
+        if (form != kSingles && rc == DQMOE_OK) rc = DQ_GEMM_LAUNCH(FP8, MODE, true, 128, ELEM); \
+        return rc;                                                                           \
+    } while (0)
+    if (elem == kElemHalf) DQ_GEMM_CASE(false, kNone, kElemHalf);
     if (elem == kElemF32)
         return gated ? launch<false, kNone, true, false, 128, kElemF32>(ma, mb, p, stream)
                      : launch<false, kNone, false, false, 128, kElemF32>(ma, mb, p, stream);
     switch (quant_mode) {
-        case DQMOE_QUANT_NONE: DQ_GEMM_CASE(false, kNone);
-        case DQMOE_QUANT_FP8_TENSOR: DQ_GEMM_CASE(true, kTensor);
-        case DQMOE_QUANT_FP8_CHANNEL: DQ_GEMM_CASE(true, kChannel);
-        default: return DQ_GEMM_LAUNCH(true, kBlock, false, 128);
+        case DQMOE_QUANT_NONE: DQ_GEMM_CASE(false, kNone, kElemBf16);
+        case DQMOE_QUANT_FP8_TENSOR: DQ_GEMM_CASE(true, kTensor, kElemBf16);
+        case DQMOE_QUANT_FP8_CHANNEL: DQ_GEMM_CASE(true, kChannel, kElemBf16);
+        default: return DQ_GEMM_LAUNCH(true, kBlock, false, 128, kElemBf16);
     }
 #undef DQ_GEMM_CASE
 #undef DQ_GEMM_LAUNCH

@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import os
+import re
 
 import numpy as np
 import torch
@@ -41,15 +42,64 @@ def bits(t: torch.Tensor) -> np.ndarray:
     return t.numpy()
 
 
-def kernels_of(fn):
-    """Names of the CUDA kernels that fn() launches, in order of their start. The profiler now and then comes back empty from a
-    short session; fn() is then called again."""
-    for _ in range(5):
-        torch.cuda.synchronize()
-        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+def _drv(result):
+    err, rest = result[0], result[1:]
+    assert int(err) == 0, err
+    return rest[0] if len(rest) == 1 else rest
+
+
+def _captured(fn):
+    """(graph, [(node, kernel name)]) of what fn() launches on the current stream; nothing is executed."""
+    from cuda.bindings import driver as drv
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        _drv(drv.cuStreamBeginCapture(stream.cuda_stream, drv.CUstreamCaptureMode.CU_STREAM_CAPTURE_MODE_RELAXED))
+        try:
             fn()
-            torch.cuda.synchronize()
-        events = [e for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
-        if events:
-            break
-    return [e.name for e in sorted(events, key=lambda e: e.time_range.start)]
+        finally:
+            graph = _drv(drv.cuStreamEndCapture(stream.cuda_stream))
+    count = _drv(drv.cuGraphGetNodes(graph))[1]
+    kernels = []
+    for node in _drv(drv.cuGraphGetNodes(graph, count))[0]:
+        if _drv(drv.cuGraphNodeGetType(node)) == drv.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            par = _drv(drv.cuGraphKernelNodeGetParams(node))
+            name = _drv(drv.cuFuncGetName(par.func)) if int(par.func) else _drv(drv.cuKernelGetName(par.kern))
+            kernels.append((node, name.decode()))
+    return graph, kernels
+
+
+def kernels_of(fn):
+    """Mangled names of the CUDA kernels that fn() launches on the current stream, by capturing them; nothing is executed."""
+    from cuda.bindings import driver as drv
+    graph, kernels = _captured(fn)
+    _drv(drv.cuGraphDestroy(graph))
+    return [name for _, name in kernels]
+
+
+def run_kernels(fn, keep):
+    """Executes those of fn()'s kernels whose name keep() accepts, and nothing else of fn()."""
+    from cuda.bindings import driver as drv
+    graph, kernels = _captured(fn)
+    for node, name in kernels:
+        if not keep(name):
+            _drv(drv.cuGraphDestroyNode(node))
+    runnable = _drv(drv.cuGraphInstantiate(graph, 0))
+    _drv(drv.cuGraphLaunch(runnable, torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    _drv(drv.cuGraphExecDestroy(runnable))
+    _drv(drv.cuGraphDestroy(graph))
+
+
+def tile_form(kernel_name):
+    """"pairs", "wide" or "narrow" for a grouped GEMM of gemm_sm100.cu, by the template arguments in its mangled name <fp8, mode,
+    gated, pair, rows per weight box, element>; None for any other kernel."""
+    m = re.search(r"GemmUniversal_tcgen05ILb\dELi\dELb\dELb(\d)ELi(\d+)ELi\dE", kernel_name)
+    if m is None:
+        return None
+    return "pairs" if m.group(1) == "1" else {"128": "wide", "64": "narrow"}[m.group(2)]
+
+
+def tile_forms(fn):
+    """Tile forms of the grouped GEMMs that fn() launches, in order."""
+    return [f for f in map(tile_form, kernels_of(fn)) if f is not None]

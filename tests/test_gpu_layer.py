@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import moe_test
-from helpers import bf16_from_bits, bits, golden, make_inputs
+from helpers import bf16_from_bits, bits, golden, make_inputs, tile_forms
 from oracle import moe_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -149,7 +149,7 @@ def test_errors_raise_runtime_error(ops, workspace):
 
 
 RAGGED = [0, 1, 127, 128, 129, 0, 300, 5]
-# mean rows per expert >= 512: the non-block modes run on CTA pairs (256-row tiles, odd tile counts included)
+# mean rows per expert >= 512 in a small launch: the non-block modes run on CTA pairs (256-row tiles, odd tile counts included)
 LARGE = [641, 0, 1300, 129]
 
 
@@ -157,10 +157,12 @@ LARGE = [641, 0, 1300, 129]
 MANY = [200, 131, 0, 256, 77, 300, 128, 129, 1, 255, 190, 260, 140, 222, 180, 250]
 
 
-@pytest.mark.parametrize("counts,N,K", [(RAGGED, 384, 640), (LARGE, 384, 640), (MANY, 1280, 256)],
-                         ids=["ragged-narrow", "pairs", "many-wide"])
+GROUPS = [(RAGGED, 384, 640, "narrow"), (LARGE, 384, 640, "pairs"), (MANY, 1280, 256, "wide")]
+
+
+@pytest.mark.parametrize("counts,N,K,form", GROUPS, ids=["ragged-narrow", "pairs", "many-wide"])
 @pytest.mark.parametrize("mode,gated", [(0, False), (0, True), (256, True), (512, False), (512, True), (1024, False), (1024, True)])
-def test_grouped_gemm_ragged_groups(ops, mode, gated, counts, N, K):
+def test_grouped_gemm_ragged_groups(ops, mode, gated, counts, N, K, form):
     """dqmoe_grouped_gemm alone on ragged expert sizes (0, 1, 127, 128, 129 rows ...); the three
     shape sets reach the three tile configurations (128-column, CTA-pair and 256-column tiles)."""
     E = len(counts)
@@ -212,6 +214,9 @@ def test_grouped_gemm_ragged_groups(ops, mode, gated, counts, N, K):
         out = torch.zeros(n, N, dtype=torch.bfloat16, device=DEV)
         ops.grouped_gemm(dev(aq), dev(asc), dev(wq), dev(wsc), off_d, mt, N, mode, False, out)
         got, want = out.cpu().float(), ref
+    if mode != 1024:
+        args = (dev(aq), dev(asc), dev(wq), dev(wsc), off_d, mt, N, mode, gated, out)
+        assert tile_forms(lambda: ops.grouped_gemm(*args, amax=amax if gated and mode else None)) == [form]
     assert ops.device_status() == 0
     # one e4m3 step of the re-quantised output at the largest magnitude is 1/16 of it: the layer tolerance applies
     assert orc.cosine(got, want) >= 0.9999 and orc.max_rel_err(got, want) <= REL_MAX
@@ -230,10 +235,9 @@ def test_profiler_sees_the_kernel_names_the_reference_script_filters_on(ops, wor
     assert gemm, names
 
 
-@pytest.mark.parametrize("counts,N,K", [(RAGGED, 384, 640), (LARGE, 384, 640), (MANY, 1280, 256)],
-                         ids=["ragged-narrow", "pairs", "many-wide"])
+@pytest.mark.parametrize("counts,N,K,form", GROUPS, ids=["ragged-narrow", "pairs", "many-wide"])
 @pytest.mark.parametrize("mode", [0, 512, 1024])
-def test_grouped_gemm_row_addresses_equal_scatter_map(ops, mode, counts, N, K):
+def test_grouped_gemm_row_addresses_equal_scatter_map(ops, mode, counts, N, K, form):
     """dqmoe_grouped_gemm_rows (stage 2 storing each row to an explicit address, the path the
     expert-parallel layer uses to write into peer memory) against the same GEMM with a scatter map."""
     import ctypes
@@ -262,8 +266,10 @@ def test_grouped_gemm_row_addresses_equal_scatter_map(ops, mode, counts, N, K):
     row_dst = torch.where(perm >= 0, got.data_ptr() + perm.to(torch.int64) * (N * 2), torch.zeros((), dtype=torch.int64, device=DEV))
     p = lambda t: None if t is None else ctypes.c_void_p(t.data_ptr())
     lib = _lib.load()
-    _lib.check(lib.dqmoe_grouped_gemm_rows(p(aq), p(asc), p(wq), p(wsc), p(offsets), p(mt), n, N, K, E, mode,
-                                           p(row_dst), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    call = lambda: _lib.check(lib.dqmoe_grouped_gemm_rows(p(aq), p(asc), p(wq), p(wsc), p(offsets), p(mt), n, N, K, E, mode,
+                                                          p(row_dst), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    call()
+    assert mode == 1024 or tile_forms(call) == [form]
     assert ops.device_status() == 0
     assert torch.equal(got, want)
 
@@ -289,18 +295,19 @@ def test_moe_block_router_to_weighted_output(ops, mode, scoring):
     assert_close(out, ref)
 
 
-@pytest.mark.parametrize("E,T,H,I,k", [(8, 64, 1024, 2048, 2), (8, 300, 512, 384, 3), (4, 2000, 512, 256, 1), (3, 5, 192, 160, 2)])
+@pytest.mark.parametrize("E,T,H,I,k", [(8, 64, 1024, 2048, 2), (8, 300, 512, 384, 3), (4, 2400, 512, 256, 1), (3, 5, 192, 160, 2)])
 def test_layer_fp16_operands(ops, workspace, E, T, H, I, k):
     """dqmoe_moe_forward_f16: fp16 activations, weights and output against the oracle's layer run on fp16
-    tensors (torch_moe_grouped of test/util.py:71-92 is dtype-generic). Includes the 2000-row-per-expert case
-    that takes the CTA-pair tiles and a ragged one."""
+    tensors (torch_moe_grouped of test/util.py:71-92 is dtype-generic). Includes a case of 600 rows per
+    expert, which takes the CTA-pair tiles, and a ragged one."""
     a, b, b1, _, m_indices = make_inputs(23, T, H, I, E, k, 1.0, 0.05)
     a, b, b1 = a.half(), b.half(), b1.half()
     ref = orc.moe_layer_bf16(a, b, b1, m_indices, E)
     assert ref.dtype == torch.float16
     d = torch.zeros(T, k, H, dtype=torch.float16, device=DEV)
-    ops.moe_forward_f16(a.to(DEV), b.to(DEV), b1.to(DEV), d, m_indices.to(DEV), workspace)
-    torch.cuda.synchronize()
+    args = (a.to(DEV), b.to(DEV), b1.to(DEV), d, m_indices.to(DEV), workspace)
+    ops.moe_forward_f16(*args)
+    assert ("pairs" in tile_forms(lambda: ops.moe_forward_f16(*args))) == (T == 2400)
     assert ops.device_status() == 0
     assert_close(d, ref)
     # fp16 has three more mantissa bits than bf16: the result must be closer to the oracle than a bf16 run is

@@ -116,15 +116,16 @@ def test_128x128_quantiser_bit_exact(ops, E, rows, cols):
 def test_1x128_quantiser_takes_strips_for_rows_that_fill_them(ops, rows, cols, strips):
     g = torch.Generator().manual_seed(cols)
     x = torch.randn(rows, cols, generator=g).to(torch.bfloat16)
-    xd, out = x.to(DEV), []
-    names = kernels_of(lambda: out.append(ops.per_token_block_cast_to_fp8(xd)))
+    xd = x.to(DEV)
+    names = kernels_of(lambda: ops.per_token_block_cast_to_fp8(xd))
     assert any("scatter_quant" in n for n in names) == strips, names
     q, s = orc.quant_block_1x128(x)
-    assert np.array_equal(bits(out[0][1]), bits(s)) and np.array_equal(bits(out[0][0]), bits(q))
+    qd, sd = ops.per_token_block_cast_to_fp8(xd)
+    assert np.array_equal(bits(sd), bits(s)) and np.array_equal(bits(qd), bits(q))
 
 
 @pytest.mark.parametrize("k", [1, 3, 5, 6, 7, 8, 9])
 def test_combine_batches_as_many_slots_as_there_are(ops, k):
     d, w = torch.randn(33, k, 264, device=DEV).to(torch.bfloat16), torch.rand(33, k, device=DEV)
     names = kernels_of(lambda: ops.finalize_weighted(d, w))
-    assert any(f"finalize_weighted_kernel<{4 if k == 3 else min(k, 8)}>" in n for n in names), names
+    assert any(f"finalize_weighted_kernelILi{4 if k == 3 else min(k, 8)}E" in n for n in names), names

@@ -1,57 +1,123 @@
-"""CTA pairs against single CTAs: row counts on both sides of the lines of the rule that chooses them, checked against the
-oracle, and a small batch bit-identical to its rows of the full one (the choice must not show in the results)."""
+"""Which tile form the grouped GEMM runs on - single CTAs, CTA pairs, chosen on the host or from the experts' row counts on the
+device - and that the choice does not show in the results; block scales by tile likewise."""
+import numpy as np
 import pytest
 import torch
 
-from helpers import kernels_of
+from helpers import kernels_of, run_kernels, tile_form, tile_forms
 from oracle import moe_oracle as orc
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
+# rows of eight experts (128 to 800 on average), the form that suits them: 2 x 256-row tiles against 1.16 x 128-row tiles
+COUNTS = {
+    "even-two-tiles": ([200] * 8, "pairs"),  # 16 against 16
+    "ragged-two-tiles": ([129, 255, 256, 130, 200, 0, 240, 129], "pairs"),
+    "odd-three-tiles": ([300] * 8, "wide"),  # 32 against 24
+    "skewed": ([1400, 20, 10, 0, 130, 64, 1, 33], "wide"),  # 24 against 18, 207 rows on average
+    "one-for-all": ([800, 90, 100, 120, 80, 70, 128, 60], "wide"),  # 22 against 14
+    "below-the-line": ([300, 400, 600, 0, 200, 700, 10, 640], "pairs"),  # 30 against 26
+    "above-the-line": ([300, 400, 600, 0, 300, 700, 10, 640], "wide"),  # 32 against 27
+}
 
-@pytest.mark.parametrize("mode", [0, 256, 512])
-@pytest.mark.parametrize("rows", [128, 129, 200, 240, 241, 385, 560])
-def test_layer_on_both_sides_of_the_pair_rule(mode, rows):
+
+@pytest.mark.parametrize("case", list(COUNTS))
+@pytest.mark.parametrize("mode,gated", [(0, True), (0, False), (256, True), (256, False), (512, True), (512, False)])
+def test_row_counts_choose_the_tile_form(mode, gated, case):
+    """The form that works is the one that suits the counts; every row is bit-identical to the same row in a launch of a few
+    rows per expert, which takes single CTAs, and four rows of every expert agree with fp64 sums."""
     from dqmoe_b200 import ops
-    E, H, I = 3, 128, 8192 if rows < 300 else 6144
-    T = E * rows
-    g = torch.Generator(device=DEV).manual_seed(rows)
-    a = torch.randn(T, H, generator=g, device=DEV).to(torch.bfloat16)
-    b = (torch.randn(E, 2 * I, H, generator=g, device=DEV) * 0.05).to(torch.bfloat16)
-    b1 = (torch.randn(E, H, I, generator=g, device=DEV) * 0.05).to(torch.bfloat16)
-    ids = (torch.arange(T, dtype=torch.int32) % E).view(T, 1)
-    ids[:40] = 0  # ragged experts
-    qs = (a, None, b, None, b1, None)
+    counts, form = COUNTS[case]
+    E, n = len(counts), sum(counts)
+    K, N = (2048 if mode == 0 else 4096), (8192 if gated else 16384)  # 32 K blocks, 64 column tiles: 30000 from 15 row tiles on
+    g = torch.Generator(device=DEV).manual_seed(n + mode)
+    a = torch.randn(n, K, generator=g, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(E, (2 if gated else 1) * N, K, generator=g, device=DEV) * 0.05).to(torch.bfloat16)
     if mode == 256:
-        qs = (*ops.per_tensor_cast_to_fp8(a), *ops.per_tensor_cast_to_fp8(b, per_expert=True), *ops.per_tensor_cast_to_fp8(b1, per_expert=True))
+        (a, sa), (w, sw) = ops.per_tensor_cast_to_fp8(a), ops.per_tensor_cast_to_fp8(w, per_expert=True)
     elif mode == 512:
-        qs = (*ops.per_token_cast_to_fp8(a), *ops.per_channel_cast_to_fp8(b), *ops.per_channel_cast_to_fp8(b1))
-
-    def run(x, xs, idx):
-        n = idx.shape[0]
-        d = torch.zeros(n, 1, H, dtype=torch.bfloat16, device=DEV)
-        ws = torch.empty(ops.moe_workspace_bytes(n, H, I, E, 1, mode), dtype=torch.uint8, device=DEV)
-        ops.moe_forward(x, xs, *qs[2:], d, idx.to(DEV), ws, mode)
-        assert ops.device_status() == 0
-        return d.cpu()
-
-    full = run(qs[0], qs[1], ids)
-    sample = torch.arange(0, T, max(1, T // 48))
-    xs = qs[1] if qs[1] is None or qs[1].numel() == 1 else qs[1].reshape(T, -1)[sample.to(DEV)].contiguous()
-    small = run(qs[0].view(torch.uint8).reshape(T, -1)[sample.to(DEV)].contiguous().view(qs[0].dtype).view(len(sample), H), xs, ids[sample])
-    if mode != 256:  # the intermediate's per-tensor scale depends on the batch
-        assert torch.equal(full[sample], small)
-    ws8 = [t.cpu() if t is not None else None for t in qs]
-    if mode == 0:
-        ref = orc.moe_layer_bf16(ws8[0][sample], ws8[2], ws8[4], ids[sample], E)
-    elif mode == 512:
-        ref = orc.moe_layer_fp8(ws8[0][sample], ws8[1].reshape(T, -1)[sample], *ws8[2:], ids[sample], E, mode)
+        (a, sa), (w, sw) = ops.per_token_cast_to_fp8(a), ops.per_channel_cast_to_fp8(w)
     else:
-        ref = orc.moe_layer_fp8(ws8[0][sample], ws8[1], *ws8[2:], ids[sample], E, mode)
-    # the layer tolerance; per-tensor mode: the sample's own intermediate scale, so the small batch is the one compared
-    got = small if mode == 256 else full[sample]
-    assert orc.cosine(got, ref) >= 0.999 and orc.max_rel_err(got, ref) <= 2e-2
+        sa = sw = None
+
+    def run(rows_of):  # rows_of[e]: rows of expert e, as indices into the full batch
+        rows = torch.cat(rows_of).to(DEV)
+        off = torch.tensor(np.concatenate([[0], np.cumsum([len(r) for r in rows_of])]), dtype=torch.int32, device=DEV)
+        ar = a.view(torch.uint8).view(n, -1)[rows].contiguous().view(a.dtype).view(len(rows), K)
+        sr = sa if mode != 512 else sa.view(n, 1)[rows].contiguous()
+        out = torch.zeros(len(rows), N, dtype=torch.bfloat16, device=DEV)
+        amax = torch.zeros(len(rows) if mode == 512 else 1, device=DEV) if gated and mode else None
+        mt = ops.mtile_prefix(off)
+        call = lambda o, m: ops.grouped_gemm(ar, sr, w, sw, off, mt, N, mode, gated, o, amax=m)
+        call(out, amax)
+        # of the launched forms those that write something when they run alone
+        working = []
+        for f in tile_forms(lambda: call(out, amax)):
+            alone, spare = torch.zeros_like(out), None if amax is None else torch.zeros_like(amax)
+            run_kernels(lambda: call(alone, spare), lambda name: tile_form(name) == f)
+            if alone.any():
+                working.append(f)
+                assert torch.equal(alone, out)
+        assert ops.device_status() == 0
+        return out, amax, working
+
+    first = np.concatenate([[0], np.cumsum(counts)])
+    every = [torch.arange(first[e], first[e + 1]) for e in range(E)]
+    out, amax, forms = run(every)
+    assert forms == [form], forms
+    few = [r[torch.linspace(0, len(r) - 1, min(len(r), 60)).long()] if len(r) else r for r in every]
+    small, amax_small, forms = run(few)
+    assert forms == ["wide"], forms
+    picked = torch.cat(few).to(DEV)
+    assert torch.equal(out[picked], small)
+    if mode == 512 and gated:
+        assert torch.equal(amax[picked], amax_small)
+        assert torch.equal(amax, out.float().abs().amax(1))
+    if mode == 256 and gated:
+        assert amax.item() == out.float().abs().max().item()
+    for e in range(E):
+        r = few[e][:: max(1, len(few[e]) // 4)].to(DEV)
+        if not len(r):
+            continue
+        x, y = a[r].double(), w[e].double()
+        if mode == 256:
+            x, y = x * sa.double(), y * sw[e].double()
+        elif mode == 512:
+            x, y = x * sa.view(n, 1)[r].double(), y * sw[e].double()
+        ref = x @ y.t()
+        if gated:
+            gate, val = ref.float().to(torch.bfloat16).chunk(2, dim=-1)
+            ref = (torch.nn.functional.silu(gate) * val).double()
+        # A flipped rounding of value, silu or product is 2^-8 of the result each, one of the gate |g| + 1 times as much (d ln
+        # silu / d ln g = 1 + g (1 - sigmoid)): 2^-5 in all up to |g| = 5, beyond which silu is below 0.034 of a typical gate
+        assert ((out[r].double() - ref).abs() <= 2.0 ** -5 * ref.abs() + 2.0 ** -6 * ref.abs().mean()).all()
+
+
+@pytest.mark.parametrize("counts,N,K,launched,form", [
+    ([127] * 8, 16384, 4096, "one", "wide"), ([256, 0] * 4, 16384, 4096, "both", "pairs"),  # from 128 rows on average: by counts
+    ([200] * 8, 4096, 4096, "one", "wide"), ([511] * 8, 1024, 512, "one", "wide"), ([512] * 8, 1024, 512, "one", "pairs"),  # small
+    ([896] * 4 + [640] * 4, 16384, 2048, "both", "wide"),  # 56 against 48
+    ([800] * 8, 16384, 2048, "one", "pairs"), ([2000] * 4 + [1] * 4 + [0], 16384, 2048, "one", "pairs")])  # from 800 on
+def test_lines_of_the_host_rule(counts, N, K, launched, form):
+    """Average row counts and sizes on both sides of the lines between which the device chooses."""
+    from dqmoe_b200 import ops
+    E = len(counts)
+    n = sum(counts)
+    a = torch.zeros(n, K, dtype=torch.uint8, device=DEV).view(ops.FP8)
+    w = torch.zeros(E, N, K, dtype=torch.uint8, device=DEV).view(ops.FP8)
+    off = torch.tensor(np.concatenate([[0], np.cumsum(counts)]), dtype=torch.int32, device=DEV)
+    out = torch.ones(n, N, dtype=torch.bfloat16, device=DEV)
+    sa, sw, mt = torch.ones(1, device=DEV), torch.ones(E, device=DEV), ops.mtile_prefix(off)
+    call = lambda: ops.grouped_gemm(a, sa, w, sw, off, mt, N, 256, False, out)
+    forms = tile_forms(call)
+    if launched == "both":
+        assert forms == ["wide", "pairs"], forms
+        run_kernels(call, lambda name: tile_form(name) == form)
+    else:
+        assert forms == [form], forms
+        call()
+    assert ops.device_status() == 0 and not out.any()
 
 
 @pytest.mark.parametrize("T,k,E,H,I", [(8192, 2, 24, 2064, 2064), (7000, 1, 5, 2048, 4368)])
@@ -75,8 +141,9 @@ def test_block_scales_by_tile(T, k, E, H, I):
         ws = torch.empty(ops.moe_workspace_bytes(n, H, I, E, k, 1024), dtype=torch.uint8, device=DEV)
         qr = q.view(torch.uint8)[rows.to(DEV)].contiguous().view(q.dtype)
         sr, idr = s[rows.to(DEV)].contiguous(), ids[rows].contiguous().to(DEV)
-        names = kernels_of(lambda: ops.moe_forward(qr, sr, *b, *b1, d, idr, ws, 1024))
+        ops.moe_forward(qr, sr, *b, *b1, d, idr, ws, 1024)
         assert ops.device_status() == 0
+        names = kernels_of(lambda: ops.moe_forward(qr, sr, *b, *b1, d, idr, ws, 1024))
         assert any("scale_tiles" in n for n in names) == tiled, names
         return d.cpu()
 
@@ -100,6 +167,7 @@ def test_scales_are_laid_out_by_tile_where_it_pays(n, H, I, E, tiled):
     ids = (torch.arange(n, device=DEV, dtype=torch.int32) % E).view(n, 1)
     ws = torch.empty(ops.moe_workspace_bytes(n, H, I, E, 1, 1024), dtype=torch.uint8, device=DEV)
     args = (z(n, H), one(n, g(H)), z(E, 2 * I, H), one(E, g(2 * I), g(H)), z(E, H, I), one(E, g(H), g(I)), d, ids, ws, 1024)
-    names = kernels_of(lambda: ops.moe_forward(*args))
+    ops.moe_forward(*args)
     assert ops.device_status() == 0 and not d.any()
+    names = kernels_of(lambda: ops.moe_forward(*args))
     assert any("scale_tiles" in k for k in names) == tiled, names
