@@ -171,3 +171,34 @@ def test_scales_are_laid_out_by_tile_where_it_pays(n, H, I, E, tiled):
     assert ops.device_status() == 0 and not d.any()
     names = kernels_of(lambda: ops.moe_forward(*args))
     assert any("scale_tiles" in k for k in names) == tiled, names
+
+
+@pytest.mark.parametrize("n_shared", [0, 1])
+def test_block_entry_point_with_scales_by_tile(n_shared):
+    """The whole MoE block lays its own workspace out and quantises on the way into expert order: with enough K blocks its scales
+    go by tile too. Sampled tokens are bit-identical to a small call and agree with the oracle."""
+    from dqmoe_b200 import ops
+    T, k, E, H, I = 8200, 2, 7, 2048, 2064
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x = torch.randn(T, H, generator=g, device=DEV).to(torch.bfloat16)
+    b = ops.per_block_cast_to_fp8((torch.randn(E + n_shared, 2 * I, H, generator=g, device=DEV) * 0.05).to(torch.bfloat16))
+    b1 = ops.per_block_cast_to_fp8((torch.randn(E + n_shared, H, I, generator=g, device=DEV) * 0.05).to(torch.bfloat16))
+    logits = torch.randn(T, E, generator=g, device=DEV)
+    logits[:, 1] += 3.0  # skewed, and one expert without rows
+    logits[:, 4] = -100.0
+
+    def run(rows, tiled):
+        args = (x[rows].contiguous(), logits[rows].contiguous(), *b, *b1, k, "sigmoid", 1024)
+        out = ops.moe_block(*args, n_shared=n_shared)
+        assert ops.device_status() == 0
+        names = kernels_of(lambda: ops.moe_block(*args, n_shared=n_shared))
+        assert any("scale_tiles" in n for n in names) == tiled, names
+        return out.cpu()
+
+    sample = torch.arange(0, T, 173)
+    full, small = run(torch.arange(T, device=DEV), True), run(sample.to(DEV), False)
+    assert torch.equal(full[sample], small)
+    xs = x.cpu()[sample]
+    ref = orc.moe_block(xs, logits.cpu()[sample], b[0].cpu(), b1[0].cpu(), k, "sigmoid", 1024, n_shared=n_shared,
+                        quantized=(*orc.quant_block_1x128(xs), *[t.cpu() for t in b], *[t.cpu() for t in b1]))
+    assert orc.cosine(small, ref) >= 0.999 and orc.max_rel_err(small, ref) <= 2e-2
