@@ -67,12 +67,15 @@ constexpr int kAmaxParts = 4096;  // floats the layer workspace holds for the pe
 // (the grouped GEMMs set up their barriers and TMEM in between): the next kernel's blocks may become resident while this
 // one runs, and no thread touches global memory before all earlier kernels of the stream have completed. What such a kernel
 // reads may therefore still be written while it is resident: its pointers are not __restrict__ and its loads are plain ones
-// (ld_stream16). Between the short
-// kernels of the layer the gap shrinks from ~2 us to below 1 us (MoE block of 5 tokens, H 1024, I 2048: 45.8 -> 34.6 us).
-// The grouped GEMMs are launched this way up to kPdlGemmRows rows only. Their blocks, one per SM, would otherwise take the
-// SMs in the order in which the kernel before leaves them instead of in the launch order, which spreads the blocks that
-// share a weight tile over both dies: 4096 tokens x 2, block FP8 1886 -> 1959 us, 8192 x 8 5312 -> 6088 us; with some
-// hundred rows nothing is shared and the gap counts (864 rows: 330 -> 326 us, 32 rows: 254 -> 245 us).
+// (ld_stream16). Between the short kernels of the layer the gap shrinks from ~2 us to below 1 us (MoE block of 5 tokens, H 1024,
+// I 2048: 45.8 -> 34.6 us).
+// The grouped GEMMs are launched this way up to kPdlGemmRows rows only. Their blocks, one per SM, otherwise take the SMs in the
+// order in which the kernel before leaves them instead of in the launch order, which spreads the blocks that share a weight
+// tile over both dies: 4096 tokens x 2, block FP8 1886 -> 1959 us, 8192 x 8 5312 -> 6088 us. Up to some 2000 rows little is shared
+// and the gap counts (layer calls, without / with: H 1024, I 2048, E 4, 512 rows 31 / 27 us, 2048 rows 41 / 36; H 4096, I 14336,
+// E 8, 864 rows 276 / 272, 2048 rows 456 / 453; H 7168, I 2048, E 32, 2048 rows 292 / 289). In between it goes either way: with
+// 128 small experts (H 2048, I 768) 2048 rows cost 141 / 147 in MXFP8, 157 / 159 in block FP8 and 153 / 152 per-channel, 4096 rows of
+// the large models 974 / 981 in block FP8 and 804 / 795 per-channel.
 constexpr int kPdlGemmRows = 2048;
 template <class... KArgs, class... Args>
 static inline int launch_pdl(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
