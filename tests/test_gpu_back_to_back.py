@@ -126,3 +126,53 @@ def weights_nvfp4(ops):
     g = torch.Generator(device=DEV).manual_seed(9)
     return [ops.nvfp4_cast_weights((torch.randn(E, r, c, generator=g, device=DEV) * 0.05).to(torch.bfloat16))
             for r, c in ((1024, H), (H, 512))]
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("kind", ["bf16", "tensor", "channel", "block", "mx"])
+def test_two_streams_with_a_workspace_each(ops, kind, captured):
+    """A program that forks: one stream quantises and runs a layer, another waits for an event and runs its own, both join and
+    the results are added; eagerly and as a captured graph whose launches cross streams."""
+    w = weights(ops, kind)
+    side, main = torch.cuda.Stream(), torch.cuda.Stream()
+    (x0, _, i0), (x1, _, i1) = inputs(11, 300), inputs(12, 300)
+    ws = [torch.empty(ops.moe_workspace_bytes(300, H, I, E, K, MODE[kind]), dtype=torch.uint8, device=DEV) for _ in range(2)]
+    want = []
+    for x, i in ((x0, i0), (x1, i1)):
+        d = torch.zeros(300, K, H, dtype=torch.bfloat16, device=DEV)
+        layer_call(ops, kind, w, x, i, d, ws[0])
+        torch.cuda.synchronize()
+        want.append(d)
+    d0, d1 = torch.zeros_like(want[0]), torch.zeros_like(want[0])
+    keep = []
+
+    def step():
+        scaled = x1 * 2.0  # work in front of the fork that the other stream must wait for
+        halved = scaled * 0.5
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            layer_call(ops, kind, w, halved, i1, d1, ws[1])
+        layer_call(ops, kind, w, x0, i0, d0, ws[0])
+        main.wait_stream(side)
+        keep.append((scaled, halved))
+        return d0 + d1
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(main):
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=main):
+                total = step()
+            for _ in range(5):
+                d0.zero_()
+                d1.zero_()
+                graph.replay()
+        else:
+            for _ in range(5):
+                d0.zero_()
+                d1.zero_()
+                total = step()
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    assert torch.equal(d0, want[0]) and torch.equal(d1, want[1])
+    assert torch.equal(total, want[0] + want[1])
