@@ -1,5 +1,7 @@
 """Which tile form the grouped GEMM runs on - single CTAs, CTA pairs, chosen on the host or from the experts' row counts on the
 device - and that the choice does not show in the results; block scales by tile likewise."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -27,7 +29,7 @@ COUNTS = {
 def test_row_counts_choose_the_tile_form(mode, gated, case):
     """The form that works is the one that suits the counts; every row is bit-identical to the same row in a launch of a few
     rows per expert, which takes single CTAs, and four rows of every expert agree with fp64 sums."""
-    from dqmoe_b200 import ops
+    from dqmoe_b200 import _lib, ops
     counts, form = COUNTS[case]
     E, n = len(counts), sum(counts)
     K, N = (2048 if mode == 0 else 4096), (8192 if gated else 16384)  # 32 K blocks, 64 column tiles: 30000 from 15 row tiles on
@@ -71,6 +73,17 @@ def test_row_counts_choose_the_tile_form(mode, gated, case):
     assert forms == ["wide"], forms
     picked = torch.cat(few).to(DEV)
     assert torch.equal(out[picked], small)
+    if not gated:  # the same rows to explicit addresses, as an expert-parallel rank stores them
+        perm = torch.randperm(n, generator=g, device=DEV)
+        spread = torch.zeros_like(out)
+        row_dst = spread.data_ptr() + perm * (N * 2)
+        off = torch.tensor(first, dtype=torch.int32, device=DEV)
+        ptr = lambda t: None if t is None else ctypes.c_void_p(t.data_ptr())
+        mt = ops.mtile_prefix(off)
+        _lib.check(_lib.load().dqmoe_grouped_gemm_rows(ptr(a), ptr(sa), ptr(w), ptr(sw), ptr(off), ptr(mt), n, N, K, E, mode,
+                                                       ptr(row_dst), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        assert ops.device_status() == 0
+        assert torch.equal(spread[perm], out)
     if mode == 512 and gated:
         assert torch.equal(amax[picked], amax_small)
         assert torch.equal(amax, out.float().abs().amax(1))
