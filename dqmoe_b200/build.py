@@ -19,7 +19,7 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libdqmoe_b200.so")
 
-SOURCES = ["common.cu", "route.cu", "permute.cu", "quant.cu", "quant_mx.cu", "gemm_sm100.cu", "gemm_mx_sm100.cu", "layer.cu",
+SOURCES = ["common.cu", "route.cu", "permute.cu", "quant.cu", "quant_mx.cu", "gemm_sm100.cu", "gemm_wm_sm100.cu", "gemm_mx_sm100.cu", "layer.cu",
            "ep.cu", "decode.cu", "plugin.cu"]
 
 NVCC_FLAGS = [

@@ -31,6 +31,12 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
 enum Elem : int { kElemBf16 = 0, kElemHalf = 1, kElemF32 = 2 };  // element type of the unquantised path
 }  // namespace gemm
 
+namespace gemm_wm {
+int grouped_gemm(const void* a, const float* a_scale, const void* w, const float* w_scale, const int* offsets, int n, int N, int K,
+                 int E, int quant_mode, int gated, void* out, float* amax, const int* dest_to_src, const float* bias,
+                 cudaStream_t stream);
+}  // namespace gemm_wm
+
 namespace gemm_mx {
 int grouped_gemm_mx(const void* a, const uint8_t* a_sf, const void* w, const uint8_t* w_sf, const int* offsets,
                     const int* mtile_prefix, int n, int N, int K, int E, int gated, void* out, uint8_t* out_sf,
@@ -233,17 +239,24 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
         rc = permute::scale_tiles(perm_a_scale, n, L.perm_scale_cols, offsets, mtile_prefix, E, perm_a_scale_t, stream);
         if (rc != DQMOE_OK) return rc;
     }
-    rc = gemm::grouped_gemm(perm_a, sa1, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1,
-                            two_pass ? act_bf16 : act, act_scale, amax, nullptr, nullptr, stream, elem, bias1, perm_a_scale_t, act_scale_t);
+    const bool wm = quant_mode != DQMOE_QUANT_FP8_BLOCK && elem == gemm::kElemBf16;
+    if (wm)
+        rc = gemm_wm::grouped_gemm(perm_a, sa1, b, b_scale, offsets, n, I, H, E, quant_mode, 1, two_pass ? act_bf16 : act, amax, nullptr,
+                                   bias1, stream);
+    else
+        rc = gemm::grouped_gemm(perm_a, sa1, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, act, act_scale, amax, nullptr,
+                                nullptr, stream, elem, bias1, perm_a_scale_t, act_scale_t);
     if (rc != DQMOE_OK) return rc;
     if (two_pass) {
         rc = dqmoe_requant_from_amax(act_bf16, n, I, amax, quant_mode == DQMOE_QUANT_FP8_CHANNEL ? 1 : 0, act,
                                      act_scale, stream);
         if (rc != DQMOE_OK) return rc;
     }
-    rc = gemm::grouped_gemm(act, act_scale, b1, b1_scale, offsets, mtile_prefix, n, H, I, E, quant_mode, 0, d, nullptr,
-                            nullptr, dest_to_src, nullptr, stream, elem, bias2, act_scale_t);
-    return rc;
+    if (wm)
+        return gemm_wm::grouped_gemm(act, act_scale, b1, b1_scale, offsets, n, H, I, E, quant_mode, 0, d, nullptr, dest_to_src, bias2,
+                                     stream);
+    return gemm::grouped_gemm(act, act_scale, b1, b1_scale, offsets, mtile_prefix, n, H, I, E, quant_mode, 0, d, nullptr, nullptr,
+                              dest_to_src, nullptr, stream, elem, bias2, act_scale_t);
 }
 
 int dqmoe_moe_forward(const void* a, const float* a_scale, const void* b, const float* b_scale, const void* b1,
@@ -453,6 +466,13 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
     else
         rc = permute::scatter_rows(x_bf16, size_t(H) * 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, nullptr, 0, stream);
     if (rc != DQMOE_OK) return rc;
+    if (!fp8) {
+        rc = gemm_wm::grouped_gemm(perm_a, nullptr, b, nullptr, offsets, n, I, H, E, quant_mode, 1, act, nullptr, nullptr, nullptr, stream);
+        if (rc == DQMOE_OK)
+            rc = gemm_wm::grouped_gemm(act, nullptr, b1, nullptr, offsets, n, H, I, E, quant_mode, 0, d, nullptr, dest_to_src, nullptr, stream);
+        if (rc != DQMOE_OK) return rc;
+        return dqmoe_finalize_weighted(d, weights, out_bf16, T, k, H, stream);
+    }
     if (perm_a_scale_t != nullptr) {
         rc = permute::scale_tiles(perm_a_scale, n, L.perm_scale_cols, offsets, mtile_prefix, E, perm_a_scale_t, stream);
         if (rc != DQMOE_OK) return rc;
