@@ -14,6 +14,7 @@
 //
 // Replaces the same reference kernels as gemm_sm100.cu (csrc/moe_gemm_template.h:72-1039, csrc/moe_kernels.h:301-444, 581-620).
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "gemm_tile.cuh"
@@ -24,12 +25,15 @@ namespace gemm_wm {
 
 constexpr int kWRows = 128;                       // weight rows per CTA = lanes of TMEM
 constexpr int kMaxTok = 256;                      // rows of an expert per tile
+constexpr int kBlockTok = 64;                     // the same in block mode
 constexpr int kKBytes = 128;                      // K bytes per stage: one 128-byte swizzle row
 constexpr int kUmmaKBytes = 32;                   // K bytes per tcgen05.mma
 constexpr int kABytes = kWRows * kKBytes;         // 16 KiB
-constexpr int kStageArea = 4 * (kABytes + kMaxTok * kKBytes);
+// Bytes of the stages: four 256-token tiles of a single CTA or six of a pair; in block mode, which needs room for scales and the
+// re-quantisation, seven of 64 tokens, ten of 16.
+constexpr int stage_area(bool block) { return block ? 180 * 1024 : 4 * (kABytes + kMaxTok * kKBytes); }
 constexpr int kMaxStages = 10;
-constexpr int kThreads = 384;                     // warp 0 TMA, warp 1 MMA, warps 2-3 idle, warps 4..11 epilogue
+constexpr int kThreads = 384;                     // warp 0 TMA, warp 1 MMA, warp 2 scale products (block mode), warp 3 idle, warps 4..11 epilogue
 constexpr int kEpiWarps = 8;
 constexpr int kMaxExperts = 1024;
 constexpr int kMaxDevices = 64;
@@ -37,7 +41,7 @@ constexpr int kTmemCols = 512;                    // two accumulator buffers of 
 constexpr int kSub = 16;                          // tokens per pass through the store buffers
 constexpr long long kWaitLimit = 1000000000LL;    // clock cycles before a wait gives up (~0.5 s)
 
-enum Mode : int { kNone = 0, kTensor = 1, kChannel = 2 };
+enum Mode : int { kNone = 0, kTensor = 1, kChannel = 2, kBlock = 3 };
 
 struct Params {
     int n_rows;               // rows of A (expanded rows n)
@@ -47,10 +51,13 @@ struct Params {
     int w_tiles;              // tiles per expert along the output columns
     int kb_count;             // ceil(K bytes / 128)
     const int* offsets;       // [E+1] first row of each expert
-    const float* sa;          // activation scales: tensor [1], channel [n]
-    const float* sb;          // weight scales: tensor [E], channel [E, w_rows]
+    const float* sa;          // activation scales: tensor [1], channel [n], block [ceil(K/128)][n_pad]
+    const float* sb;          // weight scales: tensor [E], channel [E, w_rows], block [E, ceil(w_rows/128), ceil(K/128)]
     void* out;
     float* amax;              // fc1: channel [n], tensor [1]
+    float* out_scale;         // fc1, block mode: [n, ceil(I/128)]
+    float* out_scale_t;       // the same by column, [ceil(I/128)][n_pad]
+    int n_pad;                // rows of the scale matrices by column
     const float* bias;        // [E, w_rows] fp32 added to the dequantised product, or nullptr
     const int* dest_to_src;   // fc2: output row of each row
     int* status;              // host-mapped status word
@@ -61,23 +68,38 @@ struct Maps {
     CUtensorMap rows[4];      // activation rows, boxes of 16, 32, 64 and 128 rows
 };
 
-struct SharedTail {
+constexpr int kProdTok = kTmemCols;               // scale products: one token per accumulator column
+constexpr int kAccBufs = 4;                       // accumulator buffers of block mode, of two or four K blocks each
+
+struct BlockTail {
+    uint64_t prod_empty[kAccBufs];                // the epilogue warps are done with the products of an accumulator buffer
+    // fc1: per pair of tokens the products of their scales with that of the gate rows (x, y) and of the value rows (z, w); the
+    // second array with the value rows' second scale block, where there is one. fc2: one product per token, packed.
+    alignas(16) float prod[2][kProdTok * 2];
+    float amax[2][kBlockTok], inv[kBlockTok];     // fc1: of each token's columns in the tile's first and second half
+};
+struct RowScaleTail {
+    float sa[2][kMaxTok];                         // channel mode: the activation scale of each token of the tile
+};
+
+template <bool kBlockMode>
+struct SharedTail : std::conditional_t<kBlockMode, BlockTail, RowScaleTail> {
     uint64_t full[kMaxStages];
     uint64_t empty[kMaxStages];
-    uint64_t tmem_full[2];
-    uint64_t tmem_empty[2];
+    uint64_t tmem_full[kAccBufs];
+    uint64_t tmem_empty[kAccBufs];
     uint32_t tmem_base;
     int abort_flag;
     int max_tok;                                  // tokens of the largest tile
     unsigned long long dst[2][kMaxTok];           // output row of each token of the tile, 0 = none
-    float sa[2][kMaxTok];                         // its activation scale (channel mode)
     alignas(16) uint4 stage[2][2][kSub * 16];     // per epilogue warpgroup: two buffers of 16 tokens x (64 or 128 columns)
     int tprefix[kMaxExperts + 1];                 // cumulative token tiles
     int offsets[kMaxExperts + 1];
 };
 
-constexpr size_t kSmemBytes = 1024 + size_t(kStageArea) + sizeof(SharedTail);
-static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
+template <bool kBlockMode>
+constexpr size_t smem_bytes() { return 1024 + size_t(stage_area(kBlockMode)) + sizeof(SharedTail<kBlockMode>); }
+static_assert(smem_bytes<false>() <= 227 * 1024 && smem_bytes<true>() <= 227 * 1024, "shared memory of one CTA");
 
 __host__ __device__ constexpr int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
@@ -87,28 +109,47 @@ __device__ __forceinline__ int tile_tokens(int count, int tiles) {
     return round_up((count + tiles - 1) / tiles, kPair ? 32 : 16);
 }
 
+// Block mode starts an expert's first tile at a multiple of four rows, so that the scales of four rows are one aligned vector;
+// the rows before the expert's own are computed and dropped.
+template <bool kBlockMode>
+__device__ __forceinline__ int expert_base(int offset) { return kBlockMode ? offset & ~3 : offset; }
+template <bool kBlockMode>
+__device__ __forceinline__ int expert_rows(int offset, int end) { return end > offset ? end - expert_base<kBlockMode>(offset) : 0; }
+
 struct Tile {
     int e, wt, row0, rows, tok;  // expert, tile along the output columns, first row, rows, tokens computed (rows rounded up)
 };
 
 // Tiles are numbered expert-major; inside an expert the token tile runs fastest, so that concurrently running CTAs share
 // one weight tile.
-template <bool kPair>
-__device__ __forceinline__ Tile decode_tile(int t, int& e_cursor, const SharedTail& st, int w_tiles) {
+template <bool kPair, bool kBlockMode>
+__device__ __forceinline__ Tile decode_tile(int t, int& e_cursor, const SharedTail<kBlockMode>& st, int w_tiles) {
     while (t >= st.tprefix[e_cursor + 1] * w_tiles) ++e_cursor;
     const int local = t - st.tprefix[e_cursor] * w_tiles;
     const int tiles = st.tprefix[e_cursor + 1] - st.tprefix[e_cursor];
-    const int count = st.offsets[e_cursor + 1] - st.offsets[e_cursor];
+    const int count = expert_rows<kBlockMode>(st.offsets[e_cursor], st.offsets[e_cursor + 1]);
     const int nt = tile_tokens<kPair>(count, tiles);
     Tile tl;
     tl.e = e_cursor;
     tl.wt = local / tiles;
     const int j = local - tl.wt * tiles;
-    tl.row0 = st.offsets[e_cursor] + j * nt;
+    tl.row0 = expert_base<kBlockMode>(st.offsets[e_cursor]) + j * nt;
     tl.rows = min(nt, count - j * nt);
     tl.tok = round_up(tl.rows, kPair ? 32 : 16);
     return tl;
 }
+
+// two fp32 FMAs in one instruction (packed fp32 of sm_100): a += x * s
+__device__ __forceinline__ void ffma2(float& a0, float& a1, uint32_t x0, uint32_t x1, float s0, float s1) {
+    const float2 r = __ffma2_rn(make_float2(__uint_as_float(x0), __uint_as_float(x1)), make_float2(s0, s1), make_float2(a0, a1));
+    a0 = r.x;
+    a1 = r.y;
+}
+
+// Block mode: accumulator columns of one K block of a tile, and K blocks per 128-column buffer. Few tokens put several K blocks
+// in one buffer, so that the hand-over between tensor core and epilogue (some 1000 cycles for a warp's wait, loads, products and
+// release, however few tokens there are) is made once for up to four of them.
+__device__ __forceinline__ int block_cols(int tok) { return tok > 32 ? 64 : 32; }
 
 __device__ __forceinline__ void group_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -120,13 +161,21 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
     pdl_launch();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    SharedTail& st = *reinterpret_cast<SharedTail*>(smem + kStageArea);
+    constexpr bool kBlockMode = kMode == kBlock;
+    constexpr int kStageArea = stage_area(kBlockMode);
+    SharedTail<kBlockMode>& st = *reinterpret_cast<SharedTail<kBlockMode>*>(smem + kStageArea);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     constexpr int kKElems = kFp8 ? kKBytes : kKBytes / 2;
     constexpr int kKind = kFp8 ? 0 : 1;               // kind::f8f6f4, kind::f16
-    constexpr int kCtaCols = kGated ? kWRows / 2 : kWRows;   // output columns per CTA
+    constexpr int kCtaCols = kGated ? kWRows / 2 : kWRows;   // output columns per CTA and pass
+    static_assert(!kBlockMode || (kFp8 && !kPair), "block mode: e4m3, single CTAs");
+    constexpr int kBufs = kBlockMode ? kAccBufs : 2;  // accumulator buffers
+    constexpr int kBufCols = kTmemCols / kBufs;
+    // fc1 in block mode re-quantises groups of 128 columns, two passes of a CTA over the same tokens
+    constexpr int kPassMax = kBlockMode && kGated ? 2 : 1;
+    constexpr int kTileCols = kCtaCols * kPassMax * (kPair ? 2 : 1);
     // In a pair, CTA 0 (the leader) issues the MMAs for both and owns the barriers they wait on.
     const int cta_rank = kPair ? int(ptx::cluster_ctarank()) : 0;
     const bool leader = cta_rank == 0;
@@ -138,9 +187,10 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
             ptx::mbar_init(&st.full[s], 1);
             ptx::mbar_init(&st.empty[s], 1);
         }
-        for (int b = 0; b < 2; ++b) {
-            ptx::mbar_init(&st.tmem_full[b], 1);
+        for (int b = 0; b < kBufs; ++b) {
+            ptx::mbar_init(&st.tmem_full[b], kBlockMode ? 2 : 1);                  // block mode: and the warp of the scale products
             ptx::mbar_init(&st.tmem_empty[b], kPair ? 2 * kEpiWarps : kEpiWarps);  // both CTAs' epilogue warps
+            if constexpr (kBlockMode) ptx::mbar_init(&st.prod_empty[b], kEpiWarps);
         }
         st.abort_flag = 0;
         ptx::fence_barrier_init();
@@ -163,8 +213,9 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
         int run = 0, largest = 0;
         for (int e0 = 0; e0 < p.E; e0 += 32) {
             const int e = e0 + lane;
-            const int count = e < p.E ? st.offsets[e + 1] - st.offsets[e] : 0;
-            const int tiles = (count + kMaxTok - 1) / kMaxTok;
+            const int count = e < p.E ? expert_rows<kBlockMode>(st.offsets[e], st.offsets[e + 1]) : 0;
+            constexpr int kLimit = kBlockMode ? kBlockTok : kMaxTok;
+            const int tiles = (count + kLimit - 1) / kLimit;
             if (tiles > 0) largest = max(largest, tile_tokens<kPair>(count, tiles));
             int sum = tiles;
 #pragma unroll
@@ -192,112 +243,449 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
     const int kb_count = p.kb_count;
     const uint32_t stage_bytes = kABytes + uint32_t(st.max_tok) * (kPair ? kKBytes / 2 : kKBytes);
     const int stages = min(kMaxStages, int(kStageArea / stage_bytes));
+    // passes of the tile at column tile wt
+    auto passes = [&](int wt) { return kPassMax == 2 && wt * kTileCols + kCtaCols < p.N ? 2 : 1; };
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
-        if (ptx::elect_one()) {
-            ptx::prefetch_tensormap(&maps.w);
-            for (int i = 0; i < 4; ++i) ptx::prefetch_tensormap(&maps.rows[i]);
-            int s = 0;
-            uint32_t ph = 0;
-            int e_cursor = 0;
-            bool ok = true;
-            for (int t = tile_first; ok && t < total_tiles; t += tile_step) {
-                const Tile tl = decode_tile<kPair>(t, e_cursor, st, p.w_tiles);
-                const int unit = tl.wt * (kPair ? 2 : 1) + cta_rank;        // this CTA's 64 or 128 output columns
-                const int rows_here = kPair ? tl.tok / 2 : tl.tok;          // each CTA of a pair loads half of the tokens
-                const int row_first = tl.row0 + (kPair ? cta_rank * rows_here : 0);
-                const uint32_t bytes = kABytes + uint32_t(rows_here) * kKBytes;
-                for (int kb = 0; kb < kb_count; ++kb) {
-                    if (!ptx::mbar_wait(&st.empty[s], ph ^ 1u, abort_flag, kWaitLimit)) {
-                        ok = false;
-                        break;
-                    }
-                    uint8_t* sw = smem + size_t(s) * stage_bytes;
-                    uint8_t* sr = sw + kABytes;
-                    const int k0 = kb * kKElems;
-                    // all bytes of a pair are credited to the leader's barrier
-                    uint32_t bar;
-                    if constexpr (kPair) {
-                        bar = ptx::map_to_cta(&st.full[s], 0);
-                        if (leader) ptx::mbar_arrive_expect_tx(&st.full[s], 2 * bytes);
-                    } else {
-                        bar = ptx::smem_u32(&st.full[s]);
-                        ptx::mbar_arrive_expect_tx(&st.full[s], bytes);
-                    }
-                    if constexpr (kGated)
-                        ptx::tma_load_5d<kPair>(sw, &maps.w, k0, 0, 0, unit * (kCtaCols / 8), tl.e, bar);
-                    else
-                        ptx::tma_load_3d<kPair>(sw, &maps.w, k0, unit * kCtaCols, tl.e, bar);
-                    int r = row_first;
-                    auto rows_box = [&](int i) {
-                        ptx::tma_load_2d_any<kPair>(sr, &maps.rows[i], k0, r, bar);
-                        sr += (kKBytes * 16) << i;
-                        r += 16 << i;
-                    };
-                    for (int left = rows_here >> 7; left > 0; --left) rows_box(3);
-                    if (rows_here & 64) rows_box(2);
-                    if (rows_here & 32) rows_box(1);
-                    if (rows_here & 16) rows_box(0);
-                    if (++s == stages) s = 0, ph ^= 1u;
+    if (warp < 4) {
+
+      if (warp == 0) {
+          // ------------------------------------------------------------ TMA producer
+          if (ptx::elect_one()) {
+              ptx::prefetch_tensormap(&maps.w);
+              for (int i = 0; i < 4; ++i) ptx::prefetch_tensormap(&maps.rows[i]);
+              int s = 0;
+              uint32_t ph = 0;
+              int e_cursor = 0;
+              bool ok = true;
+              for (int t = tile_first; ok && t < total_tiles; t += tile_step) {
+                  const Tile tl = decode_tile<kPair, kMode == kBlock>(t, e_cursor, st, p.w_tiles);
+                  const int rows_here = kPair ? tl.tok / 2 : tl.tok;          // each CTA of a pair loads half of the tokens
+                  const int row_first = tl.row0 + (kPair ? cta_rank * rows_here : 0);
+                  const uint32_t bytes = kABytes + uint32_t(rows_here) * kKBytes;
+                  for (int pass = 0; ok && pass < passes(tl.wt); ++pass) {
+                      const int col = tl.wt * kTileCols + (pass + cta_rank) * kCtaCols;  // this CTA's 64 or 128 output columns
+                      for (int kb = 0; kb < kb_count; ++kb) {
+                          if (!ptx::mbar_wait(&st.empty[s], ph ^ 1u, abort_flag, kWaitLimit)) {
+                              ok = false;
+                              break;
+                          }
+                          uint8_t* sw = smem + size_t(s) * stage_bytes;
+                          uint8_t* sr = sw + kABytes;
+                          const int k0 = kb * kKElems;
+                          // all bytes of a pair are credited to the leader's barrier
+                          uint32_t bar;
+                          if constexpr (kPair) {
+                              bar = ptx::map_to_cta(&st.full[s], 0);
+                              if (leader) ptx::mbar_arrive_expect_tx(&st.full[s], 2 * bytes);
+                          } else {
+                              bar = ptx::smem_u32(&st.full[s]);
+                              ptx::mbar_arrive_expect_tx(&st.full[s], bytes);
+                          }
+                          if constexpr (kGated)
+                              ptx::tma_load_5d<kPair>(sw, &maps.w, k0, 0, 0, col / 8, tl.e, bar);
+                          else
+                              ptx::tma_load_3d<kPair>(sw, &maps.w, k0, col, tl.e, bar);
+                          int r = row_first;
+                          auto rows_box = [&](int i) {
+                              ptx::tma_load_2d_any<kPair>(sr, &maps.rows[i], k0, r, bar);
+                              sr += (kKBytes * 16) << i;
+                              r += 16 << i;
+                          };
+                          for (int left = rows_here >> 7; left > 0; --left) rows_box(3);
+                          if (rows_here & 64) rows_box(2);
+                          if (rows_here & 32) rows_box(1);
+                          if (rows_here & 16) rows_box(0);
+                          if (++s == stages) s = 0, ph ^= 1u;
+                      }
+                  }
+              }
+          }
+          __syncwarp();
+      } else if (warp == 1) {
+          // ------------------------------------------------------------ MMA issuer
+          if (leader && ptx::elect_one()) {
+              // operand format code: e4m3 = 0 (kind::f8f6f4); bf16 = 1 (kind::f16)
+              constexpr uint32_t idesc0 = ptx::make_idesc(kFp8 ? 0u : 1u, kPair ? 2 * kWRows : kWRows, 0);
+              const uint64_t desc0 = ptx::smem_desc_sw128(ptx::smem_u32(smem));
+              // completion of everything issued so far -> one barrier (of both CTAs in a pair)
+              auto commit = [&](uint64_t* bar) {
+                  if constexpr (kPair) {
+                      ptx::umma_commit_pair(ptx::map_to_cta(bar, 0));
+                      ptx::umma_commit_pair(ptx::map_to_cta(bar, 1));
+                  } else {
+                      ptx::umma_commit(bar);
+                  }
+              };
+              auto mma_stage = [&](uint32_t d_tmem, int s, uint32_t idesc, bool first) {
+                  const uint64_t dw = ptx::smem_desc_advance(desc0, uint32_t(s) * stage_bytes);
+                  const uint64_t dr = ptx::smem_desc_advance(dw, kABytes);
+#pragma unroll
+                  for (int k = 0; k < kKBytes / kUmmaKBytes; ++k) {
+                      const uint32_t accumulate = first && k == 0 ? 0u : 1u;
+                      if constexpr (kPair)
+                          ptx::umma_pair<kKind>(d_tmem, ptx::smem_desc_advance(dw, k * kUmmaKBytes),
+                                                ptx::smem_desc_advance(dr, k * kUmmaKBytes), idesc, accumulate);
+                      else
+                          ptx::umma<kKind>(d_tmem, ptx::smem_desc_advance(dw, k * kUmmaKBytes),
+                                           ptx::smem_desc_advance(dr, k * kUmmaKBytes), idesc, accumulate);
+                  }
+              };
+              int s = 0, buf = 0;
+              uint32_t ph = 0, buf_ph = 0;
+              auto next_buf = [&] {
+                  if (++buf == kBufs) buf = 0, buf_ph ^= 1u;
+              };
+              int e_cursor = 0;
+              bool ok = true;
+              for (int t = tile_first; ok && t < total_tiles; t += tile_step) {
+                  const Tile tl = decode_tile<kPair, kMode == kBlock>(t, e_cursor, st, p.w_tiles);
+                  const uint32_t idesc = idesc0 | (uint32_t(tl.tok) >> 3) << 17;
+                  if constexpr (!kBlockMode) {
+                      if (!ptx::mbar_wait(&st.tmem_empty[buf], buf_ph ^ 1u, abort_flag, kWaitLimit)) break;
+                      ptx::tc_fence_after();
+                  }
+                  const int cols = block_cols(tl.tok);
+                  for (int pass = 0; ok && pass < passes(tl.wt); ++pass) {
+                      for (int kb = 0, col = 0; kb < kb_count; ++kb) {
+                          // block mode: the stage first - its barrier is long over - so that the MMAs follow the buffer's at once
+                          if (!ptx::mbar_wait(&st.full[s], ph, abort_flag, kWaitLimit) ||
+                              (kBlockMode && col == 0 && !ptx::mbar_wait(&st.tmem_empty[buf], buf_ph ^ 1u, abort_flag, kWaitLimit))) {
+                              ok = false;
+                              break;
+                          }
+                          ptx::tc_fence_after();
+                          mma_stage(tmem_base + uint32_t(buf * kBufCols + col), s, idesc, kBlockMode || kb == 0);
+                          commit(&st.empty[s]);
+                          if (++s == stages) s = 0, ph ^= 1u;
+                          if constexpr (kBlockMode) {
+                              col += cols;
+                              if (col == kBufCols || kb + 1 == kb_count) {
+                                  commit(&st.tmem_full[buf]);
+                                  next_buf();
+                                  col = 0;
+                              }
+                          }
+                      }
+                  }
+                  if constexpr (!kBlockMode) {
+                      if (!ok) break;
+                      commit(&st.tmem_full[buf]);
+                      next_buf();
+                  }
+              }
+          }
+          __syncwarp();
+      } else if (warp == 2) {
+          // ------------------------------------------------------------ scale products (block mode)
+          // Four tokens of one of a buffer's K blocks per lane: their activation scales, fetched four buffers ahead, times the
+          // scales of this CTA's weight rows. The epilogue warps then read finished products, two tokens at a time, where each of them would
+          // multiply the same pairs again. They find them behind the accumulator buffer's barrier, on which these warps arrive too.
+          if constexpr (kBlockMode) {
+              const int KB = kb_count, NB = (p.w_rows + 127) / 128;
+              const int at_buf = lane * 4;  // place in a buffer's products
+              int buf = 0;
+              uint32_t buf_ph = 0;
+              int e_cursor = 0;
+              bool ok = true;
+              for (int t = tile_first; ok && t < total_tiles; t += tile_step) {
+                  const Tile tl = decode_tile<kPair, kBlockMode>(t, e_cursor, st, p.w_tiles);
+                  const int cols = block_cols(tl.tok), group = kBufCols / cols;
+                  const int kb_mine = at_buf / cols, tok = at_buf % cols;
+                  const bool mine = tok < tl.tok;
+                  const float* sa = p.sa + tl.row0 + tok;
+                  const float* sb = p.sb + size_t(tl.e) * NB * KB;
+                  const int v0 = p.N + tl.wt * 128;  // fc1: first value row of the tile
+                  const float* sb0 = sb + size_t(min(tl.wt, NB - 1)) * KB;
+                  const float* sb1 = sb + size_t(min(v0 >> 7, NB - 1)) * KB;
+                  const float* sb2 = sb + size_t(min((v0 >> 7) + 1, NB - 1)) * KB;
+                  const bool split = kGated && (v0 & 127) != 0;
+                  for (int pass = 0; ok && pass < passes(tl.wt); ++pass) {
+                      auto load_sa = [&](int kb) {
+                          return mine && kb < KB ? *reinterpret_cast<const float4*>(sa + size_t(kb) * p.n_pad) : make_float4(0.f, 0.f, 0.f, 0.f);
+                      };
+                      float4 ahead[4];
+#pragma unroll
+                      for (int u = 0; u < 4; ++u) ahead[u] = load_sa(u * group + kb_mine);
+                      float w0 = 0.f, w1 = 0.f, w2 = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;  // weight scales of 32 K blocks, one per lane; the next 32
+                      auto load_sb = [&](int kb) {
+                          if (kb >= KB) return;
+                          n0 = sb0[kb];
+                          if constexpr (kGated) n1 = sb1[kb];
+                          if (split) n2 = sb2[kb];
+                      };
+                      load_sb(lane);
+                      for (int kb0 = 0; ok && kb0 < KB;) {
+#pragma unroll
+                          for (int u = 0; u < 4; ++u) {
+                              if (kb0 >= KB) break;
+                              if ((kb0 & 31) == 0) {
+                                  w0 = n0, w1 = n1, w2 = n2;
+                                  load_sb(kb0 + 32 + lane);
+                              }
+                              const float4 a = ahead[u];
+                              ahead[u] = load_sa(kb0 + 4 * group + kb_mine);
+                              const int from = (kb0 + kb_mine) & 31;
+                              const float f0 = __shfl_sync(0xffffffffu, w0, from);
+                              const float f1 = kGated ? __shfl_sync(0xffffffffu, w1, from) : 0.f;
+                              const float f2 = split ? __shfl_sync(0xffffffffu, w2, from) : 0.f;
+                              ok = ptx::mbar_wait_warp(&st.prod_empty[buf], buf_ph ^ 1u, abort_flag, kWaitLimit);
+                              if (!ok) break;
+                              if (mine) {
+                                  const int at = buf * kBufCols + at_buf;
+                                  if constexpr (kGated) {
+                                      float4* d0 = reinterpret_cast<float4*>(st.prod[0] + at * 2);
+                                      d0[0] = make_float4(a.x * f0, a.y * f0, a.x * f1, a.y * f1);
+                                      d0[1] = make_float4(a.z * f0, a.w * f0, a.z * f1, a.w * f1);
+                                      if (split) {
+                                          float4* d1 = reinterpret_cast<float4*>(st.prod[1] + at * 2);
+                                          d1[0] = make_float4(a.x * f0, a.y * f0, a.x * f2, a.y * f2);
+                                          d1[1] = make_float4(a.z * f0, a.w * f0, a.z * f2, a.w * f2);
+                                      }
+                                  } else {
+                                      *reinterpret_cast<float4*>(st.prod[0] + at) = make_float4(a.x * f0, a.y * f0, a.z * f0, a.w * f0);
+                                  }
+                              }
+                              __syncwarp();
+                              if (lane == 0) ptx::mbar_arrive(&st.tmem_full[buf]);
+                              if (++buf == kBufs) buf = 0, buf_ph ^= 1u;
+                              kb0 += group;
+                          }
+                      }
+                  }
+              }
+          }
+      }
+    } else if constexpr (kBlockMode) {
+        // ------------------------------------------------------------ epilogue warps, block mode
+        // The first warpgroup has the first half of the tile's tokens, the second the other: up to 64 sums per thread.
+        const int q = warp & 3;
+        const int h = (warp - 4) >> 2;
+        const int wg_thread = threadIdx.x & 127;
+        const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+        constexpr int kPieces = kCtaCols / 8;
+        const int tok_st = ((lane >> 3) & 1) * 8 + (lane & 7);                  // token of 16 and 16-byte piece that this thread
+        const int tok_ld = wg_thread / kPieces, piece_ld = wg_thread % kPieces;  // writes to and reads from the store buffers
+        int buf = 0;
+        uint32_t buf_ph = 0;
+        uint32_t sub_it = 0, tile_it = 0;
+        int e_cursor = 0;
+        bool ok = true;
+        // one arrival per warp, after all of its lanes are done: the accumulator buffer to the MMA thread, its products to their warps
+        auto release = [&](uint64_t* bar) {
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(bar);
+        };
+
+        for (int t = tile_first; t < total_tiles; t += tile_step, ++tile_it) {
+            int count, tok0, group, n_pass, out_row = -1;  // out_row: fc2: where this thread's token of the tile goes; used after the K loop
+            int split_at = 128;                     // fc1: column of the tile from which the value rows are in their second scale block
+            {
+                const Tile tl = decode_tile<kPair, kBlockMode>(t, e_cursor, st, p.w_tiles);
+                const int first = (tl.tok / kSub + 1) / 2 * kSub;
+                tok0 = h == 0 ? 0 : first;
+                count = h == 0 ? first : tl.tok - first;
+                group = kBufCols / block_cols(tl.tok);
+                n_pass = passes(tl.wt);
+                if constexpr (kGated) {
+                    split_at = 128 - ((p.N + tl.wt * 128) & 127);
+                } else {
+                    const int tok = int(threadIdx.x) - 128, row = tl.row0 + tok;
+                    if (tok < tl.rows && row >= st.offsets[tl.e] && row < st.offsets[tl.e + 1]) out_row = p.dest_to_src[row];
                 }
             }
-        }
-        __syncwarp();
-    } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer
-        if (leader && ptx::elect_one()) {
-            // operand format code: e4m3 = 0 (kind::f8f6f4); bf16 = 1 (kind::f16)
-            constexpr uint32_t idesc0 = ptx::make_idesc(kFp8 ? 0u : 1u, kPair ? 2 * kWRows : kWRows, 0);
-            const uint64_t desc0 = ptx::smem_desc_sw128(ptx::smem_u32(smem));
-            // completion of everything issued so far -> one barrier (of both CTAs in a pair)
-            auto commit = [&](uint64_t* bar) {
-                if constexpr (kPair) {
-                    ptx::umma_commit_pair(ptx::map_to_cta(bar, 0));
-                    ptx::umma_commit_pair(ptx::map_to_cta(bar, 1));
-                } else {
-                    ptx::umma_commit(bar);
+
+            // kUnits: 16-token units of this warpgroup; kGroup: K blocks per buffer
+            auto tile_work = [&](auto units_tag, auto group_tag) {
+                constexpr int kUnits = decltype(units_tag)::value, kGroup = decltype(group_tag)::value;
+                constexpr int kCols = kBufCols / kGroup;
+                [[maybe_unused]] uint4 act[kPassMax][kUnits];  // fc1: eight columns of a token per unit, bf16
+#pragma unroll
+                for (int pass = 0; pass < kPassMax; ++pass) {
+                    if (pass >= n_pass) break;
+                    const float* prod = st.prod[kGated && pass * kCtaCols + q * 16 >= split_at ? 1 : 0];
+                    // acc[u][i][4g ..]: as the fragment registers, group i of 16 weight rows
+                    float acc[kUnits][2][8];
+#pragma unroll
+                    for (int u = 0; u < kUnits; ++u)
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+#pragma unroll
+                            for (int r = 0; r < 8; ++r) acc[u][i][r] = 0.0f;
+                    bool ready = false;
+                    for (int kb = 0; kb < kb_count; kb += kGroup) {
+                        if (ok && !ready) ok = ptx::mbar_wait_warp(&st.tmem_full[buf], buf_ph, abort_flag, kWaitLimit);
+                        ptx::tc_fence_after();
+                        const int this_buf = buf;
+                        uint32_t x[kGroup * kUnits][2][8];
+                        const uint32_t t_buf = t_lane + uint32_t(this_buf * kBufCols + tok0);
+#pragma unroll
+                        for (int u = 0; u < kGroup * kUnits; ++u) {  // columns of K blocks past the last hold old sums, not used
+                            const uint32_t at = t_buf + (u / kUnits) * kCols + (u % kUnits) * kSub;
+                            ptx::tmem_ld_16x256b_x2(at, x[u][0]);
+                            ptx::tmem_ld_16x256b_x2(at + (16u << 16), x[u][1]);
+                        }
+                        ptx::tmem_wait_ld_units(x);
+                        ptx::tc_fence_before();
+                        release(&st.tmem_empty[this_buf]);
+                        if (++buf == kBufs) buf = 0, buf_ph ^= 1u;
+                        // ask for the next buffer now: the answers arrive under the FMAs, and the lanes agree on one
+                        const bool over = ptx::mbar_test_wait(&st.tmem_full[buf], buf_ph);
+                        const float* prod_buf = prod + (this_buf * kBufCols + tok0 + 2 * (lane & 3)) * (kGated ? 2 : 1);
+#pragma unroll
+                        for (int b = 0; b < kGroup; ++b) {
+                            if (b > 0 && kb + b >= kb_count) break;
+#pragma unroll
+                            for (int u = 0; u < kUnits; ++u)
+#pragma unroll
+                                for (int g = 0; g < 2; ++g) {
+                                    float4 f;
+                                    if constexpr (kGated) {
+                                        f = *reinterpret_cast<const float4*>(prod_buf + (b * kCols + u * kSub + 8 * g) * 2);
+                                    } else {
+                                        const float2 f2 = *reinterpret_cast<const float2*>(prod_buf + b * kCols + u * kSub + 8 * g);
+                                        f = make_float4(f2.x, f2.y, f2.x, f2.y);
+                                    }
+#pragma unroll
+                                    for (int i = 0; i < 2; ++i) {
+                                        const uint32_t* y = &x[b * kUnits + u][i][4 * g];
+                                        ffma2(acc[u][i][4 * g], acc[u][i][4 * g + 1], y[0], y[1], f.x, f.y);
+                                        ffma2(acc[u][i][4 * g + 2], acc[u][i][4 * g + 3], y[2], y[3], f.z, f.w);
+                                    }
+                                }
+                        }
+                        ready = __all_sync(0xffffffffu, over);
+                        release(&st.prod_empty[this_buf]);
+                    }
+
+                    // ---- the sums of the pass are complete. What follows needs the tile again: in the K loop the registers are sums.
+                    const Tile tl = decode_tile<kPair, kBlockMode>(t, e_cursor, st, p.w_tiles);
+                    const int col_cta = tl.wt * kTileCols + pass * kCtaCols;
+                    if constexpr (!kGated) {
+                        st.dst[tile_it & 1u][threadIdx.x - 128] =
+                            out_row >= 0 ? reinterpret_cast<unsigned long long>(p.out) + size_t(out_row) * p.N * 2 : 0ull;
+                        group_sync(3, kEpiWarps * 32);
+                    }
+                    float bw[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+                    if (p.bias != nullptr) {
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+#pragma unroll
+                            for (int v = 0; v < 2; ++v) {
+                                const int wr = kGated ? min(col_cta + q * 16 + i * 8 + (lane >> 2), p.N - 1) + v * p.N
+                                                      : min(col_cta + q * 32 + i * 16 + v * 8 + (lane >> 2), p.N - 1);
+                                bw[i][v] = p.bias[size_t(tl.e) * p.w_rows + wr];
+                            }
+                    }
+#pragma unroll
+                    for (int sub = 0; sub < kUnits; ++sub) {
+                        uint4* stage = st.stage[h][sub_it & 1u];
+                        ++sub_it;
+                        uint32_t o[2][2][2];
+#pragma unroll
+                        for (int g = 0; g < 2; ++g)
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const float* y = &acc[sub][i][g * 4];
+                                if constexpr (kGated) {
+                                    o[i][0][g] = swiglu_bf16x2(y[0] + bw[i][0], y[1] + bw[i][0], y[2] + bw[i][1], y[3] + bw[i][1]);
+                                } else {
+                                    o[i][0][g] = pack_bf16x2(y[0] + bw[i][0], y[1] + bw[i][0]);
+                                    o[i][1][g] = pack_bf16x2(y[2] + bw[i][1], y[3] + bw[i][1]);
+                                }
+                            }
+                        if constexpr (kGated) {
+                            const int piece = q * 2 + (lane >> 4);
+                            ptx::stmatrix_x4_trans(&stage[tok_st * kPieces + (piece ^ (tok_st & 7))], o[0][0][0], o[0][0][1], o[1][0][0],
+                                                   o[1][0][1]);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const int piece = q * 4 + i * 2 + (lane >> 4);
+                                ptx::stmatrix_x4_trans(&stage[tok_st * kPieces + (piece ^ (tok_st & 7))], o[i][0][0], o[i][0][1],
+                                                       o[i][1][0], o[i][1][1]);
+                            }
+                        }
+                        group_sync(1 + h, 128);
+                        if constexpr (kGated) {
+                            act[pass][sub] = stage[tok_ld * kPieces + (piece_ld ^ (tok_ld & 7))];
+                            uint32_t m2 = 0;
+                            if (col_cta + piece_ld * 8 < p.N) {
+                                amax_bf16x2(m2, act[pass][sub].x);
+                                amax_bf16x2(m2, act[pass][sub].y);
+                                amax_bf16x2(m2, act[pass][sub].z);
+                                amax_bf16x2(m2, act[pass][sub].w);
+                            }
+#pragma unroll
+                            for (int d = 1; d < 8; d <<= 1) amax_bf16x2(m2, __shfl_xor_sync(0xffffffffu, m2, d));
+                            if (piece_ld == 0) st.amax[pass][tok0 + sub * kSub + tok_ld] = amax_bf16x2_value(m2);
+                        } else {
+#pragma unroll
+                            for (int u = 0; u < kSub * kPieces / 128; ++u) {
+                                const int tok = u * (128 / kPieces) + tok_ld;
+                                const uint4 v = stage[tok * kPieces + (piece_ld ^ (tok & 7))];
+                                const unsigned long long dst = st.dst[tile_it & 1u][tok0 + sub * kSub + tok];
+                                const int col = col_cta + piece_ld * 8;
+                                if (ok && dst != 0 && col < p.N)
+                                    st16(reinterpret_cast<uint8_t*>(dst) + size_t(col) * 2, Vec16{v.x, v.y, v.z, v.w});
+                            }
+                        }
+                    }
+                }
+                if constexpr (kGated) {  // scale of each token's 128 columns, one token per thread; then the quantised rows
+                    const Tile tl = decode_tile<kPair, kBlockMode>(t, e_cursor, st, p.w_tiles);
+                    const int row_lo = st.offsets[tl.e], row_hi = st.offsets[tl.e + 1];
+                    group_sync(1 + h, 128);
+                    if (wg_thread < count) {
+                        const int tok = tok0 + wg_thread, row = tl.row0 + tok;
+                        const float sf = scale_from_amax(n_pass == 2 ? fmaxf(st.amax[0][tok], st.amax[1][tok]) : st.amax[0][tok]);
+                        st.inv[tok] = inv_scale(sf);
+                        if (ok && row >= row_lo && row < row_hi && tok < tl.rows) {
+                            p.out_scale[size_t(row) * ((p.N + 127) / 128) + tl.wt] = sf;
+                            p.out_scale_t[size_t(tl.wt) * p.n_pad + row] = sf;
+                        }
+                    }
+                    group_sync(1 + h, 128);
+#pragma unroll
+                    for (int sub = 0; sub < kUnits; ++sub) {
+                        const int tok = tok0 + sub * kSub + tok_ld, row = tl.row0 + tok;
+                        const float inv = st.inv[tok];
+#pragma unroll
+                        for (int pass = 0; pass < 2; ++pass) {
+                            const int col = tl.wt * kTileCols + pass * kCtaCols + piece_ld * 8;
+                            const uint4 a = act[pass][sub];
+                            if (ok && row >= row_lo && row < row_hi && tok < tl.rows && col < p.N)
+                                *reinterpret_cast<uint2*>(static_cast<uint8_t*>(p.out) + size_t(row) * p.N + col) =
+                                    make_uint2(f2e4m3x4(bf16_lo(a.x) * inv, bf16_hi(a.x) * inv, bf16_lo(a.y) * inv, bf16_hi(a.y) * inv),
+                                               f2e4m3x4(bf16_lo(a.z) * inv, bf16_hi(a.z) * inv, bf16_lo(a.w) * inv, bf16_hi(a.w) * inv));
+                        }
+                    }
                 }
             };
-            int s = 0;
-            uint32_t ph = 0;
-            uint32_t acc_it = 0;
-            int e_cursor = 0;
-            bool ok = true;
-            for (int t = tile_first; ok && t < total_tiles; t += tile_step, ++acc_it) {
-                const Tile tl = decode_tile<kPair>(t, e_cursor, st, p.w_tiles);
-                const uint32_t idesc = idesc0 | (uint32_t(tl.tok) >> 3) << 17;
-                const uint32_t buf = acc_it & 1u;
-                if (!ptx::mbar_wait(&st.tmem_empty[buf], ((acc_it >> 1) & 1u) ^ 1u, abort_flag, kWaitLimit)) break;
-                ptx::tc_fence_after();
-                const uint32_t d_tmem = tmem_base + buf * kMaxTok;
-                for (int kb = 0; kb < kb_count; ++kb) {
-                    if (!ptx::mbar_wait(&st.full[s], ph, abort_flag, kWaitLimit)) {
-                        ok = false;
-                        break;
-                    }
-                    ptx::tc_fence_after();
-                    const uint64_t dw = ptx::smem_desc_advance(desc0, uint32_t(s) * stage_bytes);
-                    const uint64_t dr = ptx::smem_desc_advance(dw, kABytes);
-#pragma unroll
-                    for (int k = 0; k < kKBytes / kUmmaKBytes; ++k) {
-                        const uint32_t accumulate = kb == 0 && k == 0 ? 0u : 1u;
-                        if constexpr (kPair)
-                            ptx::umma_pair<kKind>(d_tmem, ptx::smem_desc_advance(dw, k * kUmmaKBytes),
-                                                  ptx::smem_desc_advance(dr, k * kUmmaKBytes), idesc, accumulate);
-                        else
-                            ptx::umma<kKind>(d_tmem, ptx::smem_desc_advance(dw, k * kUmmaKBytes),
-                                             ptx::smem_desc_advance(dr, k * kUmmaKBytes), idesc, accumulate);
-                    }
-                    commit(&st.empty[s]);
-                    if (++s == stages) s = 0, ph ^= 1u;
+            const auto one = std::integral_constant<int, 1>{};
+            const auto two = std::integral_constant<int, 2>{};
+            const auto four = std::integral_constant<int, 4>{};
+            const int units = count / kSub;
+            if (units == 0) {  // 16 tokens: none for this warpgroup, which hands the buffers on
+                for (int trip = 0; trip < (kb_count + group - 1) / group * n_pass; ++trip) {
+                    if (ok) ok = ptx::mbar_wait_warp(&st.tmem_full[buf], buf_ph, abort_flag, kWaitLimit);
+                    release(&st.tmem_empty[buf]);
+                    release(&st.prod_empty[buf]);
+                    if (++buf == kBufs) buf = 0, buf_ph ^= 1u;
                 }
-                if (!ok) break;
-                commit(&st.tmem_full[buf]);
+                if constexpr (!kGated) {
+                    st.dst[tile_it & 1u][threadIdx.x - 128] =
+                        out_row >= 0 ? reinterpret_cast<unsigned long long>(p.out) + size_t(out_row) * p.N * 2 : 0ull;
+                    group_sync(3, kEpiWarps * 32);
+                }
+            } else if (group == 4) {
+                tile_work(one, four);
+            } else if (units == 1) {
+                tile_work(one, two);
+            } else {
+                tile_work(two, two);
             }
         }
-        __syncwarp();
-    } else if (warp >= 4) {
+    } else {
         // ------------------------------------------------------------ epilogue warps
         // Two warpgroups share a tile: each takes every other 32 tokens, 16 at a time through its store buffers. A
         // warpgroup's warps meet at named barriers; a warp whose wait gave up goes on to all of them without storing.
@@ -319,38 +707,49 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
                 ptx::mbar_arrive(&st.tmem_empty[b]);
         };
 
-        for (int t = tile_first; t < total_tiles; t += tile_step, ++acc_it) {
-            const Tile tl = decode_tile<kPair>(t, e_cursor, st, p.w_tiles);
-            const uint32_t buf = acc_it & 1u;
-            const int col_cta = (tl.wt * (kPair ? 2 : 1) + cta_rank) * kCtaCols;
-            {   // where the tile's tokens go, and their scales: one token per thread
-                const int tok = threadIdx.x - 4 * 32;
-                unsigned long long dst = 0;
-                if (tok < tl.rows) {
-                    const int row = tl.row0 + tok;
-                    const int out_row = kGated ? row : p.dest_to_src[row];
-                    if (out_row >= 0) dst = reinterpret_cast<unsigned long long>(p.out) + size_t(out_row) * p.N * 2;
-                    if constexpr (kMode == kChannel) st.sa[buf][tok] = p.sa[row];
-                }
-                st.dst[buf][tok] = dst;
+        // What the epilogue of a tile reads from global memory, fetched while the tile before is worked on: where this thread's
+        // token goes and its scale, scale and bias of this thread's weight rows r and r + 8 of the warp's two 16-row groups.
+        struct TileData {
+            Tile tl;
+            int col_cta, out_row;
+            float sa, sw[2][2], bw[2][2];
+        };
+        const int tok_mine = threadIdx.x - 4 * 32;
+        auto fetch = [&](int t, TileData& d) {
+            d.tl = decode_tile<kPair, kMode == kBlock>(t, e_cursor, st, p.w_tiles);
+            d.col_cta = (d.tl.wt * (kPair ? 2 : 1) + cta_rank) * kCtaCols;
+            d.out_row = -1;
+            if (tok_mine < d.tl.rows) {
+                const int row = d.tl.row0 + tok_mine;
+                d.out_row = kGated ? row : p.dest_to_src[row];
+                if constexpr (kMode == kChannel) d.sa = p.sa[row];
             }
-            // this thread's weight rows r and r + 8 of the warp's two 16-row groups: scale and bias
-            const bool has_bias = p.bias != nullptr;
-            float sw[2][2], bw[2][2];
 #pragma unroll
             for (int i = 0; i < 2; ++i)
 #pragma unroll
                 for (int v = 0; v < 2; ++v) {
                     int wr;
                     if constexpr (kGated)
-                        wr = min(col_cta + q * 16 + i * 8 + (lane >> 2), p.N - 1) + v * p.N;
+                        wr = min(d.col_cta + q * 16 + i * 8 + (lane >> 2), p.N - 1) + v * p.N;
                     else
-                        wr = min(col_cta + q * 32 + i * 16 + v * 8 + (lane >> 2), p.N - 1);
-                    sw[i][v] = 1.0f;
-                    if constexpr (kMode == kChannel) sw[i][v] = p.sb[size_t(tl.e) * p.w_rows + wr];
-                    if constexpr (kMode == kTensor) sw[i][v] = p.sa[0] * p.sb[tl.e];
-                    bw[i][v] = has_bias ? p.bias[size_t(tl.e) * p.w_rows + wr] : 0.0f;
+                        wr = min(d.col_cta + q * 32 + i * 16 + v * 8 + (lane >> 2), p.N - 1);
+                    d.sw[i][v] = 1.0f;
+                    if constexpr (kMode == kChannel) d.sw[i][v] = p.sb[size_t(d.tl.e) * p.w_rows + wr];
+                    if constexpr (kMode == kTensor) d.sw[i][v] = p.sa[0] * p.sb[d.tl.e];
+                    d.bw[i][v] = p.bias != nullptr ? p.bias[size_t(d.tl.e) * p.w_rows + wr] : 0.0f;
                 }
+        };
+        TileData next;
+        if (tile_first < total_tiles) fetch(tile_first, next);
+
+        for (int t = tile_first; t < total_tiles; t += tile_step, ++acc_it) {
+            const TileData td = next;
+            const Tile& tl = td.tl;
+            const uint32_t buf = acc_it & 1u;
+            const int col_cta = td.col_cta;
+            st.dst[buf][tok_mine] = td.out_row >= 0 ? reinterpret_cast<unsigned long long>(p.out) + size_t(td.out_row) * p.N * 2 : 0ull;
+            if constexpr (kMode == kChannel) st.sa[buf][tok_mine] = td.sa;
+            if (t + tile_step < total_tiles) fetch(t + tile_step, next);
             group_sync(3, kEpiWarps * 32);
             if (ok) ok = ptx::mbar_wait_warp(&st.tmem_full[buf], (acc_it >> 1) & 1u, abort_flag, kWaitLimit);
             ptx::tc_fence_after();
@@ -389,8 +788,8 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
                             float y[2][2];
 #pragma unroll
                             for (int v = 0; v < 2; ++v) {
-                                y[v][0] = __uint_as_float(x[2 * v]) * (s0 * sw[i][v]) + bw[i][v];
-                                y[v][1] = __uint_as_float(x[2 * v + 1]) * (s1 * sw[i][v]) + bw[i][v];
+                                y[v][0] = __uint_as_float(x[2 * v]) * (s0 * td.sw[i][v]) + td.bw[i][v];
+                                y[v][1] = __uint_as_float(x[2 * v + 1]) * (s1 * td.sw[i][v]) + td.bw[i][v];
                             }
                             if constexpr (kGated) {
                                 o[i][0][g] = swiglu_bf16x2(y[0][0], y[0][1], y[1][0], y[1][1]);
@@ -486,14 +885,14 @@ static int launch(const Maps& maps, const Params& p, cudaStream_t stream) {
     {
         std::lock_guard<std::mutex> lk(mu);
         if (!configured[dev]) {
-            DQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes)));
+            DQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes<kMode == kBlock>())));
             configured[dev] = true;
         }
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(kPair ? sm_count() & ~1 : sm_count()), 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
-    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.dynamicSmemBytes = smem_bytes<kMode == kBlock>();
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -538,32 +937,38 @@ static int make_weight_map(CUtensorMap* map, const void* w, int esz, int E, int 
 // Arguments as gemm::grouped_gemm takes them; bf16 and per-tensor / per-channel FP8 operands.
 int grouped_gemm(const void* a, const float* a_scale, const void* w, const float* w_scale, const int* offsets, int n, int N, int K,
                  int E, int quant_mode, int gated, void* out, float* amax, const int* dest_to_src, const float* bias,
-                 cudaStream_t stream) {
-    DQ_CHECK(quant_mode == DQMOE_QUANT_NONE || quant_mode == DQMOE_QUANT_FP8_TENSOR || quant_mode == DQMOE_QUANT_FP8_CHANNEL);
+                 float* out_scale, float* out_scale_t, int n_pad, cudaStream_t stream) {
+    const bool block = quant_mode == DQMOE_QUANT_FP8_BLOCK;
+    DQ_CHECK(quant_mode == DQMOE_QUANT_NONE || quant_mode == DQMOE_QUANT_FP8_TENSOR || quant_mode == DQMOE_QUANT_FP8_CHANNEL || block);
     DQ_CHECK(n >= 0 && N > 0 && K > 0 && E > 0 && E <= kMaxExperts);
     if (n == 0) return DQMOE_OK;
     const bool fp8 = quant_mode != DQMOE_QUANT_NONE;
     const int esz = fp8 ? 1 : 2;
     DQ_CHECK_FMT((size_t(K) * esz) % 16 == 0, "K=%d: rows must be a multiple of 16 bytes", K);
-    DQ_CHECK_FMT(N % 8 == 0, "N=%d: output rows must be 16-byte vectors", N);
+    DQ_CHECK_FMT(N % (gated && block ? 16 : 8) == 0, "N=%d: output rows must be 16-byte vectors", N);
     DQ_CHECK(is_aligned(a, 16) && is_aligned(w, 16) && is_aligned(out, 16));
     DQ_CHECK(a != nullptr && w != nullptr && out != nullptr && offsets != nullptr && (gated || dest_to_src != nullptr));
-    if (fp8) DQ_CHECK(a_scale != nullptr && w_scale != nullptr && (!gated || amax != nullptr));
+    if (fp8) DQ_CHECK(a_scale != nullptr && w_scale != nullptr && (block || !gated || amax != nullptr));
+    // a tile's scales are read four rows at a time, up to its rows rounded up to 16
+    if (block) DQ_CHECK(n_pad % 4 == 0 && n_pad >= n + 15 && is_aligned(a_scale, 16) && (!gated || (out_scale != nullptr && out_scale_t != nullptr)));
 
-    const bool pair = n / E >= 24;
+    const bool pair = !block && n / E >= 24;
     const int cta_cols = gated ? kWRows / 2 : kWRows;
     Params p;
     p.n_rows = n;
     p.N = N;
     p.E = E;
     p.w_rows = gated ? 2 * N : N;
-    p.w_tiles = ceil_div(N, pair ? 2 * cta_cols : cta_cols);
+    p.w_tiles = ceil_div(N, pair || (block && gated) ? 2 * cta_cols : cta_cols);
     p.kb_count = ceil_div(K * esz, kKBytes);
     p.offsets = offsets;
     p.sa = a_scale;
     p.sb = w_scale;
     p.out = out;
     p.amax = amax;
+    p.out_scale = out_scale;
+    p.out_scale_t = out_scale_t;
+    p.n_pad = n_pad;
     p.bias = bias;
     p.dest_to_src = dest_to_src;
     p.status = device_status_word();
@@ -579,7 +984,8 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
     switch (quant_mode) {
         case DQMOE_QUANT_NONE: return DQ_WM_LAUNCH(false, kNone);
         case DQMOE_QUANT_FP8_TENSOR: return DQ_WM_LAUNCH(true, kTensor);
-        default: return DQ_WM_LAUNCH(true, kChannel);
+        case DQMOE_QUANT_FP8_CHANNEL: return DQ_WM_LAUNCH(true, kChannel);
+        default: return gated ? launch<true, kBlock, true, false>(maps, p, stream) : launch<true, kBlock, false, false>(maps, p, stream);
     }
 #undef DQ_WM_LAUNCH
 }

@@ -18,10 +18,11 @@ int route_topk(const float* logits, int T, int E, int k, int n_shared, int scori
 }  // namespace route
 namespace permute {
 int scatter_rows(const void* src, size_t row_bytes, int T, int k, const int* src_to_dest, void* dst, const float* src_scale,
-                 int scale_cols, float* dst_scale, float* amax, int amax_per_row, cudaStream_t stream);
+                 int scale_cols, float* dst_scale, float* scale_t, int n_pad, float* amax, int amax_per_row, cudaStream_t stream);
 int scale_tiles(const float* scale, int n, int cols, const int* offsets, const int* mtile_prefix, int E, float* out,
                 cudaStream_t stream);
-int scatter_quant_1x128(const void* x_bf16, int T, int k, int H, const int* src_to_dest, void* q, float* scale, cudaStream_t stream);
+int scatter_quant_1x128(const void* x_bf16, int T, int k, int H, const int* src_to_dest, void* q, float* scale, float* scale_t, int n_pad,
+                        cudaStream_t stream);
 }  // namespace permute
 namespace gemm {
 int grouped_gemm(const void* a, const float* a_scale, const void* w, const float* w_scale, const int* offsets,
@@ -34,7 +35,7 @@ enum Elem : int { kElemBf16 = 0, kElemHalf = 1, kElemF32 = 2 };  // element type
 namespace gemm_wm {
 int grouped_gemm(const void* a, const float* a_scale, const void* w, const float* w_scale, const int* offsets, int n, int N, int K,
                  int E, int quant_mode, int gated, void* out, float* amax, const int* dest_to_src, const float* bias,
-                 cudaStream_t stream);
+                 float* out_scale, float* out_scale_t, int n_pad, cudaStream_t stream);
 }  // namespace gemm_wm
 
 namespace gemm_mx {
@@ -69,6 +70,12 @@ static bool tiled_scales(int64_t n, int H, int I, int E, int quant_mode) {
     const int64_t kh = ceil_div(H, 128), ki = ceil_div(I, 128);
     return tiles * (ki * kh + ceil_div(H, 256) * ki) >= kTiledTrips;
 }
+// Which grouped GEMMs have the weights on the M side (gemm_wm_sm100.cu).
+constexpr int kWmBlockRows = 40;
+static bool weights_on_m(int64_t n, int E, int quant_mode, int elem) {
+    if (quant_mode == DQMOE_QUANT_FP8_BLOCK) return n < kWmBlockRows * int64_t(E);
+    return elem == gemm::kElemBf16;
+}
 constexpr int kDecodeRows = 8;  // up to this many expanded rows the GEMV path of decode.cu is used (bf16, per-tensor FP8)
 
 struct Layout {
@@ -77,6 +84,7 @@ struct Layout {
     size_t total;
     size_t sort_ws_bytes;
     int perm_scale_cols;
+    int n_pad;  // block mode: rows of the scale matrices by column
 };
 
 static bool valid_mode(int q) {
@@ -119,11 +127,13 @@ static Layout make_layout(int T, int H, int I, int E, int k, int quant_mode, int
                                    : quant_mode == DQMOE_QUANT_FP8_CHANNEL ? n
                                    : quant_mode == DQMOE_QUANT_FP8_TENSOR ? 1 : 0;
     L.act_scale = add(act_scale_elems * sizeof(float));
-    // block mode: the scale matrices a second time by tile, for the grouped GEMMs (every expert may add a partly filled tile)
+    // block mode: the scale matrices a second time for the grouped GEMMs, by tile (every expert may add a partly filled one) or by
+    // column (n_pad rows: a tile reads on to a multiple of 16)
     const bool tiled = tiled_scales(int64_t(n), H, I, E, quant_mode);
-    const size_t tile_rows = tiled ? ((n + 127) / 128 + (size_t(E) < n ? size_t(E) : n)) * 128 : 0;
-    L.perm_a_scale_t = add(tile_rows * ceil_div(H, 128) * sizeof(float));
-    L.act_scale_t = add(tile_rows * ceil_div(I, 128) * sizeof(float));
+    L.n_pad = quant_mode == DQMOE_QUANT_FP8_BLOCK ? int(align_up(n + 16, 4)) : 0;
+    const size_t scale_rows = tiled ? ((n + 127) / 128 + (size_t(E) < n ? size_t(E) : n)) * 128 : size_t(L.n_pad);
+    L.perm_a_scale_t = add(scale_rows * ceil_div(H, 128) * sizeof(float));
+    L.act_scale_t = add(scale_rows * ceil_div(I, 128) * sizeof(float));
     const bool two_pass = quant_mode == DQMOE_QUANT_FP8_TENSOR || quant_mode == DQMOE_QUANT_FP8_CHANNEL;
     L.act_bf16 = add(two_pass ? n * I * 2 : 0);
     L.amax = add(quant_mode == DQMOE_QUANT_FP8_CHANNEL ? n * sizeof(float)
@@ -200,8 +210,11 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
     float* perm_a_scale = reinterpret_cast<float*>(ws + L.perm_a_scale);
     void* act = ws + L.act;
     float* act_scale = reinterpret_cast<float*>(ws + L.act_scale);
-    float* perm_a_scale_t = layer::tiled_scales(n, H, I, E, quant_mode) ? reinterpret_cast<float*>(ws + L.perm_a_scale_t) : nullptr;
-    float* act_scale_t = perm_a_scale_t != nullptr ? reinterpret_cast<float*>(ws + L.act_scale_t) : nullptr;
+    const bool block = quant_mode == DQMOE_QUANT_FP8_BLOCK;
+    const bool wm = layer::weights_on_m(n, E, quant_mode, elem);
+    const bool tiled = !wm && layer::tiled_scales(n, H, I, E, quant_mode);
+    float* perm_a_scale_t = (block && wm) || tiled ? reinterpret_cast<float*>(ws + L.perm_a_scale_t) : nullptr;
+    float* act_scale_t = (block && wm) || tiled ? reinterpret_cast<float*>(ws + L.act_scale_t) : nullptr;
     void* act_bf16 = ws + L.act_bf16;
     float* amax = reinterpret_cast<float*>(ws + L.amax);
 
@@ -216,7 +229,7 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
 
     const bool two_pass = quant_mode == DQMOE_QUANT_FP8_TENSOR || quant_mode == DQMOE_QUANT_FP8_CHANNEL;
     rc = permute::scatter_rows(a, size_t(H) * esz, T, k, src_to_dest, perm_a, a_scale, L.perm_scale_cols, perm_a_scale,
-                               two_pass ? amax : nullptr, quant_mode == DQMOE_QUANT_FP8_CHANNEL, stream);
+                               wm ? perm_a_scale_t : nullptr, L.n_pad, two_pass ? amax : nullptr, quant_mode == DQMOE_QUANT_FP8_CHANNEL, stream);
     if (rc != DQMOE_OK) return rc;
 
     if (quant_mode == DQMOE_QUANT_FP8_MX) {
@@ -235,16 +248,15 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
                                         nullptr, dest_to_src, nullptr, bias2, false, nullptr, nullptr, nullptr, stream);
     }
     const float* sa1 = quant_mode == DQMOE_QUANT_FP8_TENSOR ? a_scale : perm_a_scale;
-    if (perm_a_scale_t != nullptr) {
+    if (tiled) {
         rc = permute::scale_tiles(perm_a_scale, n, L.perm_scale_cols, offsets, mtile_prefix, E, perm_a_scale_t, stream);
         if (rc != DQMOE_OK) return rc;
     }
-    const bool wm = quant_mode != DQMOE_QUANT_FP8_BLOCK && elem == gemm::kElemBf16;
     if (wm)
-        rc = gemm_wm::grouped_gemm(perm_a, sa1, b, b_scale, offsets, n, I, H, E, quant_mode, 1, two_pass ? act_bf16 : act, amax, nullptr,
-                                   bias1, stream);
+        rc = gemm_wm::grouped_gemm(perm_a, block ? perm_a_scale_t : sa1, b, b_scale, offsets, n, I, H, E, quant_mode, 1,
+                                   two_pass ? act_bf16 : act, amax, nullptr, bias1, act_scale, act_scale_t, L.n_pad, stream);
     else
-        rc = gemm::grouped_gemm(perm_a, sa1, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, act, act_scale, amax, nullptr,
+        rc = gemm::grouped_gemm(perm_a, sa1, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, act, act_scale, nullptr, nullptr,
                                 nullptr, stream, elem, bias1, perm_a_scale_t, act_scale_t);
     if (rc != DQMOE_OK) return rc;
     if (two_pass) {
@@ -253,8 +265,8 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
         if (rc != DQMOE_OK) return rc;
     }
     if (wm)
-        return gemm_wm::grouped_gemm(act, act_scale, b1, b1_scale, offsets, n, H, I, E, quant_mode, 0, d, nullptr, dest_to_src, bias2,
-                                     stream);
+        return gemm_wm::grouped_gemm(act, block ? act_scale_t : act_scale, b1, b1_scale, offsets, n, H, I, E, quant_mode, 0, d, nullptr,
+                                     dest_to_src, bias2, nullptr, nullptr, L.n_pad, stream);
     return gemm::grouped_gemm(act, act_scale, b1, b1_scale, offsets, mtile_prefix, n, H, I, E, quant_mode, 0, d, nullptr, nullptr,
                               dest_to_src, nullptr, stream, elem, bias2, act_scale_t);
 }
@@ -311,7 +323,7 @@ int dqmoe_moe_forward_nvfp4(const void* a, const uint8_t* a_sf, const float* a_g
     int rc = route::route_sort(m_indices, n, E, counts, offsets, mtile_prefix, dest_to_src, src_to_dest, ws + L.sort_ws,
                                L.sort_ws_bytes, stream);
     if (rc != DQMOE_OK) return rc;
-    rc = permute::scatter_rows(a, size_t(H) / 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, nullptr, 0, stream);
+    rc = permute::scatter_rows(a, size_t(H) / 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, nullptr, 0, nullptr, 0, stream);
     if (rc != DQMOE_OK) return rc;
     // one scale byte per 16 elements: the tiling kernel sees them as the scales of a row twice as long
     rc = dqmoe_mx_tile_scales(a_sf, n, 2 * H, dest_to_src, k, offsets, mtile_prefix, E, perm_a_sf, stream);
@@ -425,8 +437,10 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
     float* perm_a_scale = reinterpret_cast<float*>(lws + L.perm_a_scale);
     void* act = lws + L.act;
     float* act_scale = reinterpret_cast<float*>(lws + L.act_scale);
-    float* perm_a_scale_t = layer::tiled_scales(n, H, I, E, quant_mode) ? reinterpret_cast<float*>(lws + L.perm_a_scale_t) : nullptr;
-    float* act_scale_t = perm_a_scale_t != nullptr ? reinterpret_cast<float*>(lws + L.act_scale_t) : nullptr;
+    const bool wm = layer::weights_on_m(n, E, quant_mode, gemm::kElemBf16);
+    const bool tiled = !wm && layer::tiled_scales(n, H, I, E, quant_mode);
+    float* perm_a_scale_t = fp8 && (wm || tiled) ? reinterpret_cast<float*>(lws + L.perm_a_scale_t) : nullptr;
+    float* act_scale_t = fp8 && (wm || tiled) ? reinterpret_cast<float*>(lws + L.act_scale_t) : nullptr;
 
     int rc = route::route_topk(logits, T, E_routed, k_routed, n_shared, scoring, indices, weights, stream);
     if (rc != DQMOE_OK) return rc;
@@ -461,27 +475,27 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
         if (rc != DQMOE_OK) return rc;
         return dqmoe_finalize_weighted(d, weights, out_bf16, T, k, H, stream);
     }
-    if (fp8)  // quantise on the way into expert order: a token is read as bf16 once, its k rows written as e4m3 + 1x128 scales
-        rc = permute::scatter_quant_1x128(x_bf16, T, k, H, src_to_dest, perm_a, perm_a_scale, stream);
-    else
-        rc = permute::scatter_rows(x_bf16, size_t(H) * 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, nullptr, 0, stream);
+    if (fp8) {  // quantise on the way into expert order: a token is read as bf16 once, its k rows written as e4m3 + 1x128 scales
+        rc = permute::scatter_quant_1x128(x_bf16, T, k, H, src_to_dest, perm_a, perm_a_scale, wm ? perm_a_scale_t : nullptr, L.n_pad, stream);
+        if (rc == DQMOE_OK && tiled)
+            rc = permute::scale_tiles(perm_a_scale, n, L.perm_scale_cols, offsets, mtile_prefix, E, perm_a_scale_t, stream);
+    } else {
+        rc = permute::scatter_rows(x_bf16, size_t(H) * 2, T, k, src_to_dest, perm_a, nullptr, 0, nullptr, nullptr, 0, nullptr, 0, stream);
+    }
     if (rc != DQMOE_OK) return rc;
-    if (!fp8) {
-        rc = gemm_wm::grouped_gemm(perm_a, nullptr, b, nullptr, offsets, n, I, H, E, quant_mode, 1, act, nullptr, nullptr, nullptr, stream);
+    if (wm) {
+        rc = gemm_wm::grouped_gemm(perm_a, perm_a_scale_t, b, b_scale, offsets, n, I, H, E, quant_mode, 1, act, nullptr, nullptr, nullptr,
+                                   act_scale, act_scale_t, L.n_pad, stream);
         if (rc == DQMOE_OK)
-            rc = gemm_wm::grouped_gemm(act, nullptr, b1, nullptr, offsets, n, H, I, E, quant_mode, 0, d, nullptr, dest_to_src, nullptr, stream);
-        if (rc != DQMOE_OK) return rc;
-        return dqmoe_finalize_weighted(d, weights, out_bf16, T, k, H, stream);
+            rc = gemm_wm::grouped_gemm(act, act_scale_t, b1, b1_scale, offsets, n, H, I, E, quant_mode, 0, d, nullptr, dest_to_src, nullptr,
+                                       nullptr, nullptr, L.n_pad, stream);
+    } else {
+        rc = gemm::grouped_gemm(perm_a, perm_a_scale, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, act, act_scale, nullptr,
+                                nullptr, nullptr, stream, gemm::kElemBf16, nullptr, perm_a_scale_t, act_scale_t);
+        if (rc == DQMOE_OK)
+            rc = gemm::grouped_gemm(act, act_scale, b1, b1_scale, offsets, mtile_prefix, n, H, I, E, quant_mode, 0, d, nullptr, nullptr,
+                                    dest_to_src, nullptr, stream, gemm::kElemBf16, nullptr, act_scale_t);
     }
-    if (perm_a_scale_t != nullptr) {
-        rc = permute::scale_tiles(perm_a_scale, n, L.perm_scale_cols, offsets, mtile_prefix, E, perm_a_scale_t, stream);
-        if (rc != DQMOE_OK) return rc;
-    }
-    rc = gemm::grouped_gemm(perm_a, perm_a_scale, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, act,
-                            act_scale, nullptr, nullptr, nullptr, stream, gemm::kElemBf16, nullptr, perm_a_scale_t, act_scale_t);
-    if (rc != DQMOE_OK) return rc;
-    rc = gemm::grouped_gemm(act, act_scale, b1, b1_scale, offsets, mtile_prefix, n, H, I, E, quant_mode, 0, d, nullptr,
-                            nullptr, dest_to_src, nullptr, stream, gemm::kElemBf16, nullptr, act_scale_t);
     if (rc != DQMOE_OK) return rc;
     return dqmoe_finalize_weighted(d, weights, out_bf16, T, k, H, stream);
 }

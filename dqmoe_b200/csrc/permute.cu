@@ -117,7 +117,8 @@ __device__ __forceinline__ int slot_dest(const int* src_to_dest, int t, int k, i
 __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* src, uint8_t* dst,
                                                                 const int* src_to_dest, int T, int k, int row_vecs,
                                                                 const float* src_scale, float* dst_scale,
-                                                                int scale_cols, float* amax, int amax_per_row) {
+                                                                int scale_cols, float* scale_t, int n_pad, float* amax,
+                                                                int amax_per_row) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     if (amax != nullptr && !amax_per_row && blockIdx.x == 0 && threadIdx.x == 0) amax[0] = 0.0f;
@@ -143,7 +144,11 @@ __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* s
                     if (v0 + 32 * u < row_vecs) st16(dst + (size_t(r) * row_vecs + v0 + 32 * u) * 16, x[u]);
                 if (amax_per_row && strip == 0 && lane == 0) amax[r] = 0.0f;
                 if (strip == 0)
-                    for (int c = lane; c < scale_cols; c += 32) dst_scale[size_t(r) * scale_cols + c] = src_scale[size_t(t) * scale_cols + c];
+                    for (int c = lane; c < scale_cols; c += 32) {
+                        const float sf = src_scale[size_t(t) * scale_cols + c];
+                        dst_scale[size_t(r) * scale_cols + c] = sf;
+                        if (scale_t != nullptr) scale_t[size_t(c) * n_pad + r] = sf;
+                    }
             }
         }
     }
@@ -152,8 +157,8 @@ __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* s
 // The same with 1x128 FP8 quantisation of the bf16 row on the way: a lane owns 16 consecutive columns per step, so a
 // 128-column group is 8 lanes; two steps of 512 columns per strip. cols is a multiple of 16.
 __global__ void __launch_bounds__(kThreads) scatter_quant_1x128_kernel(const uint8_t* x, int T, int k, int cols,
-                                                                       const int* src_to_dest, uint8_t* q,
-                                                                       float* scale) {
+                                                                       const int* src_to_dest, uint8_t* q, float* scale,
+                                                                       float* scale_t, int n_pad) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int groups = (cols + 127) / 128;
@@ -200,7 +205,10 @@ __global__ void __launch_bounds__(kThreads) scatter_quant_1x128_kernel(const uin
                     const int c = c0 + 512 * s;
                     if (c < cols) {
                         st16(q + size_t(r) * cols + c, o[s]);
-                        if ((lane & 7) == 0) scale[size_t(r) * groups + (c >> 7)] = sf[s];
+                        if ((lane & 7) == 0) {
+                            scale[size_t(r) * groups + (c >> 7)] = sf[s];
+                            if (scale_t != nullptr) scale_t[size_t(c >> 7) * n_pad + r] = sf[s];
+                        }
                     }
                 }
             }
@@ -294,18 +302,19 @@ int scale_tiles(const float* scale, int n, int cols, const int* offsets, const i
     return DQMOE_OK;
 }
 int scatter_rows(const void* src, size_t row_bytes, int T, int k, const int* src_to_dest, void* dst, const float* src_scale,
-                 int scale_cols, float* dst_scale, float* amax, int amax_per_row, cudaStream_t stream) {
+                 int scale_cols, float* dst_scale, float* scale_t, int n_pad, float* amax, int amax_per_row, cudaStream_t stream) {
     const int row_vecs = int(row_bytes / 16);
     DQ_CHECK(is_aligned(src, 16) && is_aligned(dst, 16));
     DQ_RC(launch_pdl(scatter_rows_kernel, dim3(grid_for_rows(int64_t(T) * ceil_div(row_vecs, 128))), kThreads, 0, stream,
                      static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), src_to_dest, T, k, row_vecs, src_scale,
-                     dst_scale, scale_cols, amax, amax_per_row));
+                     dst_scale, scale_cols, scale_t, n_pad, amax, amax_per_row));
     return DQMOE_OK;
 }
-int scatter_quant_1x128(const void* x_bf16, int T, int k, int H, const int* src_to_dest, void* q, float* scale, cudaStream_t stream) {
+int scatter_quant_1x128(const void* x_bf16, int T, int k, int H, const int* src_to_dest, void* q, float* scale, float* scale_t, int n_pad,
+                        cudaStream_t stream) {
     DQ_CHECK(is_aligned(x_bf16, 16) && is_aligned(q, 16) && H % 16 == 0);
     DQ_RC(launch_pdl(scatter_quant_1x128_kernel, dim3(grid_for_rows(int64_t(T) * ceil_div(H, 1024))), kThreads, 0, stream,
-                     static_cast<const uint8_t*>(x_bf16), T, k, H, src_to_dest, static_cast<uint8_t*>(q), scale));
+                     static_cast<const uint8_t*>(x_bf16), T, k, H, src_to_dest, static_cast<uint8_t*>(q), scale, scale_t, n_pad));
     return DQMOE_OK;
 }
 
@@ -375,7 +384,7 @@ int dqmoe_quant_fp8_block_1x128(const void* x_bf16, int64_t rows, int cols, void
     // strip stays empty or more, and the row form is as fast or faster (100000 rows of 512 41.5 / 39.9, 20000 rows of 512
     // 8.3 / 8.6, 100000 rows of 256 20.9 / 36.1).
     if (cols > 512 && cols % 16 == 0 && is_aligned(q, 16) && rows < (int64_t(1) << 31))
-        return permute::scatter_quant_1x128(x_bf16, int(rows), 1, cols, nullptr, q, scale, static_cast<cudaStream_t>(stream));
+        return permute::scatter_quant_1x128(x_bf16, int(rows), 1, cols, nullptr, q, scale, nullptr, 0, static_cast<cudaStream_t>(stream));
     DQ_RC(launch_pdl(permute::quant_1x128_kernel, dim3(permute::grid_for_rows(rows)), permute::kThreads, 0,
                      static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(x_bf16), rows, cols, 1, nullptr,
                      static_cast<uint8_t*>(q), scale));

@@ -516,6 +516,25 @@ __device__ __forceinline__ void tmem_wait_ld16(uint32_t (&a)[16], uint32_t (&b)[
                  : "memory");
 }
 
+// The same for 16 columns.
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+// Wait for this thread's outstanding tcgen05.ld; the registers of all units pass through statements behind the wait.
+template <int kUnits>
+__device__ __forceinline__ void tmem_wait_ld_units(uint32_t (&x)[kUnits][2][8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int u = 0; u < kUnits; ++u)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            asm volatile("" : "+r"(x[u][i][0]), "+r"(x[u][i][1]), "+r"(x[u][i][2]), "+r"(x[u][i][3]), "+r"(x[u][i][4]), "+r"(x[u][i][5]),
+                              "+r"(x[u][i][6]), "+r"(x[u][i][7])::"memory");
+}
+
 // Four 8x8 matrices of 16-bit values, each lane holding row lane / 4, columns 2 (lane % 4) + {0, 1} of each, stored transposed:
 // lane l gives the address of the 16 bytes that take column l % 8 of matrix l / 8.
 __device__ __forceinline__ void stmatrix_x4_trans(void* smem_dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
