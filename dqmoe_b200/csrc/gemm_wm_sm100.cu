@@ -101,12 +101,14 @@ template <bool kBlockMode>
 constexpr size_t smem_bytes() { return 1024 + size_t(stage_area(kBlockMode)) + sizeof(SharedTail<kBlockMode>); }
 static_assert(smem_bytes<false>() <= 227 * 1024 && smem_bytes<true>() <= 227 * 1024, "shared memory of one CTA");
 
-__host__ __device__ constexpr int round_up(int x, int m) { return (x + m - 1) / m * m; }
-
-// Rows of one expert per tile when its `count` rows go to ceil(count / 256) tiles.
+// An expert's rows in units of 16 (32 on a pair) are spread over its tiles as evenly as whole units allow: the first tiles take one
+// more than the others. With tiles of one size, rounded up, 780 rows on pairs were 4 x 224 = 896, now 224 + 3 x 192 = 800.
 template <bool kPair>
-__device__ __forceinline__ int tile_tokens(int count, int tiles) {
-    return round_up((count + tiles - 1) / tiles, kPair ? 32 : 16);
+constexpr int kUnit = kPair ? 32 : 16;
+template <bool kPair>
+__device__ __forceinline__ int largest_tile(int count, int tiles) {
+    const int units = (count + kUnit<kPair> - 1) / kUnit<kPair>;
+    return (units + tiles - 1) / tiles * kUnit<kPair>;
 }
 
 // Block mode starts an expert's first tile at a multiple of four rows, so that the scales of four rows are one aligned vector;
@@ -128,14 +130,16 @@ __device__ __forceinline__ Tile decode_tile(int t, int& e_cursor, const SharedTa
     const int local = t - st.tprefix[e_cursor] * w_tiles;
     const int tiles = st.tprefix[e_cursor + 1] - st.tprefix[e_cursor];
     const int count = expert_rows<kBlockMode>(st.offsets[e_cursor], st.offsets[e_cursor + 1]);
-    const int nt = tile_tokens<kPair>(count, tiles);
+    const int units = (count + kUnit<kPair> - 1) / kUnit<kPair>;
+    const int each = units / tiles, more = units - each * tiles;
     Tile tl;
     tl.e = e_cursor;
     tl.wt = local / tiles;
     const int j = local - tl.wt * tiles;
-    tl.row0 = expert_base<kBlockMode>(st.offsets[e_cursor]) + j * nt;
-    tl.rows = min(nt, count - j * nt);
-    tl.tok = round_up(tl.rows, kPair ? 32 : 16);
+    const int first = (j * each + min(j, more)) * kUnit<kPair>;
+    tl.row0 = expert_base<kBlockMode>(st.offsets[e_cursor]) + first;
+    tl.tok = (each + (j < more ? 1 : 0)) * kUnit<kPair>;
+    tl.rows = min(tl.tok, count - first);
     return tl;
 }
 
@@ -216,7 +220,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
             const int count = e < p.E ? expert_rows<kBlockMode>(st.offsets[e], st.offsets[e + 1]) : 0;
             constexpr int kLimit = kBlockMode ? kBlockTok : kMaxTok;
             const int tiles = (count + kLimit - 1) / kLimit;
-            if (tiles > 0) largest = max(largest, tile_tokens<kPair>(count, tiles));
+            if (tiles > 0) largest = max(largest, largest_tile<kPair>(count, tiles));
             int sum = tiles;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -952,7 +956,7 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
     // a tile's scales are read four rows at a time, up to its rows rounded up to 16
     if (block) DQ_CHECK(n_pad % 4 == 0 && n_pad >= n + 15 && is_aligned(a_scale, 16) && (!gated || (out_scale != nullptr && out_scale_t != nullptr)));
 
-    const bool pair = !block && n / E >= 24;
+    const bool pair = !block && n / E >= 48;
     const int cta_cols = gated ? kWRows / 2 : kWRows;
     Params p;
     p.n_rows = n;
