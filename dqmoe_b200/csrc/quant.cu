@@ -146,24 +146,28 @@ __global__ void __launch_bounds__(kThreads) requant_rows_kernel(const uint8_t* x
     }
 }
 
-// One block per 128x128 weight block: 256 threads = 16 column-vectors x 16 row lanes. A thread's eight 16-byte vectors
-// are fetched together and stay in registers between the amax and the conversion, and the next block's are on their way
-// while this one is reduced and written (HBM-bound: 3 B per element; 8 x 4096 x 14336: fetched one by one and read a second
-// time for the conversion 417 us, in one pass 284 us, with the next block's loads ahead 269 us = 5.2 TB/s).
-__global__ void __launch_bounds__(kThreads) block128_kernel(const uint8_t* w, int e, int rows, int cols, uint8_t* q,
-                                                            float* scale) {
+// kWide neighbouring 128x128 weight blocks per thread block: 16 row lanes x kWide x 16 column vectors. A thread's eight 16-byte
+// vectors are fetched together and stay in registers between the amax and the conversion, and the next blocks' are on their way
+// while these are reduced and written (HBM-bound: 3 B per element; 8 x 4096 x 14336: fetched one by one and read a second
+// time for the conversion 417 us, in one pass 284 us, with the next block's loads ahead 269 us = 5.2 TB/s, two blocks side by side
+// 225 us = 6.3 TB/s: rows are then read in pieces of 512 bytes by one warp each and written in pieces of 256). One thread block of
+// 512 per SM: with two the loads ahead spill (512 us); four blocks wide leave 64 registers per thread.
+template <int kWide>
+__global__ void __launch_bounds__(kThreads * kWide) block128_kernel(const uint8_t* w, int e, int rows, int cols, uint8_t* q,
+                                                                    float* scale) {
     pdl_enter();
-    __shared__ float s_red[kThreads / 32];
-    const int bc = (cols + 127) / 128, br = (rows + 127) / 128;
-    const int64_t blocks = int64_t(e) * br * bc;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    __shared__ float s_red[2][16 * kWide];
+    const int bc = (cols + 127) / 128, br = (rows + 127) / 128, gc = (bc + kWide - 1) / kWide;
+    const int64_t groups = int64_t(e) * br * gc;
+    const int half_warp = threadIdx.x >> 4;  // 16 lanes: one row's 128 columns
+    const int tx = threadIdx.x & 15, cb = half_warp % kWide, ty = half_warp / kWide;
     struct Place {
         size_t first;   // this thread's first element
         int rows_left;  // rows of the matrix from it on, 0 beyond the last column
     };
-    auto place = [&](int64_t b) {
-        const int ei = int(b / (int64_t(br) * bc));
-        const int r0 = int((b / bc) % br) * 128 + ty, c = int(b % bc) * 128 + tx * 8;
+    auto place = [&](int64_t g) {
+        const int ei = int(g / (int64_t(br) * gc));
+        const int r0 = int((g / gc) % br) * 128 + ty, c = (int(g % gc) * kWide + cb) * 128 + tx * 8;
         return Place{(size_t(ei) * rows + r0) * cols + c, c < cols ? max(0, rows - r0) : 0};
     };
     auto fetch = [&](const Place& pl, Vec16 (&raw)[8]) {
@@ -172,11 +176,11 @@ __global__ void __launch_bounds__(kThreads) block128_kernel(const uint8_t* w, in
             raw[i] = 16 * i < pl.rows_left ? ld_stream16(w + (pl.first + size_t(16 * i) * cols) * 2) : Vec16{0, 0, 0, 0};
     };
     Vec16 raw[8];
-    int64_t b = blockIdx.x;
-    if (b >= blocks) return;
-    Place pl = place(b);
+    int64_t g = blockIdx.x;
+    if (g >= groups) return;
+    Place pl = place(g);
     fetch(pl, raw);
-    while (true) {
+    for (int parity = 0;; parity ^= 1) {
         float m = 0.0f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -184,18 +188,25 @@ __global__ void __launch_bounds__(kThreads) block128_kernel(const uint8_t* w, in
             unpack8(raw[i], v);
             m = amax8(v, m);
         }
-        const int64_t next = b + gridDim.x;
-        const bool more = next < blocks;
+        const int64_t next = g + gridDim.x;
+        const bool more = next < groups;
         Place pn{0, 0};
         Vec16 ahead[8];
         if (more) {
             pn = place(next);
             fetch(pn, ahead);
         }
-        const float amax = block_max(m, s_red);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (tx == 0) s_red[parity][half_warp] = m;
+        __syncthreads();  // one per round: the other buffer was last read before the round in between
+        float amax = 0.0f;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) amax = fmaxf(amax, s_red[parity][r * kWide + cb]);
         const float sf = scale_from_amax(amax);
         const float inv = inv_scale(sf);
-        if (threadIdx.x == 0) scale[b] = sf;
+        const int col_block = int(g % gc) * kWide + cb;
+        if (tx == 0 && ty == 0 && col_block < bc) scale[(g / gc) * bc + col_block] = sf;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             if (16 * i < pl.rows_left) {
@@ -205,7 +216,7 @@ __global__ void __launch_bounds__(kThreads) block128_kernel(const uint8_t* w, in
             }
         }
         if (!more) break;
-        b = next;
+        g = next;
         pl = pn;
 #pragma unroll
         for (int i = 0; i < 8; ++i) raw[i] = ahead[i];
@@ -410,8 +421,11 @@ int dqmoe_quant_fp8_block_128x128(const void* w_bf16, int e, int rows, int cols,
     DQ_CHECK(w_bf16 != nullptr && q != nullptr && scale != nullptr);
     DQ_CHECK_FMT(cols % 8 == 0, "cols=%d must be a multiple of 8", cols);
     DQ_CHECK(is_aligned(w_bf16, 16) && is_aligned(q, 8));
-    const int64_t blocks = int64_t(e) * ((rows + 127) / 128) * ((cols + 127) / 128);
-    DQ_RC(launch_pdl(quant::block128_kernel, dim3(quant::grid_cap(blocks, 3)), quant::kThreads, 0,
+    // Two wide everywhere: one / two wide, us: 4096 x 4096 18.2 / 17.8, 3 x 1000 x 5000 15.8 / 15.4, 16 x 600 x 512 15.6 / 15.4,
+    // 5 x 2000 x 7000 42.1 / 38.6, 8 x 4096 x 14336 269 / 225.
+    constexpr int kWide = 2;
+    const int64_t groups = int64_t(e) * ((rows + 127) / 128) * ((cols + 128 * kWide - 1) / (128 * kWide));
+    DQ_RC(launch_pdl(quant::block128_kernel<kWide>, dim3(quant::grid_cap(groups, 1)), quant::kThreads * kWide, 0,
                      static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(w_bf16), e, rows, cols,
                      static_cast<uint8_t*>(q), scale));
     return DQMOE_OK;
