@@ -283,12 +283,8 @@ def launches_per_step(n, mode, H, I, E):
     kh, ki = -(-H // 128), -(-I // 128)
     # block FP8 lays the activation scales out by tile in calls of many K blocks (tiled_scales in layer.cu)
     tiled = mode == 1024 and min(H, I) >= 2048 and n >= 192 * E and (n // 128 + E // 2) * (ki * kh + -(-H // 256) * ki) >= 44000
-    # both tile forms of a GEMM are launched where the experts' row counts choose (tile_form in gemm_sm100.cu)
-    esz, mtiles = (2 if mode == 0 else 1), -(-n // 128) + min(E, n) - 1
-    both = [mode in (0, 256, 512) and 128 <= n // E < 800 and mtiles * cols >= 296 and mtiles * cols * -(-k * esz // 128) >= 30000
-            for cols, k in ((ki, H), (-(-H // 256), I))]
     # sort, scatter into expert order, [scale tiling: MXFP8, block FP8 where it pays], fc1, [re-quantisation pass], fc2
-    return sort + 1 + 1 + (1 if mode in (256, 512, 2048) or tiled else 0) + 1 + sum(both)
+    return sort + 1 + 1 + (1 if mode in (256, 512, 2048) or tiled else 0) + 1
 
 
 def config_of(name, wl, world, T=None):

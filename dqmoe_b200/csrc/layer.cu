@@ -13,8 +13,8 @@ namespace route {
 size_t sort_workspace_bytes(int n, int E);
 int route_sort(const int* ids, int n, int E, int* counts, int* offsets, int* mtile_prefix, int* dest_to_src,
                int* src_to_dest, void* ws, size_t ws_bytes, cudaStream_t stream);
-int route_topk(const float* logits, int T, int E, int k, int n_shared, int scoring, int* indices, float* weights,
-               cudaStream_t stream);
+int route_and_sort(const float* logits, int T, int E, int k, int n_shared, int scoring, int* indices, float* weights, int* counts,
+                   int* offsets, int* mtile_prefix, int* dest_to_src, int* src_to_dest, void* ws, size_t ws_bytes, cudaStream_t stream);
 }  // namespace route
 namespace permute {
 int scatter_rows(const void* src, size_t row_bytes, int T, int k, const int* src_to_dest, void* dst, const float* src_scale,
@@ -70,7 +70,13 @@ static bool tiled_scales(int64_t n, int H, int I, int E, int quant_mode) {
     const int64_t kh = ceil_div(H, 128), ki = ceil_div(I, 128);
     return tiles * (ki * kh + ceil_div(H, 256) * ki) >= kTiledTrips;
 }
-// Which grouped GEMMs have the weights on the M side (gemm_wm_sm100.cu).
+// Which grouped GEMMs have the weights on the M side (gemm_wm_sm100.cu): all of bf16 and per-tensor / per-channel FP8, and block
+// mode up to an average of 40 rows per expert. There the row tiles of 128 are mostly empty; beyond, an expert takes several tiles of
+// 64 rows, each of which reads the weights through L2 again. Row tiles / weights on M, us per call: MoE block of H 7168, I 2048, k 8:
+// E 32 + 1 shared 16 tokens (5 rows) 287 / 243, 96 (26) 309 / 267; E 256 300 tokens (9) 2022 / 1693, 1000 (31) 2173 / 1845; H 2048, I 768,
+// E 128, k 8 500 tokens (31) 174 / 160; H 4096, I 14336, E 8, k 2 100 tokens (25) 286 / 250. The line is where skewed routing (Zipf 1.1)
+// begins to lose: 31 rows 1264 / 1266 and 146 / 148, 37 rows 298 / 290, 44 rows 1509 / 1656 and 150 / 160, 50 rows 271 / 299, although even
+// routing still gains there (50 rows 315 / 279, 298 / 278); at 75 rows 290 / 425.
 constexpr int kWmBlockRows = 40;
 static bool weights_on_m(int64_t n, int E, int quant_mode, int elem) {
     if (quant_mode == DQMOE_QUANT_FP8_BLOCK) return n < kWmBlockRows * int64_t(E);
@@ -173,11 +179,12 @@ void* dqmoe_moe_workspace_ptr(void* workspace, int which, int T, int H, int I, i
 }
 
 // elem: the operands and the output are bf16, IEEE half or fp32 (the last two with quant_mode NONE only);
-// bias1 [E, 2I] / bias2 [E, H]: fp32 biases of fc1 / fc2 added to the dequantised products, or nullptr.
+// bias1 [E, 2I] / bias2 [E, H]: fp32 biases of fc1 / fc2 added to the dequantised products, or nullptr; sorted: the workspace
+// already holds the expert sort of m_indices.
 static int moe_forward_impl(const void* a, const float* a_scale, const void* b, const float* b_scale, const void* b1,
                             const float* b1_scale, void* d, const int32_t* m_indices, void* workspace,
                             size_t workspace_bytes, int T, int H, int I, int E, int k, int quant_mode, int elem,
-                            const float* bias1, const float* bias2, cudaStream_t stream) {
+                            const float* bias1, const float* bias2, cudaStream_t stream, bool sorted = false) {
     DQ_CHECK(T >= 0 && H > 0 && I > 0 && E > 0 && k > 0);
     DQ_CHECK_FMT(layer::valid_mode(quant_mode), "quant_mode_value=%d is not one of 0, 256, 512, 1024, 2048", quant_mode);
     if (quant_mode == DQMOE_QUANT_FP8_MX)
@@ -223,8 +230,8 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
         return decode::forward(a, a_scale, b, b_scale, b1, b1_scale, d, m_indices, fp8 ? act_bf16 : act, amax, T, H, I,
                                E, k, fp8, stream);
 
-    int rc = route::route_sort(m_indices, n, E, counts, offsets, mtile_prefix, dest_to_src, src_to_dest, ws + L.sort_ws,
-                               L.sort_ws_bytes, stream);
+    int rc = sorted ? DQMOE_OK : route::route_sort(m_indices, n, E, counts, offsets, mtile_prefix, dest_to_src, src_to_dest,
+                                                   ws + L.sort_ws, L.sort_ws_bytes, stream);
     if (rc != DQMOE_OK) return rc;
 
     const bool two_pass = quant_mode == DQMOE_QUANT_FP8_TENSOR || quant_mode == DQMOE_QUANT_FP8_CHANNEL;
@@ -442,7 +449,8 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
     float* perm_a_scale_t = fp8 && (wm || tiled) ? reinterpret_cast<float*>(lws + L.perm_a_scale_t) : nullptr;
     float* act_scale_t = fp8 && (wm || tiled) ? reinterpret_cast<float*>(lws + L.act_scale_t) : nullptr;
 
-    int rc = route::route_topk(logits, T, E_routed, k_routed, n_shared, scoring, indices, weights, stream);
+    int rc = route::route_and_sort(logits, T, E_routed, k_routed, n_shared, scoring, indices, weights, counts, offsets, mtile_prefix,
+                                   dest_to_src, src_to_dest, lws + L.sort_ws, L.sort_ws_bytes, stream);
     if (rc != DQMOE_OK) return rc;
     if (quant_mode == DQMOE_QUANT_FP8_TENSOR || quant_mode == DQMOE_QUANT_FP8_CHANNEL) {
         // dynamic quantisation of the activations (per tensor or per token), then the layer as the drop-in call runs it
@@ -452,14 +460,11 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
                  ? dqmoe_quant_fp8_rowwise(x_bf16, T, H, xq, xs, stream)
                  : dqmoe_quant_fp8_tensor(x_bf16, 1, int64_t(T) * H, xq, xs, reinterpret_cast<float*>(ws + B.xamax), stream);
         if (rc != DQMOE_OK) return rc;
-        rc = dqmoe_moe_forward(xq, xs, b, b_scale, b1, b1_scale, d, indices, lws, L.total, T, H, I, E, k, quant_mode, 1,
-                               stream);
+        rc = moe_forward_impl(xq, xs, b, b_scale, b1, b1_scale, d, indices, lws, L.total, T, H, I, E, k, quant_mode, gemm::kElemBf16,
+                              nullptr, nullptr, stream, true);
         if (rc != DQMOE_OK) return rc;
         return dqmoe_finalize_weighted(d, weights, out_bf16, T, k, H, stream);
     }
-    rc = route::route_sort(indices, n, E, counts, offsets, mtile_prefix, dest_to_src, src_to_dest, lws + L.sort_ws,
-                           L.sort_ws_bytes, stream);
-    if (rc != DQMOE_OK) return rc;
     if (quant_mode == DQMOE_QUANT_FP8_MX) {  // the same fusion with 1x32 power-of-two scales
         rc = dqmoe_permute_quant_mxfp8(x_bf16, H, k, dest_to_src, n, offsets, mtile_prefix, E, perm_a,
                                        reinterpret_cast<uint8_t*>(perm_a_scale), stream);

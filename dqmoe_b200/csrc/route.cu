@@ -308,13 +308,8 @@ int route_sort(const int* ids, int n, int E, int* counts, int* offsets, int* mti
 // normalised to sum 1. Output rows have `slots` >= k entries: entries k.. name the shared
 // experts E, E+1, ... (every token, weight 1), which the layer then treats like routed ones.
 template <int kPerLane>
-__global__ void __launch_bounds__(256) route_topk_kernel(const float* logits, int T, int E, int k, int slots,
-                                                         int scoring, int* indices, float* weights) {
-    pdl_enter();
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= T) return;
-    const float* row = logits + size_t(warp) * E;
+__device__ __forceinline__ void topk_of_token(const float* row, int E, int k, int slots, int scoring, int lane, int* indices,
+                                              float* weights) {
     float x[kPerLane];
     float m = -INFINITY;
 #pragma unroll
@@ -361,22 +356,108 @@ __global__ void __launch_bounds__(256) route_topk_kernel(const float* logits, in
         }
     }
     if (lane < k) {
-        indices[size_t(warp) * slots + lane] = sel_idx;
-        weights[size_t(warp) * slots + lane] = sel_score / denom;
+        indices[lane] = sel_idx;
+        weights[lane] = sel_score / denom;
     } else if (lane < slots) {
-        indices[size_t(warp) * slots + lane] = E + (lane - k);
-        weights[size_t(warp) * slots + lane] = 1.0f;
+        indices[lane] = E + (lane - k);
+        weights[lane] = 1.0f;
     }
+}
+
+template <int kPerLane>
+__global__ void __launch_bounds__(256) route_topk_kernel(const float* logits, int T, int E, int k, int slots,
+                                                         int scoring, int* indices, float* weights) {
+    pdl_enter();
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (warp >= T) return;
+    topk_of_token<kPerLane>(logits + size_t(warp) * E, E, k, slots, scoring, threadIdx.x & 31, indices + size_t(warp) * slots,
+                            weights + size_t(warp) * slots);
+}
+
+// Router and expert sort of a small call in one block: 32 warps take a token each in turn, then sort the rows they have just
+// named (32 at a time, in row order; the same stable order as the kernels above).
+constexpr int kRouteSortThreads = 1024;
+constexpr int kRouteSortWarps = kRouteSortThreads / 32;
+template <int kPerLane>
+__global__ void __launch_bounds__(kRouteSortThreads) route_sort_small_kernel(const float* logits, int T, int E, int k, int slots,
+                                                                             int scoring, int* indices, float* weights, int* counts,
+                                                                             int* offsets, int* mtile_prefix, int* dest_to_src,
+                                                                             int* src_to_dest) {
+    pdl_enter();
+    extern __shared__ int s_mem[];
+    const int E_all = E + slots - k, n = T * slots;
+    int* s_warp_hist = s_mem;                                   // [warp][E_all + 1]: rows of a bucket in the warps before
+    int* s_base = s_warp_hist + kRouteSortWarps * (E_all + 1);  // [E_all + 2]
+    int* s_tiles = s_base + E_all + 2;                          // [E_all + 2]
+    __shared__ int s_warp_tot[33];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < kRouteSortWarps * (E_all + 1); i += kRouteSortThreads) s_warp_hist[i] = 0;
+    for (int t = warp; t < T; t += kRouteSortWarps)
+        topk_of_token<kPerLane>(logits + size_t(t) * E, E, k, slots, scoring, lane, indices + size_t(t) * slots, weights + size_t(t) * slots);
+    __syncthreads();  // the block's own stores to `indices` are visible to it
+    // consecutive rows per warp, 32 at a time
+    const int per_warp = (n + kRouteSortThreads - 1) / kRouteSortThreads * 32;
+    const int base = warp * per_warp;
+    int* my_hist = s_warp_hist + warp * (E_all + 1);
+    constexpr int kPasses = kChunk / kRouteSortThreads;
+    int bucket[kPasses], rank[kPasses];
+#pragma unroll
+    for (int it = 0; it < kPasses; ++it) {
+        const int r = base + it * 32 + lane;
+        const bool live = it * 32 < per_warp && r < n;
+        const int b = live ? bucket_of(indices[r], E_all) : -1;  // a row without a choice (NaN logits) sorts behind every expert
+        const unsigned peers = __match_any_sync(0xffffffffu, b);
+        const int before = __popc(peers & ((1u << lane) - 1u));
+        int seen = 0;
+        if (live) seen = my_hist[b];
+        __syncwarp();
+        if (live && before == 0) my_hist[b] = seen + __popc(peers);
+        __syncwarp();
+        bucket[it] = b;
+        rank[it] = seen + before;
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b <= E_all; b += kRouteSortThreads) {
+        int run = 0;
+        for (int w = 0; w < kRouteSortWarps; ++w) {
+            const int v = s_warp_hist[w * (E_all + 1) + b];
+            s_warp_hist[w * (E_all + 1) + b] = run;
+            run += v;
+        }
+        s_base[b] = run;
+        s_tiles[b] = b < E_all ? (run + 127) / 128 : 0;
+        if (b < E_all) counts[b] = run;
+    }
+    __syncthreads();
+    block_exclusive_scan(s_base, E_all + 1, s_warp_tot);
+    block_exclusive_scan(s_tiles, E_all + 1, s_warp_tot);
+    for (int b = threadIdx.x; b <= E_all; b += kRouteSortThreads) {
+        offsets[b] = s_base[b];
+        mtile_prefix[b] = s_tiles[b];
+    }
+#pragma unroll
+    for (int it = 0; it < kPasses; ++it) {
+        if (bucket[it] < 0) continue;
+        const int r = base + it * 32 + lane;
+        const int dest = s_base[bucket[it]] + my_hist[bucket[it]] + rank[it];
+        dest_to_src[dest] = bucket[it] < E_all ? r : -1;
+        src_to_dest[r] = bucket[it] < E_all ? dest : -1;
+    }
+}
+
+static int check_topk(const float* logits, int T, int E, int k, int n_shared, int scoring, const int* indices, const float* weights) {
+    DQ_CHECK(T >= 0 && E > 0 && E <= kMaxExperts && k > 0 && k <= 32 && k <= E);
+    DQ_CHECK_FMT(n_shared >= 0 && k + n_shared <= 32 && E + n_shared <= kMaxExperts, "n_shared=%d", n_shared);
+    DQ_CHECK(scoring == DQMOE_SCORE_SOFTMAX || scoring == DQMOE_SCORE_SIGMOID);
+    if (T > 0) DQ_CHECK(logits != nullptr && indices != nullptr && weights != nullptr);
+    return DQMOE_OK;
 }
 
 int route_topk(const float* logits, int T, int E, int k, int n_shared, int scoring, int* indices, float* weights,
                cudaStream_t stream) {
-    DQ_CHECK(T >= 0 && E > 0 && E <= kMaxExperts && k > 0 && k <= 32 && k <= E);
-    DQ_CHECK_FMT(n_shared >= 0 && k + n_shared <= 32 && E + n_shared <= kMaxExperts, "n_shared=%d", n_shared);
+    DQ_RC(check_topk(logits, T, E, k, n_shared, scoring, indices, weights));
     const int slots = k + n_shared;
-    DQ_CHECK(scoring == DQMOE_SCORE_SOFTMAX || scoring == DQMOE_SCORE_SIGMOID);
     if (T == 0) return DQMOE_OK;
-    DQ_CHECK(logits != nullptr && indices != nullptr && weights != nullptr);
     const int blocks = ceil_div(T, 8);
     if (E <= 32) DQ_RC(launch_pdl(route_topk_kernel<1>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring,
                                   indices, weights));
@@ -390,6 +471,26 @@ int route_topk(const float* logits, int T, int E, int k, int n_shared, int scori
                                         indices, weights));
     else DQ_RC(launch_pdl(route_topk_kernel<32>, dim3(blocks), 256, 0, stream, logits, T, E, k, slots, scoring, indices,
                           weights));
+    return DQMOE_OK;
+}
+
+// Router, then the expert sort of the rows it names (E routed experts, n_shared shared ones behind them).
+// In one launch up to 256 choices (T k): it saves a launch, but a warp takes its T / 32 tokens one choice after the other. Two
+// kernels / one, us per MoE block: 10 choices (H 1024, I 2048, E 8) 30.4 / 29.6; 768 (H 7168, I 2048, E 33) 277 / 285.
+constexpr int kRouteSortChoices = 256;
+int route_and_sort(const float* logits, int T, int E, int k, int n_shared, int scoring, int* indices, float* weights, int* counts,
+                   int* offsets, int* mtile_prefix, int* dest_to_src, int* src_to_dest, void* ws, size_t ws_bytes, cudaStream_t stream) {
+    const int slots = k + n_shared, E_all = E + n_shared;
+    const size_t smem = (size_t(kRouteSortWarps) * (E_all + 1) + 2 * (E_all + 2)) * sizeof(int);
+    if (T == 0 || int64_t(T) * k > kRouteSortChoices || int64_t(T) * slots > kChunk || E > 256 || smem > 48 * 1024) {
+        DQ_RC(route_topk(logits, T, E, k, n_shared, scoring, indices, weights, stream));
+        return route_sort(indices, T * slots, E_all, counts, offsets, mtile_prefix, dest_to_src, src_to_dest, ws, ws_bytes, stream);
+    }
+    DQ_RC(check_topk(logits, T, E, k, n_shared, scoring, indices, weights));
+    auto kern = E <= 32 ? route_sort_small_kernel<1> : E <= 64 ? route_sort_small_kernel<2> : E <= 128 ? route_sort_small_kernel<4>
+                                                                                                       : route_sort_small_kernel<8>;
+    DQ_RC(launch_pdl(kern, dim3(1), kRouteSortThreads, smem, stream, logits, T, E, k, slots, scoring, indices, weights, counts, offsets,
+                     mtile_prefix, dest_to_src, src_to_dest));
     return DQMOE_OK;
 }
 
