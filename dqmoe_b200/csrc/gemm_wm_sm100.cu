@@ -256,7 +256,6 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
           // ------------------------------------------------------------ TMA producer
           if (ptx::elect_one()) {
               ptx::prefetch_tensormap(&maps.w);
-              for (int i = 0; i < 4; ++i) ptx::prefetch_tensormap(&maps.rows[i]);
               int s = 0;
               uint32_t ph = 0;
               int e_cursor = 0;
@@ -982,9 +981,10 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
     p.status = device_status_word();
     if (p.status == nullptr) return DQMOE_ERR_CUDA;
 
-    Maps maps;
+    // Only the boxes that a tile of this call can need: encoding a map takes 0.5 us (MoE block of 5 tokens: C++ 23.3 -> 20.3 us).
+    Maps maps = {};
     DQ_RC(make_weight_map(&maps.w, w, esz, E, N, K, gated != 0));
-    for (int i = 0; i < 4; ++i) DQ_RC(gemm::make_map(&maps.rows[i], a, esz, uint64_t(n), uint64_t(K), 16 << i));
+    for (int i = 0; i < 4 && (i == 0 || (16 << i) <= n + 31); ++i) DQ_RC(gemm::make_map(&maps.rows[i], a, esz, uint64_t(n), uint64_t(K), 16 << i));
 
 #define DQ_WM_LAUNCH(FP8, MODE)                                                                                         \
     (gated ? (pair ? launch<FP8, MODE, true, true>(maps, p, stream) : launch<FP8, MODE, true, false>(maps, p, stream))  \
