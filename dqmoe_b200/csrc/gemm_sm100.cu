@@ -9,6 +9,10 @@
 // and accumulated in registers while the next K block runs on the tensor cores
 // into the other TMEM buffer.
 //
+// Rows on M. The layer runs its bf16, per-tensor and per-channel GEMMs, and block mode with few rows per expert, on the form with the
+// weights on M (gemm_wm_sm100.cu); this one serves the stand-alone operators, fp16 / fp32 operands, expert-parallel ranks and block
+// mode from 40 rows per expert on.
+//
 // Replaces the six CUTLASS grouped-GEMM variants of the reference and their
 // per-expert "configure" kernels (csrc/moe_gemm_template.h:72-1039) together
 // with doGatedActivationKernel, scale_1x128_kernel and finalizeScatterKernel
