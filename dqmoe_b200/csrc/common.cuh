@@ -64,7 +64,8 @@ constexpr int kAmaxParts = 4096;  // floats the layer workspace holds for the pe
 }
 
 // Programmatic dependent launch. Every kernel launched through launch_pdl calls pdl_launch() and pdl_wait() first thing
-// (the grouped GEMMs set up their barriers and TMEM in between): the next kernel's blocks may become resident while this
+// (the grouped GEMMs set up their barriers and TMEM in between; the row scatter and the weights-on-M GEMM call pdl_launch() after
+// their wait, and the latter fetches weights before it: gemm_wm_sm100.cu): the next kernel's blocks may become resident while this
 // one runs, and no thread touches global memory before all earlier kernels of the stream have completed. What such a kernel
 // reads may therefore still be written while it is resident: its pointers are not __restrict__ and its loads are plain ones
 // (ld_stream16). Between the short kernels of the layer the gap shrinks from ~2 us to below 1 us (MoE block of 5 tokens, H 1024,

@@ -167,7 +167,8 @@ __device__ __forceinline__ void group_sync(int id, int threads) {
 template <bool kFp8, int kMode, bool kGated, bool kPair>
 __global__ void __launch_bounds__(kThreads, 1)
 moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, const Params p) {
-    pdl_launch();
+    constexpr bool kEarly = !kPair;  // see below
+    if constexpr (!kEarly) pdl_launch();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr bool kBlockMode = kMode == kBlock;
@@ -215,7 +216,13 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
             ptx::tmem_relinquish();
         }
     }
-    pdl_wait();  // from here on global memory is read
+    // kEarly: launched as a dependent, this kernel starts while the one before it still runs, but not before the expert sort and all
+    // that came before it are complete, since the kernels in between (the row scatter, fc1) let their dependents start only after
+    // their own wait. So the row counts are there, and so are the weights: the first stages' weights are fetched before the wait, and
+    // every role that touches what the kernel before reads or writes waits for itself. Without / with, us per call: per-tensor
+    // 9 tokens at the Mixtral shape 235.5 / 227.0, bf16 438 / 421, MoE block of 5 tokens (H 1024, I 2048) 30.4 / 27.7, 96 tokens
+    // (H 7168, I 2048, E 33) 278 / 278. Not on pairs: 777 tokens 389 / 396, the weights then contend with the re-quantisation pass.
+    if constexpr (!kEarly) pdl_wait();
     for (int i = threadIdx.x; i <= p.E; i += kThreads) st.offsets[i] = p.offsets[i];
     __syncthreads();
     if (warp == 2) {  // token tiles per expert, cumulative, and the largest
@@ -261,38 +268,57 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
           // ------------------------------------------------------------ TMA producer
           if (ptx::elect_one()) {
               ptx::prefetch_tensormap(&maps.w);
+              // announces a stage's bytes (all those of a pair to the leader's barrier) and fetches its weights
+              auto load_weights = [&](const Tile& tl, int pass, int kb, int s) {
+                  const int col = tl.wt * kTileCols + (pass + cta_rank) * kCtaCols;  // this CTA's 64 or 128 output columns
+                  const uint32_t bytes = kABytes + uint32_t(kPair ? tl.tok / 2 : tl.tok) * kKBytes;
+                  uint8_t* sw = smem + size_t(s) * stage_bytes;
+                  uint32_t bar;
+                  if constexpr (kPair) {
+                      bar = ptx::map_to_cta(&st.full[s], 0);
+                      if (leader) ptx::mbar_arrive_expect_tx(&st.full[s], 2 * bytes);
+                  } else {
+                      bar = ptx::smem_u32(&st.full[s]);
+                      ptx::mbar_arrive_expect_tx(&st.full[s], bytes);
+                  }
+                  if constexpr (kGated)
+                      ptx::tma_load_5d<kPair>(sw, &maps.w, kb * kKElems, 0, 0, col / 8, tl.e, bar);
+                  else
+                      ptx::tma_load_3d<kPair>(sw, &maps.w, kb * kKElems, col, tl.e, bar);
+              };
+              int ahead = 0;  // stages whose weights are on their way before the wait
+              for (int t = tile_first, cursor = 0; kEarly && ahead < stages && t < total_tiles; t += tile_step) {
+                  const Tile tl = decode_tile<kPair, kBlockMode>(t, cursor, st, p.w_tiles);
+                  for (int pass = 0; pass < passes(tl.wt); ++pass)
+                      for (int kb = 0; ahead < stages && kb < kb_count; ++kb, ++ahead) load_weights(tl, pass, kb, ahead);
+              }
+              pdl_wait();
               int s = 0;
               uint32_t ph = 0;
               int e_cursor = 0;
               bool ok = true;
               for (int t = tile_first; ok && t < total_tiles; t += tile_step) {
-                  const Tile tl = decode_tile<kPair, kMode == kBlock>(t, e_cursor, st, p.w_tiles);
+                  const Tile tl = decode_tile<kPair, kBlockMode>(t, e_cursor, st, p.w_tiles);
                   const int rows_here = kPair ? tl.tok / 2 : tl.tok;          // each CTA of a pair loads half of the tokens
                   const int row_first = tl.row0 + (kPair ? cta_rank * rows_here : 0);
-                  const uint32_t bytes = kABytes + uint32_t(rows_here) * kKBytes;
                   for (int pass = 0; ok && pass < passes(tl.wt); ++pass) {
-                      const int col = tl.wt * kTileCols + (pass + cta_rank) * kCtaCols;  // this CTA's 64 or 128 output columns
                       for (int kb = 0; kb < kb_count; ++kb) {
-                          if (!ptx::mbar_wait(&st.empty[s], ph ^ 1u, abort_flag, kWaitLimit)) {
-                              ok = false;
-                              break;
-                          }
-                          uint8_t* sw = smem + size_t(s) * stage_bytes;
-                          uint8_t* sr = sw + kABytes;
-                          const int k0 = kb * kKElems;
-                          // all bytes of a pair are credited to the leader's barrier
-                          uint32_t bar;
-                          if constexpr (kPair) {
-                              bar = ptx::map_to_cta(&st.full[s], 0);
-                              if (leader) ptx::mbar_arrive_expect_tx(&st.full[s], 2 * bytes);
+                          if (ahead > 0) {
+                              --ahead;
                           } else {
-                              bar = ptx::smem_u32(&st.full[s]);
-                              ptx::mbar_arrive_expect_tx(&st.full[s], bytes);
+                              if (!ptx::mbar_wait(&st.empty[s], ph ^ 1u, abort_flag, kWaitLimit)) {
+                                  ok = false;
+                                  break;
+                              }
+                              load_weights(tl, pass, kb, s);
                           }
-                          if constexpr (kGated)
-                              ptx::tma_load_5d<kPair>(sw, &maps.w, k0, 0, 0, col / 8, tl.e, bar);
+                          uint8_t* sr = smem + size_t(s) * stage_bytes + kABytes;
+                          const int k0 = kb * kKElems;
+                          uint32_t bar;
+                          if constexpr (kPair)
+                              bar = ptx::map_to_cta(&st.full[s], 0);
                           else
-                              ptx::tma_load_3d<kPair>(sw, &maps.w, k0, col, tl.e, bar);
+                              bar = ptx::smem_u32(&st.full[s]);
                           int r = row_first;
                           auto rows_box = [&](int i) {
                               ptx::tma_load_2d_any<kPair>(sr, &maps.rows[i], k0, r, bar);
@@ -389,6 +415,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
           // scales of this CTA's weight rows. The epilogue warps then read finished products, two tokens at a time, where each of them would
           // multiply the same pairs again. They find them behind the accumulator buffer's barrier, on which these warps arrive too.
           if constexpr (kBlockMode) {
+              pdl_wait();
               const int KB = kb_count, NB = (p.w_rows + 127) / 128;
               const int at_buf = lane * 4;  // place in a buffer's products
               int buf = 0;
@@ -464,6 +491,8 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
           }
       }
     } else if constexpr (kBlockMode) {
+        pdl_wait();
+        if constexpr (kEarly) pdl_launch();  // after the wait: see above
         // ------------------------------------------------------------ epilogue warps, block mode
         // The first warpgroup has the first half of the tile's tokens, the second the other: up to 64 sums per thread.
         const int q = warp & 3;
@@ -694,6 +723,8 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
             }
         }
     } else {
+        pdl_wait();
+        if constexpr (kEarly) pdl_launch();  // after the wait: see above
         // ------------------------------------------------------------ epilogue warps
         // Two warpgroups share a tile: each takes every other 32 tokens, 16 at a time through its store buffers. A
         // warpgroup's warps meet at named barriers; a warp whose wait gave up goes on to all of them without storing.

@@ -119,7 +119,8 @@ __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* s
                                                                 const float* src_scale, float* dst_scale,
                                                                 int scale_cols, float* scale_t, int n_pad, float* amax,
                                                                 int amax_per_row) {
-    pdl_enter();
+    pdl_wait();
+    pdl_launch();  // after the wait: the grouped GEMM behind relies on the sort before this kernel being complete
     const int lane = threadIdx.x & 31;
     if (amax != nullptr && !amax_per_row && blockIdx.x == 0 && threadIdx.x == 0) amax[0] = 0.0f;
     const int strips = (row_vecs + 127) / 128;
@@ -159,7 +160,8 @@ __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint8_t* s
 __global__ void __launch_bounds__(kThreads) scatter_quant_1x128_kernel(const uint8_t* x, int T, int k, int cols,
                                                                        const int* src_to_dest, uint8_t* q, float* scale,
                                                                        float* scale_t, int n_pad) {
-    pdl_enter();
+    pdl_wait();
+    pdl_launch();  // after the wait: the grouped GEMM behind relies on the sort before this kernel being complete
     const int lane = threadIdx.x & 31;
     const int groups = (cols + 127) / 128;
     const int strips = (cols + 1023) / 1024;
