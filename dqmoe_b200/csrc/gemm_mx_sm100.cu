@@ -143,7 +143,7 @@ __device__ __forceinline__ uint32_t mx_scale_byte(float amax, float* inv) {
 
 template <bool kGated, bool kFp4>
 __global__ void __launch_bounds__(kThreads, 1)
-moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma_a,
+moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ gemm::RowMaps rows_a,
                                          const __grid_constant__ CUtensorMap tma_b, const Params p) {
     using F = Fmt<kFp4>;
     constexpr int kSfAtoms = F::kSfAtoms, kSfStage = F::kSfStage, kSfCols = F::kSfCols, kSfCol = F::kSfCol,
@@ -195,7 +195,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
       if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         if (ptx::elect_one()) {
-            ptx::prefetch_tensormap(&tma_a);
+            ptx::prefetch_tensormap(&rows_a.all);
             ptx::prefetch_tensormap(&tma_b);
             uint32_t it = 0;
             int e_cursor = 0;
@@ -204,6 +204,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
                 const Tile tl = decode_tile(t, e_cursor, st, p.n_tiles);
                 const int wrow0 = tl.e * p.w_rows + tl.nt * p.tile_w_rows;
                 const int wrow1 = wrow0 + p.box2_off;
+                const int rows = gemm::rows_to_load(tl.row_end - tl.row0);
                 const uint8_t* sf_a = p.sfa + size_t(tl.mtile) * kb_count * kSfPart;
                 const uint8_t* sf_b0 = p.sfb + size_t(min(wrow0 >> 7, p.w_blocks - 1)) * kb_count * kSfPart;
                 const uint8_t* sf_b1 = p.sfb + size_t(min(wrow1 >> 7, p.w_blocks - 1)) * kb_count * kSfPart;
@@ -215,8 +216,8 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
                     }
                     uint8_t* sa = smem + size_t(s) * kStageBytes;
                     uint8_t* sb = sa + kABytes;
-                    ptx::mbar_arrive_expect_tx(&st.full[s], kStageBytes + kSfStage);
-                    ptx::tma_load_2d(sa, &tma_a, kb * kBK, tl.row0, &st.full[s]);
+                    ptx::mbar_arrive_expect_tx(&st.full[s], kStageBytes - uint32_t(kBM - rows) * 128 + kSfStage);
+                    gemm::load_rows(sa, rows_a, kb * kBK, tl.row0, rows, &st.full[s]);
                     ptx::tma_load_2d(sb, &tma_b, kb * kBK, wrow0, &st.full[s]);
                     ptx::tma_load_2d(sb + kBox * kBK, &tma_b, kb * kBK, wrow1, &st.full[s]);
                     ptx::bulk_load(&st.sf[s][0], sf_a + size_t(kb) * kSfPart, kSfPart, &st.full[s]);
@@ -540,7 +541,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ CUtensorMap tma
 }
 
 template <bool kGated, bool kFp4>
-static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, cudaStream_t stream) {
+static int launch(const gemm::RowMaps& ma, const CUtensorMap& mb, const Params& p, cudaStream_t stream) {
     auto kern = moe_GemmGrouped_GemmUniversal_tcgen05_mx<kGated, kFp4>;
     static std::mutex mu;
     static bool configured[kMaxDevices] = {};
@@ -605,8 +606,9 @@ int grouped_gemm_mx(const void* a, const uint8_t* a_sf, const void* w, const uin
     p.status = device_status_word();
     if (p.status == nullptr) return DQMOE_ERR_CUDA;
     const uint64_t row_bytes = fp4 ? uint64_t(K) / 2 : uint64_t(K);  // both formats as byte matrices
-    CUtensorMap ma, mb;
-    int rc = gemm::make_map(&ma, a, 1, uint64_t(n), row_bytes, kBM);
+    gemm::RowMaps ma;
+    CUtensorMap mb;
+    int rc = gemm::make_row_maps(&ma, a, 1, uint64_t(n), row_bytes);
     if (rc != DQMOE_OK) return rc;
     rc = gemm::make_map(&mb, w, 1, uint64_t(E) * p.w_rows, row_bytes, kBox);
     if (rc != DQMOE_OK) return rc;

@@ -227,7 +227,7 @@ __device__ __forceinline__ bool pairs_suit(const int* mtile_prefix, int E, int l
 // throughput, 64 when a launch would otherwise have fewer tiles than SMs (decode shapes).
 template <bool kFp8, int kMode, bool kGated, bool kPair, int kBox, int kElem = kElemBf16>
 __global__ void __launch_bounds__(kThreads, 1)
-moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
+moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ RowMaps rows_a,
                                       const __grid_constant__ CUtensorMap tma_b, const Params p) {
     pdl_launch();
     extern __shared__ uint8_t smem_raw[];
@@ -317,7 +317,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
       if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         if (ptx::elect_one()) {
-            ptx::prefetch_tensormap(&tma_a);
+            ptx::prefetch_tensormap(&rows_a.all);
             ptx::prefetch_tensormap(&tma_b);
             uint32_t it = 0;
             int e_cursor = 0;
@@ -326,6 +326,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                 const Tile tl = decode_tile<kPair>(t, e_cursor, st, p.n_tiles, cta_rank);
                 const int wrow0 = tl.e * p.w_rows + tl.nt * p.tile_w_rows;
                 const int wrow1 = wrow0 + p.box2_off;
+                [[maybe_unused]] const int rows = rows_to_load(tl.row_end - tl.row0);  // single CTAs
                 for (int kb = 0; kb < kb_count; ++kb, ++it) {
                     const int s = it % kNumStages;
                     const uint32_t ph = (it / kNumStages) & 1u;
@@ -341,19 +342,20 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
                         // first 128 rows, CTA 1 the second); all bytes are credited to the leader's barrier.
                         const uint32_t full_leader = ptx::map_to_cta(&st.full[s], 0);
                         if (leader) ptx::mbar_arrive_expect_tx(&st.full[s], 2 * kStageBytesPair);
-                        ptx::tma_load_2d_pair(sa, &tma_a, k0, tl.row0, full_leader);
+                        ptx::tma_load_2d_pair(sa, &rows_a.all, k0, tl.row0, full_leader);
                         ptx::tma_load_2d_pair(sb, &tma_b, k0, leader ? wrow0 : wrow1, full_leader);
                     } else {
+                        const uint32_t bytes = kStageSz - uint32_t(kBM - rows) * kBKBytes;
                         if constexpr (kMode == kBlock) {
                             const bool tiled = p.sa_t != nullptr;
-                            ptx::mbar_arrive_expect_tx(&st.full[s], kStageSz + (tiled ? uint32_t(sizeof(st.sc_a[0])) : 0u));
+                            ptx::mbar_arrive_expect_tx(&st.full[s], bytes + (tiled ? uint32_t(sizeof(st.sc_a[0])) : 0u));
                             if (tiled)
                                 ptx::bulk_load(st.sc_a[it % kScaleSlots], p.sa_t + (size_t(tl.mtile) * kb_count + kb) * kBM,
                                                sizeof(st.sc_a[0]), &st.full[s]);
                         } else {
-                            ptx::mbar_arrive_expect_tx(&st.full[s], kStageSz);
+                            ptx::mbar_arrive_expect_tx(&st.full[s], bytes);
                         }
-                        ptx::tma_load_2d(sa, &tma_a, k0, tl.row0, &st.full[s]);
+                        load_rows(sa, rows_a, k0, tl.row0, rows, &st.full[s]);
                         ptx::tma_load_2d(sb, &tma_b, k0, wrow0, &st.full[s]);
                         ptx::tma_load_2d(sb + kBox * kBKBytes, &tma_b, k0, wrow1, &st.full[s]);
                     }
@@ -859,7 +861,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ CUtensorMap tma_a,
 // ---------------------------------------------------------------- host side
 
 template <bool kFp8, int kMode, bool kGated, bool kPair, int kBox, int kElem = kElemBf16>
-static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, cudaStream_t stream) {
+static int launch(const RowMaps& ma, const CUtensorMap& mb, const Params& p, cudaStream_t stream) {
     auto kern = moe_GemmGrouped_GemmUniversal_tcgen05<kFp8, kMode, kGated, kPair, kBox, kElem>;
     // the shared-memory opt-in is per function and per device
     static std::mutex mu;
@@ -981,8 +983,9 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
     p.status = device_status_word();
     if (p.status == nullptr) return DQMOE_ERR_CUDA;
 
-    CUtensorMap ma, mb;
-    int rc = make_map(&ma, a, esz, uint64_t(n), uint64_t(K), kBM);
+    RowMaps ma;
+    CUtensorMap mb;
+    int rc = make_row_maps(&ma, a, esz, uint64_t(n), uint64_t(K));
     if (rc != DQMOE_OK) return rc;
     rc = make_map(&mb, w, esz, uint64_t(E) * p.w_rows, uint64_t(K), box);
     if (rc != DQMOE_OK) return rc;
