@@ -72,6 +72,7 @@ struct Fmt {
 constexpr long long kWaitLimit = 1000000000LL;  // clock cycles before a wait gives up (~0.5 s)
 
 struct Params {
+    int early;           // launched by the layer: the sort is complete when this kernel starts
     int n_rows, N, K, E;
     int n_tiles;         // column tiles per row tile
     int w_rows;          // weight rows per expert (stage 1: 2I, stage 2: H)
@@ -149,7 +150,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ gemm::RowMaps r
     constexpr int kSfAtoms = F::kSfAtoms, kSfStage = F::kSfStage, kSfCols = F::kSfCols, kSfCol = F::kSfCol,
                   kAccCol1 = F::kAccCol1;
     constexpr int kSfPart = kSfAtoms * kSfBlock;  // scale bytes of 128 rows and one stage
-    pdl_launch();
+    if (!p.early) pdl_launch();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     Shared<kFp4>& st = *reinterpret_cast<Shared<kFp4>*>(smem + size_t(kStages) * kStageBytes);
@@ -175,7 +176,11 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ gemm::RowMaps r
         ptx::tmem_alloc(&st.tmem_base, kTmemCols);
         ptx::tmem_relinquish();
     }
-    pdl_wait();  // from here on global memory is read
+    // early (the layer's calls): the kernels between the expert sort and this one let their dependents start only after their own
+    // wait, so when this kernel starts the sort and all before it are complete. The row counts and the weights are there, and the
+    // first stages' weights and their scales are fetched before the wait (as in gemm_wm_sm100.cu). Without / with, us per MoE block:
+    // 30 tokens (H 1024, I 2048, E 8) 42.5 / 39, 20 tokens (H 7168, I 2048, E 32) 277 / 269, 100 tokens (E 33) 291.5 / 284.
+    if (!p.early) pdl_wait();
     for (int i = threadIdx.x; i <= p.E; i += kThreads) {
         st.mprefix[i] = p.mtile_prefix[i];
         st.offsets[i] = p.offsets[i];
@@ -197,32 +202,46 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ gemm::RowMaps r
         if (ptx::elect_one()) {
             ptx::prefetch_tensormap(&rows_a.all);
             ptx::prefetch_tensormap(&tma_b);
+            // announces a stage's bytes and fetches its weights and their scales
+            auto load_weights = [&](const Tile& tl, int rows, int kb, int s) {
+                const int wrow0 = tl.e * p.w_rows + tl.nt * p.tile_w_rows;
+                const int wrow1 = wrow0 + p.box2_off;
+                const uint8_t* sf_b0 = p.sfb + (size_t(min(wrow0 >> 7, p.w_blocks - 1)) * kb_count + kb) * kSfPart;
+                const uint8_t* sf_b1 = p.sfb + (size_t(min(wrow1 >> 7, p.w_blocks - 1)) * kb_count + kb) * kSfPart;
+                uint8_t* sb = smem + size_t(s) * kStageBytes + kABytes;
+                ptx::mbar_arrive_expect_tx(&st.full[s], kStageBytes - uint32_t(kBM - rows) * 128 + kSfStage);
+                ptx::tma_load_2d(sb, &tma_b, kb * kBK, wrow0, &st.full[s]);
+                ptx::tma_load_2d(sb + kBox * kBK, &tma_b, kb * kBK, wrow1, &st.full[s]);
+                ptx::bulk_load(&st.sf[s][kSfPart], sf_b0, kSfPart, &st.full[s]);
+                ptx::bulk_load(&st.sf[s][2 * kSfPart], sf_b1, kSfPart, &st.full[s]);
+            };
+            int ahead = 0;  // stages whose weights are on their way before the wait
+            for (int t = tile_first, cursor = 0; p.early && ahead < kStages && t < total_tiles; t += tile_step) {
+                const Tile tl = decode_tile(t, cursor, st, p.n_tiles);
+                const int rows = gemm::rows_to_load(tl.row_end - tl.row0);
+                for (int kb = 0; ahead < kStages && kb < kb_count; ++kb, ++ahead) load_weights(tl, rows, kb, ahead);
+            }
+            pdl_wait();
             uint32_t it = 0;
             int e_cursor = 0;
             bool ok = true;
             for (int t = tile_first; ok && t < total_tiles; t += tile_step) {
                 const Tile tl = decode_tile(t, e_cursor, st, p.n_tiles);
-                const int wrow0 = tl.e * p.w_rows + tl.nt * p.tile_w_rows;
-                const int wrow1 = wrow0 + p.box2_off;
                 const int rows = gemm::rows_to_load(tl.row_end - tl.row0);
                 const uint8_t* sf_a = p.sfa + size_t(tl.mtile) * kb_count * kSfPart;
-                const uint8_t* sf_b0 = p.sfb + size_t(min(wrow0 >> 7, p.w_blocks - 1)) * kb_count * kSfPart;
-                const uint8_t* sf_b1 = p.sfb + size_t(min(wrow1 >> 7, p.w_blocks - 1)) * kb_count * kSfPart;
                 for (int kb = 0; kb < kb_count; ++kb, ++it) {
                     const int s = it % kStages;
-                    if (!ptx::mbar_wait(&st.empty[s], ((it / kStages) & 1u) ^ 1u, abort_flag, kWaitLimit)) {
-                        ok = false;
-                        break;
+                    if (ahead > 0) {
+                        --ahead;
+                    } else {
+                        if (!ptx::mbar_wait(&st.empty[s], ((it / kStages) & 1u) ^ 1u, abort_flag, kWaitLimit)) {
+                            ok = false;
+                            break;
+                        }
+                        load_weights(tl, rows, kb, s);
                     }
-                    uint8_t* sa = smem + size_t(s) * kStageBytes;
-                    uint8_t* sb = sa + kABytes;
-                    ptx::mbar_arrive_expect_tx(&st.full[s], kStageBytes - uint32_t(kBM - rows) * 128 + kSfStage);
-                    gemm::load_rows(sa, rows_a, kb * kBK, tl.row0, rows, &st.full[s]);
-                    ptx::tma_load_2d(sb, &tma_b, kb * kBK, wrow0, &st.full[s]);
-                    ptx::tma_load_2d(sb + kBox * kBK, &tma_b, kb * kBK, wrow1, &st.full[s]);
+                    gemm::load_rows(smem + size_t(s) * kStageBytes, rows_a, kb * kBK, tl.row0, rows, &st.full[s]);
                     ptx::bulk_load(&st.sf[s][0], sf_a + size_t(kb) * kSfPart, kSfPart, &st.full[s]);
-                    ptx::bulk_load(&st.sf[s][kSfPart], sf_b0 + size_t(kb) * kSfPart, kSfPart, &st.full[s]);
-                    ptx::bulk_load(&st.sf[s][2 * kSfPart], sf_b1 + size_t(kb) * kSfPart, kSfPart, &st.full[s]);
                 }
             }
         }
@@ -286,6 +305,8 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ gemm::RowMaps r
       }
     } else {
         ptx::setmaxnreg_inc<kRegsEpilogue>();
+        pdl_wait();
+        if (p.early) pdl_launch();  // after the wait: see above
         // ------------------------------------------------------------ epilogue warps
         const int q = warp & 3;            // TMEM lane quarter this warp may read
         const int h = (warp - 4) >> 2;     // which 64-column half of each 128-column group
@@ -566,7 +587,7 @@ static int launch(const gemm::RowMaps& ma, const CUtensorMap& mb, const Params& 
 int grouped_gemm_mx(const void* a, const uint8_t* a_sf, const void* w, const uint8_t* w_sf, const int* offsets,
                     const int* mtile_prefix, int n, int N, int K, int E, int gated, void* out, uint8_t* out_sf,
                     const int* dest_to_src, const void* row_dst, const float* bias, bool fp4, const float* ga,
-                    const float* gw, const float* gout, cudaStream_t stream) {
+                    const float* gw, const float* gout, cudaStream_t stream, bool early) {
     DQ_CHECK(n >= 0 && N > 0 && K > 0 && E > 0 && E <= kMaxExperts);
     if (n == 0) return DQMOE_OK;
     const char* mode = fp4 ? "NVFP4" : "MXFP8";
@@ -580,6 +601,7 @@ int grouped_gemm_mx(const void* a, const uint8_t* a_sf, const void* w, const uin
     if (gated) DQ_CHECK(out_sf != nullptr && is_aligned(out_sf, 16));
     if (fp4) DQ_CHECK(ga != nullptr && gw != nullptr && (!gated || gout != nullptr));
     Params p;
+    p.early = early ? 1 : 0;
     p.n_rows = n;
     p.N = N;
     p.K = K;
@@ -625,14 +647,14 @@ extern "C" int dqmoe_grouped_gemm_mx(const void* a, const uint8_t* a_sf, const v
                                      dqmoe_stream_t stream) {
     return dq::gemm_mx::grouped_gemm_mx(a, a_sf, w, w_sf, offsets, mtile_prefix, n, N, K, E, gated, out, out_sf,
                                         dest_to_src, nullptr, nullptr, false, nullptr, nullptr, nullptr,
-                                        static_cast<cudaStream_t>(stream));
+                                        static_cast<cudaStream_t>(stream), false);
 }
 
 extern "C" int dqmoe_grouped_gemm_mx_rows(const void* a, const uint8_t* a_sf, const void* w, const uint8_t* w_sf,
                                           const int32_t* offsets, const int32_t* mtile_prefix, int n, int N, int K, int E,
                                           const void* row_dst, dqmoe_stream_t stream) {
     return dq::gemm_mx::grouped_gemm_mx(a, a_sf, w, w_sf, offsets, mtile_prefix, n, N, K, E, 0, nullptr, nullptr, nullptr,
-                                        row_dst, nullptr, false, nullptr, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+                                        row_dst, nullptr, false, nullptr, nullptr, nullptr, static_cast<cudaStream_t>(stream), false);
 }
 
 extern "C" int dqmoe_grouped_gemm_nvfp4(const void* a, const uint8_t* a_sf, const float* a_gscale, const void* w,
@@ -642,5 +664,5 @@ extern "C" int dqmoe_grouped_gemm_nvfp4(const void* a, const uint8_t* a_sf, cons
                                         dqmoe_stream_t stream) {
     return dq::gemm_mx::grouped_gemm_mx(a, a_sf, w, w_sf, offsets, mtile_prefix, n, N, K, E, gated, out, out_sf,
                                         dest_to_src, nullptr, nullptr, true, a_gscale, w_gscale, out_gscale,
-                                        static_cast<cudaStream_t>(stream));
+                                        static_cast<cudaStream_t>(stream), false);
 }

@@ -42,7 +42,7 @@ namespace gemm_mx {
 int grouped_gemm_mx(const void* a, const uint8_t* a_sf, const void* w, const uint8_t* w_sf, const int* offsets,
                     const int* mtile_prefix, int n, int N, int K, int E, int gated, void* out, uint8_t* out_sf,
                     const int* dest_to_src, const void* row_dst, const float* bias, bool fp4, const float* ga,
-                    const float* gw, const float* gout, cudaStream_t stream);
+                    const float* gw, const float* gout, cudaStream_t stream, bool early);
 }  // namespace gemm_mx
 
 namespace decode {
@@ -248,11 +248,11 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
         rc = gemm_mx::grouped_gemm_mx(perm_a, reinterpret_cast<const uint8_t*>(perm_a_scale), b,
                                       reinterpret_cast<const uint8_t*>(b_scale), offsets, mtile_prefix, n, I, H, E, 1, act,
                                       reinterpret_cast<uint8_t*>(act_scale), nullptr, nullptr, bias1, false, nullptr, nullptr,
-                                      nullptr, stream);
+                                      nullptr, stream, true);
         if (rc != DQMOE_OK) return rc;
         return gemm_mx::grouped_gemm_mx(act, reinterpret_cast<const uint8_t*>(act_scale), b1,
                                         reinterpret_cast<const uint8_t*>(b1_scale), offsets, mtile_prefix, n, H, I, E, 0, d,
-                                        nullptr, dest_to_src, nullptr, bias2, false, nullptr, nullptr, nullptr, stream);
+                                        nullptr, dest_to_src, nullptr, bias2, false, nullptr, nullptr, nullptr, stream, true);
     }
     const float* sa1 = quant_mode == DQMOE_QUANT_FP8_TENSOR ? a_scale : perm_a_scale;
     if (tiled) {
@@ -336,10 +336,10 @@ int dqmoe_moe_forward_nvfp4(const void* a, const uint8_t* a_sf, const float* a_g
     rc = dqmoe_mx_tile_scales(a_sf, n, 2 * H, dest_to_src, k, offsets, mtile_prefix, E, perm_a_sf, stream);
     if (rc != DQMOE_OK) return rc;
     rc = gemm_mx::grouped_gemm_mx(perm_a, perm_a_sf, b, b_sf, offsets, mtile_prefix, n, I, H, E, 1, act, act_sf, nullptr,
-                                  nullptr, bias1, true, a_gscale, b_gscale, act_gscale, stream);
+                                  nullptr, bias1, true, a_gscale, b_gscale, act_gscale, stream, true);
     if (rc != DQMOE_OK) return rc;
     return gemm_mx::grouped_gemm_mx(act, act_sf, b1, b1_sf, offsets, mtile_prefix, n, H, I, E, 0, d, nullptr, dest_to_src,
-                                    nullptr, bias2, true, act_gscale, b1_gscale, nullptr, stream);
+                                    nullptr, bias2, true, act_gscale, b1_gscale, nullptr, stream, true);
 }
 
 int dqmoe_moe_forward_f16(const void* a, const void* b, const void* b1, void* d, const int32_t* m_indices,
@@ -472,11 +472,11 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
         rc = gemm_mx::grouped_gemm_mx(perm_a, reinterpret_cast<const uint8_t*>(perm_a_scale), b,
                                       reinterpret_cast<const uint8_t*>(b_scale), offsets, mtile_prefix, n, I, H, E, 1, act,
                                       reinterpret_cast<uint8_t*>(act_scale), nullptr, nullptr, nullptr, false, nullptr, nullptr,
-                                      nullptr, stream);
+                                      nullptr, stream, true);
         if (rc != DQMOE_OK) return rc;
         rc = gemm_mx::grouped_gemm_mx(act, reinterpret_cast<const uint8_t*>(act_scale), b1,
                                       reinterpret_cast<const uint8_t*>(b1_scale), offsets, mtile_prefix, n, H, I, E, 0, d,
-                                      nullptr, dest_to_src, nullptr, nullptr, false, nullptr, nullptr, nullptr, stream);
+                                      nullptr, dest_to_src, nullptr, nullptr, false, nullptr, nullptr, nullptr, stream, true);
         if (rc != DQMOE_OK) return rc;
         return dqmoe_finalize_weighted(d, weights, out_bf16, T, k, H, stream);
     }

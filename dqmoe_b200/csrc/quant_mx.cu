@@ -55,7 +55,8 @@ template <bool kGather>
 __global__ void __launch_bounds__(kThreads) quant_rows_kernel(const uint8_t* x, int64_t rows, int cols,
                                                               const int* dest_to_src, int k, const int* offsets,
                                                               const int* mtile_prefix, int E, uint8_t* q, uint8_t* sf) {
-    pdl_enter();
+    pdl_wait();
+    pdl_launch();  // after the wait: the layer's grouped GEMM behind relies on the sort before this kernel being complete
     extern __shared__ int s_tab[];  // kGather: offsets[E+1] then mtile_prefix[E+1]
     if constexpr (kGather) {
         for (int i = threadIdx.x; i <= E; i += kThreads) {
@@ -119,7 +120,8 @@ __global__ void __launch_bounds__(kThreads) quant_rows_kernel(const uint8_t* x, 
 __global__ void __launch_bounds__(kThreads) tile_scales_kernel(const uint32_t* sf_rows, int64_t rows, int kblocks,
                                                                const int* dest_to_src, int k, const int* offsets,
                                                                const int* mtile_prefix, int E, uint8_t* tiled) {
-    pdl_enter();
+    pdl_wait();
+    pdl_launch();  // after the wait: the layer's grouped GEMM behind relies on the sort before this kernel being complete
     extern __shared__ int s_tab[];
     const bool sorted = offsets != nullptr;
     if (sorted) {
