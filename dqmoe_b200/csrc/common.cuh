@@ -129,6 +129,14 @@ __device__ __forceinline__ Vec16 ld_stream16(const void* p) {
                  : "l"(p));
     return v;
 }
+// For the few words that a programmatic dependent reads before its own pdl_wait, written by a kernel that is known to be over by
+// then. Its end makes them visible at gpu scope, but only the wait covers what this SM's L1 may still hold of an earlier call
+// that used the same workspace: a relaxed load at gpu scope is served from L2. Volatile, like the others.
+__device__ __forceinline__ int ld_relaxed_gpu(const int* p) {
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void st16(void* p, const Vec16& v) {
     asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                  : "memory");

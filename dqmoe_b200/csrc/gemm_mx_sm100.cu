@@ -182,8 +182,8 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ gemm::RowMaps r
     // 30 tokens (H 1024, I 2048, E 8) 42.5 / 39, 20 tokens (H 7168, I 2048, E 32) 277 / 269, 100 tokens (E 33) 291.5 / 284.
     if (!p.early) pdl_wait();
     for (int i = threadIdx.x; i <= p.E; i += kThreads) {
-        st.mprefix[i] = p.mtile_prefix[i];
-        st.offsets[i] = p.offsets[i];
+        st.mprefix[i] = ld_relaxed_gpu(p.mtile_prefix + i);  // early: past L1
+        st.offsets[i] = ld_relaxed_gpu(p.offsets + i);
     }
     ptx::tc_fence_before();
     __syncthreads();

@@ -218,12 +218,13 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
     }
     // kEarly: launched as a dependent, this kernel starts while the one before it still runs, but not before the expert sort and all
     // that came before it are complete, since the kernels in between (the row scatter, fc1) let their dependents start only after
-    // their own wait. So the row counts are there, and so are the weights: the first stages' weights are fetched before the wait, and
-    // every role that touches what the kernel before reads or writes waits for itself. Without / with, us per call: per-tensor
+    // their own wait (the re-quantisation pass between fc1 and fc2 before it, but it starts only after fc1's). So the row counts are
+    // there, and are read past L1, and so are the weights: the first stages' weights are fetched before the wait, by TMA and so from
+    // L2 on, and every role that touches what the kernel before reads or writes waits for itself. Without / with, us per call: per-tensor
     // 9 tokens at the Mixtral shape 235.5 / 227.0, bf16 438 / 421, MoE block of 5 tokens (H 1024, I 2048) 30.4 / 27.7, 96 tokens
     // (H 7168, I 2048, E 33) 278 / 278. Not on pairs: 777 tokens 389 / 396, the weights then contend with the re-quantisation pass.
     if constexpr (!kEarly) pdl_wait();
-    for (int i = threadIdx.x; i <= p.E; i += kThreads) st.offsets[i] = p.offsets[i];
+    for (int i = threadIdx.x; i <= p.E; i += kThreads) st.offsets[i] = ld_relaxed_gpu(p.offsets + i);
     __syncthreads();
     if (warp == 2) {  // token tiles per expert, cumulative, and the largest
         int run = 0, largest = 0;

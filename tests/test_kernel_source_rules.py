@@ -82,3 +82,15 @@ def test_block_scales_are_passed_on_by_a_release():
         assert f"commit(&st.{bar})" in block and f"mbar_arrive(&st.{bar})" in block, bar
     for bar in ("empty[s]", "tmem_full[b]"):
         assert f"mbar_init(&st.{bar}, kMode == kBlock ? 2 : 1)" in text, bar
+
+
+def test_what_is_read_before_the_wait_comes_past_l1():
+    """The weights-on-M GEMM and the layer's block-scaled one copy the sort's table before their own griddepcontrol.wait. The sort is
+    over by then, but only the wait covers lines of an earlier call's table that are still in L1."""
+    for name, tables in (("gemm_wm_sm100.cu", ["offsets"]), ("gemm_mx_sm100.cu", ["offsets", "mtile_prefix"])):
+        text = source(name)
+        kernel = braces(text, text.index("__global__"))
+        for table in tables:
+            reads = re.findall(r"[\w ]*\(?\bp\." + table + r"\b", kernel)
+            assert reads and all(r.endswith("ld_relaxed_gpu(p." + table) for r in reads), (name, reads)
+    assert "ld.relaxed.gpu.global" in source("common.cuh")
