@@ -249,6 +249,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ gemm::RowMaps r
       } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         if (ptx::elect_one()) {
+            pdl_wait();  // no rows come before it, and the limit of the waits below is for this kernel's own time
             constexpr uint32_t idesc = kFp4 ? ptx::make_idesc_nvf4(kBM, kN) : ptx::make_idesc_mx(kBM, kN);
             const uint64_t desc0 = ptx::smem_desc_sw128(ptx::smem_u32(smem));
             const uint64_t desc_sf0 = ptx::smem_desc_sf(ptx::smem_u32(&st.sf[0][0]));

@@ -339,6 +339,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_wm(const __grid_constant__ Maps maps, cons
       } else if (warp == 1) {
           // ------------------------------------------------------------ MMA issuer
           if (leader && ptx::elect_one()) {
+              pdl_wait();  // no rows come before it, and the limit of the waits below is for this kernel's own time
               // operand format code: e4m3 = 0 (kind::f8f6f4); bf16 = 1 (kind::f16)
               constexpr uint32_t idesc0 = ptx::make_idesc(kFp8 ? 0u : 1u, kPair ? 2 * kWRows : kWRows, 0);
               const uint64_t desc0 = ptx::smem_desc_sw128(ptx::smem_u32(smem));

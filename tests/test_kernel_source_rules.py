@@ -94,3 +94,23 @@ def test_what_is_read_before_the_wait_comes_past_l1():
             reads = re.findall(r"[\w ]*\(?\bp\." + table + r"\b", kernel)
             assert reads and all(r.endswith("ld_relaxed_gpu(p." + table) for r in reads), (name, reads)
     assert "ld.relaxed.gpu.global" in source("common.cuh")
+
+
+def test_roles_wait_for_the_kernel_before_before_they_wait_at_a_barrier():
+    """A wait at a barrier gives up after a time that is meant for this kernel. Launched early, a role that has not yet waited for
+    the kernel before would count that one's rest, however long it is held up, against it."""
+    for name in ("gemm_wm_sm100.cu", "gemm_mx_sm100.cu"):
+        text = source(name)
+        kernel = braces(text, text.index("__global__"))
+        roles = kernel[kernel.index("if (warp < 4) {"):]
+        at = [m.start() for m in re.finditer(r"if \(warp == \d\)|else if constexpr \(kBlockMode\) \{\s*pdl_wait|"
+                                             r"else \{\s*(?:ptx::setmaxnreg_inc<\w+>\(\);\s*)?pdl_wait", roles)] + [len(roles)]
+        waits = 0
+        for first, end in zip(at, at[1:]):
+            role = roles[first:end]
+            m = re.search(r"\bmbar_wait(_warp)?\(", role)
+            if m:
+                waits += 1
+                assert "pdl_wait()" in role[:m.start()], (name, role[:200])
+        assert waits == {"gemm_wm_sm100.cu": 5, "gemm_mx_sm100.cu": 3}[name], name
+        assert not re.search(r"\bmbar_wait(_warp)?\(", kernel[:kernel.index("if (warp < 4) {")]), name
