@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import moe_test
-from helpers import bf16_from_bits, bits, golden, make_inputs, tile_forms
+from helpers import bf16_from_bits, bits, golden, kernels_of, make_inputs, tile_forms
 from oracle import moe_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -389,3 +389,27 @@ def test_decode_path_ragged_sizes(ops, workspace, mode, E, T, H, I, k):
     assert_close(d, ref)
     if T > 1:
         assert torch.count_nonzero(d[1, 0]) == 0
+
+
+@pytest.mark.parametrize("T,E,k,n_shared", [(1, 4, 2, 0), (4, 8, 2, 0), (8, 3, 1, 0), (4, 300, 1, 1), (9, 3, 1, 0), (3, 5, 2, 1)])
+def test_block_calls_of_the_decode_path_are_not_sorted(ops, T, E, k, n_shared):
+    """Up to eight rows the per-tensor block runs on the GEMV path, which takes the router's indices as they are: no sort is launched,
+    and the result is that of the four operators in turn."""
+    H, I, E_all, slots = 256, 192, E + n_shared, k + n_shared
+    g = torch.Generator(device=DEV).manual_seed(T * E)
+    x = torch.randn(T, H, generator=g, device=DEV).to(torch.bfloat16)
+    logits = torch.randn(T, E, generator=g, device=DEV)
+    w = ops.per_tensor_cast_to_fp8((torch.randn(E_all, 2 * I, H, generator=g, device=DEV) * 0.05).to(torch.bfloat16), per_expert=True)
+    w1 = ops.per_tensor_cast_to_fp8((torch.randn(E_all, H, I, generator=g, device=DEV) * 0.05).to(torch.bfloat16), per_expert=True)
+    block = lambda: ops.moe_block(x, logits, *w, *w1, k, "softmax", 256, n_shared=n_shared)
+    out = block()
+    assert any("sort" in name for name in kernels_of(block)) == (T * slots > 8)
+    idx, wt = ops.route_topk(logits, k, "softmax")
+    idx = torch.cat([idx, torch.arange(E, E_all, dtype=torch.int32, device=DEV).expand(T, n_shared)], 1).contiguous()
+    wt = torch.cat([wt, torch.ones(T, n_shared, device=DEV)], 1).contiguous()
+    q, s = ops.per_tensor_cast_to_fp8(x)
+    d = torch.zeros(T, slots, H, dtype=torch.bfloat16, device=DEV)
+    ws = torch.empty(ops.moe_workspace_bytes(T, H, I, E_all, slots, 256), dtype=torch.uint8, device=DEV)
+    ops.moe_forward(q, s, *w, *w1, d, idx, ws, 256)
+    assert ops.device_status() == 0
+    assert torch.equal(out, ops.finalize_weighted(d, wt))
