@@ -994,11 +994,17 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
     if (block) DQ_CHECK(n_pad % 4 == 0 && n_pad >= n + 15 && is_aligned(a_scale, 16) && (!gated || (out_scale != nullptr && out_scale_t != nullptr)));
 
     // A pair shares each row between two CTAs, half the bytes through L2 for wide tiles, and computes rows in steps of 32 instead of
-    // 16. Pairs / singles, us per layer call: 31 rows per expert (H 2048, I 768, E 128, per-channel) 150 / 140; 50 (H 7168, I 2048,
-    // E 32, per-tensor) 254 / 253; 62 (E 128) 153 / 152; 100 (E 32) 280 / 290; 125 (H 4096, I 14336, E 8) 285 / 295; 250 (E 32, bf16)
-    // 701 / 793. Block mode hands its accumulators over every few K blocks, which across two SMs takes twice as long.
-    const bool pair = !block && n / E >= 48;
+    // 16. Pairs / singles, us per layer call. Even routing, rows per expert on average: 20 (H 2048, I 1408, E 64, k 6, per-tensor) 120 /
+    // 111; 30 (H 2048, I 768, E 128, k 8) per-tensor 145 / 141, per-channel 139 / 138, bf16 224 / 227; 30 (H 7168, I 2048, E 32) 246 / 243;
+    // 47 (E 128, per-channel) 146 / 142, bf16 235 / 235; 100 (E 32) 280 / 290; 125 (H 4096, I 14336, E 8) 285 / 295; 250 (E 32, bf16)
+    // 701 / 793. Skewed routing (Zipf 1.1), where a few experts have several hundred rows: 30 (E 128) per-tensor 125 / 134, per-channel
+    // 123 / 132, bf16 183 / 199; 30 (H 2880, I 2880, E 64, k 3, bf16) 352 / 381; 47 (E 128) 138 / 148, 137 / 145, 206 / 223. So from 30
+    // rows on, but from 48 where a tile per expert does not fill the chip and the singles' smaller ones spread further (H 2048, I 3072,
+    // E 3, k 1, bf16: 30 rows 38 / 35, 47 rows 39 / 35). Block mode hands its accumulators over every few K blocks, which across two SMs
+    // takes twice as long.
     const int cta_cols = gated ? kWRows / 2 : kWRows;
+    const bool fills = 2 * int64_t(E) * ceil_div(N, 2 * cta_cols) >= sm_count();
+    const bool pair = !block && n / E >= (fills ? 30 : 48);
     Params p;
     p.n_rows = n;
     p.N = N;

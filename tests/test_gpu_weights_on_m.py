@@ -1,6 +1,8 @@
 """The layer's grouped GEMM with the weights on M at the edges of its tiles: units of 16 rows (32 on CTA pairs), tiles of 64 rows in
 block mode and 256 otherwise, two or four K blocks per accumulator buffer, value rows that change weight-scale block inside a tile,
 output columns that end inside one. Also the router and the sort of a small block call in one launch."""
+import re
+
 import numpy as np
 import pytest
 import torch
@@ -10,7 +12,7 @@ from helpers import kernels_of
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
-# rows per expert: around the units and tiles of single CTAs (below 48 rows on average, block mode below 40) and of pairs
+# rows per expert: around the units and tiles of single CTAs (below 30 rows on average, block mode below 40) and of pairs
 FEW = [1, 15, 16, 17, 31, 32, 33, 0, 48, 63, 64, 65, 3, 97, 2, 30, 1, 0]
 FEWEST = [1, 0, 5, 16, 2, 13, 1, 4]
 MANY = [255, 256, 257, 288, 0, 289, 31, 33, 511, 513, 780, 1, 64, 1030]
@@ -80,6 +82,28 @@ def test_rows_equal_those_of_row_tiles(mode, rows, H, I):
     assert torch.equal(d, want)
     on_m = any("tcgen05_wm" in name for name in kernels_of(lambda: ops.moe_forward(*args)))
     assert on_m == (mode != 1024 or n < 40 * E)
+
+
+@pytest.mark.parametrize("rows,E,H,I,pairs", [(29, 37, 256, 192, [False, False]), (30, 37, 256, 192, [True, False]),
+                                              (30, 38, 512, 256, [True, True]), (47, 9, 512, 256, [False, False]),
+                                              (48, 9, 512, 256, [True, True])])
+@pytest.mark.parametrize("mode", [0, 256, 512])
+def test_lines_between_single_ctas_and_pairs(mode, rows, E, H, I, pairs):
+    """fc1 and fc2 run on CTA pairs from 30 rows per expert on if a tile of 128 or 256 columns per expert fills the 74 pairs (fc1: I /
+    128 tiles, fc2: H / 256), otherwise from 48."""
+    from dqmoe_b200 import ops
+    T = rows * E
+    z = lambda *shape: torch.zeros(*shape, dtype=torch.bfloat16 if mode == 0 else torch.uint8, device=DEV).view(torch.bfloat16 if mode == 0 else ops.FP8)
+    one = lambda n: torch.ones(n, device=DEV) if mode else None
+    ids = (torch.arange(T, dtype=torch.int32, device=DEV) % E).view(T, 1)
+    ws = torch.empty(ops.moe_workspace_bytes(T, H, I, E, 1, mode), dtype=torch.uint8, device=DEV)
+    d = torch.ones(T, 1, H, dtype=torch.bfloat16, device=DEV)
+    args = (z(T, H), one(1 if mode == 256 else T), z(E, 2 * I, H), one(E if mode == 256 else E * 2 * I), z(E, H, I),
+            one(E if mode == 256 else E * H), d, ids, ws, mode)
+    ops.moe_forward(*args)
+    assert ops.device_status() == 0 and not d.any()
+    forms = [m.group(1) == "1" for m in (re.search(r"tcgen05_wmILb\dELi\dELb\dELb(\d)E", name) for name in kernels_of(lambda: ops.moe_forward(*args))) if m]
+    assert forms == pairs
 
 
 @pytest.mark.parametrize("T,E,k,n_shared", [(1, 3, 1, 0), (5, 8, 2, 0), (31, 33, 8, 1), (32, 32, 8, 1), (33, 32, 8, 1), (85, 20, 3, 2),
