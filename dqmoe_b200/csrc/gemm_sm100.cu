@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "gemm_tile.cuh"
+#include "gemm_wm.cuh"
 #include "ptx_sm100.cuh"
 
 namespace dq {
@@ -226,9 +227,7 @@ __device__ __forceinline__ bool pairs_suit(const int* mtile_prefix, int E, int l
 // kBox = weight rows per TMA box (two boxes per stage, 2*kBox accumulator columns): 128 for
 // throughput, 64 when a launch would otherwise have fewer tiles than SMs (decode shapes).
 template <bool kFp8, int kMode, bool kGated, bool kPair, int kBox, int kElem = kElemBf16>
-__global__ void __launch_bounds__(kThreads, 1)
-moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ RowMaps rows_a,
-                                      const __grid_constant__ CUtensorMap tma_b, const Params p) {
+__device__ __forceinline__ void row_tiles(const RowMaps& rows_a, const CUtensorMap& tma_b, const Params& p) {
     pdl_launch();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -858,6 +857,56 @@ moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ RowMaps rows_a,
     }
 }
 
+template <bool kFp8, int kMode, bool kGated, bool kPair, int kBox, int kElem = kElemBf16>
+__global__ void __launch_bounds__(kThreads, 1)
+moe_GemmGrouped_GemmUniversal_tcgen05(const __grid_constant__ RowMaps rows_a, const __grid_constant__ CUtensorMap tma_b,
+                                      const __grid_constant__ Params p) {
+    row_tiles<kFp8, kMode, kGated, kPair, kBox, kElem>(rows_a, tma_b, p);
+}
+
+// Block mode with few rows per expert on average, both forms in one kernel: an expert of up to 64 rows is one tile for either, and
+// then the weights belong on M (gemm_wm.cuh). Beyond, it takes a tile of 64 rows after the other, each of which reads the weights
+// through L2 again, where a row tile takes 128 rows at once. The average does not tell: with skewed routing or experts without rows
+// some have far more. So the kernel counts both kinds of tile and takes the weights on M up to line / 10 x as many 64-row as 128-row
+// tiles. Row tiles always / weights on M always, us per MoE block, k 8 but where said, by that ratio: 1.00 (even routing) 80 tokens (H
+// 7168, I 2048, E 32) 299 / 260, 208 (H 2048, I 768, E 128) 153 / 123; 1.13 (Zipf 1.1) 107 (H 2048, I 1408, E 64 + 2 shared, k 6) 120 /
+// 100; 1.16 (Zipf) 120 (E 32) 313 / 295; 1.17 (Zipf) 320 (E 128) 127 / 131; 1.21 (Zipf) 416 (H 7168, E 256) 926 / 985; 1.31 800 (E 256)
+// 1202 / 1337; 1.38 1248 (E 256) 1558 / 1802; 1.96 (half the experts empty) 1248 (E 256) 1115 / 1854; 2.0 (every token to the same
+// eight) 80 (E 32) 113 / 146. That is a line of 1.2, but 1.5 where a reduction is below 2048: there the row tiles of this kernel take 5
+// to 15 % longer than those of a kernel of their own (480 tokens, E 128, row tiles alone / weights on M / row tiles here: Zipf, 1.23,
+// 146 / 148 / 162; half empty, 1.3, 116 / 127 / 133; 624 tokens, half empty, 1.97, 120 / 155 / 137), whichever body comes second in it.
+// Both in one launch, since a second one that leaves costs 2 to 4 us per GEMM. The choice is the same in every block, and in fc1 and
+// fc2. It reads the row counts before the wait, as the weights-on-M form does.
+__device__ __forceinline__ bool weights_on_m_suit(const int* offsets, int E, int line) {
+    extern __shared__ uint8_t smem_raw[];
+    int* balance = reinterpret_cast<int*>(smem_raw);
+    if (threadIdx.x == 0) *balance = 0;
+    __syncthreads();
+    int mine = 0;
+    for (int e = threadIdx.x; e < E; e += kThreads) {
+        const int rows = ld_relaxed_gpu(offsets + e + 1) - ld_relaxed_gpu(offsets + e);
+        mine += 10 * ((rows + 63) >> 6) - line * ((rows + 127) >> 7);
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31) == 0) atomicAdd(balance, mine);
+    __syncthreads();
+    const bool suit = *balance <= 0;
+    __syncthreads();  // the forms' own shared memory begins here
+    return suit;
+}
+
+template <bool kGated>
+__global__ void __launch_bounds__(kThreads, 1)
+moe_GemmGrouped_GemmUniversal_tcgen05_wm_by_counts(const __grid_constant__ gemm_wm::Maps maps, const __grid_constant__ gemm_wm::Params wm,
+                                                   const __grid_constant__ RowMaps rows_a, const __grid_constant__ CUtensorMap tma_b,
+                                                   const __grid_constant__ Params p, int line) {
+    static_assert(kThreads == gemm_wm::kThreads, "both forms run on the same block");
+    if (weights_on_m_suit(p.offsets, p.E, line))
+        gemm_wm::weights_on_m<true, gemm_wm::kBlock, kGated, false>(maps, wm);
+    else
+        row_tiles<true, kBlock, kGated, false, kBoxRows>(rows_a, tma_b, p);
+}
+
 // ---------------------------------------------------------------- host side
 
 template <bool kFp8, int kMode, bool kGated, bool kPair, int kBox, int kElem = kElemBf16>
@@ -922,6 +971,71 @@ static TileForm tile_form(int n, int E, int quant_mode, int elem, int wide_tiles
     return rows >= 512 ? kPairs : kSingles;
 }
 
+static Params sizes(int n, int N, int K, int E, int gated, int box, int kb_count) {
+    Params p = {};
+    p.n_rows = n;
+    p.N = N;
+    p.K = K;
+    p.E = E;
+    p.w_rows = gated ? 2 * N : N;
+    p.n_tiles = gated ? ceil_div(N, box) : ceil_div(N, 2 * box);
+    p.tile_w_rows = gated ? box : 2 * box;
+    p.box2_off = gated ? N : box;
+    p.kb_count = kb_count;
+    return p;
+}
+
+// Block mode, the form by the experts' row counts: wm is the launch with the weights on M, whose operands and outputs the row tiles
+// share; a_scale: the activation scales by row.
+template <bool kGated>
+static int launch_by_counts(const gemm_wm::Form& wm, const RowMaps& ma, const CUtensorMap& mb, const Params& p, int line,
+                            cudaStream_t stream) {
+    auto kern = moe_GemmGrouped_GemmUniversal_tcgen05_wm_by_counts<kGated>;
+    constexpr size_t kSmem = kSmemBytes > gemm_wm::smem_bytes<true>() ? kSmemBytes : gemm_wm::smem_bytes<true>();
+    static std::mutex mu;
+    static bool configured[kMaxDevices] = {};
+    int dev = 0;
+    DQ_CUDA(cudaGetDevice(&dev));
+    DQ_CHECK(dev >= 0 && dev < kMaxDevices);
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!configured[dev]) {
+            DQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmem)));
+            configured[dev] = true;
+        }
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(sm_count()), 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = kSmem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = p.n_rows <= kPdlGemmRows ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    DQ_CUDA(cudaLaunchKernelEx(&cfg, kern, wm.maps, wm.p, ma, mb, p, line));
+    return DQMOE_OK;
+}
+int grouped_gemm_by_counts(const gemm_wm::Form& wm, const float* a_scale, const void* w, const int* mtile_prefix, int K, int gated,
+                           int line, cudaStream_t stream) {
+    DQ_CHECK(a_scale != nullptr && mtile_prefix != nullptr);
+    Params p = sizes(wm.p.n_rows, wm.p.N, K, wm.p.E, gated, kBoxRows, wm.p.kb_count);
+    p.offsets = wm.p.offsets;
+    p.mtile_prefix = mtile_prefix;
+    p.sa = a_scale;
+    p.sb = wm.p.sb;
+    p.out = wm.p.out;
+    p.out_scale = wm.p.out_scale;
+    p.bias = wm.p.bias;
+    p.dest_to_src = wm.p.dest_to_src;
+    p.status = wm.p.status;
+    const RowMaps ma = {wm.maps.rows[3], wm.maps.rows[1]};
+    CUtensorMap mb;
+    DQ_RC(make_map(&mb, w, 1, uint64_t(p.E) * p.w_rows, uint64_t(K), kBoxRows));
+    return gated ? launch_by_counts<true>(wm, ma, mb, p, line, stream) : launch_by_counts<false>(wm, ma, mb, p, line, stream);
+}
+
 // elem: element type of the unquantised path (kElemBf16 / kElemHalf / kElemF32); bias: [E, gated ? 2N : N] fp32 or nullptr.
 int grouped_gemm(const void* a, const float* a_scale, const void* w, const float* w_scale, const int* offsets,
                  const int* mtile_prefix, int n, int N, int K, int E, int quant_mode, int gated, void* out,
@@ -957,16 +1071,7 @@ int grouped_gemm(const void* a, const float* a_scale, const void* w, const float
                         (2 * wide_tiles <= sm_count() || (mtiles_max <= 2 && wide_tiles < 2 * sm_count()));
     const int box = narrow ? 64 : kBoxRows;
 
-    Params p;
-    p.n_rows = n;
-    p.N = N;
-    p.K = K;
-    p.E = E;
-    p.w_rows = gated ? 2 * N : N;
-    p.n_tiles = gated ? ceil_div(N, box) : ceil_div(N, 2 * box);
-    p.tile_w_rows = gated ? box : 2 * box;
-    p.box2_off = gated ? N : box;
-    p.kb_count = kb_count;
+    Params p = sizes(n, N, K, E, gated, box, kb_count);
     p.by_counts = form == kByCounts ? 1 : 0;
     p.offsets = offsets;
     p.mtile_prefix = mtile_prefix;

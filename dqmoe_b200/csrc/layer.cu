@@ -37,7 +37,8 @@ enum Elem : int { kElemBf16 = 0, kElemHalf = 1, kElemF32 = 2 };  // element type
 namespace gemm_wm {
 int grouped_gemm(const void* a, const float* a_scale, const void* w, const float* w_scale, const int* offsets, int n, int N, int K,
                  int E, int quant_mode, int gated, void* out, float* amax, const int* dest_to_src, const float* bias,
-                 float* out_scale, float* out_scale_t, int n_pad, cudaStream_t stream);
+                 float* out_scale, float* out_scale_t, int n_pad, int line, const float* a_scale_rows, const int* mtile_prefix,
+                 cudaStream_t stream);
 }  // namespace gemm_wm
 
 namespace gemm_mx {
@@ -72,14 +73,23 @@ static bool tiled_scales(int64_t n, int H, int I, int E, int quant_mode) {
     const int64_t kh = ceil_div(H, 128), ki = ceil_div(I, 128);
     return tiles * (ki * kh + ceil_div(H, 256) * ki) >= kTiledTrips;
 }
-// Which grouped GEMMs have the weights on the M side (gemm_wm_sm100.cu): all of bf16 and per-tensor / per-channel FP8, and block
-// mode up to an average of 40 rows per expert. There the row tiles of 128 are mostly empty; beyond, an expert takes several tiles of
-// 64 rows, each of which reads the weights through L2 again. Row tiles / weights on M, us per call: MoE block of H 7168, I 2048, k 8:
-// E 32 + 1 shared 16 tokens (5 rows) 287 / 243, 96 (26) 309 / 267; E 256 300 tokens (9) 2022 / 1693, 1000 (31) 2173 / 1845; H 2048, I 768,
-// E 128, k 8 500 tokens (31) 174 / 160; H 4096, I 14336, E 8, k 2 100 tokens (25) 286 / 250. The line is where skewed routing (Zipf 1.1)
-// begins to lose: 31 rows 1264 / 1266 and 146 / 148, 37 rows 298 / 290, 44 rows 1509 / 1656 and 150 / 160, 50 rows 271 / 299, although even
-// routing still gains there (50 rows 315 / 279, 298 / 278); at 75 rows 290 / 425.
+// Which grouped GEMMs have the weights on the M side (gemm_wm.cuh): all of bf16 and per-tensor / per-channel FP8, and block mode up
+// to an average of 40 rows per expert. There the row tiles of 128 are mostly empty; beyond, an expert takes several tiles of 64 rows,
+// each of which reads the weights through L2 again. Row tiles / weights on M, us per call, even routing: MoE block of H 7168, I 2048,
+// k 8: E 32 + 1 shared 16 tokens (5 rows) 287 / 243, 96 (26) 309 / 267; E 256 300 tokens (9) 2022 / 1693, 1000 (31) 2173 / 1845; H 2048,
+// I 768, E 128, k 8 500 tokens (31) 174 / 160; H 4096, I 14336, E 8, k 2 100 tokens (25) 286 / 250; 50 rows 315 / 279 and 298 / 278, 75
+// rows 290 / 425.
+// With up to 64 tokens no expert has a second tile, whatever the routing (a token names an expert once), and weights that stay in L2
+// (126 MB) are read again for little: H 1024, I 2048, E 8, k 2, every token to the same two, 120 tokens, row tiles / weights on M 38 /
+// 31. In all other calls the kernel itself falls back on row tiles where skewed routing gives the experts too many tiles of 64 rows
+// (weights_on_m_suit in gemm_sm100.cu, where the two lines are explained).
 constexpr int kWmBlockRows = 40;
+constexpr int kWmBlockTokens = 64;
+constexpr int64_t kWmL2Weights = int64_t(1) << 27;
+static int counts_line(int T, int H, int I, int E) {
+    if (T <= kWmBlockTokens || 3 * int64_t(E) * H * I <= kWmL2Weights) return 0;
+    return H >= 2048 && I >= 2048 ? 12 : 15;
+}
 static bool weights_on_m(int64_t n, int E, int quant_mode, int elem) {
     if (quant_mode == DQMOE_QUANT_FP8_BLOCK) return n < kWmBlockRows * int64_t(E);
     return elem == gemm::kElemBf16;
@@ -226,6 +236,7 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
     float* act_scale = reinterpret_cast<float*>(ws + L.act_scale);
     const bool block = quant_mode == DQMOE_QUANT_FP8_BLOCK;
     const bool wm = layer::weights_on_m(n, E, quant_mode, elem);
+    const int line = block ? layer::counts_line(T, H, I, E) : 0;
     const bool tiled = !wm && layer::tiled_scales(n, H, I, E, quant_mode);
     float* perm_a_scale_t = (block && wm) || tiled ? reinterpret_cast<float*>(ws + L.perm_a_scale_t) : nullptr;
     float* act_scale_t = (block && wm) || tiled ? reinterpret_cast<float*>(ws + L.act_scale_t) : nullptr;
@@ -267,7 +278,8 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
     }
     if (wm)
         rc = gemm_wm::grouped_gemm(perm_a, block ? perm_a_scale_t : sa1, b, b_scale, offsets, n, I, H, E, quant_mode, 1,
-                                   two_pass ? act_bf16 : act, amax, nullptr, bias1, act_scale, act_scale_t, L.n_pad, stream);
+                                   two_pass ? act_bf16 : act, amax, nullptr, bias1, act_scale, act_scale_t, L.n_pad, line, perm_a_scale,
+                                   mtile_prefix, stream);
     else
         rc = gemm::grouped_gemm(perm_a, sa1, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, act, act_scale, nullptr, nullptr,
                                 nullptr, stream, elem, bias1, perm_a_scale_t, act_scale_t);
@@ -279,7 +291,7 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
     }
     if (wm)
         return gemm_wm::grouped_gemm(act, block ? act_scale_t : act_scale, b1, b1_scale, offsets, n, H, I, E, quant_mode, 0, d, nullptr,
-                                     dest_to_src, bias2, nullptr, nullptr, L.n_pad, stream);
+                                     dest_to_src, bias2, nullptr, nullptr, L.n_pad, line, act_scale, mtile_prefix, stream);
     return gemm::grouped_gemm(act, act_scale, b1, b1_scale, offsets, mtile_prefix, n, H, I, E, quant_mode, 0, d, nullptr, nullptr,
                               dest_to_src, nullptr, stream, elem, bias2, act_scale_t);
 }
@@ -451,6 +463,7 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
     void* act = lws + L.act;
     float* act_scale = reinterpret_cast<float*>(lws + L.act_scale);
     const bool wm = layer::weights_on_m(n, E, quant_mode, gemm::kElemBf16);
+    const int line = fp8 ? layer::counts_line(T, H, I, E) : 0;  // block mode, where it comes to it
     const bool tiled = !wm && layer::tiled_scales(n, H, I, E, quant_mode);
     float* perm_a_scale_t = fp8 && (wm || tiled) ? reinterpret_cast<float*>(lws + L.perm_a_scale_t) : nullptr;
     float* act_scale_t = fp8 && (wm || tiled) ? reinterpret_cast<float*>(lws + L.act_scale_t) : nullptr;
@@ -500,10 +513,10 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
     if (rc != DQMOE_OK) return rc;
     if (wm) {
         rc = gemm_wm::grouped_gemm(perm_a, perm_a_scale_t, b, b_scale, offsets, n, I, H, E, quant_mode, 1, act, nullptr, nullptr, nullptr,
-                                   act_scale, act_scale_t, L.n_pad, stream);
+                                   act_scale, act_scale_t, L.n_pad, line, perm_a_scale, mtile_prefix, stream);
         if (rc == DQMOE_OK)
             rc = gemm_wm::grouped_gemm(act, act_scale_t, b1, b1_scale, offsets, n, H, I, E, quant_mode, 0, d, nullptr, dest_to_src, nullptr,
-                                       nullptr, nullptr, L.n_pad, stream);
+                                       nullptr, nullptr, L.n_pad, line, act_scale, mtile_prefix, stream);
     } else {
         rc = gemm::grouped_gemm(perm_a, perm_a_scale, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, act, act_scale, nullptr,
                                 nullptr, nullptr, stream, gemm::kElemBf16, nullptr, perm_a_scale_t, act_scale_t);

@@ -106,6 +106,61 @@ def test_lines_between_single_ctas_and_pairs(mode, rows, E, H, I, pairs):
     assert forms == pairs
 
 
+LONG, SHORT, TINY = (4112, 2832), (6160, 1936), (640, 144)  # both reductions from 2048 on; one below; by their many experts
+
+
+@pytest.mark.parametrize("rows,shapes", [
+    ([30] * 8, {LONG: True, SHORT: True}),
+    ([10, 20, 30, 64, 65], {LONG: True, SHORT: True}),   # 6 tiles of 64 rows against 5 of 128
+    ([10, 20, 30, 65], {LONG: False, SHORT: True}),      # 5 against 4
+    ([10, 65, 0, 0], {LONG: False, SHORT: True}),        # 3 against 2
+    ([0, 300] + [0] * 8, {LONG: False, SHORT: False}),   # 5 against 3
+    ([300] + [3] * 20, {LONG: True, SHORT: True}),
+    ([128, 0, 0, 0], {LONG: False, SHORT: False}), ([129, 0, 0, 64, 0], {LONG: False, SHORT: True}), ([64, 64, 0, 0], {LONG: True, SHORT: True}),
+    ([1] * 700 + [65] * 170 + [0] * 40, {TINY: True}), ([65] * 300 + [1] * 350 + [0] * 10, {TINY: True}),
+    ([65] * 300 + [1] * 200 + [0] * 30, {TINY: False}),
+    ([300] + [0] * 9, {TINY: None})])                    # weights that stay in L2: on M without a count
+def test_row_counts_choose_the_form_of_block_calls(rows, shapes):
+    for (H, I), on_m in shapes.items():
+        check_block_form(rows, H, I, on_m)
+
+
+def check_block_form(rows, H, I, on_m):
+    """Block mode with more than 64 tokens and fewer than 40 rows per expert: the kernel takes row tiles where there are more than 1.2
+    (short reductions: 1.5) times as many tiles of 64 rows as of 128. Either way the result is that of calls of up to 64 tokens, which
+    have the weights on M, bit for bit, with biases too. The form shows in the intermediate's scales by column, which end the workspace
+    and only one writes."""
+    from dqmoe_b200 import ops
+    E, T = len(rows), sum(rows)
+    g = torch.Generator(device=DEV).manual_seed(T + H)
+    x = torch.randn(T, H, generator=g, device=DEV).to(torch.bfloat16)
+    b = ops.per_block_cast_to_fp8((torch.randn(E, 2 * I, H, generator=g, device=DEV) * 0.05).to(torch.bfloat16))
+    b1 = ops.per_block_cast_to_fp8((torch.randn(E, H, I, generator=g, device=DEV) * 0.05).to(torch.bfloat16))
+    bias1, bias2 = torch.randn(E, 2 * I, generator=g, device=DEV) * 0.1, torch.randn(E, H, generator=g, device=DEV) * 0.1
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(rows))[torch.randperm(T, generator=torch.Generator().manual_seed(T))]
+    ids = ids.to(torch.int32).view(T, 1).to(DEV)
+    q, s = ops.per_token_block_cast_to_fp8(x)
+
+    def run(first, last):
+        n = last - first
+        ws = torch.full((ops.moe_workspace_bytes(n, H, I, E, 1, 1024),), 0xAB, dtype=torch.uint8, device=DEV)
+        d = torch.zeros(n, 1, H, dtype=torch.bfloat16, device=DEV)
+        part = lambda t: t[first:last].contiguous()
+        args = (part(q.view(torch.uint8)).view(q.dtype), part(s), *b, *b1, d, part(ids), ws, 1024)
+        ops.moe_forward(*args, bias1=bias1, bias2=bias2)
+        assert ops.device_status() == 0
+        names = kernels_of(lambda: ops.moe_forward(*args, bias1=bias1, bias2=bias2))
+        assert sum("by_counts" in name for name in names) == (2 if n > 64 and on_m is not None else 0), names
+        by_column = (n + 16 + 3) // 4 * 4 * ((I + 127) // 128) * 4
+        return d, bool((ws[-(-(-by_column // 256) * 256):] != 0xAB).any())
+
+    d, used = run(0, T)
+    assert used == (on_m is not False)
+    for first in range(0, min(T, 512), 64):
+        small, used = run(first, min(T, first + 64))
+        assert used and torch.equal(d[first:first + 64], small)
+
+
 @pytest.mark.parametrize("T,E,k,n_shared", [(1, 3, 1, 0), (5, 8, 2, 0), (31, 33, 8, 1), (32, 32, 8, 1), (33, 32, 8, 1), (85, 20, 3, 2),
                                             (256, 70, 1, 5), (257, 70, 1, 5), (16, 256, 4, 0)])
 @pytest.mark.parametrize("scoring", ["softmax", "sigmoid"])

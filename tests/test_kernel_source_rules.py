@@ -84,24 +84,37 @@ def test_block_scales_are_passed_on_by_a_release():
         assert f"mbar_init(&st.{bar}, kMode == kBlock ? 2 : 1)" in text, bar
 
 
+def test_bodies_of_the_grouped_gemms_read_with_plain_loads():
+    """The same for the two forms whose kernels only call them."""
+    for name, entry in (("gemm_sm100.cu", "void row_tiles("), ("gemm_wm.cuh", "void weights_on_m(")):
+        text = source(name)
+        body = braces(text, text.index(entry))
+        assert "pdl_wait(" in body
+        for word in ("__restrict__", "__ldg", "ld_nc16", ".nc"):
+            assert word not in body, (name, word)
+
+
 def test_what_is_read_before_the_wait_comes_past_l1():
     """The weights-on-M GEMM and the layer's block-scaled one copy the sort's table before their own griddepcontrol.wait. The sort is
     over by then, but only the wait covers lines of an earlier call's table that are still in L1."""
-    for name, tables in (("gemm_wm_sm100.cu", ["offsets"]), ("gemm_mx_sm100.cu", ["offsets", "mtile_prefix"])):
+    for name, entry, tables in (("gemm_wm.cuh", "void weights_on_m(", ["offsets"]),
+                                ("gemm_mx_sm100.cu", "__global__", ["offsets", "mtile_prefix"])):
         text = source(name)
-        kernel = braces(text, text.index("__global__"))
+        kernel = braces(text, text.index(entry))
         for table in tables:
             reads = re.findall(r"[\w ]*\(?\bp\." + table + r"\b", kernel)
             assert reads and all(r.endswith("ld_relaxed_gpu(p." + table) for r in reads), (name, reads)
     assert "ld.relaxed.gpu.global" in source("common.cuh")
+    choice = braces(source("gemm_sm100.cu"), source("gemm_sm100.cu").index("bool weights_on_m_suit("))
+    assert len(re.findall(r"ld_relaxed_gpu\(offsets \+", choice)) == len(re.findall(r"\boffsets\b", choice)) == 2
 
 
 def test_roles_wait_for_the_kernel_before_before_they_wait_at_a_barrier():
     """A wait at a barrier gives up after a time that is meant for this kernel. Launched early, a role that has not yet waited for
     the kernel before would count that one's rest, however long it is held up, against it."""
-    for name in ("gemm_wm_sm100.cu", "gemm_mx_sm100.cu"):
+    for name, entry in (("gemm_wm.cuh", "void weights_on_m("), ("gemm_mx_sm100.cu", "__global__")):
         text = source(name)
-        kernel = braces(text, text.index("__global__"))
+        kernel = braces(text, text.index(entry))
         roles = kernel[kernel.index("if (warp < 4) {"):]
         at = [m.start() for m in re.finditer(r"if \(warp == \d\)|else if constexpr \(kBlockMode\) \{\s*pdl_wait|"
                                              r"else \{\s*(?:ptx::setmaxnreg_inc<\w+>\(\);\s*)?pdl_wait", roles)] + [len(roles)]
@@ -112,5 +125,5 @@ def test_roles_wait_for_the_kernel_before_before_they_wait_at_a_barrier():
             if m:
                 waits += 1
                 assert "pdl_wait()" in role[:m.start()], (name, role[:200])
-        assert waits == {"gemm_wm_sm100.cu": 5, "gemm_mx_sm100.cu": 3}[name], name
+        assert waits == {"gemm_wm.cuh": 5, "gemm_mx_sm100.cu": 3}[name], name
         assert not re.search(r"\bmbar_wait(_warp)?\(", kernel[:kernel.index("if (warp < 4) {")]), name
