@@ -73,8 +73,8 @@ static bool tiled_scales(int64_t n, int H, int I, int E, int quant_mode) {
     const int64_t kh = ceil_div(H, 128), ki = ceil_div(I, 128);
     return tiles * (ki * kh + ceil_div(H, 256) * ki) >= kTiledTrips;
 }
-// Which grouped GEMMs have the weights on the M side (gemm_wm.cuh): all of bf16 and per-tensor / per-channel FP8, and block mode up
-// to an average of 40 rows per expert. There the row tiles of 128 are mostly empty; beyond, an expert takes several tiles of 64 rows,
+// Which grouped GEMMs have the weights on the M side (gemm_wm.cuh): bf16 and per-tensor / per-channel FP8 but for small models, and
+// block mode up to an average of 40 rows per expert. There the row tiles of 128 are mostly empty; beyond, an expert takes several tiles of 64 rows,
 // each of which reads the weights through L2 again. Row tiles / weights on M, us per call, even routing: MoE block of H 7168, I 2048,
 // k 8: E 32 + 1 shared 16 tokens (5 rows) 287 / 243, 96 (26) 309 / 267; E 256 300 tokens (9) 2022 / 1693, 1000 (31) 2173 / 1845; H 2048,
 // I 768, E 128, k 8 500 tokens (31) 174 / 160; H 4096, I 14336, E 8, k 2 100 tokens (25) 286 / 250; 50 rows 315 / 279 and 298 / 278, 75
@@ -90,9 +90,18 @@ static int counts_line(int T, int H, int I, int E) {
     if (T <= kWmBlockTokens || 3 * int64_t(E) * H * I <= kWmL2Weights) return 0;
     return H >= 2048 && I >= 2048 ? 12 : 15;
 }
-static bool weights_on_m(int64_t n, int E, int quant_mode, int elem) {
+// Small models otherwise: where one tile per expert leaves most SMs without work in fc2 and the weights stay in L2, a launch is a chain of
+// latencies, in which the row tiles' shorter MMAs and their prologue under the kernel before count. Row tiles / weights on M, us per call
+// by rows per expert: bf16 H 2048, I 3072, E 1 (16 tiles) 30 rows 28 / 28, 60 27 / 31, 200 28 / 38; per-tensor block 100 rows 34 / 39,
+// 200 36 / 47; bf16 H 768, I 1536, E 5, k 2 (30) 24 rows 20 / 20, 60 23 / 24, 240 25 / 30; H 512, I 2048, E 8, k 2 (32) 15 rows 24 / 22,
+// 75 24 / 28, per-channel 375 47 / 56; below 24 rows the weights on M gain (E 8, 3 rows 25 / 22; E 5, 5 rows 23 / 20). With 48 tiles (H
+// 2048, I 3072, E 3) 60 rows 44 / 36, and with weights from HBM (H 4096, I 14336, E 1, 32 tiles) 129 rows 125 / 110.
+constexpr int kWmTiles = 36, kWmSmallRows = 24;
+static bool weights_on_m(int64_t n, int H, int I, int E, int quant_mode, int elem) {
     if (quant_mode == DQMOE_QUANT_FP8_BLOCK) return n < kWmBlockRows * int64_t(E);
-    return elem == gemm::kElemBf16;
+    if (elem != gemm::kElemBf16) return false;
+    const int64_t weight_bytes = 3 * int64_t(E) * H * I * (quant_mode == DQMOE_QUANT_NONE ? 2 : 1);
+    return int64_t(E) * ceil_div(H, 128) >= kWmTiles || weight_bytes > kWmL2Weights || n < kWmSmallRows * int64_t(E);
 }
 constexpr int kDecodeRows = 8;  // up to this many expanded rows the GEMV path of decode.cu is used (bf16, per-tensor FP8)
 static bool on_decode_path(int n, int H, int I, int quant_mode, int elem, bool biased) {
@@ -235,7 +244,7 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
     void* act = ws + L.act;
     float* act_scale = reinterpret_cast<float*>(ws + L.act_scale);
     const bool block = quant_mode == DQMOE_QUANT_FP8_BLOCK;
-    const bool wm = layer::weights_on_m(n, E, quant_mode, elem);
+    const bool wm = layer::weights_on_m(n, H, I, E, quant_mode, elem);
     const int line = block ? layer::counts_line(T, H, I, E) : 0;
     const bool tiled = !wm && layer::tiled_scales(n, H, I, E, quant_mode);
     float* perm_a_scale_t = (block && wm) || tiled ? reinterpret_cast<float*>(ws + L.perm_a_scale_t) : nullptr;
@@ -281,8 +290,8 @@ static int moe_forward_impl(const void* a, const float* a_scale, const void* b, 
                                    two_pass ? act_bf16 : act, amax, nullptr, bias1, act_scale, act_scale_t, L.n_pad, line, perm_a_scale,
                                    mtile_prefix, stream);
     else
-        rc = gemm::grouped_gemm(perm_a, sa1, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, act, act_scale, nullptr, nullptr,
-                                nullptr, stream, elem, bias1, perm_a_scale_t, act_scale_t);
+        rc = gemm::grouped_gemm(perm_a, sa1, b, b_scale, offsets, mtile_prefix, n, I, H, E, quant_mode, 1, two_pass ? act_bf16 : act,
+                                act_scale, amax, nullptr, nullptr, stream, elem, bias1, perm_a_scale_t, act_scale_t);
     if (rc != DQMOE_OK) return rc;
     if (two_pass) {
         rc = dqmoe_requant_from_amax(act_bf16, n, I, amax, quant_mode == DQMOE_QUANT_FP8_CHANNEL ? 1 : 0, act,
@@ -462,7 +471,7 @@ static int moe_block_impl(const void* x_bf16, const float* logits, const void* b
     float* perm_a_scale = reinterpret_cast<float*>(lws + L.perm_a_scale);
     void* act = lws + L.act;
     float* act_scale = reinterpret_cast<float*>(lws + L.act_scale);
-    const bool wm = layer::weights_on_m(n, E, quant_mode, gemm::kElemBf16);
+    const bool wm = layer::weights_on_m(n, H, I, E, quant_mode, gemm::kElemBf16);
     const int line = fp8 ? layer::counts_line(T, H, I, E) : 0;  // block mode, where it comes to it
     const bool tiled = !wm && layer::tiled_scales(n, H, I, E, quant_mode);
     float* perm_a_scale_t = fp8 && (wm || tiled) ? reinterpret_cast<float*>(lws + L.perm_a_scale_t) : nullptr;

@@ -161,6 +161,34 @@ def check_block_form(rows, H, I, on_m):
         assert used and torch.equal(d[first:first + 64], small)
 
 
+@pytest.mark.parametrize("T,E,k,H,I,on_m", [
+    (23, 1, 1, 2048, 512, True), (24, 1, 1, 2048, 512, False), (200, 1, 1, 2048, 512, False),  # rows per expert
+    (200, 3, 1, 1408, 512, False), (200, 3, 1, 1536, 512, True),                               # 33 and 36 tiles
+    (300, 2, 2, 2048, 10912, False), (300, 2, 2, 2048, 10928, None)])                          # weights of 128 MiB in FP8; in bf16 beyond
+@pytest.mark.parametrize("mode", [0, 256, 512])
+def test_layers_of_small_models_have_row_tiles(mode, T, E, k, H, I, on_m):
+    """On both sides of the lines the results are those of the row tiles, bit for bit, with biases as without (of zero)."""
+    from dqmoe_b200 import ops
+    if I > 10000:
+        on_m = mode == 0 or on_m is None
+    g = torch.Generator(device=DEV).manual_seed(T + H + mode)
+    x = torch.randn(T, H, generator=g, device=DEV).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E, generator=torch.Generator().manual_seed(t))[:k] for t in range(T)]).to(torch.int32).to(DEV)
+    w = (torch.randn(E, 2 * I, H, generator=g, device=DEV) * 0.05).to(torch.bfloat16)
+    w1 = (torch.randn(E, H, I, generator=g, device=DEV) * 0.05).to(torch.bfloat16)
+    cast = {0: lambda t: (t, None), 256: lambda t: ops.per_tensor_cast_to_fp8(t, per_expert=True), 512: ops.per_channel_cast_to_fp8}[mode]
+    b, b1 = cast(w), cast(w1)
+    q, s, want = by_row_tiles(ops, mode, x, b, b1, ids, E)
+    bs, b1s = (b[1].reshape(-1), b1[1].reshape(-1)) if mode == 512 else (b[1], b1[1])
+    ws = torch.empty(ops.moe_workspace_bytes(T, H, I, E, k, mode), dtype=torch.uint8, device=DEV)
+    for bias in ({}, dict(bias1=torch.zeros(E, 2 * I, device=DEV), bias2=torch.zeros(E, H, device=DEV))):
+        d = torch.zeros(T, k, H, dtype=torch.bfloat16, device=DEV)
+        call = lambda: ops.moe_forward(q, s, b[0], bs, b1[0], b1s, d, ids, ws, mode, **bias)
+        call()
+        assert ops.device_status() == 0 and torch.equal(d, want)
+        assert any("tcgen05_wm" in name for name in kernels_of(call)) == on_m
+
+
 @pytest.mark.parametrize("T,E,k,n_shared", [(1, 3, 1, 0), (5, 8, 2, 0), (31, 33, 8, 1), (32, 32, 8, 1), (33, 32, 8, 1), (85, 20, 3, 2),
                                             (256, 70, 1, 5), (257, 70, 1, 5), (16, 256, 4, 0)])
 @pytest.mark.parametrize("scoring", ["softmax", "sigmoid"])
