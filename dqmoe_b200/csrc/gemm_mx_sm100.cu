@@ -218,7 +218,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ gemm::RowMaps r
             int ahead = 0;  // stages whose weights are on their way before the wait
             for (int t = tile_first, cursor = 0; p.early && ahead < kStages && t < total_tiles; t += tile_step) {
                 const Tile tl = decode_tile(t, cursor, st, p.n_tiles);
-                const int rows = gemm::rows_to_load(tl.row_end - tl.row0);
+                const int rows = gemm::rows_to_load(tl.row_end - tl.row0, total_tiles <= tile_step);
                 for (int kb = 0; ahead < kStages && kb < kb_count; ++kb, ++ahead) load_weights(tl, rows, kb, ahead);
             }
             pdl_wait();
@@ -227,7 +227,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ gemm::RowMaps r
             bool ok = true;
             for (int t = tile_first; ok && t < total_tiles; t += tile_step) {
                 const Tile tl = decode_tile(t, e_cursor, st, p.n_tiles);
-                const int rows = gemm::rows_to_load(tl.row_end - tl.row0);
+                const int rows = gemm::rows_to_load(tl.row_end - tl.row0, total_tiles <= tile_step);
                 const uint8_t* sf_a = p.sfa + size_t(tl.mtile) * kb_count * kSfPart;
                 for (int kb = 0; kb < kb_count; ++kb, ++it) {
                     const int s = it % kStages;

@@ -325,7 +325,7 @@ __device__ __forceinline__ void row_tiles(const RowMaps& rows_a, const CUtensorM
                 const Tile tl = decode_tile<kPair>(t, e_cursor, st, p.n_tiles, cta_rank);
                 const int wrow0 = tl.e * p.w_rows + tl.nt * p.tile_w_rows;
                 const int wrow1 = wrow0 + p.box2_off;
-                [[maybe_unused]] const int rows = rows_to_load(tl.row_end - tl.row0);  // single CTAs
+                [[maybe_unused]] const int rows = rows_to_load(tl.row_end - tl.row0, total_tiles <= tile_step);  // single CTAs
                 for (int kb = 0; kb < kb_count; ++kb, ++it) {
                     const int s = it % kNumStages;
                     const uint32_t ph = (it / kNumStages) & 1u;

@@ -10,7 +10,7 @@ DEV = "cuda"
 ROWS = [1, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 0, 161]
 
 
-@pytest.mark.parametrize("H,I", [(256, 384), (640, 128)])
+@pytest.mark.parametrize("H,I", [(256, 384), (640, 128), (4096, 1280)])  # one tile per block at most in both GEMMs; in fc2; in none
 @pytest.mark.parametrize("mode", [1024, 2048])
 def test_partly_filled_row_tiles(mode, H, I):
     from dqmoe_b200 import ops
