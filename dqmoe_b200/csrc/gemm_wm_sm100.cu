@@ -131,10 +131,14 @@ static int form(const void* a, const float* a_scale, const void* w, const float*
     p.status = device_status_word();
     if (p.status == nullptr) return DQMOE_ERR_CUDA;
 
-    // Only the boxes that a tile of this call can need: encoding a map takes 0.5 us (MoE block of 5 tokens: C++ 23.3 -> 20.3 us).
+    // Only the boxes that a tile of this call can need (each CTA of a pair loads half of one): encoding a map takes 0.5 us (MoE block
+    // of 5 tokens: C++ 23.3 -> 20.3 us).
+    const int unit = pair ? 32 : 16;
+    const int limit = block ? kBlockTok : kMaxTok;
+    const int most = (n < limit ? ceil_div(n, unit) * unit : limit) / (pair ? 2 : 1);
     f->maps = {};
     DQ_RC(make_weight_map(&f->maps.w, w, esz, E, N, K, gated != 0));
-    for (int i = 0; i < 4 && (i == 0 || row_tiles_too || (16 << i) <= n + 31); ++i) DQ_RC(gemm::make_map(&f->maps.rows[i], a, esz, uint64_t(n), uint64_t(K), 16 << i));
+    for (int i = 0; i < 4 && (row_tiles_too || (16 << i) <= most); ++i) DQ_RC(gemm::make_map(&f->maps.rows[i], a, esz, uint64_t(n), uint64_t(K), 16 << i));
     return DQMOE_OK;
 }
 
