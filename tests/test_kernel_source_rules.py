@@ -127,3 +127,41 @@ def test_roles_wait_for_the_kernel_before_before_they_wait_at_a_barrier():
                 assert "pdl_wait()" in role[:m.start()], (name, role[:200])
         assert waits == {"gemm_wm.cuh": 5, "gemm_mx_sm100.cu": 3}[name], name
         assert not re.search(r"\bmbar_wait(_warp)?\(", kernel[:kernel.index("if (warp < 4) {")]), name
+
+
+def test_whole_warps_of_the_weights_on_m_form():
+    """The same two rules there: the warp of the scale products and both epilogues wait together, and one lane arrives for a warp that
+    has met."""
+    text = source("gemm_wm.cuh")
+    kernel = braces(text, text.index("void weights_on_m("))
+    products = braces(kernel, kernel.index("else if (warp == 2)"))
+    block = braces(kernel, kernel.index("else if constexpr (kBlockMode)", kernel.index("else if (warp == 2)")))
+    plain = braces(kernel, kernel.index("else {", kernel.index(block) + len(block)))
+    for role in (products, block, plain):
+        assert "mbar_wait_warp(" in role and not re.search(r"\bmbar_wait\(", role), role[:100]
+    for role, name in ((block, "auto release"), (plain, "auto release_tmem")):
+        release = braces(role, role.index(name))
+        assert release.index("__syncwarp()") < release.index("mbar_arrive")
+        assert "mbar_arrive" not in role.replace(release, "")
+    arrivals = [m.start() for m in re.finditer("mbar_arrive", products)]
+    assert len(arrivals) == 1 and "__syncwarp()" in products[arrivals[0] - 100:arrivals[0]]
+
+
+def test_kernels_before_an_early_gemm_start_it_after_their_own_wait():
+    """An early grouped GEMM reads the sort's table and the weights before its own wait. That holds if it cannot start before the sort is
+    over: a kernel that may stand right behind the sort lets its dependents start only after its wait, and so does an early GEMM
+    itself. Others may stand between two of these, since they start behind the first: the re-quantisation pass and fc1's row tiles."""
+    for name, kernels in (("permute.cu", ["scatter_rows_kernel", "scatter_quant_1x128_kernel"]),
+                          ("quant_mx.cu", ["quant_rows_kernel", "tile_scales_kernel"])):
+        text = source(name)
+        for kernel in kernels:
+            body = braces(text, text.index(kernel + "("))
+            assert re.match(r"{\s*pdl_wait\(\);\s*pdl_launch\(\);", body) and body.count("pdl_") == 2, kernel
+    wm = source("gemm_wm.cuh")
+    wm = braces(wm, wm.index("void weights_on_m("))
+    assert re.findall(r"if constexpr \((!?kEarly)\) pdl_launch\(\)", wm) == ["!kEarly", "kEarly", "kEarly"]
+    assert len(re.findall(r"pdl_wait\(\);\s*if constexpr \(kEarly\) pdl_launch\(\)", wm)) == 2 and wm.count("pdl_launch()") == 3
+    mx = source("gemm_mx_sm100.cu")
+    mx = braces(mx, mx.index("__global__"))
+    assert re.findall(r"if \((!?p\.early)\) pdl_launch\(\)", mx) == ["!p.early", "p.early"] and mx.count("pdl_launch()") == 2
+    assert len(re.findall(r"pdl_wait\(\);\s*if \(p\.early\) pdl_launch\(\)", mx)) == 1
