@@ -5,6 +5,7 @@ import torch
 
 from helpers import kernels_of
 from oracle import moe_oracle as orc
+from test_gpu_weights_on_m import by_row_tiles
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -14,6 +15,7 @@ ROWS = [1, 31, 32, 33, 0, 64, 65, 96, 97, 127, 128, 129, 160, 161]
 @pytest.mark.parametrize("H,I", [(128, 256), (64, 144), (640, 1152), (1344, 192)])
 @pytest.mark.parametrize("mode", [0, 256, 512, 1024])
 def test_ragged_row_counts_match_oracle(mode, H, I):
+    """The layer: row tiles in block mode, the weights on M in the others, whose row tiles the next test has."""
     from dqmoe_b200 import ops
     E, T = len(ROWS), sum(ROWS)
     g = torch.Generator().manual_seed(H + I)
@@ -34,6 +36,31 @@ def test_ragged_row_counts_match_oracle(mode, H, I):
         ops.moe_forward(*q, d, ids.to(DEV), ws, mode)
     assert ops.device_status() == 0
     # the layer tolerance: a rounding of the intermediate that flips moves one e4m3 step (2^-3 relative) of one of I terms
+    assert orc.cosine(d.cpu(), ref) >= 0.999 and orc.max_rel_err(d.cpu(), ref) <= 2e-2
+
+
+@pytest.mark.parametrize("H,I", [(128, 256), (640, 1152)])
+@pytest.mark.parametrize("mode", [0, 256, 512])
+def test_ragged_row_counts_of_the_stand_alone_operators(mode, H, I):
+    """The stand-alone grouped GEMM has its row tiles in every mode."""
+    from dqmoe_b200 import ops
+    E, T = len(ROWS), sum(ROWS)
+    g = torch.Generator().manual_seed(H + I)
+    a = torch.randn(T, H, generator=g).to(torch.bfloat16)
+    b = (torch.randn(E, 2 * I, H, generator=g) * 0.05).to(torch.bfloat16)
+    b1 = (torch.randn(E, H, I, generator=g) * 0.05).to(torch.bfloat16)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(ROWS))[torch.randperm(T, generator=g)]
+    ids = ids.to(torch.int32).view(T, 1)
+    if mode == 0:
+        ref = orc.moe_layer_bf16(a, b, b1, ids, E)
+        w = (b.to(DEV), None), (b1.to(DEV), None)
+    else:
+        qs = orc.quantize_inputs(a, b, b1, mode)
+        ref = orc.moe_layer_fp8(*qs, ids, E, mode)
+        w = [tuple(t.to(DEV).contiguous() for t in pair) for pair in (qs[2:4], qs[4:6])]
+    _, _, d = by_row_tiles(ops, mode, a.to(DEV), *w, ids.to(DEV), E)
+    assert ops.device_status() == 0
+    # the layer tolerance (see above)
     assert orc.cosine(d.cpu(), ref) >= 0.999 and orc.max_rel_err(d.cpu(), ref) <= 2e-2
 
 
