@@ -86,8 +86,8 @@ static inline int make_row_maps(RowMaps* maps, const void* base, int esz, uint64
     return make_map(&maps->all, base, esz, rows, cols, 128);
 }
 // In a launch of at most one tile per block nothing waits for L2, and every further copy that the producer thread issues lengthens the
-// K loop: there all 128 rows come in one. Boxes / one copy, us per call: bf16 layer of H 2048, I 3072, E 1, 60 tokens 32 / 27, 200 tokens
-// 33 / 28, 300 tokens 33 / 28.
+// K loop: there all 128 rows come in one. Boxes / one copy, us per call: bf16 layer of H 2048, I 3072, E 1, 60 tokens 32 / 28, 200 tokens
+// 33 / 30, 300 tokens 33 / 30.
 // rows that a tile with `left` >= 1 rows of its expert ahead loads, and the loads
 __device__ __forceinline__ int rows_to_load(int left, bool one_wave) { return one_wave || left > 96 ? 128 : (left + 31) & ~31; }
 __device__ __forceinline__ void load_rows(uint8_t* smem_dst, const RowMaps& maps, int k0, int row0, int rows, uint64_t* bar) {

@@ -160,7 +160,8 @@ static Layout make_layout(int T, int H, int I, int E, int k, int quant_mode, int
                                    : quant_mode == DQMOE_QUANT_FP8_TENSOR ? 1 : 0;
     L.act_scale = add(act_scale_elems * sizeof(float));
     // block mode: the scale matrices a second time for the grouped GEMMs, by tile (every expert may add a partly filled one) or by
-    // column (n_pad rows: a tile reads on to a multiple of 16)
+    // column (n_pad rows: a tile reads on to a multiple of 16). The latter also between the two ranges that use them, so that the size
+    // never falls as T grows: a workspace taken for the most tokens serves any number.
     const bool tiled = tiled_scales(int64_t(n), H, I, E, quant_mode);
     L.n_pad = quant_mode == DQMOE_QUANT_FP8_BLOCK ? int(align_up(n + 16, 4)) : 0;
     const size_t scale_rows = tiled ? ((n + 127) / 128 + (size_t(E) < n ? size_t(E) : n)) * 128 : size_t(L.n_pad);

@@ -30,6 +30,16 @@ def test_workspace_size_is_host_arithmetic():
     assert lib.dqmoe_moe_workspace_bytes(64, 1024, 2048, 8, 2, 512) > small
 
 
+@pytest.mark.parametrize("mode", [0, 256, 512, 1024, 2048, 4096])
+@pytest.mark.parametrize("H,I,E,k", [(2048, 2048, 2, 1), (7168, 2048, 33, 9), (4096, 14336, 8, 2), (128, 128, 700, 1)])
+def test_workspace_for_the_most_tokens_serves_fewer(mode, H, I, E, k):
+    """Programs allocate for their largest batch, and the plugin lays its own out by each call's: the size must not fall anywhere as T
+    grows, also where a call changes its form (block mode: 40 and some 192 rows per expert)."""
+    lib = _lib.load()
+    sizes = [lib.dqmoe_moe_workspace_bytes(T, H, I, E, k, mode) for T in [*range(1, 1200), *range(1200, 20000, 37)]]
+    assert all(0 < a <= b for a, b in zip(sizes, sizes[1:]))
+
+
 def test_argument_errors_have_reference_format():
     lib = _lib.load()
     rc = lib.dqmoe_route_topk(None, 4, 8, 9, 0, None, None, None)  # k > E
