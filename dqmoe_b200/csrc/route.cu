@@ -475,14 +475,16 @@ int route_topk(const float* logits, int T, int E, int k, int n_shared, int scori
 }
 
 // Router, then the expert sort of the rows it names (E routed experts, n_shared shared ones behind them).
-// In one launch up to 256 choices (T k): it saves a launch, but a warp takes its T / 32 tokens one choice after the other. Two
-// kernels / one, us per MoE block: 10 choices (H 1024, I 2048, E 8) 30.4 / 29.6; 768 (H 7168, I 2048, E 33) 277 / 285.
-constexpr int kRouteSortChoices = 256;
+// In one launch while a warp has at most two tokens, and up to 192 choices (T k): it saves a launch, but a warp takes its T / 32 tokens one
+// choice after the other. Two kernels / one, us per MoE block: 10 choices (H 1024, I 2048, E 8, k 2) 30.4 / 29.6, 64 tokens 30.9 / 27.9,
+// 96 30.8 / 30.1, 128 30.7 / 32.5; H 2048, I 3072, E 3, k 1 64 tokens 31.1 / 31.1, 96 33.7 / 35.7, 192 42.1 / 46.3; H 2048, I 1408, E 64,
+// k 6 32 tokens 105.7 / 105.7, 43 105.6 / 108.3; 768 choices (H 7168, I 2048, E 33) 277 / 285.
+constexpr int kRouteSortTokens = 64, kRouteSortChoices = 192;
 int route_and_sort(const float* logits, int T, int E, int k, int n_shared, int scoring, int* indices, float* weights, int* counts,
                    int* offsets, int* mtile_prefix, int* dest_to_src, int* src_to_dest, void* ws, size_t ws_bytes, cudaStream_t stream) {
     const int slots = k + n_shared, E_all = E + n_shared;
     const size_t smem = (size_t(kRouteSortWarps) * (E_all + 1) + 2 * (E_all + 2)) * sizeof(int);
-    if (T == 0 || int64_t(T) * k > kRouteSortChoices || int64_t(T) * slots > kChunk || E > 256 || smem > 48 * 1024) {
+    if (T == 0 || T > kRouteSortTokens || int64_t(T) * k > kRouteSortChoices || int64_t(T) * slots > kChunk || E > 256 || smem > 48 * 1024) {
         DQ_RC(route_topk(logits, T, E, k, n_shared, scoring, indices, weights, stream));
         return route_sort(indices, T * slots, E_all, counts, offsets, mtile_prefix, dest_to_src, src_to_dest, ws, ws_bytes, stream);
     }

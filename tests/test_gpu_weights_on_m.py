@@ -190,10 +190,11 @@ def test_layers_of_small_models_have_row_tiles(mode, T, E, k, H, I, on_m):
 
 
 @pytest.mark.parametrize("T,E,k,n_shared", [(1, 3, 1, 0), (5, 8, 2, 0), (31, 33, 8, 1), (32, 32, 8, 1), (33, 32, 8, 1), (85, 20, 3, 2),
-                                            (256, 70, 1, 5), (257, 70, 1, 5), (16, 256, 4, 0)])
+                                            (256, 70, 1, 5), (257, 70, 1, 5), (16, 256, 4, 0), (64, 9, 3, 0),
+                                            (64, 9, 4, 0), (65, 9, 1, 0), (32, 40, 6, 2)])
 @pytest.mark.parametrize("scoring", ["softmax", "sigmoid"])
 def test_router_and_sort_of_a_small_block_call(T, E, k, n_shared, scoring):
-    """The block's router and sort in one launch (up to 256 choices) name the same experts, weights and order as the two operators:
+    """The block's router and sort, in one launch up to 64 tokens and 192 choices, name the same experts, weights and order as the two operators:
     the block's result is that of the layer on the operators' routing, weighted."""
     from dqmoe_b200 import ops
     H, I = 128, 64
@@ -213,7 +214,7 @@ def test_router_and_sort_of_a_small_block_call(T, E, k, n_shared, scoring):
     block = lambda: ops.moe_block(x, logits, *b, *b1, k, scoring, 1024, workspace=ws, n_shared=n_shared)
     out = block()
     names = kernels_of(block)
-    assert any("route_sort_small" in nm for nm in names) == (T * k <= 256), names
+    assert any("route_sort_small" in nm for nm in names) == (T <= 64 and T * k <= 192), names
     idx, wt = ops.route_topk(logits, k, scoring)
     shared = torch.arange(E, E_all, dtype=torch.int32, device=DEV).expand(T, n_shared)
     idx = torch.cat([idx, shared], 1).contiguous()
