@@ -63,12 +63,16 @@ namespace decode {
 constexpr int kAmaxParts = 4096;  // floats the layer workspace holds for the per-block amax values of the decode path's fc1
 }
 
-// Programmatic dependent launch. Every kernel launched through launch_pdl calls pdl_launch() and pdl_wait() first thing
-// (the grouped GEMMs set up their barriers and TMEM in between; the row scatter and the weights-on-M GEMM call pdl_launch() after
-// their wait, and the latter fetches weights before it: gemm_wm_sm100.cu): the next kernel's blocks may become resident while this
-// one runs, and no thread touches global memory before all earlier kernels of the stream have completed. What such a kernel
-// reads may therefore still be written while it is resident: its pointers are not __restrict__ and its loads are plain ones
-// (ld_stream16). Between the short kernels of the layer the gap shrinks from ~2 us to below 1 us (MoE block of 5 tokens, H 1024,
+// Programmatic dependent launch. A kernel launched through launch_pdl calls pdl_launch() and pdl_wait() first thing (the grouped
+// GEMMs set up their barriers and TMEM in between): the next kernel's blocks may become resident while this one runs, and no thread
+// touches global memory before all earlier kernels of the stream have completed. What such a kernel reads may therefore still be
+// written while it is resident: its pointers are not __restrict__ and its loads are plain ones (ld_stream16).
+// Early GEMMs are the exception: the weights-on-M form on single CTAs, block mode by counts, and the block-scaled GEMM as the layer
+// launches it. Before their wait they read the expert sort's table, past L1 (ld_relaxed_gpu), and their weights with the weights'
+// tiled scales. That is sound because they start only when the sort and all before it are complete: the kernels that may stand right
+// behind the sort (both row scatters, the MXFP8 quantiser, the scale tiling) and the early GEMMs themselves call pdl_launch() after
+// their wait. The re-quantisation pass and fc1's row tiles call it first, but start behind one of those.
+// Between the short kernels of the layer the gap shrinks from ~2 us to below 1 us (MoE block of 5 tokens, H 1024,
 // I 2048: 45.8 -> 34.6 us).
 // The grouped GEMMs are launched this way up to kPdlGemmRows rows only. Their blocks, one per SM, otherwise take the SMs in the
 // order in which the kernel before leaves them instead of in the launch order, which spreads the blocks that share a weight

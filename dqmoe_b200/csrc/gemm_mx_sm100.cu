@@ -178,7 +178,7 @@ moe_GemmGrouped_GemmUniversal_tcgen05_mx(const __grid_constant__ gemm::RowMaps r
     }
     // early (the layer's calls): the kernels between the expert sort and this one let their dependents start only after their own
     // wait, so when this kernel starts the sort and all before it are complete. The row counts and the weights are there, and the
-    // first stages' weights and their scales are fetched before the wait (as in gemm_wm_sm100.cu). Without / with, us per MoE block:
+    // first stages' weights and their scales are fetched before the wait (as in gemm_wm.cuh). Without / with, us per MoE block:
     // 30 tokens (H 1024, I 2048, E 8) 42.5 / 39, 20 tokens (H 7168, I 2048, E 32) 277 / 269, 100 tokens (E 33) 291.5 / 284.
     if (!p.early) pdl_wait();
     for (int i = threadIdx.x; i <= p.E; i += kThreads) {

@@ -10,8 +10,8 @@
 // into the other TMEM buffer.
 //
 // Rows on M. The layer runs its bf16, per-tensor and per-channel GEMMs, and block mode with few rows per expert, on the form with the
-// weights on M (gemm_wm_sm100.cu); this one serves the stand-alone operators, fp16 / fp32 operands, expert-parallel ranks and block
-// mode from 40 rows per expert on.
+// weights on M (gemm_wm.cuh); this one serves the stand-alone operators, fp16 / fp32 operands, expert-parallel ranks, small models
+// (weights_on_m in layer.cu) and block mode from 40 rows per expert on or with skewed routing (weights_on_m_suit below).
 //
 // Replaces the six CUTLASS grouped-GEMM variants of the reference and their
 // per-expert "configure" kernels (csrc/moe_gemm_template.h:72-1039) together
@@ -949,7 +949,9 @@ static int launch(const RowMaps& ma, const CUtensorMap& mb, const Params& p, cud
 // expert takes every token. So where it can go either way both forms are launched, and each kernel compares, from the sort's
 // table, the numbers of 256-row and 128-row tiles before it sets anything up: the pairs work up to 2 x 256-row tiles = 1.16 x
 // 128-row tiles, the singles beyond, and the other kernel leaves at once.
-// Measured, singles / pairs in us per layer call, by that ratio: 1.00 per-tensor (H 4096, I 14336, E 8, 194 rows per expert)
+// This serves the stand-alone operators, fp16 layers, the layers of small models and expert-parallel ranks. Measured, singles / pairs in
+// us per layer call, while all bf16, per-tensor and per-channel layers ran on this form (two of these GEMMs and what goes with them),
+// by that ratio: 1.00 per-tensor (H 4096, I 14336, E 8, 194 rows per expert)
 // 430 / 391, bf16 (7168 x 2048, E 32, 192) 883 / 788, per-channel (2880 x 2880, E 64, 178) 581 / 479; 1.13 per-channel (2880 x
 // 2880, 690, skewed) 1528 / 1342, bf16 (7168 x 2048, 801) 2235 / 2267; 1.20 per-channel (7168 x 2048, 297, half the experts empty)
 // 484 / 502, per-tensor (4096 x 14336, 511, one expert for every token) 811 / 866; 1.33 per-tensor (2880 x 2880, 284) 751 / 791;

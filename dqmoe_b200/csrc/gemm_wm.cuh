@@ -1,7 +1,8 @@
 // Grouped GEMM with the weights on the M side of the tensor core: D[weight row][token] = W A^T. A tile is 128 weight
 // rows per CTA (64 gate and 64 value rows in fc1) by up to 256 rows of one expert, in steps of 16 (32 on a CTA pair), so
 // an expert of 300 rows computes 304 or 320 of them, where tiles with the rows on M compute 384 or 512. Used by the layer
-// for bf16 and per-tensor / per-channel FP8 operands; gemm_sm100.cu has the form with the rows on M.
+// for bf16 and per-tensor / per-channel FP8 operands, and in block mode (tiles of up to 64 rows) for few rows per expert; gemm_sm100.cu
+// has the form with the rows on M.
 //
 // What bounds it: for many rows per expert the tensor pipe under the power limit, for few rows the weights from HBM.
 // Everything else is meant to stay out of their way:

@@ -25,7 +25,7 @@ def _have_scripts():
 
 @pytest.mark.skipif(not _have_scripts(), reason="baseline/_ref/test is not populated (run tests/reference_drivers/fetch.py)")
 @pytest.mark.parametrize("module_dir", ["dropin", "dropin_ext"])
-def test_reference_torch_test_runs_unmodified_on_the_drop_in(module_dir):
+def test_reference_torch_test_runs_unmodified_on_the_drop_in(module_dir, tmp_path):
     """module_dir: dropin = the ctypes moe_test.py, dropin_ext = the compiled pybind11 moe_test extension."""
     mod_path = os.path.join(ROOT, "dqmoe_b200", module_dir)
     if module_dir == "dropin_ext" and not any(f.startswith("moe_test") and f.endswith(".so") for f in os.listdir(mod_path)):
@@ -35,10 +35,8 @@ def test_reference_torch_test_runs_unmodified_on_the_drop_in(module_dir):
     res = subprocess.run([sys.executable, "torch_test.py"], cwd=REF_TEST, env=env, capture_output=True, text=True,
                          timeout=1500)
     out = res.stdout
-    log_dir = os.path.join(ROOT, "gpurun_out")
-    if os.path.isdir(log_dir):
-        with open(os.path.join(log_dir, f"reference_torch_test_{module_dir}.log"), "w") as f:
-            f.write(out + "\n--- stderr ---\n" + res.stderr[-4000:])
+    with open(tmp_path / f"reference_torch_test_{module_dir}.log", "w") as f:
+        f.write(out + "\n--- stderr ---\n" + res.stderr[-4000:])
     assert res.returncode == 0, res.stderr[-2000:]
     assert "Eror in perf measurement" not in out
     # one TFLOPS line per shape of enumerate_m_grouped_contiguous
